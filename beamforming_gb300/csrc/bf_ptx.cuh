@@ -33,6 +33,17 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
   return t;
 }
 
+// True in one lane of a converged warp, always the same one.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(p));
+  return p != 0;
+}
+
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
@@ -213,9 +224,9 @@ __device__ __forceinline__ void mma_f8f6f4_ts(uint32_t d_tmem, uint32_t a_tmem, 
 
 // The eight MMAs of one K stage (two 128-byte W boxes, b0 and b1): K step kk
 // reads TMEM columns a + 8 kk and box kk / 4 at byte 32 (kk % 4) of its rows
-// (descriptor address field in 16 B units).  One asm block and one predicate:
-// the issuing thread's instruction stream, not the tensor pipe, is the limit
-// at N = 192, so it carries nothing else.
+// (descriptor address field in 16 B units).  One asm block and one predicate;
+// call it from a warp-uniform loop behind elect_one(), so that the operands
+// stay in uniform registers.
 __device__ __forceinline__ void mma_ts_stage8(uint32_t d_tmem, uint32_t a_tmem, uint64_t b0, uint64_t b1,
                                               uint32_t idesc) {
   asm volatile(

@@ -308,7 +308,7 @@ __global__ void __launch_bounds__(Roles<kEpiW, kGroups>::kThreads, kHalf ? 2 : 1
   auto d_empty = [&](int i) { return bar0 + 8u * (2 * R + 2 * SW + 2 * S + 4 + kDigSlots + i); };
   uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(smem + sp.off_bar + 8 * sp.nbar);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);  // known to be warp-uniform
   const int lane = threadIdx.x & 31;
   const int ncols = 2 * p.max_nb_pass;                 // accumulator columns reserved (largest GEMM N)
   const int per_half = (kAcc - ncols) / kStageCols;  // unpacked stages beside each accumulator
@@ -468,7 +468,14 @@ __global__ void __launch_bounds__(Roles<kEpiW, kGroups>::kThreads, kHalf ? 2 : 1
     }
   } else if (warp == kMmaWarp) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    // The whole warp runs the loop and waits together; one elected lane issues.
+    // Kept warp-uniform, the descriptors, the stage addresses and the loop live
+    // in uniform registers, which is where tcgen05.mma takes them from.  Inside
+    // a single-lane branch every operand of every MMA was moved there first: a
+    // stage of 8 MMAs then cost 401 cycles at N <= 64 without commit and wait
+    // and 715 with them, against 163 / 257 (N = 32 / 64, the tensor core's own
+    // 128 / 256) and 309 / 365 in this form (152 SMs, 400 stages, clock64).
+    {
       Ring ar(S), wr(SW), dr(kDigSlots);
       const uint64_t a_const = smem_desc_sw32(smem_u32(sA));
       const uint64_t w_desc0 = smem_desc_sw128(smem_u32(sW));
@@ -484,33 +491,39 @@ __global__ void __launch_bounds__(Roles<kEpiW, kGroups>::kThreads, kHalf ? 2 : 1
         const int wbox = 2 * P.nb_pass * kKC;
         const uint32_t ab = local & 1u;
         const uint32_t aph = (local >> 1) & 1u;
-        if (!mbar_wait(accempty(ab), aph ^ 1u, err, kDevTimeoutAccEmpty)) break;
+        if (!__all_sync(0xffffffffu, mbar_wait(accempty(ab), aph ^ 1u, err, kDevTimeoutAccEmpty))) break;
         const int ds = static_cast<int>(dr.idx);
-        if (!mbar_wait(d_full(ds), dr.phase, err, kDevTimeoutFull)) break;
+        if (!__all_sync(0xffffffffu, mbar_wait(d_full(ds), dr.phase, err, kDevTimeoutFull))) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + ab * kAcc;
         // the offset MMA starts the accumulator at -8 sum_k W[n][k] / 512
-        mma_f8f6f4(d_tmem, a_const, smem_desc_sw32(smem_u32(sD + ds * sp.dbytes)), idesc, 0u);
-        mma_commit(d_empty(ds));
+        if (elect_one()) {
+          mma_f8f6f4(d_tmem, a_const, smem_desc_sw32(smem_u32(sD + ds * sp.dbytes)), idesc, 0u);
+          mma_commit(d_empty(ds));
+        }
+        __syncwarp();
         ++ndig;
         dr.advance();
         for (int ks = 0; ks < p.nk; ++ks, ar.advance(), wr.advance()) {
           const int s = static_cast<int>(ar.idx);
           const int sw = static_cast<int>(wr.idx);
           // the unpack arrives on a_full only once this stage's W slot has landed too
-          if (!mbar_wait(a_full(s), ar.phase, err, kDevTimeoutUnpacked)) {
+          if (!__all_sync(0xffffffffu, mbar_wait(a_full(s), ar.phase, err, kDevTimeoutUnpacked))) {
             ok = false;
             break;
           }
           tc_fence_after();
           const uint32_t a_tmem = tmem_base + stage_col(s, ncols, per_half, kAcc);
           const uint64_t b_desc = w_desc0 + static_cast<uint64_t>((sw * sp.wbytes) >> 4);
-          mma_ts_stage8(d_tmem, a_tmem, b_desc, b_desc + static_cast<uint64_t>(wbox >> 4), idesc);
-          mma_commit(empty(s));  // also frees the W slot: the unpack passes it on
+          if (elect_one()) {
+            mma_ts_stage8(d_tmem, a_tmem, b_desc, b_desc + static_cast<uint64_t>(wbox >> 4), idesc);
+            mma_commit(empty(s));  // also frees the W slot: the unpack passes it on
+            if (ks + 1 == p.nk) mma_commit(accfull(ab));
+          }
+          __syncwarp();
           ++nstage;
         }
         if (!ok) break;
-        mma_commit(accfull(ab));
         ++nacc;
       }
       // A commit's arrival is an asynchronous write into this CTA's shared
@@ -525,6 +538,7 @@ __global__ void __launch_bounds__(Roles<kEpiW, kGroups>::kThreads, kHalf ? 2 : 1
         mbar_wait_drain(d_empty(static_cast<int>(k % uD)), (k / uD) & 1u);
       for (uint32_t k = nacc > 2u ? nacc - 2u : 0u; k < nacc; ++k)
         mbar_wait_drain(accfull(static_cast<int>(k & 1u)), (k >> 1) & 1u);
+      __syncwarp();
     }
   } else if (RL::kForwarder && warp == RL::kFwdWarp) {
     // ------------------------------------------------------------ W forwarder
