@@ -24,16 +24,16 @@
 // and every partial sum are integer multiples of 2^-9 below 2^10 in magnitude
 // (at most 19 significant bits), exact in the f32 accumulator.  The
 // requantisation clamp(lrint(G * float(raw)), -7, 7) of cpu.cxx:37-39 is one
-// IEEE multiply by 512 G (exactly G * raw) and a round-half-even conversion.
+// IEEE multiply by 512 G (exactly G * raw) and a round-half-even step.
 //
 // Warp roles (one CTA per SM, persistent over tiles; warp numbers for the
 // layout of 8 epilogue warps, 480 threads; with 12 epilogue warps, 608
 // threads, the roles after the epilogue move up by four):
-//   warps 0-7    epilogue: TMEM accumulator -> registers -> requantise (multiply,
-//                clamp, convert, saturating nibble pack) -> 4x4 byte transpose
-//                across lanes -> 32-bit stores of 4 consecutive times of one beam
+//   warps 0-7    epilogue: TMEM accumulator -> registers (four rows of a beam to a
+//                thread) -> requantise (multiply, convert, saturating nibble pack)
+//                -> 32-bit stores of 4 consecutive bytes of J
 //   warp  8      E producer: TMA of raw E boxes into a deep ring released by the unpack
-//   warp  9      TMEM allocator and single-thread MMA issuer (A operand from TMEM)
+//   warp  9      TMEM allocator and MMA issuer (A operand from TMEM)
 //   warp  10     W producer: TMA of each tile's digit rows and of the W slice of
 //                each K stage, released by the MMA
 //   warps 11-14  unpack (groups of four take K stages in turn): raw E bytes ->
@@ -46,8 +46,8 @@
 // has landed, so the unpack warps carry no W hand-over, and the W producer
 // reuses a slot as soon as the tensor core has finished the stage that used it.
 //
-// GEMM row r of a tile (TMEM lane r) is (t, p) = (r / 2, r % 2) for the 64 times
-// of the tile.  TMEM columns: accumulators at [0, N) and [256, 256 + N), unpacked
+// Which of the tile's 64 times and 2 polarizations a GEMM row (TMEM lane) holds:
+// RowMap.  TMEM columns: accumulators at [0, N) and [256, 256 + N), unpacked
 // E stages (64 columns = 256 K bytes each) in the remaining columns.
 #include "bf_internal.h"
 #include "bf_ptx.cuh"
@@ -266,13 +266,34 @@ __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
   return r;
 }
 
-// (c << 8) | (sat4(re) << 4) | sat4(im): two integers saturated to [-8, 7] and
+// (c << 8) | (sat(re) << 4) | sat(im): two integers saturated to [0, 15] and
 // packed as the nibbles of one byte below the bytes of c.
-__device__ __forceinline__ uint32_t pack_s4x2(int re, int im, uint32_t c) {
+__device__ __forceinline__ uint32_t pack_u4x2(uint32_t re, uint32_t im, uint32_t c) {
   uint32_t r;
-  asm("cvt.pack.sat.s4.s32.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(re), "r"(im), "r"(c));
+  asm("cvt.pack.sat.u4.s32.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(re), "r"(im), "r"(c));
   return r;
 }
+
+// GEMM row r (0..31) of a lane quarter q <-> time and polarization of the tile.
+// The epilogue's loads give thread (g, c) = (lane / 4, lane % 4) the four rows
+// g, g + 8, g + 16, g + 24, so those hold four consecutive bytes of J: four
+// times of one polarization (Jlinear, arraysizes.hxx:92; quarter q holds 32
+// times of polarization q % 2), or two times of both (J2linear,
+// arraysizes.hxx:103; 16 times).  Which of the four sits in which row depends
+// on g through `swap`, which spreads the raw rows that 8 lanes of the unpack
+// read together over all 8 positions of the 128-byte swizzle (no bank
+// conflicts); the epilogue undoes it with one byte permute.
+template <bool kJ2>
+struct RowMap {
+  __device__ static __forceinline__ uint32_t swap(uint32_t g) { return kJ2 ? 2u * (g >> 2) : g >> 1; }
+  __device__ static __forceinline__ uint32_t time(uint32_t q, uint32_t r) {
+    const uint32_t g = r & 7u, j = (r >> 3) ^ swap(g);
+    return kJ2 ? 16u * q + 2u * g + (j >> 1) : 32u * (q >> 1) + 4u * g + j;
+  }
+  __device__ static __forceinline__ uint32_t pol(uint32_t q, uint32_t r) {
+    return kJ2 ? ((r >> 3) ^ swap(r & 7u)) & 1u : q & 1u;
+  }
+};
 
 // Byte offset of 16-byte chunk j of row r in a 128B-swizzled tile (TMA layout).
 __device__ __forceinline__ uint32_t sw128_offset(uint32_t r, uint32_t j) {
@@ -557,13 +578,13 @@ __global__ void __launch_bounds__(Roles<kEpiW, kGroups>::kThreads, kHalf ? 2 : 1
     }
   } else if (warp >= kUnpackWarp0) {
     // ------------------------------------------------------------ unpack
-    // Group g takes the K stages with it % kUnpackGroups == g.  Lane pair
-    // (2u, 2u+1) of quarter q holds rows (t, p=0) and (t, p=1) of time
-    // t = 16q + u: both lanes read the raw row and keep their polarization.
+    // Group g takes the K stages with it % kUnpackGroups == g.  Each lane fills
+    // one GEMM row: it reads the raw row of its time, which holds both
+    // polarizations, and keeps its own (RowMap).
     const int group = (warp - kUnpackWarp0) >> 2;
     const int q = warp & 3;
-    const uint32_t pp = lane & 1u;
-    const uint32_t tl = 16u * q + (lane >> 1);
+    const uint32_t pp = RowMap<kJ2>::pol(q, lane);
+    const uint32_t tl = RowMap<kJ2>::time(q, lane);
     const uint32_t lane_addr = static_cast<uint32_t>(32 * q) << 16;
     const uint32_t sel = pp ? 0x7531u : 0x6420u;  // odd or even bytes: polarization 1 or 0
     // this CTA's K stages: its tiles (TileRange) times nk
@@ -646,12 +667,14 @@ __global__ void __launch_bounds__(Roles<kEpiW, kGroups>::kThreads, kHalf ? 2 : 1
     }
   } else {
     // ------------------------------------------------------------ epilogue
-    // Warp w reads TMEM lane quarter w % 4 (times 16q..16q+15, both
-    // polarizations interleaved by lane) and column part w / 4.
+    // Warp w reads TMEM lane quarter w % 4 and column part w / 4; thread
+    // (g, c) of it takes rows g, g + 8, g + 16, g + 24 (four consecutive bytes of
+    // J, RowMap) of every fourth beam.
     const int q = warp & 3;
     const int part = warp >> 2;
-    const uint32_t pol = lane & 1u;
+    const uint32_t g = lane >> 2, cb = lane & 3u;
     const uint32_t lane_addr = static_cast<uint32_t>(32 * q) << 16;
+    const uint32_t osel = 0x3210u ^ (0x1111u * RowMap<kJ2>::swap(g));  // rows' bytes into J's order
 
     // The warps of the epilogue share no barrier: each reads its chunks' gains
     // straight from the scaled-gain rows gs = 512 * G (L1-resident) and waits for
@@ -677,39 +700,27 @@ __global__ void __launch_bounds__(Roles<kEpiW, kGroups>::kThreads, kHalf ? 2 : 1
       // 512 * G[f][b0 ..] (zero beyond B): the accumulator ends at raw / 512
       // exactly and the power-of-two scaling is exact, so (512 G) * (raw / 512)
       // rounds like G * raw (cpu.cxx:37)
-      const float *gcur = P.gs + static_cast<int64_t>(f) * P.npass * P.nb_pass + b0;
+      const float *gcur = P.gs + static_cast<int64_t>(f) * P.npass * P.nb_pass + b0 + cb;
       // huge or non-finite gains of this frequency: requantise with the
       // narrowing of cpu.cxx:38 (tile-uniform branch, normally not taken)
       const bool wide = __ldg(P.gwide + f) != 0;
       if (!__all_sync(0xffffffffu, mbar_wait(accfull(ab), aph, err, kDevTimeoutAccFull))) break;
       tc_fence_after();
       const uint32_t acc_addr = tmem_base + ab * kAcc + lane_addr;
-      // A 4x4 byte transpose among 4 lanes turns "4 beams of one row" into "4
-      // rows of one beam" in each lane.  Jlinear (arraysizes.hxx:92): the 4 lanes
-      // of equal polarization and consecutive times (lane bits 1 and 2) exchange,
-      // and a lane stores J[b][f][p][t..t+3].  J2linear (arraysizes.hxx:103): 4
-      // consecutive rows (t, p), (t, p+1), (t+1, p), (t+1, p+1) (lane bits 0 and
-      // 1) exchange, and a lane stores those 4 bytes of J2[b][f][t][p].
-      constexpr bool j2 = kJ2;
-      const uint32_t j4 = j2 ? (lane & 3u) : ((lane >> 1) & 3u);  // place among the 4 = beam offset after
-      const int xd1 = j2 ? 1 : 2, xd2 = j2 ? 2 : 4;
-      const uint32_t sel1 = (j4 & 1) ? 0x3715u : 0x6240u;
-      const uint32_t sel2 = (j4 & 2) ? 0x3276u : 0x5410u;
-      const int64_t bj = static_cast<int64_t>(b0 + static_cast<int>(j4)) * P.F + f;  // beam row b0 + j4
-      int64_t t;      // first time of the lane's 4 bytes
-      uint8_t *jrow;  // the lane's bytes for beam b0 + j4
-      if (!j2) {
-        t = static_cast<int64_t>(tt) * kTT + 16 * q + 4 * (lane >> 3);
-        jrow = P.J + (bj * 2 + pol) * P.jpitch + t;
+      const int64_t bj = static_cast<int64_t>(b0 + static_cast<int>(cb)) * P.F + f;  // beam row b0 + cb
+      int64_t t;      // first time of the thread's 4 bytes
+      uint8_t *jrow;  // the thread's bytes for beam b0 + cb
+      if constexpr (!kJ2) {
+        t = static_cast<int64_t>(tt) * kTT + RowMap<kJ2>::time(q, 8 * RowMap<kJ2>::swap(g) + g);
+        jrow = P.J + (bj * 2 + (q & 1)) * P.jpitch + t;
       } else {
-        const int r0 = 32 * q + static_cast<int>(lane & ~3u);  // first of the 4 rows in the tile
-        t = static_cast<int64_t>(tt) * kTT + r0 / 2;
-        jrow = P.J + bj * 2 * P.jpitch + 2 * static_cast<int64_t>(tt) * kTT + r0;
+        t = static_cast<int64_t>(tt) * kTT + 16 * q + 2 * static_cast<int>(g);
+        jrow = P.J + bj * 2 * P.jpitch + 2 * t;
       }
       const bool t_ok = t < P.T;
       const int64_t bstride = static_cast<int64_t>(P.F) * 2 * P.jpitch;  // bytes between beams, both layouts
-      const int blim = P.B - b0 - static_cast<int>(j4);  // beam offsets below this exist
-      uint8_t *dst = jrow + static_cast<int64_t>(8 * c_begin) * bstride;  // beam 8 c + j4 of the lane's chunk c
+      const int blim = P.B - b0 - static_cast<int>(cb);  // beam offsets below this exist
+      uint8_t *dst = jrow + static_cast<int64_t>(8 * c_begin) * bstride;  // beam 8 c + cb of chunk c
       // fused adler32: word h of the lane's chunk c_begin + cc sits at byte
       // position base + cc * step + h * half (mod 65521), so the tile needs only
       // a0 = sum of its bytes, a1 = sum cc * (bytes of chunk cc), a2 = sum of the
@@ -718,37 +729,46 @@ __global__ void __launch_bounds__(Roles<kEpiW, kGroups>::kThreads, kHalf ? 2 : 1
       // bytes <= 255, at most 16 words; the products are taken in 64 bits)
       uint32_t ad_a0 = 0, ad_a1 = 0, ad_a2 = 0, ad_a3 = 0;
 
+      // Beams 8 c + cb and 8 c + 4 + cb, four rows each.  With the earlier 4x4 byte
+      // transpose across lanes and scalar clamps and conversions the epilogue took
+      // 86 instructions for 32 rows x 8 beams, now about 55: full chunk 956 -> 886
+      // us, wide array 812 -> 780 us, 128-problem batch 376 -> 355 us.  What bounds the epilogue
+      // is the issue rate and above all the integer pipe, so the arithmetic runs
+      // two values to an instruction on the float pipe: acc = raw / 512 exactly;
+      // x = (512 G) acc is one IEEE multiply, equal to G * raw (cpu.cxx:37); then
+      // x 2^-149 + 8 2^-149 is rounded once, to a multiple of the smallest
+      // subnormal, so its bit pattern is the integer lrint(x) + 8 (ties to even:
+      // 8 is even), a large positive integer above the range and a negative one
+      // below it.  The saturating pack clamps that to [0, 15] -- the nibble that
+      // ucomplex4 stores (icomplex4.hxx:33) -- and the one value below the lower
+      // clamp of cpu.cxx:38, nibble 0 (-8), becomes 1 (-7) for eight nibbles at once.
       auto process = [&](int c, const uint32_t (&r)[16]) {
-        const float4 ga = __ldg(reinterpret_cast<const float4 *>(gcur + 8 * c));
-        const float4 gb = __ldg(reinterpret_cast<const float4 *>(gcur + 8 * c + 4));
-        const float gv[8] = {ga.x, ga.y, ga.z, ga.w, gb.x, gb.y, gb.z, gb.w};
-        // clamp(lrint(G * raw), -7, 7) with acc = raw / 512 exactly: one IEEE
-        // multiply, the lower clamp (to -7.25: same result after rounding), a
-        // round-half-even conversion, and the upper clamp by the saturating pack
-        int qre[8], qim[8];
-        if (!wide) {
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            qre[i] = __float2int_rn(fmaxf(__fmul_rn(gv[i], __uint_as_float(r[i])), -7.25f));
-            qim[i] = __float2int_rn(fmaxf(__fmul_rn(gv[i], __uint_as_float(r[8 + i])), -7.25f));
-          }
-        } else {
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            qre[i] = requant_narrow(__fmul_rn(gv[i], __uint_as_float(r[i])));
-            qim[i] = requant_narrow(__fmul_rn(gv[i], __uint_as_float(r[8 + i])));
-          }
-        }
-        // ucomplex4 bytes of beams 0-3 and 4-7 for this lane's time
         uint32_t w[2];
 #pragma unroll
-        for (int h2 = 0; h2 < 2; ++h2) {
+        for (int k = 0; k < 2; ++k) {
+          const float gn = __ldg(gcur + 8 * c + 4 * k);
           uint32_t x = 0;
+          if (!wide) {
+            const uint64_t g2 = f32x2(__float_as_uint(gn), __float_as_uint(gn));
+            const uint64_t tiny = f32x2(1u, 1u), eight = f32x2(8u, 8u);  // 2^-149 and 8 2^-149
 #pragma unroll
-          for (int j = 3; j >= 0; --j) x = pack_s4x2(qre[4 * h2 + j], qim[4 * h2 + j], x);
-          x ^= 0x88888888u;  // byte j = ucomplex4 of beam 4 * h2 + j (icomplex4.hxx:33)
-          const uint32_t x1 = prmt(x, __shfl_xor_sync(0xffffffffu, x, xd1), sel1);
-          w[h2] = prmt(x1, __shfl_xor_sync(0xffffffffu, x1, xd2), sel2);  // beam 4*h2 + j4, the 4 rows
+            for (int j = 3; j >= 0; --j) {
+              const int at = 4 * k + 2 * (j & 1) + 8 * (j >> 1);
+              const uint64_t y = fma_f32x2(mul_f32x2(g2, f32x2(r[at], r[at + 1])), tiny, eight);
+              x = pack_u4x2(static_cast<uint32_t>(y), static_cast<uint32_t>(y >> 32), x);
+            }
+            uint32_t v = x | (x >> 1);
+            v |= v >> 2;
+            x |= ~v & 0x11111111u;
+          } else {
+#pragma unroll
+            for (int j = 3; j >= 0; --j) {
+              const int at = 4 * k + 2 * (j & 1) + 8 * (j >> 1);
+              x = pack_u4x2(static_cast<uint32_t>(requant_narrow(__fmul_rn(gn, __uint_as_float(r[at]))) + 8),
+                            static_cast<uint32_t>(requant_narrow(__fmul_rn(gn, __uint_as_float(r[at + 1]))) + 8), x);
+            }
+          }
+          w[k] = prmt(x, 0u, osel);
         }
         if (t_ok) {
           if (8 * c < blim) __stcs(reinterpret_cast<uint32_t *>(dst), w[0]);
@@ -770,16 +790,16 @@ __global__ void __launch_bounds__(Roles<kEpiW, kGroups>::kThreads, kHalf ? 2 : 1
       // accumulator columns in chunks of 16, the next chunk's TMEM load in flight
       uint32_t ra[16], rb[16];
       if (c_begin < c_end) {
-        tmem_ld_32x32b_x16(acc_addr + 16u * c_begin, ra);
+        tmem_ld_rows4_x2(acc_addr + 16u * c_begin, ra);
         tmem_ld_wait(ra);
       }
       for (int c = c_begin; c < c_end; c += 2) {
         const bool has1 = c + 1 < c_end, has2 = c + 2 < c_end;
-        if (has1) tmem_ld_32x32b_x16(acc_addr + 16u * (c + 1), rb);
+        if (has1) tmem_ld_rows4_x2(acc_addr + 16u * (c + 1), rb);
         process(c, ra);
         if (has1) {
           tmem_ld_wait(rb);
-          if (has2) tmem_ld_32x32b_x16(acc_addr + 16u * (c + 2), ra);
+          if (has2) tmem_ld_rows4_x2(acc_addr + 16u * (c + 2), ra);
           process(c + 1, rb);
           if (has2) tmem_ld_wait(ra);
         }
@@ -820,7 +840,7 @@ __global__ void __launch_bounds__(Roles<kEpiW, kGroups>::kThreads, kHalf ? 2 : 1
 
 // Builds the E4M3 operand W[f][n][k] and the digit rows of the row sums
 // sum_k W[f][n][k] from A[f][b][d]; one warp per row n, four k per lane-step.
-//   n = 16*(b/8) + 8*cj + b%8      (cj: 0 = real output, 1 = imaginary output)
+//   n = 2*b + cj                   (cj: 0 = real output, 1 = imaginary output)
 //   k = 8*(d/4)  + 4*c  + d%4      (c:  0 = real input,  1 = imaginary input)
 // W = Ar, -Ai for the real output and Ai, Ar for the imaginary output.
 constexpr int kPrepRows = 8;  // rows per 256-thread block
@@ -854,8 +874,8 @@ __global__ void __launch_bounds__(32 * kPrepRows) bf_prep_weights(const uint8_t 
   if (n >= nw_pad) return;  // the whole warp
   int sum = 0;
   if (n < nw) {
-    const int b = 8 * (n / 16) + (n % 8);
-    const int cj = (n / 8) & 1;
+    const int b = n >> 1;
+    const int cj = n & 1;
     // rows of 2D bytes, D % 8 == 0: 4-byte aligned words
     uint32_t *wrow = reinterpret_cast<uint32_t *>(W + (static_cast<int64_t>(f) * nw + n) * (2 * D));
     for (int k4 = lane; k4 < D / 2; k4 += 32) {  // k = 4 k4 .. 4 k4 + 3: dishes d0 .. d0 + 3, input part c
