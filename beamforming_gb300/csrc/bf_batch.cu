@@ -60,12 +60,18 @@ int status_of(cudaError_t e) {
     if (e_ != cudaSuccess) return status_of(e_);   \
   } while (0)
 
+// A problem's records for the two kinds of launch: one CTA per tile, or pairs of SMs.
+struct Records {
+  TcProblem one, pair;
+};
+
 // A schedule: the problem table in launch order (tile_begin counted from the
 // start of each launch) and its launches.
 struct Schedule {
   std::vector<TcProblem> table;
   int nlaunch = 0;
   BatchLaunch launches[kMaxLaunches];
+  bool ring_plans = false;  // a launch reads the ring plan (those on pairs of SMs plan their own)
 };
 
 // Pass-width class of a problem: 0 wide, 1 narrow (<= kNarrowPass beams),
@@ -77,20 +83,23 @@ int launch_of(int cls, int cuts) { return (cls >= 1 && (cuts & 1)) + (cls >= 2 &
 
 // Problems in `order`, one launch per group of classes that `cuts` keeps
 // together (wider classes first); empty launches are dropped.
-Schedule schedule_of(const std::vector<TcProblem> &probs, const std::vector<int> &order, int cuts) {
+Schedule schedule_of(const std::vector<Records> &probs, const std::vector<int> &order, int cuts) {
   Schedule sc;
   for (int l = 0; l < kMaxLaunches; ++l) {
     BatchLaunch L;
     L.first = static_cast<int>(sc.table.size());
+    for (int i : order)
+      if (launch_of(class_of(probs[i].one), cuts) == l) L.max_nb_pass = std::max(L.max_nb_pass, probs[i].one.nb_pass);
+    const bool pair = tc_pair_launch(L.max_nb_pass);
     int64_t begin = 0;
     for (int i : order) {
-      if (launch_of(class_of(probs[i]), cuts) != l) continue;
-      TcProblem P = probs[i];
+      if (launch_of(class_of(probs[i].one), cuts) != l) continue;
+      TcProblem P = pair ? probs[i].pair : probs[i].one;
       P.tile_begin = static_cast<int>(begin);
       begin += tc_problem_tiles(P);
-      L.max_nb_pass = std::max(L.max_nb_pass, P.nb_pass);
       sc.table.push_back(P);
     }
+    sc.ring_plans |= !pair && static_cast<int>(sc.table.size()) > L.first;
     L.nprob = static_cast<int>(sc.table.size()) - L.first;
     L.ntiles = static_cast<int>(begin);
     if (L.nprob > 0) sc.launches[sc.nlaunch++] = L;
@@ -129,7 +138,7 @@ int bf_batch_create(bf_batch **out, const bf_problem *problems, int nproblems, b
   *out = nullptr;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   int64_t D = -1;
-  std::vector<TcProblem> probs(static_cast<size_t>(nproblems));
+  std::vector<Records> probs(static_cast<size_t>(nproblems));
   bool present[3] = {false, false, false};
   for (int i = 0; i < nproblems; ++i) {
     const bf_problem &q = problems[i];
@@ -139,8 +148,9 @@ int bf_batch_create(bf_batch **out, const bf_problem *problems, int nproblems, b
     const bf_dims d{q.ntimes, w.F, w.D, 2, w.B};
     if (w.D != D || !tc_supported(d)) return BF_ERR_UNSUPPORTED;
     if ((reinterpret_cast<uintptr_t>(q.E) | reinterpret_cast<uintptr_t>(q.J)) & 15u) return BF_ERR_UNSUPPORTED;
-    BF_TRY(tc_make_problem(probs[i], w, q.ntimes, q.J, q.E, 0));
-    present[class_of(probs[i])] = true;
+    BF_TRY(tc_make_problem(probs[i].one, w, q.ntimes, q.J, q.E, 0, kJLinear, false));
+    BF_TRY(tc_make_problem(probs[i].pair, w, q.ntimes, q.J, q.E, 0, kJLinear, true));
+    present[class_of(probs[i].one)] = true;
   }
   int *err = nullptr;
   int st = device_error_word(&err);
@@ -163,7 +173,7 @@ int bf_batch_create(bf_batch **out, const bf_problem *problems, int nproblems, b
   std::iota(given.begin(), given.end(), 0);
   std::vector<int> largest = given;
   std::stable_sort(largest.begin(), largest.end(), [&](int x, int y) {
-    return tc_problem_tiles(probs[x]) > tc_problem_tiles(probs[y]);
+    return tc_problem_tiles(probs[x].one) > tc_problem_tiles(probs[y].one);
   });
   const std::vector<int> *orders[2] = {&given, &largest};
   const bool cut_ok[2] = {present[0] && (present[1] || present[2]), present[2] && (present[0] || present[1])};
@@ -172,6 +182,7 @@ int bf_batch_create(bf_batch **out, const bf_problem *problems, int nproblems, b
   plans[1].raw = 8;
   plans[2].wslots = 2;
   plans[2].raw = 12;
+  for (TcRingPlan &plan : plans) plan.pair_groups = 1;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
@@ -183,7 +194,7 @@ int bf_batch_create(bf_batch **out, const bf_problem *problems, int nproblems, b
       const Schedule sc = schedule_of(probs, *orders[o], cuts);
       cudaError_t e = cudaMemcpyAsync(b->table, sc.table.data(), sizeof(TcProblem) * sc.table.size(),
                                       cudaMemcpyHostToDevice, s);
-      for (int pl = 0; pl < 3 && e == cudaSuccess; ++pl) {
+      for (int pl = 0; pl < (sc.ring_plans ? 3 : 1) && e == cudaSuccess; ++pl) {
         e = launch_schedule(b, sc.launches, sc.nlaunch, plans[pl], s);  // warm-up
         if (e != cudaSuccess) break;
         cudaEventRecord(e0, s);

@@ -105,8 +105,10 @@ inline void tc_set_extra(TcWeights &w, uint8_t *p) {
 // True when the tensor-core kernel handles this shape.
 bool tc_supported(const bf_dims &d);
 
-// Beams per pass and number of passes for B beams.
-void tc_plan_beams(int64_t B, int *nb_pass, int *npass);
+// Beams per pass and number of passes for B beams.  Passes of a multiple of 16
+// beams fill the GEMM N of a pair launch (a multiple of 32) exactly: 512 beams
+// are five passes of 96 and one of 32 instead of six of 88, each padded to 96.
+void tc_plan_beams(int64_t B, int *nb_pass, int *npass, int granule = 16);
 
 // Fills w.W, w.dig and w.gs from device A and w.G (w's sizes and buffers already set).
 cudaError_t launch_prep_weights(const TcWeights &w, const uint8_t *A, cudaStream_t s, int a_layout = kALinear);
@@ -152,17 +154,23 @@ struct TcProblem {  // 128-byte aligned through its tensor maps
   int ntt;           // time tiles per frequency
   int nw_pad;        // digit rows per frequency
   int tile_begin;    // first tile of this problem in the launch
+  int pair;          // nonzero: made for a launch on pairs of SMs, whose tiles are 128 times
+  int w_rows;        // rows of the W and digit boxes: the pass's 2 * nb_pass, or a CTA's half of N in a pair launch
 };
 
 // Shared-memory ring depths of a launch (0: planner default).
 struct TcRingPlan {
   int wslots = 0;
   int raw = 0;
+  int pair_groups = 2;  // unpack groups of a pair launch with two TMEM stages (passes wider than 64 beams)
 };
 
-// Fills a problem record (tile_begin left 0) for T times of E with weights w.
+// Whether a launch whose widest pass has max_nb_pass beams runs on pairs of SMs.
+bool tc_pair_launch(int max_nb_pass);
+// Fills a problem record (tile_begin left 0) for T times of E with weights w,
+// for a launch on pairs of SMs or not.
 cudaError_t tc_make_problem(TcProblem &P, const TcWeights &w, int64_t T, uint8_t *J, const uint8_t *E,
-                            int64_t jpitch, int j_layout = kJLinear);
+                            int64_t jpitch, int j_layout, bool pair);
 // Tiles of a problem, and K stages per tile for D dishes.
 int64_t tc_problem_tiles(const TcProblem &P);
 int tc_stages_per_tile(int64_t D);
@@ -178,6 +186,15 @@ cudaError_t launch_tc_grouped(const TcProblem *table, int nprob, int ntiles, int
 // column of the second accumulator, stages beside each accumulator, one past
 // the last TMEM column a stage uses.
 cudaError_t tc_plan_rings(int64_t D, int max_nb_pass, const TcRingPlan &plan, int *out);
+
+// Pair launches (bf_tc_pair.cu): clusters of two CTAs the device runs at once
+// (0: none), the GEMM N of a pass, the TMEM stages of a launch, and the launches.
+int pair_clusters();
+int pair_cols(int nb_pass);
+cudaError_t pair_launch_shape(int64_t D, int max_nb_pass, int *stages);
+cudaError_t launch_pair(const TcProblem &one, int64_t D, int test_stall, int *err, cudaStream_t s);
+cudaError_t launch_pair_grouped(const TcProblem *table, int nprob, int ntiles, int64_t D, int max_nb_pass, int groups,
+                                int test_stall, int *err, cudaStream_t s);
 
 // TMEM stages, unpack groups and CTAs per SM of a grouped launch with these sizes.
 cudaError_t tc_launch_shape(int64_t D, int max_nb_pass, const TcRingPlan &plan, int *stages, int *groups,

@@ -44,6 +44,16 @@ __device__ __forceinline__ bool elect_one() {
   return p != 0;
 }
 
+// Registers of the executing warpgroup (all four warps of it call this).
+template <int kRegs>
+__device__ __forceinline__ void regs_more() {
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegs));
+}
+template <int kRegs>
+__device__ __forceinline__ void regs_less() {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegs));
+}
+
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
@@ -60,32 +70,6 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
                : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
-// try_wait that lets the hardware suspend the thread until the phase completes
-// or `hint_ns` nanoseconds pass, so waiting warps do not take issue slots.
-__device__ __forceinline__ bool mbar_try_wait_sleep(uint32_t bar, uint32_t parity, uint32_t hint_ns) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity), "r"(hint_ns)
-      : "memory");
-  return ok != 0;
 }
 
 // Bounded wait for the phase with the given parity to complete.  Returns false
@@ -111,17 +95,39 @@ __device__ __forceinline__ bool wait_expired(uint64_t &t0, uint32_t polls) {
   return polls >= kMinTimeoutPolls && now - t0 > kWaitTimeoutNs;
 }
 
+// kPollCheck polls (fewer when the phase completes): the loop every waiting
+// warp of a kernel sits in, so it holds nothing but the polls and a counter.
+// The hardware suspends the warp in each poll for a while; a longer suspend
+// hint adds a sleep to every poll instead (full chunk 665 -> 659 us, wide array
+// 703 -> 677 us without it).
+__device__ __forceinline__ bool mbar_poll(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t.reg .u32 n;\n\t"
+      "mov.u32 n, %3;\n"
+      "AGAIN:\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "@p bra DONE;\n\t"
+      "add.u32 n, n, -1;\n\t"
+      "setp.ne.u32 q, n, 0;\n\t"
+      "@q bra AGAIN;\n"
+      "DONE:\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity), "n"(kPollCheck)
+      : "memory");
+  return ok != 0;
+}
+
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int *err, int code) {
-  if (mbar_try_wait(bar, parity)) return true;
+  if (mbar_poll(bar, parity)) return true;
   uint64_t t0 = globaltimer_ns();
-  for (uint32_t i = 1;; ++i) {
-    if (mbar_try_wait_sleep(bar, parity, 200000u)) return true;
-    if (i % kPollCheck == 0) {
-      if (*reinterpret_cast<volatile int *>(err) != 0) return false;
-      if (wait_expired(t0, i)) {
-        atomicCAS(err, 0, code);
-        return false;
-      }
+  for (uint32_t i = kPollCheck;; i += kPollCheck) {
+    if (mbar_poll(bar, parity)) return true;
+    if (*reinterpret_cast<volatile int *>(err) != 0) return false;
+    if (wait_expired(t0, i)) {
+      atomicCAS(err, 0, code);
+      return false;
     }
   }
 }
@@ -130,12 +136,44 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int *er
 // gives up waits with it for the copies it already issued to land before the
 // CTA exits (at most kWaitTimeoutNs per barrier).
 __device__ __forceinline__ bool mbar_wait_drain(uint32_t bar, uint32_t parity) {
-  if (mbar_try_wait(bar, parity)) return true;
+  if (mbar_poll(bar, parity)) return true;
   uint64_t t0 = globaltimer_ns();
-  for (uint32_t i = 1;; ++i) {
-    if (mbar_try_wait_sleep(bar, parity, 200000u)) return true;
-    if (i % kPollCheck == 0 && wait_expired(t0, i)) return false;
+  for (uint32_t i = kPollCheck;; i += kPollCheck) {
+    if (mbar_poll(bar, parity)) return true;
+    if (wait_expired(t0, i)) return false;
   }
+}
+
+// ---------------------------------------------------------------- clusters
+__device__ __forceinline__ uint32_t cluster_ctarank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// Address, in the cluster's shared window, of this CTA's shared address in CTA `rank`.
+__device__ __forceinline__ uint32_t map_cta(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+// Arrive on a barrier of another CTA of the cluster.
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t mapped) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(mapped) : "memory");
+}
+// The same where all it orders is this thread's tensor-memory accesses (behind
+// tcgen05.wait and tcgen05.fence::before_thread_sync).  A release at cluster
+// scope would also wait until the thread's J stores reach L2: with it on every
+// stage and tile the full chunk took 1424 us, with this 650.
+__device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t mapped) {
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(mapped) : "memory");
+}
+__device__ __forceinline__ void st_cluster_u32(uint32_t mapped, uint32_t v) {
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(mapped), "r"(v) : "memory");
+}
+// Every thread of both CTAs arrives and waits.
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 // ---------------------------------------------------------------- proxies
@@ -248,6 +286,55 @@ __device__ __forceinline__ void mma_ts_stage8(uint32_t d_tmem, uint32_t a_tmem, 
       "add.u32 a, %1, 56;\n\tadd.s64 b, %3, 6;\n\t"
       "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], [a], b, %4, p;\n\t}" ::"r"(d_tmem),
       "r"(a_tmem), "l"(b0), "l"(b1), "r"(idesc)
+      : "memory");
+}
+
+// The forms for a pair of CTAs (cta_group::2): the issuing CTA's tensor core
+// and its peer's each take 128 of the M = 256 rows from their own tensor memory
+// (or shared memory) and share B, of which each CTA holds one half of the N
+// columns' rows at the same shared-memory offset.
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t dst_smem, uint32_t ncols) {
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem), "r"(ncols)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_relinquish_pair() {
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+__device__ __forceinline__ void mma_f8f6f4_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                                uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// The four MMAs of one 128-byte W box: K step kk reads TMEM columns a + 8 kk
+// and byte 32 kk of the box's rows.
+__device__ __forceinline__ void mma_ts_box_pair(uint32_t d_tmem, uint32_t a_tmem, uint64_t b0, uint32_t idesc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 b;\n\t.reg .b32 a, l, h;\n\t"
+      "setp.ne.b32 p, %3, 0;\n\t"
+      "mov.b64 {l, h}, %2;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], [%1], %2, %3, p;\n\t"
+      "add.u32 a, %1, 8;\n\tadd.u32 l, l, 2;\n\tmov.b64 b, {l, h};\n\t"
+      "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], [a], b, %3, p;\n\t"
+      "add.u32 a, %1, 16;\n\tadd.u32 l, l, 2;\n\tmov.b64 b, {l, h};\n\t"
+      "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], [a], b, %3, p;\n\t"
+      "add.u32 a, %1, 24;\n\tadd.u32 l, l, 2;\n\tmov.b64 b, {l, h};\n\t"
+      "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], [a], b, %3, p;\n\t}" ::"r"(d_tmem),
+      "r"(a_tmem), "l"(b0), "r"(idesc)
+      : "memory");
+}
+// Arrive once on the mbarrier at this offset in both CTAs of the pair when
+// every tcgen05 operation this thread issued before has completed.
+__device__ __forceinline__ void mma_commit_pair(uint32_t bar) {
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+      "h"(static_cast<uint16_t>(3))
       : "memory");
 }
 

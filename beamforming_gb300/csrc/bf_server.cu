@@ -218,6 +218,7 @@ void CUDART_CB flight_landed(void *arg) {
 // host function that marks the flight landed.  Runs without the mutex.
 bool bf_server::launch(Flight &fl, const std::vector<Request> &reqs, int *ntiles) {
   const TcWeights &w = weights->tc;
+  const bool pair = tc_pair_launch(w.nb_pass);
   int64_t begin = 0;
   unsigned waited = 0;  // versions whose refresh this stream already waits for
   for (size_t i = 0; i < reqs.size(); ++i) {
@@ -231,7 +232,8 @@ bool bf_server::launch(Flight &fl, const std::vector<Request> &reqs, int *ntiles
       return false;
     const TcWeights v = channel_view(vr.w->tc, r.channel, r.nchannels);
     TcProblem &P = fl.table_host[i];
-    if (tc_make_problem(P, v, r.ntimes, r.dJ, r.e_on_device ? r.E : r.dE, 0) != cudaSuccess) return false;
+    if (tc_make_problem(P, v, r.ntimes, r.dJ, r.e_on_device ? r.E : r.dE, 0, kJLinear, pair) != cudaSuccess)
+      return false;
     P.tile_begin = static_cast<int>(begin);
     begin += tc_problem_tiles(P);
   }

@@ -50,7 +50,7 @@
 // RowMap.  TMEM columns: accumulators at [0, N) and [256, 256 + N), unpacked
 // E stages (64 columns = 256 K bytes each) in the remaining columns.
 #include "bf_internal.h"
-#include "bf_ptx.cuh"
+#include "bf_tc_common.cuh"
 
 #include <algorithm>
 #include <atomic>
@@ -81,14 +81,6 @@ struct Roles {
   static constexpr int kFwdWarp = kUnpackWarp0 + 4 * kUnpackGroups;
   static constexpr int kThreads = 32 * (kFwdWarp + (kForwarder ? 1 : 0));
 };
-constexpr int kTT = 64;                 // times per tile
-constexpr int kBM = 128;                // GEMM rows per tile
-constexpr int kKC = 128;                // K bytes per TMA box / swizzle atom (64 dishes x re/im)
-constexpr int kSub = 2;                 // boxes per pipeline stage
-constexpr int kStageK = kSub * kKC;     // K bytes per stage (128 dishes x re/im): 8 MMAs
-static_assert(kSub == 2, "mma_ts_stage8 issues the eight MMAs of two W boxes");
-constexpr int kRawBox = kTT * kKC;      // raw E per box: 64 times x 64 dishes x 2 pol
-constexpr int kRawBytes = kSub * kRawBox;
 constexpr int kAccCols = 256;           // TMEM column offset of the second accumulator
 // Beam passes of at most kHalfPass beams run the half-SM layout: 4 epilogue
 // warps, 256 TMEM columns (second accumulator at column 128) and at most
@@ -96,19 +88,8 @@ constexpr int kAccCols = 256;           // TMEM column offset of the second accu
 // each SM has two MMA issuers, two unpack chains and two epilogues.
 constexpr int kAccColsHalf = 128;
 constexpr int kSmemLimitHalf = 115712;  // half of the SM's 228 KiB less the 1 KiB each block reserves
-constexpr int kStageCols = kStageK / 4;  // TMEM columns per unpacked stage
 constexpr int kSmemLimit = 232448;      // 227 KiB opt-in per block
 constexpr int kMaxStages = 8;
-constexpr int kDigSlots = 2;            // digit-row slots (one per tile in flight)
-// Offset correction: one extra MMA per tile, issued first (it also clears the
-// accumulator), multiplies a constant A tile by the tile's digit rows.  The
-// constant row holds -2^-6, -2^-2, -4, -64, -256 at K = 0..4 (again at 16..20,
-// so the 32-byte swizzle cannot move them), the digit row of n holds d0..d3 and
-// 4 d4 with sum_k W[n][k] = d0 + 16 d1 + 256 d2 + 4096 d3 + 65536 d4, so the
-// accumulator starts at -sum_k W[n][k] / 64 = -8 sum_k W[n][k] / 512 exactly.
-constexpr uint32_t kDigitScaleLo = 0xE8C8A888u;  // E4M3 -2^-6, -2^-2, -4, -64
-constexpr uint32_t kDigitScaleHi = 0x000000F8u;  // E4M3 -256
-constexpr int kConstABytes = kBM * kDigitRow;
 constexpr int kMaxWSlots = 6;
 constexpr int kMinRaw = 4;
 constexpr int kMaxRaw = 16;
@@ -246,58 +227,6 @@ __host__ __device__ inline SmemPlan smem_plan(int stages, int wslots, int raw, i
 __host__ __device__ inline uint32_t stage_col(int i, int ncols, int per_half, int acc_cols) {
   return i < per_half ? static_cast<uint32_t>(ncols + kStageCols * i)
                       : static_cast<uint32_t>(acc_cols + ncols + kStageCols * (i - per_half));
-}
-
-// Position in a ring of n slots: slot index and the parity of the pass over the ring.
-struct Ring {
-  uint32_t idx = 0, phase = 0, n;
-  __device__ explicit Ring(int n_) : n(static_cast<uint32_t>(n_)) {}
-  __device__ __forceinline__ void advance() {
-    if (++idx == n) {
-      idx = 0;
-      phase ^= 1u;
-    }
-  }
-};
-
-__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
-  uint32_t r;
-  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
-  return r;
-}
-
-// (c << 8) | (sat(re) << 4) | sat(im): two integers saturated to [0, 15] and
-// packed as the nibbles of one byte below the bytes of c.
-__device__ __forceinline__ uint32_t pack_u4x2(uint32_t re, uint32_t im, uint32_t c) {
-  uint32_t r;
-  asm("cvt.pack.sat.u4.s32.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(re), "r"(im), "r"(c));
-  return r;
-}
-
-// GEMM row r (0..31) of a lane quarter q <-> time and polarization of the tile.
-// The epilogue's loads give thread (g, c) = (lane / 4, lane % 4) the four rows
-// g, g + 8, g + 16, g + 24, so those hold four consecutive bytes of J: four
-// times of one polarization (Jlinear, arraysizes.hxx:92; quarter q holds 32
-// times of polarization q % 2), or two times of both (J2linear,
-// arraysizes.hxx:103; 16 times).  Which of the four sits in which row depends
-// on g through `swap`, which spreads the raw rows that 8 lanes of the unpack
-// read together over all 8 positions of the 128-byte swizzle (no bank
-// conflicts); the epilogue undoes it with one byte permute.
-template <bool kJ2>
-struct RowMap {
-  __device__ static __forceinline__ uint32_t swap(uint32_t g) { return kJ2 ? 2u * (g >> 2) : g >> 1; }
-  __device__ static __forceinline__ uint32_t time(uint32_t q, uint32_t r) {
-    const uint32_t g = r & 7u, j = (r >> 3) ^ swap(g);
-    return kJ2 ? 16u * q + 2u * g + (j >> 1) : 32u * (q >> 1) + 4u * g + j;
-  }
-  __device__ static __forceinline__ uint32_t pol(uint32_t q, uint32_t r) {
-    return kJ2 ? ((r >> 3) ^ swap(r & 7u)) & 1u : q & 1u;
-  }
-};
-
-// Byte offset of 16-byte chunk j of row r in a 128B-swizzled tile (TMA layout).
-__device__ __forceinline__ uint32_t sw128_offset(uint32_t r, uint32_t j) {
-  return (r >> 3) * 1024u + (r & 7u) * 128u + ((j ^ (r & 7u)) << 4);
 }
 
 template <bool kGrouped, bool kJ2, int kEpiW, bool kAdler, int kGroups, bool kHalf>
@@ -586,6 +515,7 @@ __global__ void __launch_bounds__(Roles<kEpiW, kGroups>::kThreads, kHalf ? 2 : 1
     const uint32_t pp = RowMap<kJ2>::pol(q, lane);
     const uint32_t tl = RowMap<kJ2>::time(q, lane);
     const uint32_t lane_addr = static_cast<uint32_t>(32 * q) << 16;
+    const UnpackRow row(tl);
     const uint32_t sel = pp ? 0x7531u : 0x6420u;  // odd or even bytes: polarization 1 or 0
     // this CTA's K stages: its tiles (TileRange) times nk
     const uint32_t my_tiles = TileRange::of<kGrouped>(p).count();
@@ -620,23 +550,7 @@ __global__ void __launch_bounds__(Roles<kEpiW, kGroups>::kThreads, kHalf ? 2 : 1
         // stores wait for the tensor core to release the stage
         uint32_t out[kSub][32];
 #pragma unroll
-        for (int h = 0; h < kSub; ++h) {
-          const uint8_t *raw = sR + r * kRawBytes + h * kRawBox;
-          uint32_t e[16];  // this lane's polarization, dishes 4m..4m+3 of the box in word m
-#pragma unroll
-          for (uint32_t j = 0; j < 8; ++j) {
-            // 16-byte chunk j: dishes 8j..8j+7, bytes [d0p0 d0p1 d1p0 d1p1 ...]
-            const uint4 w = *reinterpret_cast<const uint4 *>(raw + sw128_offset(tl, j));
-            e[2 * j] = prmt(w.x, w.y, sel);
-            e[2 * j + 1] = prmt(w.z, w.w, sel);
-          }
-          const uint32_t msk = 0x0F0F0F0Fu;
-#pragma unroll
-          for (int m = 0; m < 16; ++m) {
-            out[h][2 * m] = (e[m] >> 4) & msk;  // real nibbles u (E4M3 bytes = u * 2^-9)
-            out[h][2 * m + 1] = e[m] & msk;     // imaginary nibbles
-          }
-        }
+        for (int h = 0; h < kSub; ++h) unpack_box(smem_u32(sR) + r * kRawBytes + h * kRawBox, row, sel, out[h]);
         // the raw slot is in registers now; the next TMA into it is an async-proxy
         // write after these generic reads, so order them across proxies first
         fence_proxy_async_smem();
@@ -667,14 +581,10 @@ __global__ void __launch_bounds__(Roles<kEpiW, kGroups>::kThreads, kHalf ? 2 : 1
     }
   } else {
     // ------------------------------------------------------------ epilogue
-    // Warp w reads TMEM lane quarter w % 4 and column part w / 4; thread
-    // (g, c) of it takes rows g, g + 8, g + 16, g + 24 (four consecutive bytes of
-    // J, RowMap) of every fourth beam.
+    // Warp w reads TMEM lane quarter w % 4 and column part w / 4.
     const int q = warp & 3;
     const int part = warp >> 2;
-    const uint32_t g = lane >> 2, cb = lane & 3u;
     const uint32_t lane_addr = static_cast<uint32_t>(32 * q) << 16;
-    const uint32_t osel = 0x3210u ^ (0x1111u * RowMap<kJ2>::swap(g));  // rows' bytes into J's order
 
     // The warps of the epilogue share no barrier: each reads its chunks' gains
     // straight from the scaled-gain rows gs = 512 * G (L1-resident) and waits for
@@ -692,142 +602,24 @@ __global__ void __launch_bounds__(Roles<kEpiW, kGroups>::kThreads, kHalf ? 2 : 1
       const TcProblem &P = pc.at(p, tile, lt);
       int pass, tt, f;
       cur.take<kGrouped>(P, lt, pass, tt, f);
-      const int nchunk = P.nb_pass / 8;
-      const int c_begin = part * nchunk / kEpiParts, c_end = (part + 1) * nchunk / kEpiParts;
       const uint32_t ab = local & 1u;
       const uint32_t aph = (local >> 1) & 1u;
-      const int b0 = pass * P.nb_pass;
-      // 512 * G[f][b0 ..] (zero beyond B): the accumulator ends at raw / 512
-      // exactly and the power-of-two scaling is exact, so (512 G) * (raw / 512)
-      // rounds like G * raw (cpu.cxx:37)
-      const float *gcur = P.gs + static_cast<int64_t>(f) * P.npass * P.nb_pass + b0 + cb;
-      // huge or non-finite gains of this frequency: requantise with the
-      // narrowing of cpu.cxx:38 (tile-uniform branch, normally not taken)
-      const bool wide = __ldg(P.gwide + f) != 0;
-      if (!__all_sync(0xffffffffu, mbar_wait(accfull(ab), aph, err, kDevTimeoutAccFull))) break;
-      tc_fence_after();
-      const uint32_t acc_addr = tmem_base + ab * kAcc + lane_addr;
-      const int64_t bj = static_cast<int64_t>(b0 + static_cast<int>(cb)) * P.F + f;  // beam row b0 + cb
-      int64_t t;      // first time of the thread's 4 bytes
-      uint8_t *jrow;  // the thread's bytes for beam b0 + cb
-      if constexpr (!kJ2) {
-        t = static_cast<int64_t>(tt) * kTT + RowMap<kJ2>::time(q, 8 * RowMap<kJ2>::swap(g) + g);
-        jrow = P.J + (bj * 2 + (q & 1)) * P.jpitch + t;
-      } else {
-        t = static_cast<int64_t>(tt) * kTT + 16 * q + 2 * static_cast<int>(g);
-        jrow = P.J + bj * 2 * P.jpitch + 2 * t;
-      }
-      const bool t_ok = t < P.T;
-      const int64_t bstride = static_cast<int64_t>(P.F) * 2 * P.jpitch;  // bytes between beams, both layouts
-      const int blim = P.B - b0 - static_cast<int>(cb);  // beam offsets below this exist
-      uint8_t *dst = jrow + static_cast<int64_t>(8 * c_begin) * bstride;  // beam 8 c + cb of chunk c
-      // fused adler32: word h of the lane's chunk c_begin + cc sits at byte
-      // position base + cc * step + h * half (mod 65521), so the tile needs only
-      // a0 = sum of its bytes, a1 = sum cc * (bytes of chunk cc), a2 = sum of the
-      // second words' bytes, a3 = sum k * byte_k within words; then
-      // sum i d_i = base a0 + step a1 + half a2 + a3 (32-bit sums per tile:
-      // bytes <= 255, at most 16 words; the products are taken in 64 bits)
-      uint32_t ad_a0 = 0, ad_a1 = 0, ad_a2 = 0, ad_a3 = 0;
-
-      // Beams 8 c + cb and 8 c + 4 + cb, four rows each.  With the earlier 4x4 byte
-      // transpose across lanes and scalar clamps and conversions the epilogue took
-      // 86 instructions for 32 rows x 8 beams, now about 55: full chunk 956 -> 886
-      // us, wide array 812 -> 780 us, 128-problem batch 376 -> 355 us.  What bounds the epilogue
-      // is the issue rate and above all the integer pipe, so the arithmetic runs
-      // two values to an instruction on the float pipe: acc = raw / 512 exactly;
-      // x = (512 G) acc is one IEEE multiply, equal to G * raw (cpu.cxx:37); then
-      // x 2^-149 + 8 2^-149 is rounded once, to a multiple of the smallest
-      // subnormal, so its bit pattern is the integer lrint(x) + 8 (ties to even:
-      // 8 is even), a large positive integer above the range and a negative one
-      // below it.  The saturating pack clamps that to [0, 15] -- the nibble that
-      // ucomplex4 stores (icomplex4.hxx:33) -- and the one value below the lower
-      // clamp of cpu.cxx:38, nibble 0 (-8), becomes 1 (-7) for eight nibbles at once.
-      auto process = [&](int c, const uint32_t (&r)[16]) {
-        uint32_t w[2];
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-          const float gn = __ldg(gcur + 8 * c + 4 * k);
-          uint32_t x = 0;
-          if (!wide) {
-            const uint64_t g2 = f32x2(__float_as_uint(gn), __float_as_uint(gn));
-            const uint64_t tiny = f32x2(1u, 1u), eight = f32x2(8u, 8u);  // 2^-149 and 8 2^-149
-#pragma unroll
-            for (int j = 3; j >= 0; --j) {
-              const int at = 4 * k + 2 * (j & 1) + 8 * (j >> 1);
-              const uint64_t y = fma_f32x2(mul_f32x2(g2, f32x2(r[at], r[at + 1])), tiny, eight);
-              x = pack_u4x2(static_cast<uint32_t>(y), static_cast<uint32_t>(y >> 32), x);
-            }
-            uint32_t v = x | (x >> 1);
-            v |= v >> 2;
-            x |= ~v & 0x11111111u;
-          } else {
-#pragma unroll
-            for (int j = 3; j >= 0; --j) {
-              const int at = 4 * k + 2 * (j & 1) + 8 * (j >> 1);
-              x = pack_u4x2(static_cast<uint32_t>(requant_narrow(__fmul_rn(gn, __uint_as_float(r[at]))) + 8),
-                            static_cast<uint32_t>(requant_narrow(__fmul_rn(gn, __uint_as_float(r[at + 1]))) + 8), x);
-            }
-          }
-          w[k] = prmt(x, 0u, osel);
-        }
-        if (t_ok) {
-          if (8 * c < blim) __stcs(reinterpret_cast<uint32_t *>(dst), w[0]);
-          if (8 * c + 4 < blim) __stcs(reinterpret_cast<uint32_t *>(dst + 4 * bstride), w[1]);
-        }
-        if constexpr (kAdler) {  // only the bytes stored count
-          const uint32_t w0 = (t_ok && 8 * c < blim) ? w[0] : 0u;
-          const uint32_t w1 = (t_ok && 8 * c + 4 < blim) ? w[1] : 0u;
-          const uint32_t s1 = __dp4a(w1, 0x01010101u, 0u);
-          const uint32_t s01 = __dp4a(w0, 0x01010101u, s1);
-          ad_a0 += s01;
-          ad_a1 += static_cast<uint32_t>(c - c_begin) * s01;
-          ad_a2 += s1;
-          ad_a3 = __dp4a(w1, 0x03020100u, __dp4a(w0, 0x03020100u, ad_a3));
-        }
-        dst += 8 * bstride;
-      };
-
-      // accumulator columns in chunks of 16, the next chunk's TMEM load in flight
-      uint32_t ra[16], rb[16];
-      if (c_begin < c_end) {
-        tmem_ld_rows4_x2(acc_addr + 16u * c_begin, ra);
-        tmem_ld_wait(ra);
-      }
-      for (int c = c_begin; c < c_end; c += 2) {
-        const bool has1 = c + 1 < c_end, has2 = c + 2 < c_end;
-        if (has1) tmem_ld_rows4_x2(acc_addr + 16u * (c + 1), rb);
-        process(c, ra);
-        if (has1) {
-          tmem_ld_wait(rb);
-          if (has2) tmem_ld_rows4_x2(acc_addr + 16u * (c + 2), ra);
-          process(c + 1, rb);
-          if (has2) tmem_ld_wait(ra);
-        }
-      }
-      tc_fence_before();
-      mbar_arrive(accempty(ab));
-      if constexpr (kAdler) {
-        const uint64_t off = static_cast<uint64_t>((jrow + static_cast<int64_t>(8 * c_begin) * bstride) - P.jbase);
-        const uint32_t base = static_cast<uint32_t>(off % kAdlerMod);
-        const uint32_t half = static_cast<uint32_t>(static_cast<uint64_t>(4 * bstride) % kAdlerMod);
-        const uint32_t step = static_cast<uint32_t>(static_cast<uint64_t>(8 * bstride) % kAdlerMod);
-        ad_s1 += ad_a0;
-        ad_s2 += static_cast<unsigned long long>(base) * ad_a0 + static_cast<unsigned long long>(step) * ad_a1 +
-                 static_cast<unsigned long long>(half) * ad_a2 + ad_a3;
-      }
+      const EpilogueTile<kJ2, kAdler> et(P, f, pass, tt, q, lane);
+      const int nchunk = P.nb_pass / 8;
+      const bool ok = et.template run<2>(
+          P, tmem_base + ab * kAcc + lane_addr, part * nchunk / kEpiParts, (part + 1) * nchunk / kEpiParts, ad_s1, ad_s2,
+          [&]() {
+            const bool full = __all_sync(0xffffffffu, mbar_wait(accfull(ab), aph, err, kDevTimeoutAccFull));
+            tc_fence_after();
+            return full;
+          },
+          [&]() {
+            tc_fence_before();
+            mbar_arrive(accempty(ab));
+          });
+      if (!ok) break;
     }
-    if constexpr (kAdler) {  // one pair of atomics per warp
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        ad_s1 += __shfl_xor_sync(0xffffffffu, ad_s1, o);
-        ad_s2 += __shfl_xor_sync(0xffffffffu, ad_s2, o);
-      }
-      if (lane == 0) {
-        const TcProblem &P0 = p.one;
-        atomicAdd(P0.adler, ad_s1);
-        atomicAdd(P0.adler + 1, ad_s2);
-      }
-    }
+    if constexpr (kAdler) add_adler(p.one.adler, ad_s1, ad_s2, lane);
   }
 
   tc_fence_before();
@@ -970,13 +762,13 @@ void tc_set_ring_plan(int wslots, int raw) {
   g_plan_raw = raw;
 }
 
-void tc_plan_beams(int64_t B, int *nb_pass, int *npass) {
+void tc_plan_beams(int64_t B, int *nb_pass, int *npass, int granule) {
   // at most 96 beams (192 accumulator columns) per pass, so that two
-  // accumulators and at least four unpacked stages fit the 512 TMEM columns;
-  // passes are balanced
+  // accumulators and at least two unpacked stages fit the 512 TMEM columns;
+  // several passes are balanced in steps of `granule` beams
   const int64_t b8 = (B + 7) / 8 * 8;
   const int64_t np = (b8 + 95) / 96;
-  const int64_t nbp = ((b8 + np - 1) / np + 7) / 8 * 8;
+  const int64_t nbp = np == 1 ? b8 : ((b8 + np - 1) / np + granule - 1) / granule * granule;
   *nb_pass = static_cast<int>(nbp);
   *npass = static_cast<int>((b8 + nbp - 1) / nbp);
 }
@@ -1002,7 +794,7 @@ cudaError_t launch_prep_weights(const TcWeights &w, const uint8_t *A, cudaStream
 
 // Fills a problem record: shape, pointers and the two tensor maps.
 static cudaError_t make_problem(TcProblem &P, const TcWeights &w, int64_t T, uint8_t *J, const uint8_t *E,
-                                int64_t jpitch, int j_layout) {
+                                int64_t jpitch, int j_layout, bool pair) {
   const int64_t F = w.F, D = w.D;
   if ((reinterpret_cast<uintptr_t>(E) & 15u) || (reinterpret_cast<uintptr_t>(J) & 15u)) return cudaErrorMisalignedAddress;
   std::memset(&P, 0, sizeof(P));
@@ -1020,6 +812,8 @@ static cudaError_t make_problem(TcProblem &P, const TcWeights &w, int64_t T, uin
   P.npass = w.npass;
   P.ntt = static_cast<int>((T + kTT - 1) / kTT);
   P.nw_pad = w.nw_pad;
+  P.pair = pair ? 1 : 0;
+  P.w_rows = pair ? pair_cols(w.nb_pass) / 2 : 2 * w.nb_pass;
   P.gs = w.gs;
   P.gwide = w.gwide;
   {  // E[t][f][d*p] bytes: dims {2D, F, T}
@@ -1033,14 +827,14 @@ static cudaError_t make_problem(TcProblem &P, const TcWeights &w, int64_t T, uin
     const cuuint64_t dims[3] = {static_cast<cuuint64_t>(2 * D), static_cast<cuuint64_t>(w.nw),
                                 static_cast<cuuint64_t>(F)};
     const cuuint64_t str[2] = {static_cast<cuuint64_t>(2 * D), static_cast<cuuint64_t>(2 * D * w.nw)};
-    const cuuint32_t box[3] = {static_cast<cuuint32_t>(kKC), static_cast<cuuint32_t>(2 * w.nb_pass), 1};
+    const cuuint32_t box[3] = {static_cast<cuuint32_t>(kKC), static_cast<cuuint32_t>(P.w_rows), 1};
     if (!make_map(&P.tm_w, w.W, 3, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B)) return cudaErrorInvalidValue;
   }
   {  // digit rows dig[f][n][32] bytes: dims {32, nw_pad, F}
     const cuuint64_t dims[3] = {static_cast<cuuint64_t>(kDigitRow), static_cast<cuuint64_t>(w.nw_pad),
                                 static_cast<cuuint64_t>(F)};
     const cuuint64_t str[2] = {static_cast<cuuint64_t>(kDigitRow), static_cast<cuuint64_t>(kDigitRow) * w.nw_pad};
-    const cuuint32_t box[3] = {static_cast<cuuint32_t>(kDigitRow), static_cast<cuuint32_t>(2 * w.nb_pass), 1};
+    const cuuint32_t box[3] = {static_cast<cuuint32_t>(kDigitRow), static_cast<cuuint32_t>(P.w_rows), 1};
     if (!make_map(&P.tm_d, w.dig, 3, dims, str, box, CU_TENSOR_MAP_SWIZZLE_32B)) return cudaErrorInvalidValue;
   }
   return cudaSuccess;
@@ -1144,12 +938,19 @@ static cudaError_t launch_kernel(const TcParams &p, int smem_bytes, cudaStream_t
   }
 }
 
+// Passes of at most kHalfPass beams run two CTAs on each SM instead: their MMAs
+// take a few cycles, so two of everything else on an SM is worth more than
+// sharing W (b = 16: DRAM at 0.87 of the copy bandwidth).
+bool tc_pair_launch(int max_nb_pass) { return max_nb_pass > kHalfPass && pair_clusters() > 0; }
+
 cudaError_t tc_make_problem(TcProblem &P, const TcWeights &w, int64_t T, uint8_t *J, const uint8_t *E,
-                            int64_t jpitch, int j_layout) {
-  return make_problem(P, w, T, J, E, jpitch, j_layout);
+                            int64_t jpitch, int j_layout, bool pair) {
+  return make_problem(P, w, T, J, E, jpitch, j_layout, pair);
 }
 
-int64_t tc_problem_tiles(const TcProblem &P) { return static_cast<int64_t>(P.ntt) * P.F * P.npass; }
+int64_t tc_problem_tiles(const TcProblem &P) {
+  return static_cast<int64_t>(P.pair ? (P.ntt + 1) / 2 : P.ntt) * P.F * P.npass;
+}
 
 int tc_stages_per_tile(int64_t D) { return static_cast<int>((D + kStageK / 2 - 1) / (kStageK / 2)); }
 
@@ -1182,6 +983,12 @@ cudaError_t tc_plan_rings(int64_t D, int max_nb_pass, const TcRingPlan &plan, in
 
 cudaError_t tc_launch_shape(int64_t D, int max_nb_pass, const TcRingPlan &plan, int *stages, int *groups,
                             int *ctas_per_sm) {
+  if (tc_pair_launch(max_nb_pass)) {
+    *ctas_per_sm = 1;
+    const cudaError_t e = pair_launch_shape(D, max_nb_pass, stages);
+    *groups = *stages >= 4 ? 2 : plan.pair_groups;
+    return e;
+  }
   TcParams p{};
   p.nk = tc_stages_per_tile(D);
   int smem_bytes = 0;
@@ -1195,6 +1002,12 @@ cudaError_t tc_launch_shape(int64_t D, int max_nb_pass, const TcRingPlan &plan, 
 
 cudaError_t launch_tc_grouped(const TcProblem *table, int nprob, int ntiles, int64_t D, int max_nb_pass,
                               const TcRingPlan &plan, int *err, cudaStream_t s) {
+  if (tc_pair_launch(max_nb_pass)) {
+    int stages = 0, groups = 0, ctas = 0;
+    const cudaError_t e = tc_launch_shape(D, max_nb_pass, plan, &stages, &groups, &ctas);
+    if (e != cudaSuccess) return e;
+    return launch_pair_grouped(table, nprob, ntiles, D, max_nb_pass, groups, g_test_stall, err, s);
+  }
   TcParams p{};
   p.table = table;
   p.nprob = nprob;
@@ -1210,11 +1023,13 @@ cudaError_t launch_tc_grouped(const TcProblem *table, int nprob, int ntiles, int
 cudaError_t launch_tc(const TcWeights &w, int64_t T, uint8_t *J, const uint8_t *E, int *err, cudaStream_t s,
                       int64_t jpitch, int j_layout, unsigned long long *adler, const uint8_t *jbase) {
   TcParams p{};
-  cudaError_t e = make_problem(p.one, w, T, J, E, jpitch, j_layout);
+  const bool pair = tc_pair_launch(w.nb_pass);
+  cudaError_t e = make_problem(p.one, w, T, J, E, jpitch, j_layout, pair);
   if (e != cudaSuccess) return e;
   p.one.adler = adler;
   if (jbase) p.one.jbase = jbase;
   if (adler && (p.one.jbase > J)) return cudaErrorInvalidValue;
+  if (pair) return launch_pair(p.one, w.D, g_test_stall, err, s);
   const int64_t ntiles = static_cast<int64_t>(p.one.ntt) * w.F * w.npass;
   if (ntiles > 0x7FFFFFFF) return cudaErrorInvalidValue;
   p.ntiles = static_cast<int>(ntiles);

@@ -1,0 +1,643 @@
+// bf_tc_pair.cu -- the tensor-core beamformer on pairs of SMs (cta_group::2).
+//
+// Same GEMM, operands and epilogue as bf_tc.cu (see there for the arithmetic),
+// but two CTAs of a cluster work on one tile of 128 times: each unpacks its own
+// 64 times into its own tensor memory and requantises them, and one thread of
+// the leader issues every MMA for both (M = 256).  Each CTA holds one half of
+// the W rows, so W costs a CTA half the shared memory: a frequency's whole W
+// (b = 96, d = 512: 96 KB) stays resident and is loaded once per frequency
+// instead of once per tile, and the tensor cores read half as many bytes of it
+// from shared memory.  In the one-CTA kernel W went through shared memory
+// twice per tile (TMA write, MMA read), 3072 of the ~4600 cycles of shared-memory
+// traffic a tile needs at 128 B per cycle, against 3072 cycles of MMA work.
+//
+// Tiles of a cluster are contiguous: beam pass fastest, then time, then
+// frequency (then problem).  W stage ks of a new (problem, frequency, pass) is
+// loaded as soon as the tensor cores finished the last tile that used slot ks.
+// Where W does not fit (deep K), or the next tile is another pass, the slots are
+// an ordinary ring.
+//
+// Warp roles of each CTA (kEpiW epilogue warps):
+//   epilogue     as in bf_tc.cu
+//   E producer   TMA of raw E boxes
+//   MMA          leader: issues for both CTAs.  Peer: tells the leader when its
+//                own W stages and digit rows have landed
+//   W producer   TMA of this CTA's half of W and of the digit rows
+//   unpack       8 warps: one group in which two warps per lane quarter take one
+//                box of each stage (passes wider than 64 beams, two TMEM stages),
+//                or two groups of four that take stages in turn
+#include "bf_internal.h"
+#include "bf_tc_common.cuh"
+
+#include <algorithm>
+#include <atomic>
+
+namespace bf {
+namespace {
+
+constexpr int kPairAcc = 256;        // TMEM column of the second accumulator
+constexpr int kPairSmem = 232448;    // 227 KiB opt-in per block
+constexpr int kPairMaxRaw = 16;
+constexpr int kPairMaxStages = 8;
+constexpr int kUnpackWarps = 8;
+constexpr int kEpiW = 8;       // epilogue warps
+constexpr int kEpiChunks = 2;  // chunks of 8 beams in flight per epilogue warp
+constexpr int kPairThreads = 32 * (kEpiW + kUnpackWarps + 3);
+
+struct PairParams {
+  TcProblem one;            // the problem of a plain launch
+  const TcProblem *table;   // grouped launch: nprob problems in device memory, by tile_begin
+  int nprob;
+  int ntiles;               // tile pairs
+  int nk;                   // K stages per tile
+  int ncols;                // widest GEMM N of the launch (a multiple of 32)
+  int stages, wslots, raw;  // TMEM stages, W slots, raw E slots
+  int test_stall;
+  int *err;
+};
+
+struct PairSmem {
+  int wbytes, dbytes;
+  int off_a, off_d, off_r, off_bar, nbar, total;
+};
+
+__host__ __device__ inline PairSmem pair_smem(int stages, int wslots, int raw, int ncols) {
+  PairSmem s{};
+  s.wbytes = kSub * (ncols / 2) * kKC;  // this CTA's half of the rows
+  s.dbytes = (ncols / 2 * kDigitRow + 1023) / 1024 * 1024;
+  s.off_a = wslots * s.wbytes;
+  s.off_d = s.off_a + kConstABytes;
+  s.off_r = s.off_d + kDigSlots * s.dbytes;
+  s.off_bar = s.off_r + raw * kRawBytes;
+  // raw_full[R] raw_empty[R] w_full[SW] w_peer[SW] w_empty[SW] a_full[S] empty[S] accfull[2] accempty[2]
+  // d_full[2] d_peer[2] d_empty[2]
+  s.nbar = 2 * raw + 3 * wslots + 2 * stages + 4 + 3 * kDigSlots;
+  s.total = s.off_bar + 8 * s.nbar + 32;  // + the TMEM address and the leader's commit counts
+  return s;
+}
+
+// A cluster's tiles, one by one.
+template <bool kGrouped>
+struct PairCursor {
+  const TcProblem *P;
+  int idx = 0, pass, tp, f, ntp;
+  __device__ __forceinline__ PairCursor(const PairParams &p, int first) : P(&p.one) {
+    int lt = first;
+    if constexpr (kGrouped) {
+      int lo = 0, hi = p.nprob - 1;
+      while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (p.table[mid].tile_begin <= first) lo = mid; else hi = mid - 1;
+      }
+      idx = lo;
+      P = p.table + lo;
+      lt -= P->tile_begin;
+    }
+    ntp = (P->ntt + 1) >> 1;
+    pass = lt % P->npass;
+    tp = (lt / P->npass) % ntp;
+    f = lt / (P->npass * ntp);
+  }
+  // the next tile has other W rows
+  __device__ __forceinline__ bool last_of_w() const { return P->npass > 1 || tp + 1 == ntp; }
+  __device__ __forceinline__ void next(const PairParams &p) {
+    if (++pass < P->npass) return;
+    pass = 0;
+    if (++tp < ntp) return;
+    tp = 0;
+    ++f;
+    if constexpr (kGrouped) {
+      if (f == P->F && idx + 1 < p.nprob) {
+        f = 0;
+        P = p.table + ++idx;
+        ntp = (P->ntt + 1) >> 1;
+      }
+    }
+  }
+  // beams of this tile's pass (a multiple of 8) and its GEMM N (a multiple of 32)
+  __device__ __forceinline__ int beams() const { return min(P->nb_pass, (P->B + 7) / 8 * 8 - pass * P->nb_pass); }
+  __device__ __forceinline__ int n() const { return (2 * beams() + 31) & ~31; }
+};
+
+// TMEM column of unpacked stage i: the columns left beside the two accumulators.
+__host__ __device__ inline uint32_t pair_stage_col(uint32_t i, int ncols, int per_half, int cols) {
+  return static_cast<uint32_t>(ncols) + i * static_cast<uint32_t>(cols) +
+         (i < static_cast<uint32_t>(per_half) ? 0u : static_cast<uint32_t>(kPairAcc - per_half * cols));
+}
+
+template <bool kGrouped, bool kJ2, bool kAdler, int kGroups>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
+    bf_form_beams_pair(const __grid_constant__ PairParams p) {
+  constexpr int kUnpackWarp0 = kEpiW, kEProdWarp = kEpiW + kUnpackWarps, kMmaWarp = kEProdWarp + 1;
+  constexpr int kWProdWarp = kEProdWarp + 2;
+  constexpr int kEpiParts = kEpiW / 4;
+  constexpr int kStageWarps = kUnpackWarps / kGroups;  // unpack warps of a stage
+  constexpr int kBoxes = kSub * 4 / kStageWarps;       // boxes of it each of them takes
+  static_assert(kGroups == 1 || kGroups == 2, "one group of 8 unpack warps or two of 4");
+  extern __shared__ uint8_t smem_dyn[];
+  // the same offset in both CTAs of the cluster
+  uint8_t *smem = smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u);
+  const int S = p.stages, SW = p.wslots, R = p.raw, nk = p.nk;
+  const PairSmem sp = pair_smem(S, SW, R, p.ncols);
+  uint8_t *sW = smem, *sA = smem + sp.off_a, *sD = smem + sp.off_d, *sR = smem + sp.off_r;
+  const uint32_t bar0 = smem_u32(smem + sp.off_bar);
+  auto raw_full = [&](int r) { return bar0 + 8u * r; };
+  auto raw_empty = [&](int r) { return bar0 + 8u * (R + r); };
+  const uint32_t bw = bar0 + 16u * R;
+  auto w_full = [&](int s) { return bw + 8u * s; };
+  auto w_peer = [&](int s) { return bw + 8u * (SW + s); };
+  auto w_empty = [&](int s) { return bw + 8u * (2 * SW + s); };
+  const uint32_t ba = bw + 24u * SW;
+  auto a_full = [&](int s) { return ba + 8u * s; };
+  auto empty = [&](int s) { return ba + 8u * (S + s); };
+  const uint32_t bc = ba + 16u * S;
+  auto accfull = [&](int i) { return bc + 8u * i; };
+  auto accempty = [&](int i) { return bc + 16u + 8u * i; };
+  auto d_full = [&](int i) { return bc + 32u + 8u * i; };
+  auto d_peer = [&](int i) { return bc + 48u + 8u * i; };
+  auto d_empty = [&](int i) { return bc + 64u + 8u * i; };
+  uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(smem + sp.off_bar + 8 * sp.nbar);
+  uint32_t *counts = tmem_holder + 1;  // commits the leader issued on empty, w_empty, d_empty, accfull
+
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);  // known to be warp-uniform
+  const int lane = threadIdx.x & 31;
+  const int rank = static_cast<int>(cluster_ctarank());
+  const int ncols = p.ncols;
+  const int per_half = (kPairAcc - ncols) / kStageCols;
+
+  if (threadIdx.x == 0) {
+    for (int r = 0; r < R; ++r) {
+      mbar_init(raw_full(r), 1);
+      mbar_init(raw_empty(r), kStageWarps);
+    }
+    for (int s = 0; s < SW; ++s) {
+      mbar_init(w_full(s), 1);
+      mbar_init(w_peer(s), 1);
+      mbar_init(w_empty(s), 1);
+    }
+    for (int s = 0; s < S; ++s) {
+      mbar_init(a_full(s), 2 * kStageWarps);  // the leader's: the unpack warps of a stage in both CTAs
+      mbar_init(empty(s), 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(accfull(i), 1);
+      mbar_init(accempty(i), 2 * kEpiW);  // the leader's: both CTAs' epilogue warps
+      mbar_init(d_full(i), 1);
+      mbar_init(d_peer(i), 1);
+      mbar_init(d_empty(i), 1);
+    }
+    for (int i = 0; i < 4; ++i) counts[i] = 0;
+    fence_barrier_init();
+  }
+  // constant A tile of the offset MMA: every row the same, so the 32-byte
+  // swizzle leaves it unchanged
+  for (int i = threadIdx.x; i < kConstABytes / 4; i += blockDim.x) {
+    const int w = i & 7;
+    reinterpret_cast<uint32_t *>(sA)[i] = (w == 0 || w == 4) ? kDigitScaleLo : (w == 1 || w == 5) ? kDigitScaleHi : 0u;
+  }
+  fence_proxy_async_smem();
+  if (warp == kMmaWarp) {
+    tmem_alloc_pair(smem_u32(tmem_holder), 512);
+    tmem_relinquish_pair();
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_holder;
+  int *err = p.err;
+
+  const int64_t ncl = gridDim.x >> 1, cl = blockIdx.x >> 1;
+  const int first = static_cast<int>(cl * p.ntiles / ncl), end = static_cast<int>((cl + 1) * p.ntiles / ncl);
+  const bool stream_w = SW < nk;  // W slots are an ordinary ring
+
+  if (warp == kEProdWarp) {
+    // ------------------------------------------------------------ E producer
+    if (lane == 0 && !p.test_stall) {
+      const uint64_t pol_e = policy_evict_first();
+      Ring rr(R);
+      uint32_t issued = 0;
+      bool ok = true;
+      const TcProblem *seen = nullptr;
+      PairCursor<kGrouped> cur(p, first);
+      for (int tile = first; ok && tile < end; ++tile, cur.next(p)) {
+        if (kGrouped && cur.P != seen) {  // a table entry the host rewrites between launches
+          tensormap_acquire(&cur.P->tm_e);
+          seen = cur.P;
+        }
+        for (int ks = 0; ks < nk; ++ks, rr.advance(), ++issued) {
+          const int r = static_cast<int>(rr.idx);
+          if (!mbar_wait(raw_empty(r), rr.phase ^ 1u, err, kDevTimeoutEmpty)) {
+            ok = false;
+            break;
+          }
+          mbar_arrive_expect_tx(raw_full(r), kRawBytes);
+#pragma unroll
+          for (int h = 0; h < kSub; ++h)
+            tma_load_3d(smem_u32(sR + r * kRawBytes + h * kRawBox), &cur.P->tm_e, raw_full(r), (ks * kSub + h) * kKC,
+                        cur.f, (2 * cur.tp + rank) * kTT, pol_e);
+        }
+      }
+      // let the copies already issued land before the CTA exits, on every exit
+      for (uint32_t k = (issued >= static_cast<uint32_t>(R) ? issued - R : 0); k < issued; ++k)
+        mbar_wait_drain(raw_full(static_cast<int>(k % R)), (k / R) & 1u);
+    }
+  } else if (warp == kWProdWarp) {
+    // ------------------------------------------------------------ W producer
+    if (lane == 0 && !p.test_stall) {
+      const uint64_t pol_w = policy_evict_last();
+      Ring wr(SW), dr(kDigSlots);
+      uint32_t it = 0, dit = 0;
+      bool ok = true, fresh = true;
+      const TcProblem *seen = nullptr;
+      PairCursor<kGrouped> cur(p, first);
+      for (int tile = first; ok && tile < end; ++tile) {
+        if (fresh || stream_w) {
+          if (kGrouped && cur.P != seen) {
+            tensormap_acquire(&cur.P->tm_w);
+            tensormap_acquire(&cur.P->tm_d);
+            seen = cur.P;
+          }
+          const int row0 = cur.pass * 2 * cur.P->nb_pass + rank * (cur.n() / 2);
+          const int wbox = cur.P->w_rows * kKC;
+          if (fresh) {  // the digit rows, for the offset MMA
+            const int ds = static_cast<int>(dr.idx);
+            if (!mbar_wait(d_empty(ds), dr.phase ^ 1u, err, kDevTimeoutEmpty)) break;
+            mbar_arrive_expect_tx(d_full(ds), cur.P->w_rows * kDigitRow);
+            tma_load_3d(smem_u32(sD + ds * sp.dbytes), &cur.P->tm_d, d_full(ds), 0, row0, cur.f, pol_w);
+            dr.advance();
+            ++dit;
+          }
+          for (int ks = 0; ks < nk; ++ks, ++it, wr.advance()) {
+            const int s = static_cast<int>(wr.idx);
+            if (!mbar_wait(w_empty(s), wr.phase ^ 1u, err, kDevTimeoutEmpty)) {
+              ok = false;
+              break;
+            }
+            mbar_arrive_expect_tx(w_full(s), kSub * wbox);
+#pragma unroll
+            for (int h = 0; h < kSub; ++h)
+              tma_load_3d(smem_u32(sW + s * sp.wbytes + h * wbox), &cur.P->tm_w, w_full(s), (ks * kSub + h) * kKC,
+                          row0, cur.f, pol_w);
+          }
+        }
+        fresh = cur.last_of_w();
+        cur.next(p);
+      }
+      for (uint32_t k = (it >= static_cast<uint32_t>(SW) ? it - SW : 0); k < it; ++k)
+        mbar_wait_drain(w_full(static_cast<int>(k % SW)), (k / SW) & 1u);
+      for (uint32_t k = (dit >= static_cast<uint32_t>(kDigSlots) ? dit - kDigSlots : 0); k < dit; ++k)
+        mbar_wait_drain(d_full(static_cast<int>(k % kDigSlots)), (k / kDigSlots) & 1u);
+    }
+  } else if (warp == kMmaWarp && rank == 1) {
+    // ------------------------------------- peer: this CTA's W and digits landed
+    if (lane == 0 && !p.test_stall) {
+      Ring wr(SW), dr(kDigSlots);
+      bool ok = true, fresh = true;
+      PairCursor<kGrouped> cur(p, first);
+      for (int tile = first; ok && tile < end; ++tile) {
+        if (fresh) {
+          if (!mbar_wait(d_full(dr.idx), dr.phase, err, kDevTimeoutFull)) break;
+          mbar_arrive_cluster(map_cta(d_peer(dr.idx), 0));
+          dr.advance();
+        }
+        if (fresh || stream_w) {
+          for (int ks = 0; ks < nk; ++ks, wr.advance()) {
+            if (!mbar_wait(w_full(wr.idx), wr.phase, err, kDevTimeoutFull)) {
+              ok = false;
+              break;
+            }
+            mbar_arrive_cluster(map_cta(w_peer(wr.idx), 0));
+          }
+        }
+        fresh = cur.last_of_w();
+        cur.next(p);
+      }
+    }
+    __syncwarp();
+  } else if (warp == kMmaWarp) {
+    // ------------------------------------------------------------ MMA issuer
+    // Warp-uniform, one elected lane issues (see bf_tc.cu).  The tensor core
+    // idles whenever a stage costs this warp more than its MMAs take, so the
+    // loop of the common tile -- resident W, neither loaded nor given back --
+    // holds nothing but the wait, the MMAs and the commit.
+    Ring ar(S), wr(SW), dr(kDigSlots);
+    const uint64_t a_const = smem_desc_sw32(smem_u32(sA));
+    const uint64_t w_desc0 = smem_desc_sw128(smem_u32(sW));
+    const uint32_t w_step = static_cast<uint32_t>(sp.wbytes) >> 4;
+    uint32_t local = 0;
+    uint32_t nstage = 0, nw = 0, ndig = 0, nacc = 0;  // commits issued on empty, w_empty, d_empty, accfull
+    bool ok = true, fresh = true;
+    PairCursor<kGrouped> cur(p, first);
+    for (int tile = first; ok && tile < end; ++tile, ++local) {
+      const uint32_t idesc = idesc_e4m3_f32(2 * kBM, static_cast<uint32_t>(cur.n()));
+      const uint32_t wbox = static_cast<uint32_t>(cur.P->w_rows * kKC) >> 4;
+      const bool last = cur.last_of_w();
+      const uint32_t ab = local & 1u;
+      if (!__all_sync(0xffffffffu, mbar_wait(accempty(ab), ((local >> 1) & 1u) ^ 1u, err, kDevTimeoutAccEmpty))) break;
+      const int ds = static_cast<int>(dr.idx);
+      if (fresh && !__all_sync(0xffffffffu, mbar_wait(d_full(ds), dr.phase, err, kDevTimeoutFull) &&
+                                                mbar_wait(d_peer(ds), dr.phase, err, kDevTimeoutFull)))
+        break;
+      tc_fence_after();
+      const uint32_t d_tmem = tmem_base + ab * kPairAcc;
+      // the offset MMA starts the accumulator at -8 sum_k W[n][k] / 512
+      if (elect_one()) {
+        mma_f8f6f4_pair(d_tmem, a_const, smem_desc_sw32(smem_u32(sD + ds * sp.dbytes)), idesc, 0u);
+        if (last) mma_commit_pair(d_empty(ds));
+      }
+      __syncwarp();
+      if (last) {
+        ++ndig;
+        dr.advance();
+      }
+      if (!fresh && !last && !stream_w) {
+        uint64_t b_desc = w_desc0;
+        for (int ks = 0; ks < nk; ++ks, b_desc += w_step) {
+          const uint32_t bar = a_full(ar.idx);
+          if (!__all_sync(0xffffffffu, mbar_wait(bar, ar.phase, err, kDevTimeoutUnpacked))) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t a_tmem = tmem_base + pair_stage_col(ar.idx, ncols, per_half, kStageCols);
+          if (elect_one()) {
+            mma_ts_box_pair(d_tmem, a_tmem, b_desc, idesc);
+            mma_ts_box_pair(d_tmem, a_tmem + 32, b_desc + wbox, idesc);
+            mma_commit_pair(bar + 8u * S);  // empty
+          }
+          __syncwarp();
+          ++nstage;
+          ar.advance();
+        }
+        if (ok && elect_one()) mma_commit_pair(accfull(ab));
+        __syncwarp();
+      } else {
+        const bool reload = fresh || stream_w, release = last || stream_w;
+        for (int ks = 0; ks < nk; ++ks, ar.advance()) {
+          // the parity of a W slot's current load: resident slots (SW == nk) step
+          // with the loads, not with the tiles
+          const int sw = stream_w ? static_cast<int>(wr.idx) : ks;
+          if (reload && !__all_sync(0xffffffffu, mbar_wait(w_full(sw), wr.phase, err, kDevTimeoutFull) &&
+                                                     mbar_wait(w_peer(sw), wr.phase, err, kDevTimeoutFull))) {
+            ok = false;
+            break;
+          }
+          const uint32_t bar = a_full(ar.idx);
+          if (!__all_sync(0xffffffffu, mbar_wait(bar, ar.phase, err, kDevTimeoutUnpacked))) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t a_tmem = tmem_base + pair_stage_col(ar.idx, ncols, per_half, kStageCols);
+          const uint64_t b_desc = w_desc0 + static_cast<uint32_t>(sw) * w_step;
+          if (elect_one()) {
+            mma_ts_box_pair(d_tmem, a_tmem, b_desc, idesc);
+            mma_ts_box_pair(d_tmem, a_tmem + 32, b_desc + wbox, idesc);
+            mma_commit_pair(bar + 8u * S);  // empty
+            if (release) mma_commit_pair(w_empty(sw));
+            if (ks + 1 == nk) mma_commit_pair(accfull(ab));
+          }
+          __syncwarp();
+          ++nstage;
+          nw += release ? 1u : 0u;
+          if (reload) wr.advance();
+        }
+      }
+      if (!ok) break;
+      ++nacc;
+      fresh = last;
+      cur.next(p);
+    }
+    // A commit's arrival is an asynchronous write into both CTAs' shared memory:
+    // wait (bounded) for the last phase committed on every barrier before the
+    // CTAs can exit, here and, from the counts, in the peer.
+    if (lane == 0) {
+      const uint32_t at = map_cta(smem_u32(counts), 1);
+      st_cluster_u32(at, nstage);
+      st_cluster_u32(at + 4, nw);
+      st_cluster_u32(at + 8, ndig);
+      st_cluster_u32(at + 12, nacc);
+      counts[0] = nstage;
+      counts[1] = nw;
+      counts[2] = ndig;
+      counts[3] = nacc;
+    }
+    __syncwarp();
+  } else if (warp >= kUnpackWarp0 && warp < kEProdWarp) {
+    // ------------------------------------------------------------ unpack
+    // Each lane fills one GEMM row: it reads the raw row of its time, which
+    // holds both polarizations, and keeps its own (RowMap).  Two groups take
+    // stages in turn (R and S are even, so a slot always belongs to one group).
+    const int group = (warp - kUnpackWarp0) / kStageWarps;
+    const int box0 = ((warp - kUnpackWarp0) % kStageWarps >> 2) * kBoxes;
+    const int q = warp & 3;
+    const UnpackRow row(RowMap<kJ2>::time(q, lane));
+    const uint32_t sel = RowMap<kJ2>::pol(q, lane) ? 0x7531u : 0x6420u;  // odd or even bytes
+    const uint32_t lane_addr = static_cast<uint32_t>(32 * q) << 16;
+    const uint32_t total = static_cast<uint32_t>(end - first) * static_cast<uint32_t>(nk);
+    Ring rr(R), ar(S);
+    for (int g = 0; g < group; ++g) {
+      rr.advance();
+      ar.advance();
+    }
+    for (uint32_t it = group; it < total; it += kGroups) {
+      const int r = static_cast<int>(rr.idx);
+      const int s = static_cast<int>(ar.idx);
+      if (!__all_sync(0xffffffffu, mbar_wait(raw_full(r), rr.phase, err, kDevTimeoutFull))) break;
+      // the stage goes to registers first, so that only the tensor-memory
+      // stores wait for the tensor core to release the stage
+      uint32_t out[kBoxes][32];
+#pragma unroll
+      for (int h = 0; h < kBoxes; ++h) unpack_box(smem_u32(sR) + r * kRawBytes + (box0 + h) * kRawBox, row, sel, out[h]);
+      // the next TMA into the slot is an async-proxy write after these generic reads
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(raw_empty(r));
+      if (!__all_sync(0xffffffffu, mbar_wait(empty(s), ar.phase ^ 1u, err, kDevTimeoutEmpty))) break;
+      const uint32_t col = tmem_base + lane_addr + pair_stage_col(s, ncols, per_half, kStageCols);
+#pragma unroll
+      for (int h = 0; h < kBoxes; ++h) tmem_st_32x32b_x32(col + 32 * (box0 + h), out[h]);
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster_relaxed(map_cta(a_full(s), 0));
+#pragma unroll
+      for (int g = 0; g < kGroups; ++g) {
+        rr.advance();
+        ar.advance();
+      }
+    }
+  } else if (warp < kEpiW) {
+    // ------------------------------------------------------------ epilogue
+    // Warp w reads TMEM lane quarter w % 4 and column part w / 4.  The warps
+    // share no barrier: a slow one does not hold up the others.
+    const int q = warp & 3;
+    const int part = warp >> 2;
+    const uint32_t lane_addr = static_cast<uint32_t>(32 * q) << 16;
+    uint32_t local = 0;
+    unsigned long long ad_s1 = 0, ad_s2 = 0;  // fused adler32 (kAdler): sums of the J bytes this lane stores
+    PairCursor<kGrouped> cur(p, first);
+    for (int tile = first; tile < end; ++tile, ++local, cur.next(p)) {
+      const uint32_t ab = local & 1u;
+      const EpilogueTile<kJ2, kAdler> et(*cur.P, cur.f, cur.pass, 2 * cur.tp + rank, q, lane);
+      const int nchunk = cur.beams() / 8;
+      const bool ok = et.template run<kEpiChunks>(
+          *cur.P, tmem_base + ab * kPairAcc + lane_addr, part * nchunk / kEpiParts, (part + 1) * nchunk / kEpiParts,
+          ad_s1, ad_s2,
+          [&]() {
+            const bool full = __all_sync(0xffffffffu, mbar_wait(accfull(ab), (local >> 1) & 1u, err, kDevTimeoutAccFull));
+            tc_fence_after();
+            return full;
+          },
+          [&]() {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster_relaxed(map_cta(accempty(ab), 0));
+          });
+      if (!ok) break;
+    }
+    if constexpr (kAdler) add_adler(p.one.adler, ad_s1, ad_s2, lane);
+  }
+
+  // Both CTAs wait for the leader's last commits to arrive (see the MMA issuer)
+  // and for each other before either frees tensor memory or exits.
+  __syncwarp();
+  cluster_sync();
+  if (warp == kMmaWarp) {
+    const uint32_t uS = static_cast<uint32_t>(S), uW = static_cast<uint32_t>(SW), uD = static_cast<uint32_t>(kDigSlots);
+    const uint32_t c0 = counts[0], c1 = counts[1], c2 = counts[2], c3 = counts[3];
+    for (uint32_t k = c0 > uS ? c0 - uS : 0; k < c0; ++k) mbar_wait_drain(empty(static_cast<int>(k % uS)), (k / uS) & 1u);
+    for (uint32_t k = c1 > uW ? c1 - uW : 0; k < c1; ++k)
+      mbar_wait_drain(w_empty(static_cast<int>(k % uW)), (k / uW) & 1u);
+    for (uint32_t k = c2 > uD ? c2 - uD : 0; k < c2; ++k)
+      mbar_wait_drain(d_empty(static_cast<int>(k % uD)), (k / uD) & 1u);
+    for (uint32_t k = c3 > 2u ? c3 - 2u : 0u; k < c3; ++k) mbar_wait_drain(accfull(static_cast<int>(k & 1u)), (k >> 1) & 1u);
+    __syncwarp();
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync();
+  if (warp == kMmaWarp) {
+    tc_fence_after();
+    tmem_dealloc_pair(tmem_base, 512);
+  }
+}
+
+// Ring depths and shared memory of a launch whose widest GEMM N is ncols.
+cudaError_t plan_pair(PairParams &p, int64_t D, int ncols, int *smem_bytes) {
+  p.nk = tc_stages_per_tile(D);
+  const int stages = std::min(kPairMaxStages, 2 * ((kPairAcc - ncols) / (kStageCols)));
+  if (stages < 2) return cudaErrorInvalidValue;
+  // W resident (all nk slots) where at least 64 KB of raw E slots fit beside it,
+  // else as many slots as that leaves: a W load takes ~2400 cycles from the
+  // commit that frees its slot to the peer's word that it landed
+  auto total = [&](int w, int r) { return pair_smem(stages, w, r, ncols).total + 1024; };
+  int wslots = p.nk;
+  if (total(wslots, 4) > kPairSmem) {
+    wslots = 2;
+    while (wslots < p.nk - 1 && total(wslots + 1, 4) <= kPairSmem) ++wslots;
+  }
+  int raw = 2;
+  while (raw < kPairMaxRaw && total(wslots, raw + 1) <= kPairSmem) ++raw;
+  raw -= raw % 2;  // a raw slot stays with one unpack group
+  p.ncols = ncols;
+  p.stages = stages;
+  p.wslots = wslots;
+  p.raw = raw;
+  *smem_bytes = total(wslots, raw);
+  return *smem_bytes > kPairSmem ? cudaErrorInvalidValue : cudaSuccess;
+}
+
+template <bool kGrouped, bool kJ2, bool kAdler, int kGroups>
+cudaError_t launch_inst(const PairParams &p, int smem_bytes, cudaStream_t s) {
+  auto kern = bf_form_beams_pair<kGrouped, kJ2, kAdler, kGroups>;
+  static std::atomic<bool> attr_set{false};
+  if (!attr_set.load()) {
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem);
+    if (e != cudaSuccess) return e;
+    attr_set.store(true);
+  }
+  const int grid = 2 * std::min(p.ntiles, pair_clusters());
+  if (grid <= 0) return cudaSuccess;
+  kern<<<grid, kPairThreads, smem_bytes, s>>>(p);
+  return cudaGetLastError();
+}
+
+}  // namespace
+
+int pair_cols(int nb_pass) { return (2 * nb_pass + 31) / 32 * 32; }
+
+int pair_clusters() {
+  static const int n = []() {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+      return 0;
+    auto kern = bf_form_beams_pair<false, false, false, 2>;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return 0;
+    }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(2);
+    cfg.blockDim = dim3(kPairThreads);
+    cfg.dynamicSmemBytes = kPairSmem;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 2;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int k = 0;
+    if (cudaOccupancyMaxActiveClusters(&k, kern, &cfg) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return 0;
+    }
+    return std::min(k, sms / 2);
+  }();
+  return n;
+}
+
+cudaError_t pair_launch_shape(int64_t D, int max_nb_pass, int *stages) {
+  PairParams p{};
+  int smem_bytes = 0;
+  const cudaError_t e = plan_pair(p, D, pair_cols(max_nb_pass), &smem_bytes);
+  *stages = p.stages;
+  return e;
+}
+
+cudaError_t launch_pair(const TcProblem &one, int64_t D, int test_stall, int *err, cudaStream_t s) {
+  PairParams p{};
+  p.one = one;
+  p.nprob = 1;
+  const int64_t ntiles = tc_problem_tiles(one);
+  if (ntiles > 0x7FFFFFFF) return cudaErrorInvalidValue;
+  p.ntiles = static_cast<int>(ntiles);
+  p.err = err;
+  p.test_stall = test_stall;
+  int smem_bytes = 0;
+  const cudaError_t e = plan_pair(p, D, pair_cols(one.nb_pass), &smem_bytes);
+  if (e != cudaSuccess) return e;
+  const bool j2 = one.jlayout == kJ2, adler = one.adler != nullptr;
+  if (j2)
+    return adler ? launch_inst<false, true, true, 2>(p, smem_bytes, s) : launch_inst<false, true, false, 2>(p, smem_bytes, s);
+  return adler ? launch_inst<false, false, true, 2>(p, smem_bytes, s) : launch_inst<false, false, false, 2>(p, smem_bytes, s);
+}
+
+cudaError_t launch_pair_grouped(const TcProblem *table, int nprob, int ntiles, int64_t D, int max_nb_pass, int groups,
+                                int test_stall, int *err, cudaStream_t s) {
+  PairParams p{};
+  p.table = table;
+  p.nprob = nprob;
+  p.ntiles = ntiles;
+  p.err = err;
+  p.test_stall = test_stall;
+  int smem_bytes = 0;
+  const cudaError_t e = plan_pair(p, D, pair_cols(max_nb_pass), &smem_bytes);
+  if (e != cudaSuccess) return e;
+  return groups == 1 ? launch_inst<true, false, false, 1>(p, smem_bytes, s)
+                     : launch_inst<true, false, false, 2>(p, smem_bytes, s);
+}
+
+}  // namespace bf
