@@ -85,7 +85,7 @@ struct TcWeights {
   int nw_pad = 0;    // digit rows per frequency: npass * 2 * nb_pass
   uint8_t *W = nullptr;      // [F][nw][2D]
   uint8_t *dig = nullptr;    // [F][nw_pad][kDigitRow]
-  float *gs = nullptr;       // [F][nw_pad / 2]: 512 * G, zero past B (the epilogue's gains)
+  float *gs = nullptr;       // [F][nw_pad / 2]: 2^18 G, zero past B (the epilogue's gains)
   int *gwide = nullptr;      // [F]: nonzero when a gain of the frequency can take |G * raw| to 2^31
   const float *G = nullptr;  // [F][B] (device; read by the weight preparation)
 };

@@ -17,14 +17,18 @@
 // value, set by one extra MMA that opens every tile (digit rows of the row
 // sums times a constant tile, see kDigitScaleLo):
 //
-//   acc[n] = -8 * sum_k W[n][k] / 512 + sum_k u_k W[n][k] / 512
-//          = sum_k (u_k - 8) W[n][k] / 512 = raw / 512
+//   acc[n] = 2^-18 (-8 sum_k W[n][k] + sum_k u_k W[n][k])
+//          = 2^-18 sum_k (u_k - 8) W[n][k] = 2^-18 raw
 //
-// W holds the integers Ar, -Ai, Ai in [-8, 8], exact in E4M3; the start value
-// and every partial sum are integer multiples of 2^-9 below 2^10 in magnitude
-// (at most 19 significant bits), exact in the f32 accumulator.  The
+// W holds the integers Ar, -Ai, Ai in [-8, 8] in the same form, w * 2^-9 (a sign
+// and the low nibble).  The start value and every partial sum are integer
+// multiples of 2^-18 below 2^1 in magnitude (at most 19 significant bits), exact
+// in the f32 accumulator.  As normal numbers (w itself) the products are just
+// as exact, but the codes' exponent bits toggle from column to column, and the
+// chip runs at its power limit: the full chunk took 745 us with them, 719
+// with subnormals (the wide array 743, 726; sustained).  The
 // requantisation clamp(lrint(G * float(raw)), -7, 7) of cpu.cxx:37-39 is one
-// IEEE multiply by 512 G (exactly G * raw) and a round-half-even step.
+// IEEE multiply by 2^18 G (exactly G * raw) and a round-half-even step.
 //
 // Warp roles (one CTA per SM, persistent over tiles; warp numbers for the
 // layout of 8 epilogue warps, 480 threads; with 12 epilogue warps, 608
@@ -446,7 +450,7 @@ __global__ void __launch_bounds__(Roles<kEpiW, kGroups>::kThreads, kHalf ? 2 : 1
         if (!__all_sync(0xffffffffu, mbar_wait(d_full(ds), dr.phase, err, kDevTimeoutFull))) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + ab * kAcc;
-        // the offset MMA starts the accumulator at -8 sum_k W[n][k] / 512
+        // the offset MMA starts the accumulator at -8 sum_k W[n][k] 2^-18
         if (elect_one()) {
           mma_f8f6f4(d_tmem, a_const, smem_desc_sw32(smem_u32(sD + ds * sp.dbytes)), idesc, 0u);
           mma_commit(d_empty(ds));
@@ -587,7 +591,7 @@ __global__ void __launch_bounds__(Roles<kEpiW, kGroups>::kThreads, kHalf ? 2 : 1
     const uint32_t lane_addr = static_cast<uint32_t>(32 * q) << 16;
 
     // The warps of the epilogue share no barrier: each reads its chunks' gains
-    // straight from the scaled-gain rows gs = 512 * G (L1-resident) and waits for
+    // straight from the scaled-gain rows gs = 2^18 G (L1-resident) and waits for
     // the accumulator on its own, so a slow warp does not hold up the others.
     uint32_t local = 0;
     // fused adler32 (kAdler): this lane's sums of the J bytes it stores,
@@ -642,13 +646,12 @@ __global__ void __launch_bounds__(32 * kPrepRows) bf_prep_weights(const uint8_t 
                                                                    const float *__restrict__ G, float *__restrict__ gs,
                                                                    int *__restrict__ gwide, int B, int D, int nw,
                                                                    int nw_pad, int a_layout) {
-  // E4M3 codes of the integers 0..8
-  const uint8_t e4m3_pos[9] = {0x00, 0x38, 0x40, 0x44, 0x48, 0x4A, 0x4C, 0x4E, 0x50};
+  // the E4M3 code of v * 2^-9, |v| <= 15, is |v| with a sign bit
   const int rblocks = (nw_pad + kPrepRows - 1) / kPrepRows;  // blocks per frequency
   const int f = static_cast<int>(blockIdx.x) / rblocks;
   const int n = (static_cast<int>(blockIdx.x) % rblocks) * kPrepRows + static_cast<int>(threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  if (static_cast<int>(blockIdx.x) % rblocks == 0) {  // the frequency's scaled gains: 512 G, zero past B
+  if (static_cast<int>(blockIdx.x) % rblocks == 0) {  // the frequency's scaled gains: 2^18 G, zero past B
     const int ng = nw_pad / 2;
     // |raw| <= 128 D, so with |G| * 128 D < 2^30 every product G * raw stays
     // below 2^31 and the plain requantisation is exact; otherwise (or for a
@@ -657,7 +660,7 @@ __global__ void __launch_bounds__(32 * kPrepRows) bf_prep_weights(const uint8_t 
     int wide = 0;
     for (int i = threadIdx.x; i < ng; i += blockDim.x) {
       const float g = i < B ? G[static_cast<int64_t>(f) * B + i] : 0.0f;
-      gs[static_cast<int64_t>(f) * ng + i] = 512.0f * g;
+      gs[static_cast<int64_t>(f) * ng + i] = 262144.0f * g;
       wide |= !(fabsf(g) < wide_at);
     }
     wide = __syncthreads_or(wide);
@@ -683,7 +686,7 @@ __global__ void __launch_bounds__(32 * kPrepRows) bf_prep_weights(const uint8_t 
           v = cj == 0 ? (c == 0 ? ar : -ai) : (c == 0 ? ai : ar);
         }
         const int av = v < 0 ? -v : v;
-        word |= static_cast<uint32_t>(e4m3_pos[av] | (v < 0 ? 0x80 : 0x00)) << (8 * j);
+        word |= static_cast<uint32_t>(av | (v < 0 ? 0x80 : 0x00)) << (8 * j);
         sum += v;
       }
       wrow[k4] = word;
@@ -703,9 +706,9 @@ __global__ void __launch_bounds__(32 * kPrepRows) bf_prep_weights(const uint8_t 
       const int dj = r >= 8 ? r - 16 : r;
       rest = (rest - dj) >> 4;
       const int av = dj < 0 ? -dj : dj;
-      w0 |= static_cast<uint32_t>(e4m3_pos[av] | (dj < 0 ? 0x80 : 0x00)) << (8 * j);
+      w0 |= static_cast<uint32_t>(av | (dj < 0 ? 0x80 : 0x00)) << (8 * j);
     }
-    w1 = rest == 0 ? 0u : (rest > 0 ? 0x48u : 0xC8u);  // 4 * d4: +-4 or 0
+    w1 = rest == 0 ? 0u : (rest > 0 ? 0x04u : 0x84u);  // 4 * d4: +-4 or 0
     uint32_t *row = reinterpret_cast<uint32_t *>(dig + (static_cast<int64_t>(f) * nw_pad + n) * kDigitRow);
     row[0] = w0;
     row[1] = w1;

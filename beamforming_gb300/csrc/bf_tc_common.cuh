@@ -23,8 +23,8 @@ constexpr int kDigSlots = 2;            // digit-row slots (one per tile in flig
 // accumulator), multiplies a constant A tile by the tile's digit rows.  The
 // constant row holds -2^-6, -2^-2, -4, -64, -256 at K = 0..4 (again at 16..20,
 // so the 32-byte swizzle cannot move them), the digit row of n holds d0..d3 and
-// 4 d4 with sum_k W[n][k] = d0 + 16 d1 + 256 d2 + 4096 d3 + 65536 d4, so the
-// accumulator starts at -sum_k W[n][k] / 64 = -8 sum_k W[n][k] / 512 exactly.
+// 4 d4, all times 2^-9, with sum_k W[n][k] = d0 + 16 d1 + 256 d2 + 4096 d3 + 65536 d4, so the
+// accumulator starts at -2^-15 sum_k W[n][k] = -8 sum_k W[n][k] 2^-18 exactly.
 constexpr uint32_t kDigitScaleLo = 0xE8C8A888u;  // E4M3 -2^-6, -2^-2, -4, -64
 constexpr uint32_t kDigitScaleHi = 0x000000F8u;  // E4M3 -256
 constexpr int kConstABytes = kBM * kDigitRow;
@@ -131,8 +131,8 @@ struct EpilogueTile {
     const uint32_t g = static_cast<uint32_t>(lane) >> 2, cb = static_cast<uint32_t>(lane) & 3u;
     osel = 0x3210u ^ (0x1111u * RowMap<kJ2>::swap(g));
     const int b0 = pass * P.nb_pass;
-    // 512 * G[f][b0 ..] (zero beyond B): the accumulator ends at raw / 512
-    // exactly and the power-of-two scaling is exact, so (512 G) * (raw / 512)
+    // 2^18 G[f][b0 ..] (zero beyond B): the accumulator ends at 2^-18 raw
+    // exactly and the power-of-two scaling is exact, so (2^18 G) * (2^-18 raw)
     // rounds like G * raw (cpu.cxx:37)
     gcur = P.gs + static_cast<int64_t>(f) * P.npass * P.nb_pass + b0 + cb;
     // huge or non-finite gains of this frequency: requantise with the
@@ -155,8 +155,8 @@ struct EpilogueTile {
   // The J words of 8 beams (one chunk: beams 8 c + cb and 8 c + 4 + cb, four rows
   // each) from their accumulators and scaled gains.  What bounds the epilogue
   // is the issue rate and above all the integer pipe, so the arithmetic runs
-  // two values to an instruction on the float pipe: acc = raw / 512 exactly;
-  // x = (512 G) acc is one IEEE multiply, equal to G * raw (cpu.cxx:37); then
+  // two values to an instruction on the float pipe: acc = 2^-18 raw exactly;
+  // x = (2^18 G) acc is one IEEE multiply, equal to G * raw (cpu.cxx:37); then
   // x 2^-149 + 8 2^-149 is rounded once, to a multiple of the smallest
   // subnormal, so its bit pattern is the integer lrint(x) + 8 (ties to even:
   // 8 is even), a large positive integer above the range and a negative one

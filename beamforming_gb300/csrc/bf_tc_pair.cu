@@ -341,7 +341,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
         break;
       tc_fence_after();
       const uint32_t d_tmem = tmem_base + ab * kPairAcc;
-      // the offset MMA starts the accumulator at -8 sum_k W[n][k] / 512
+      // the offset MMA starts the accumulator at -8 sum_k W[n][k] 2^-18
       if (elect_one()) {
         mma_f8f6f4_pair(d_tmem, a_const, smem_desc_sw32(smem_u32(sD + ds * sp.dbytes)), idesc, 0u);
         if (last) mma_commit_pair(d_empty(ds));
