@@ -182,7 +182,7 @@ int bf_batch_create(bf_batch **out, const bf_problem *problems, int nproblems, b
   plans[1].raw = 8;
   plans[2].wslots = 2;
   plans[2].raw = 12;
-  for (TcRingPlan &plan : plans) plan.pair_groups = 1;
+  for (TcRingPlan &plan : plans) plan.one_group = true;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);

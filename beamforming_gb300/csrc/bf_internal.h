@@ -162,7 +162,7 @@ struct TcProblem {  // 128-byte aligned through its tensor maps
 struct TcRingPlan {
   int wslots = 0;
   int raw = 0;
-  int pair_groups = 2;  // unpack groups of a pair launch with two TMEM stages (passes wider than 64 beams)
+  bool one_group = false;  // one unpack group beside two TMEM stages, also on pairs of SMs
 };
 
 // Whether a launch whose widest pass has max_nb_pass beams runs on pairs of SMs.
@@ -191,7 +191,7 @@ cudaError_t tc_plan_rings(int64_t D, int max_nb_pass, const TcRingPlan &plan, in
 // (0: none), the GEMM N of a pass, the TMEM stages of a launch, and the launches.
 int pair_clusters();
 int pair_cols(int nb_pass);
-cudaError_t pair_launch_shape(int64_t D, int max_nb_pass, int *stages);
+cudaError_t pair_launch_shape(int64_t D, int max_nb_pass, int groups, int *stages);
 cudaError_t launch_pair(const TcProblem &one, int64_t D, int test_stall, int *err, cudaStream_t s);
 cudaError_t launch_pair_grouped(const TcProblem *table, int nprob, int ntiles, int64_t D, int max_nb_pass, int groups,
                                 int test_stall, int *err, cudaStream_t s);

@@ -984,13 +984,17 @@ cudaError_t tc_plan_rings(int64_t D, int max_nb_pass, const TcRingPlan &plan, in
   return cudaSuccess;
 }
 
+// Unpack groups of a pair launch.
+static int pair_groups(int max_nb_pass, const TcRingPlan &plan) {
+  return plan.one_group && max_nb_pass > kNarrowPass ? 1 : 2;
+}
+
 cudaError_t tc_launch_shape(int64_t D, int max_nb_pass, const TcRingPlan &plan, int *stages, int *groups,
                             int *ctas_per_sm) {
   if (tc_pair_launch(max_nb_pass)) {
     *ctas_per_sm = 1;
-    const cudaError_t e = pair_launch_shape(D, max_nb_pass, stages);
-    *groups = *stages >= 4 ? 2 : plan.pair_groups;
-    return e;
+    *groups = pair_groups(max_nb_pass, plan);
+    return pair_launch_shape(D, max_nb_pass, *groups, stages);
   }
   TcParams p{};
   p.nk = tc_stages_per_tile(D);
@@ -1005,12 +1009,9 @@ cudaError_t tc_launch_shape(int64_t D, int max_nb_pass, const TcRingPlan &plan, 
 
 cudaError_t launch_tc_grouped(const TcProblem *table, int nprob, int ntiles, int64_t D, int max_nb_pass,
                               const TcRingPlan &plan, int *err, cudaStream_t s) {
-  if (tc_pair_launch(max_nb_pass)) {
-    int stages = 0, groups = 0, ctas = 0;
-    const cudaError_t e = tc_launch_shape(D, max_nb_pass, plan, &stages, &groups, &ctas);
-    if (e != cudaSuccess) return e;
-    return launch_pair_grouped(table, nprob, ntiles, D, max_nb_pass, groups, g_test_stall, err, s);
-  }
+  if (tc_pair_launch(max_nb_pass))
+    return launch_pair_grouped(table, nprob, ntiles, D, max_nb_pass, pair_groups(max_nb_pass, plan), g_test_stall, err,
+                               s);
   TcParams p{};
   p.table = table;
   p.nprob = nprob;

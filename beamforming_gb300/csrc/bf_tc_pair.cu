@@ -23,9 +23,14 @@
 //   MMA          leader: issues for both CTAs.  Peer: tells the leader when its
 //                own W stages and digit rows have landed
 //   W producer   TMA of this CTA's half of W and of the digit rows
-//   unpack       8 warps: one group in which two warps per lane quarter take one
-//                box of each stage (passes wider than 64 beams, two TMEM stages),
-//                or two groups of four that take stages in turn
+//   unpack       8 warps: two groups of four that take stages in turn, or (batches
+//                of passes wider than 64 beams) one group in which two warps per
+//                lane quarter take one box of each stage.  With two stages in
+//                tensor memory a stage must be stored, announced and waited for
+//                within the 768 cycles of the other's MMAs; two groups overlap
+//                the rest of their work (664 against 703 us on the full chunk
+//                in short bursts).  More warps only contend for the integer pipe
+//                (16 unpack warps 712, 12 epilogue warps 693 us).
 #include "bf_internal.h"
 #include "bf_tc_common.cuh"
 
@@ -39,9 +44,9 @@ constexpr int kPairAcc = 256;        // TMEM column of the second accumulator
 constexpr int kPairSmem = 232448;    // 227 KiB opt-in per block
 constexpr int kPairMaxRaw = 16;
 constexpr int kPairMaxStages = 8;
-constexpr int kUnpackWarps = 8;
 constexpr int kEpiW = 8;       // epilogue warps
 constexpr int kEpiChunks = 2;  // chunks of 8 beams in flight per epilogue warp
+constexpr int kUnpackWarps = 8;
 constexpr int kPairThreads = 32 * (kEpiW + kUnpackWarps + 3);
 
 struct PairParams {
@@ -133,7 +138,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
   constexpr int kEpiParts = kEpiW / 4;
   constexpr int kStageWarps = kUnpackWarps / kGroups;  // unpack warps of a stage
   constexpr int kBoxes = kSub * 4 / kStageWarps;       // boxes of it each of them takes
-  static_assert(kGroups == 1 || kGroups == 2, "one group of 8 unpack warps or two of 4");
   extern __shared__ uint8_t smem_dyn[];
   // the same offset in both CTAs of the cluster
   uint8_t *smem = smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u);
@@ -427,8 +431,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
   } else if (warp >= kUnpackWarp0 && warp < kEProdWarp) {
     // ------------------------------------------------------------ unpack
     // Each lane fills one GEMM row: it reads the raw row of its time, which
-    // holds both polarizations, and keeps its own (RowMap).  Two groups take
-    // stages in turn (R and S are even, so a slot always belongs to one group).
+    // holds both polarizations, and keeps its own (RowMap).  The groups take
+    // stages in turn (R and S are multiples of their number, so a slot always
+    // belongs to one group).
     const int group = (warp - kUnpackWarp0) / kStageWarps;
     const int box0 = ((warp - kUnpackWarp0) % kStageWarps >> 2) * kBoxes;
     const int q = warp & 3;
@@ -445,19 +450,24 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
       const int r = static_cast<int>(rr.idx);
       const int s = static_cast<int>(ar.idx);
       if (!__all_sync(0xffffffffu, mbar_wait(raw_full(r), rr.phase, err, kDevTimeoutFull))) break;
-      // the stage goes to registers first, so that only the tensor-memory
-      // stores wait for the tensor core to release the stage
-      uint32_t out[kBoxes][32];
+      // box by box: the first box's words are made before the stage is free, the
+      // others' while the stores of the one before are under way
+      const uint32_t raw = smem_u32(sR) + static_cast<uint32_t>(r * kRawBytes + box0 * kRawBox);
+      const uint32_t col = tmem_base + lane_addr + pair_stage_col(s, ncols, per_half, kStageCols) + 32u * box0;
+      bool free = true;
 #pragma unroll
-      for (int h = 0; h < kBoxes; ++h) unpack_box(smem_u32(sR) + r * kRawBytes + (box0 + h) * kRawBox, row, sel, out[h]);
+      for (int h = 0; h < kBoxes; ++h) {
+        uint32_t out[32];
+        unpack_box(raw + h * kRawBox, row, sel, out);
+        if (h == 0) free = __all_sync(0xffffffffu, mbar_wait(empty(s), ar.phase ^ 1u, err, kDevTimeoutEmpty));
+        if (!free) break;
+        tmem_st_32x32b_x32(col + 32 * h, out);
+      }
+      if (!free) break;
       // the next TMA into the slot is an async-proxy write after these generic reads
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(raw_empty(r));
-      if (!__all_sync(0xffffffffu, mbar_wait(empty(s), ar.phase ^ 1u, err, kDevTimeoutEmpty))) break;
-      const uint32_t col = tmem_base + lane_addr + pair_stage_col(s, ncols, per_half, kStageCols);
-#pragma unroll
-      for (int h = 0; h < kBoxes; ++h) tmem_st_32x32b_x32(col + 32 * (box0 + h), out[h]);
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
@@ -525,9 +535,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 }
 
 // Ring depths and shared memory of a launch whose widest GEMM N is ncols.
-cudaError_t plan_pair(PairParams &p, int64_t D, int ncols, int *smem_bytes) {
+cudaError_t plan_pair(PairParams &p, int64_t D, int ncols, int groups, int *smem_bytes) {
   p.nk = tc_stages_per_tile(D);
-  const int stages = std::min(kPairMaxStages, 2 * ((kPairAcc - ncols) / (kStageCols)));
+  int stages = std::min(kPairMaxStages, 2 * ((kPairAcc - ncols) / kStageCols));
+  stages -= stages % groups;  // so does a TMEM stage
   if (stages < 2) return cudaErrorInvalidValue;
   // W resident (all nk slots) where at least 64 KB of raw E slots fit beside it,
   // else as many slots as that leaves: a W load takes ~2400 cycles from the
@@ -540,7 +551,7 @@ cudaError_t plan_pair(PairParams &p, int64_t D, int ncols, int *smem_bytes) {
   }
   int raw = 2;
   while (raw < kPairMaxRaw && total(wslots, raw + 1) <= kPairSmem) ++raw;
-  raw -= raw % 2;  // a raw slot stays with one unpack group
+  raw -= raw % groups;  // a raw slot stays with one unpack group
   p.ncols = ncols;
   p.stages = stages;
   p.wslots = wslots;
@@ -599,10 +610,10 @@ int pair_clusters() {
   return n;
 }
 
-cudaError_t pair_launch_shape(int64_t D, int max_nb_pass, int *stages) {
+cudaError_t pair_launch_shape(int64_t D, int max_nb_pass, int groups, int *stages) {
   PairParams p{};
   int smem_bytes = 0;
-  const cudaError_t e = plan_pair(p, D, pair_cols(max_nb_pass), &smem_bytes);
+  const cudaError_t e = plan_pair(p, D, pair_cols(max_nb_pass), groups, &smem_bytes);
   *stages = p.stages;
   return e;
 }
@@ -617,7 +628,7 @@ cudaError_t launch_pair(const TcProblem &one, int64_t D, int test_stall, int *er
   p.err = err;
   p.test_stall = test_stall;
   int smem_bytes = 0;
-  const cudaError_t e = plan_pair(p, D, pair_cols(one.nb_pass), &smem_bytes);
+  const cudaError_t e = plan_pair(p, D, pair_cols(one.nb_pass), 2, &smem_bytes);
   if (e != cudaSuccess) return e;
   const bool j2 = one.jlayout == kJ2, adler = one.adler != nullptr;
   if (j2)
@@ -634,7 +645,7 @@ cudaError_t launch_pair_grouped(const TcProblem *table, int nprob, int ntiles, i
   p.err = err;
   p.test_stall = test_stall;
   int smem_bytes = 0;
-  const cudaError_t e = plan_pair(p, D, pair_cols(max_nb_pass), &smem_bytes);
+  const cudaError_t e = plan_pair(p, D, pair_cols(max_nb_pass), groups, &smem_bytes);
   if (e != cudaSuccess) return e;
   return groups == 1 ? launch_inst<true, false, false, 1>(p, smem_bytes, s)
                      : launch_inst<true, false, false, 2>(p, smem_bytes, s);
