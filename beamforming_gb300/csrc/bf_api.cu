@@ -70,6 +70,11 @@ struct DeviceCtx {
   DevBuf W, dig;            // tensor-core operand for non-resident calls
   DevBuf partials;          // adler32 partial sums
   DevBuf adl;               // fused adler32 sums {sum d_i, sum i d_i} of the last checked call
+  // Scratch of the padded route (run_padded): operand and E copy of the call
+  // that used it last, on whatever stream; the next one waits for pad_done.
+  DevBuf padE, padW, padDig;
+  cudaEvent_t pad_done = nullptr;
+  bool pad_used = false;
 };
 
 constexpr int kMaxDevices = 64;
@@ -122,12 +127,13 @@ void plan_weights(TcWeights &w, int64_t F, int64_t B, int64_t D) {
   w.F = F;
   w.B = B;
   w.D = D;
+  w.Dk = (D + 7) / 8 * 8;
   tc_plan_beams(B, &w.nb_pass, &w.npass);
   w.nw = static_cast<int>((B + 7) / 8 * 8 * 2);
   w.nw_pad = w.npass * 2 * w.nb_pass;
 }
 
-size_t weights_bytes(const TcWeights &w) { return static_cast<size_t>(w.F) * w.nw * 2 * w.D; }
+size_t weights_bytes(const TcWeights &w) { return static_cast<size_t>(w.F) * w.nw * 2 * w.Dk; }
 
 
 int choose_tensor(const bf_dims &d, bool *use_tc) {
@@ -148,10 +154,89 @@ int run_device_bufs(const bf_dims &d, uint8_t *J, const uint8_t *E, const uint8_
                     DevBuf &dig, int *err, cudaStream_t s, int a_layout = kALinear, int j_layout = kJLinear,
                     unsigned long long *adl = nullptr, bool *fused = nullptr);
 
+// A shape the tensor-core kernel does not take in place, on it all the same
+// (TcPadded); *ran = false where the dp4a kernel has to take it: the rule or the
+// memory says so, or the stream is being captured (the scratch is shared with
+// later calls, which a graph cannot wait for).  `rw`: resident weights, whose
+// operand is used instead of preparing A.  The caller holds c.mu.
+int run_padded(DeviceCtx &c, const bf_dims &d, uint8_t *J, const uint8_t *E, const uint8_t *A, const float *G,
+               const TcWeights *rw, cudaStream_t s, int a_layout, int j_layout, unsigned long long *adl, bool *fused,
+               bool *ran) {
+  *ran = false;
+  const TcPadded r = tc_padded(d, E);
+  if (!r.ok) return BF_OK;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+    (void)cudaGetLastError();
+    return BF_OK;
+  }
+  TcWeights w;
+  if (rw) {
+    w = *rw;
+  } else {
+    plan_weights(w, d.nfrequencies, d.nbeams, d.ndishes);
+  }
+  if (!c.pad_done) BF_TRY(cudaEventCreateWithFlags(&c.pad_done, cudaEventDisableTiming));
+  if (c.pad_used) BF_TRY(cudaStreamWaitEvent(s, c.pad_done, 0));
+  cudaError_t e = r.copy ? c.padE.reserve(r.bytes) : cudaSuccess;
+  if (!rw && e == cudaSuccess) e = c.padW.reserve(weights_bytes(w));
+  if (!rw && e == cudaSuccess) e = c.padDig.reserve(tc_extra_bytes(w));
+  if (e == cudaErrorMemoryAllocation) {
+    (void)cudaGetLastError();
+    return BF_OK;
+  }
+  BF_TRY(e);
+  *ran = true;
+  t_last_kernel = "tensor";
+  c.pad_used = true;
+  const int st = [&]() -> int {
+    if (!rw) {
+      w.W = c.padW.as<uint8_t>();
+      tc_set_extra(w, c.padDig.as<uint8_t>());
+      w.G = G;
+      BF_TRY(launch_prep_weights(w, A, s, a_layout));
+    }
+    if (adl) {
+      BF_TRY(cudaMemsetAsync(adl, 0, 2 * sizeof(unsigned long long), s));
+      if (fused) *fused = true;
+    }
+    const int64_t P = d.npolarizations, per_t = d.nfrequencies * d.ndishes * P;
+    for (int64_t t0 = 0; t0 < d.ntimes; t0 += r.times) {
+      const int64_t nt = std::min(r.times, d.ntimes - t0);
+      const uint8_t *Ec = E + t0 * per_t;
+      if (r.copy) {
+        BF_TRY(launch_pad_e(d, Ec, esize(d) - static_cast<size_t>(t0 * per_t), nt, c.padE.as<uint8_t>(), s));
+        Ec = c.padE.as<uint8_t>();
+      }
+      if (P == 1) {
+        const TcRows rows{d.ntimes, nt};
+        const int64_t pairs = (nt + 1) / 2;
+        BF_TRY(launch_tc(w, pairs, J + t0, Ec, c.err, s, (d.ntimes + 1) / 2, kJ2, adl, J, &rows));
+      } else {
+        BF_TRY(launch_tc(w, nt, J + (j_layout == kJ2 ? 2 * t0 : t0), Ec, c.err, s, d.ntimes, j_layout, adl, J));
+      }
+    }
+    return BF_OK;
+  }();
+  const cudaError_t re = cudaEventRecord(c.pad_done, s);
+  return st != BF_OK ? st : to_status(re);
+}
+
 // All four arrays on the device.  Operand scratch comes from ctx (caller holds ctx.mu).
 int run_device(DeviceCtx &c, const bf_dims &d, uint8_t *J, const uint8_t *E, const uint8_t *A, const float *G,
                cudaStream_t s, int a_layout = kALinear, int j_layout = kJLinear, unsigned long long *adl = nullptr,
                bool *fused = nullptr) {
+  if (fused) *fused = false;
+  if (jsize(d) == 0) return BF_OK;
+  bool use_tc = false;
+  const int st = choose_tensor(d, &use_tc);
+  if (st != BF_OK) return st;
+  const bool aligned = ((reinterpret_cast<uintptr_t>(E) | reinterpret_cast<uintptr_t>(J)) & 15u) == 0;
+  if (g_kernel.load() == BF_KERNEL_AUTO && !(use_tc && aligned)) {
+    bool ran = false;
+    const int ps = run_padded(c, d, J, E, A, G, nullptr, s, a_layout, j_layout, adl, fused, &ran);
+    if (ran || ps != BF_OK) return ps;
+  }
   return run_device_bufs(d, J, E, A, G, c.W, c.dig, c.err, s, a_layout, j_layout, adl, fused);
 }
 
@@ -618,6 +703,12 @@ int bf_form_beams_resident(const bf_weights *w, int64_t ntimes, uint8_t *J, cons
   if (use_tc) {
     t_last_kernel = "tensor";
     return to_status(launch_tc(w->tc, ntimes, J, E, c->err, s));
+  }
+  if (g_kernel.load() == BF_KERNEL_AUTO) {
+    std::lock_guard<std::mutex> lk(c->mu);
+    bool ran = false;
+    const int ps = run_padded(*c, d, J, E, nullptr, nullptr, &w->tc, s, kALinear, kJLinear, nullptr, nullptr, &ran);
+    if (ran || ps != BF_OK) return ps;
   }
   t_last_kernel = simt_name();
   return to_status(launch_simt(d, J, E, w->A, w->G, s));

@@ -79,11 +79,12 @@ cudaError_t launch_simt(const bf_dims &d, uint8_t *J, const uint8_t *E, const ui
 constexpr int kDigitRow = 32;  // bytes per digit row
 struct TcWeights {
   int64_t F = 0, B = 0, D = 0;
+  int64_t Dk = 0;    // dishes in a W row: D rounded up to 8 (TMA row strides), zero past D
   int nb_pass = 0;   // beams per tensor-core pass (multiple of 8, <= 128)
   int npass = 0;     // passes over the beams
   int nw = 0;        // W rows per frequency holding data: 2 * roundup(B, 8)
   int nw_pad = 0;    // digit rows per frequency: npass * 2 * nb_pass
-  uint8_t *W = nullptr;      // [F][nw][2D]
+  uint8_t *W = nullptr;      // [F][nw][2 Dk]
   uint8_t *dig = nullptr;    // [F][nw_pad][kDigitRow]
   float *gs = nullptr;       // [F][nw_pad / 2]: 2^18 G, zero past B (the epilogue's gains)
   int *gwide = nullptr;      // [F]: nonzero when a gain of the frequency can take |G * raw| to 2^31
@@ -102,8 +103,23 @@ inline void tc_set_extra(TcWeights &w, uint8_t *p) {
   w.gwide = reinterpret_cast<int *>(w.gs + static_cast<size_t>(w.F) * w.nw_pad / 2);
 }
 
-// True when the tensor-core kernel handles this shape.
+// True when the tensor-core kernel handles this shape in place.
 bool tc_supported(const bf_dims &d);
+
+// The tensor-core kernel on shapes it does not take in place (tc_supported):
+// any times, up to 2048 dishes, one or two polarizations, any alignment of E and
+// J.  E goes through a padded copy where its rows do not suit TMA, in chunks of
+// times.  With one polarization the copy makes times 2 t and 2 t + 1 the two
+// polarizations of time t, and J2's rows of them are J's rows.
+struct TcPadded {
+  bool ok = false;     // this route takes the shape, and faster than the dp4a kernel
+  bool copy = false;   // E needs the copy
+  int64_t times = 0;   // times per chunk
+  size_t bytes = 0;    // of the copy of one chunk
+};
+TcPadded tc_padded(const bf_dims &d, const uint8_t *E);
+// The padded copy of `times` times of E (`avail` bytes from E to the end of the array).
+cudaError_t launch_pad_e(const bf_dims &d, const uint8_t *E, size_t avail, int64_t times, uint8_t *out, cudaStream_t s);
 
 // Beams per pass and number of passes for B beams.  Passes of a multiple of 16
 // beams fill the GEMM N of a pair launch (a multiple of 32) exactly: 512 beams
@@ -121,9 +137,14 @@ cudaError_t launch_prep_weights(const TcWeights &w, const uint8_t *A, cudaStream
 // adler32 sums adler[0] += d_i, adler[1] += i * d_i (i = byte position from
 // jbase, taken mod 65521); the caller zeroes them first and finishes the
 // checksum with adler_finish().
+// `rows` (J2 only) gives the rows of J in bytes where they are not 2 * jpitch and
+// 2 * T (an odd number of times as pairs).
+struct TcRows {
+  int64_t pitch, len;
+};
 cudaError_t launch_tc(const TcWeights &w, int64_t T, uint8_t *J, const uint8_t *E, int *err, cudaStream_t s,
                       int64_t jpitch = 0, int j_layout = kJLinear, unsigned long long *adler = nullptr,
-                      const uint8_t *jbase = nullptr);
+                      const uint8_t *jbase = nullptr, const TcRows *rows = nullptr);
 constexpr uint32_t kAdlerMod = 65521;
 // adler32 of n bytes from S1 = sum d_i and S2 = sum i d_i (i from 0, both taken
 // mod 65521 or not): a = 1 + S1, b = n + n S1 - S2 (adler32.c:7-20 unrolled).
@@ -146,7 +167,9 @@ struct TcProblem {  // 128-byte aligned through its tensor maps
   unsigned long long *adler;   // null, or the fused adler32 sums {sum d_i, sum i * d_i} (device)
   const float *gs;   // scaled gains [F][npass * nb_pass]
   const int *gwide;  // [F]: the frequency needs the narrowing requantisation (huge or non-finite gains)
-  int64_t jpitch;    // bytes between consecutive (b, f, p) rows of J (J2: (b, f) rows are 2 * jpitch apart)
+  int64_t rpitch;    // bytes between consecutive rows of J: (b, f, p), or (b, f) for J2
+  int64_t rlen;      // bytes of such a row that belong to this problem
+  int bytes;         // nonzero: rows without 4-byte alignment, stored byte by byte
   int jlayout;       // JLayout
   int T, F, B;
   int nb_pass;       // beams per pass

@@ -83,6 +83,7 @@ extern "C" int bf_form_beams_noalloc(const bf_dims *dims, uint8_t *J, const uint
   w.F = d.nfrequencies;
   w.B = d.nbeams;
   w.D = d.ndishes;
+  w.Dk = d.ndishes;  // a multiple of 8 (tc_supported)
   tc_plan_beams(d.nbeams, &w.nb_pass, &w.npass, 8);  // the documented size limit counts passes of 8
   w.nw = static_cast<int>((d.nbeams + 7) / 8 * 8 * 2);
   w.nw_pad = w.npass * 2 * w.nb_pass;

@@ -192,7 +192,7 @@ namespace {
 TcWeights channel_view(const TcWeights &w, int c0, int n) {
   TcWeights v = w;
   v.F = n;
-  v.W = w.W + static_cast<int64_t>(c0) * w.nw * 2 * w.D;
+  v.W = w.W + static_cast<int64_t>(c0) * w.nw * 2 * w.Dk;
   v.dig = w.dig + static_cast<int64_t>(c0) * w.nw_pad * kDigitRow;
   v.gs = w.gs + static_cast<int64_t>(c0) * (w.nw_pad / 2);
   v.gwide = w.gwide + c0;

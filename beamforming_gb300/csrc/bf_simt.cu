@@ -1,8 +1,9 @@
 // bf_simt.cu -- exact integer beamformer on the CUDA cores (dp4a).
 //
 // Handles every shape (any ntimes, ndishes, nbeams; 1 or 2 polarizations).
-// It is the fallback for shapes the tensor-core kernel does not take and an
-// independent second GPU implementation for the parity tests.  Same
+// It takes what the tensor-core kernel does not, in place or through a padded
+// copy (TcPadded, bf_tc.cu: small problems mostly), and is an independent second
+// GPU implementation for the parity tests.  Same
 // arithmetic as cpu.cxx:24-41: int32 sums of 4-bit products, then
 // clamp(lrint(G * float(raw)), -7, 7).
 //

@@ -58,6 +58,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <cudaTypedefs.h>
@@ -644,7 +645,7 @@ __global__ void __launch_bounds__(32 * kPrepRows) bf_prep_weights(const uint8_t 
                                                                    uint8_t *__restrict__ W,
                                                                    uint8_t *__restrict__ dig,
                                                                    const float *__restrict__ G, float *__restrict__ gs,
-                                                                   int *__restrict__ gwide, int B, int D, int nw,
+                                                                   int *__restrict__ gwide, int B, int D, int Dk, int nw,
                                                                    int nw_pad, int a_layout) {
   // the E4M3 code of v * 2^-9, |v| <= 15, is |v| with a sign bit
   const int rblocks = (nw_pad + kPrepRows - 1) / kPrepRows;  // blocks per frequency
@@ -671,16 +672,16 @@ __global__ void __launch_bounds__(32 * kPrepRows) bf_prep_weights(const uint8_t 
   if (n < nw) {
     const int b = n >> 1;
     const int cj = n & 1;
-    // rows of 2D bytes, D % 8 == 0: 4-byte aligned words
-    uint32_t *wrow = reinterpret_cast<uint32_t *>(W + (static_cast<int64_t>(f) * nw + n) * (2 * D));
-    for (int k4 = lane; k4 < D / 2; k4 += 32) {  // k = 4 k4 .. 4 k4 + 3: dishes d0 .. d0 + 3, input part c
+    // rows of 2 Dk bytes, Dk % 8 == 0: 4-byte aligned words
+    uint32_t *wrow = reinterpret_cast<uint32_t *>(W + (static_cast<int64_t>(f) * nw + n) * (2 * Dk));
+    for (int k4 = lane; k4 < Dk / 2; k4 += 32) {  // k = 4 k4 .. 4 k4 + 3: dishes d0 .. d0 + 3, input part c
       const int c = k4 & 1;
       const int d0 = 4 * (k4 >> 1);
       uint32_t word = 0;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         int v = 0;
-        if (b < B) {
+        if (b < B && d0 + j < D) {
           int ar, ai;
           load_a(A, a_layout, f, b, d0 + j, B, D, ar, ai);
           v = cj == 0 ? (c == 0 ? ar : -ai) : (c == 0 ? ai : ar);
@@ -787,19 +788,126 @@ bool tc_supported(const bf_dims &d) {
   return true;
 }
 
+// 16 bytes of E from byte `off`, `valid` of them (the rest 0).  Unaligned words
+// where all of them lie inside the array, else byte by byte.
+__device__ __forceinline__ uint4 load16_any(const uint8_t *__restrict__ E, int64_t off, int valid, int64_t avail) {
+  uint32_t w[4];
+  if (valid >= 16 && off >= 4 && off + 20 <= avail) {
+    const uintptr_t at = reinterpret_cast<uintptr_t>(E + off);
+    const uint32_t *p = reinterpret_cast<const uint32_t *>(at & ~uintptr_t(3));
+    const uint32_t sh = 8u * static_cast<uint32_t>(at & 3u);
+    uint32_t v[5];
+#pragma unroll
+    for (int i = 0; i < 5; ++i) v[i] = __ldg(p + i);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = __funnelshift_r(v[i], v[i + 1], sh);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      w[i] = 0;
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (4 * i + k < valid) w[i] |= static_cast<uint32_t>(__ldg(E + off + 4 * i + k)) << (8 * k);
+    }
+  }
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// The padded copy of E (TcPadded): rows [t][f] of Dk dishes x 2 bytes.  One
+// polarization: row [t'][f] interleaves the rows of times 2 t' and 2 t' + 1.
+// One warp per row, 16 bytes per lane and step: bound by the bytes it moves.
+__global__ void __launch_bounds__(256) bf_pad_e(const uint8_t *__restrict__ E, int64_t avail, uint8_t *__restrict__ out,
+                                                int64_t T, int64_t F, int64_t D, int64_t Dk, int P) {
+  const int64_t rows = (P == 2 ? T : (T + 1) / 2) * F;
+  const int lane = threadIdx.x & 31;
+  for (int64_t row = blockIdx.x * 8ll + (threadIdx.x >> 5); row < rows; row += gridDim.x * 8ll) {
+    uint4 *dst = reinterpret_cast<uint4 *>(out + row * 2 * Dk);
+    if (P == 2) {
+      for (int64_t c = lane; c < Dk / 8; c += 32) {
+        const int64_t left = 2 * D - 16 * c;
+        dst[c] = load16_any(E, row * 2 * D + 16 * c, static_cast<int>(left < 16 ? (left < 0 ? 0 : left) : 16), avail);
+      }
+    } else {
+      const int64_t t = row / F, f = row - t * F;
+      for (int64_t c = lane; c < Dk / 8; c += 32) {  // dishes 8 c .. 8 c + 7 of both times
+        const int64_t left = D - 8 * c;
+        const int valid = static_cast<int>(left < 8 ? (left < 0 ? 0 : left) : 8);
+        uint32_t w[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          if (2 * t + q >= T) continue;
+          const int64_t off = ((2 * t + q) * F + f) * D + 8 * c;
+#pragma unroll
+          for (int k = 0; k < 8; ++k)
+            if (k < valid) w[k >> 1] |= static_cast<uint32_t>(__ldg(E + off + k)) << (16 * (k & 1) + 8 * q);
+        }
+        dst[c] = make_uint4(w[0], w[1], w[2], w[3]);
+      }
+    }
+  }
+}
+
+TcPadded tc_padded(const bf_dims &d, const uint8_t *E) {
+  TcPadded r;
+  if (d.npolarizations < 1 || d.npolarizations > 2 || d.ndishes <= 0 || d.ndishes > 2048) return r;
+  if (d.ntimes <= 0 || d.nbeams <= 0 || d.nfrequencies <= 0) return r;
+  if (d.ntimes > (1ll << 31) || d.nfrequencies > (1 << 20) || d.nbeams > (1 << 16)) return r;
+  const int64_t Dk = (d.ndishes + 7) / 8 * 8;
+  // This route costs three launches and an event, ~22 us, before it computes.
+  // The dp4a kernel takes about 6 + 7.5 us per 128 dishes for a wave of three
+  // blocks of 64 rows x 32 beams per SM, fitted to 60 shapes measured with both:
+  // e.g. t=1001 f=1 d=250 b=45 21 against 22 us, f=9 46 against 25; d=510 b=96
+  // 36 against 25, f=9 122 against 30; t=8001 f=16 1520 against 116; d=31 b=7 f=9
+  // 16 against 21.  Below 256 times (two tile pairs) the pairs of SMs stay empty.
+  if (d.ntimes < 256) return r;
+  const int64_t rows = 64 / d.npolarizations;
+  const double blocks = static_cast<double>((d.ntimes + rows - 1) / rows) * d.nfrequencies * ((d.nbeams + 31) / 32);
+  const double waves = std::ceil(blocks / (3.0 * num_sms()));
+  if (waves * (6.0 + 7.5 * static_cast<double>((d.ndishes + 127) / 128)) < 26.0) return r;
+  // the operand and one chunk of the copy stay below 1 GiB
+  if (static_cast<double>(d.nfrequencies) * (d.nbeams + 7) * 4.0 * Dk > 1073741824.0) return r;
+  r.copy = d.npolarizations == 1 || Dk != d.ndishes || (reinterpret_cast<uintptr_t>(E) & 15u) != 0;
+  r.times = d.ntimes;
+  if (r.copy) {
+    const int64_t per_t = d.nfrequencies * Dk * d.npolarizations;  // bytes of the copy per time
+    r.times = std::max<int64_t>(128, (int64_t(256) << 20) / per_t / 128 * 128);
+    r.times = std::min(r.times, d.ntimes);
+    r.bytes = static_cast<size_t>((r.times + 1) / 2 * 2 * per_t);
+    if (r.bytes > (size_t(1) << 30)) return r;
+  }
+  r.ok = true;
+  return r;
+}
+
+cudaError_t launch_pad_e(const bf_dims &d, const uint8_t *E, size_t avail, int64_t times, uint8_t *out,
+                         cudaStream_t s) {
+  const int64_t Dk = (d.ndishes + 7) / 8 * 8;
+  const int64_t rows = (d.npolarizations == 2 ? times : (times + 1) / 2) * d.nfrequencies;
+  const int64_t blocks = std::min<int64_t>((rows + 7) / 8, 16ll * num_sms());
+  bf_pad_e<<<static_cast<unsigned>(blocks), 256, 0, s>>>(E, static_cast<int64_t>(avail), out, times, d.nfrequencies,
+                                                         d.ndishes, Dk, static_cast<int>(d.npolarizations));
+  return cudaGetLastError();
+}
+
 cudaError_t launch_prep_weights(const TcWeights &w, const uint8_t *A, cudaStream_t s, int a_layout) {
   const int64_t blocks = static_cast<int64_t>((w.nw_pad + kPrepRows - 1) / kPrepRows) * w.F;
   if (blocks > 0x7FFFFFFF) return cudaErrorInvalidValue;
   bf_prep_weights<<<static_cast<unsigned>(blocks), 32 * kPrepRows, 0, s>>>(
-      A, w.W, w.dig, w.G, w.gs, w.gwide, static_cast<int>(w.B), static_cast<int>(w.D), w.nw, w.nw_pad, a_layout);
+      A, w.W, w.dig, w.G, w.gs, w.gwide, static_cast<int>(w.B), static_cast<int>(w.D), static_cast<int>(w.Dk),
+      w.nw, w.nw_pad, a_layout);
   return cudaGetLastError();
+}
+
+// Rows that start or end between words are stored byte by byte.
+static void set_row_stores(TcProblem &P) {
+  P.bytes = ((reinterpret_cast<uintptr_t>(P.J) | static_cast<uintptr_t>(P.rpitch) | static_cast<uintptr_t>(P.rlen)) & 3u) ? 1 : 0;
 }
 
 // Fills a problem record: shape, pointers and the two tensor maps.
 static cudaError_t make_problem(TcProblem &P, const TcWeights &w, int64_t T, uint8_t *J, const uint8_t *E,
                                 int64_t jpitch, int j_layout, bool pair) {
-  const int64_t F = w.F, D = w.D;
-  if ((reinterpret_cast<uintptr_t>(E) & 15u) || (reinterpret_cast<uintptr_t>(J) & 15u)) return cudaErrorMisalignedAddress;
+  const int64_t F = w.F, D = w.Dk;  // E rows hold Dk dishes too: they are D, or E is a padded copy
+  if (reinterpret_cast<uintptr_t>(E) & 15u) return cudaErrorMisalignedAddress;
   std::memset(&P, 0, sizeof(P));
   P.T = static_cast<int>(T);
   P.F = static_cast<int>(F);
@@ -807,10 +915,13 @@ static cudaError_t make_problem(TcProblem &P, const TcWeights &w, int64_t T, uin
   P.J = J;
   P.jbase = J;
   P.adler = nullptr;
-  P.jpitch = jpitch > 0 ? jpitch : T;
-  if (P.jpitch < T || (P.jpitch & 3)) return cudaErrorInvalidValue;
+  if (jpitch <= 0) jpitch = T;
+  if (jpitch < T) return cudaErrorInvalidValue;
   if (j_layout != kJLinear && j_layout != kJ2) return cudaErrorInvalidValue;
   P.jlayout = j_layout;
+  P.rpitch = j_layout == kJ2 ? 2 * jpitch : jpitch;
+  P.rlen = j_layout == kJ2 ? 2 * T : T;
+  set_row_stores(P);
   P.nb_pass = w.nb_pass;
   P.npass = w.npass;
   P.ntt = static_cast<int>((T + kTT - 1) / kTT);
@@ -1025,7 +1136,8 @@ cudaError_t launch_tc_grouped(const TcProblem *table, int nprob, int ntiles, int
 }
 
 cudaError_t launch_tc(const TcWeights &w, int64_t T, uint8_t *J, const uint8_t *E, int *err, cudaStream_t s,
-                      int64_t jpitch, int j_layout, unsigned long long *adler, const uint8_t *jbase) {
+                      int64_t jpitch, int j_layout, unsigned long long *adler, const uint8_t *jbase,
+                      const TcRows *rows) {
   TcParams p{};
   const bool pair = tc_pair_launch(w.nb_pass);
   cudaError_t e = make_problem(p.one, w, T, J, E, jpitch, j_layout, pair);
@@ -1033,12 +1145,17 @@ cudaError_t launch_tc(const TcWeights &w, int64_t T, uint8_t *J, const uint8_t *
   p.one.adler = adler;
   if (jbase) p.one.jbase = jbase;
   if (adler && (p.one.jbase > J)) return cudaErrorInvalidValue;
-  if (pair) return launch_pair(p.one, w.D, g_test_stall, err, s);
+  if (rows) {
+    p.one.rpitch = rows->pitch;
+    p.one.rlen = rows->len;
+    set_row_stores(p.one);
+  }
+  if (pair) return launch_pair(p.one, w.Dk, g_test_stall, err, s);
   const int64_t ntiles = static_cast<int64_t>(p.one.ntt) * w.F * w.npass;
   if (ntiles > 0x7FFFFFFF) return cudaErrorInvalidValue;
   p.ntiles = static_cast<int>(ntiles);
   p.nprob = 1;
-  p.nk = tc_stages_per_tile(w.D);
+  p.nk = tc_stages_per_tile(w.Dk);
   p.err = err;
   int smem_bytes = 0;
   e = plan_launch(p, w.nb_pass, TcRingPlan{}, &smem_bytes);

@@ -124,8 +124,9 @@ struct EpilogueTile {
   uint8_t *jrow;  // the thread's bytes for beam b0 + cb
   int64_t bstride;
   int blim;
+  int nbytes;     // of the thread's 4 bytes, those inside the row
   uint32_t osel;  // the rows' bytes into J's order
-  bool wide, t_ok;
+  bool wide, bytes;
 
   __device__ __forceinline__ EpilogueTile(const TcProblem &P, int f, int pass, int tt, int q, int lane) {
     const uint32_t g = static_cast<uint32_t>(lane) >> 2, cb = static_cast<uint32_t>(lane) & 3u;
@@ -139,16 +140,18 @@ struct EpilogueTile {
     // narrowing of cpu.cxx:38 (tile-uniform branch, normally not taken)
     wide = __ldg(P.gwide + f) != 0;
     const int64_t bj = static_cast<int64_t>(b0 + static_cast<int>(cb)) * P.F + f;  // beam row b0 + cb
-    int64_t t;  // first time of the thread's 4 bytes
+    int64_t at;  // the thread's 4 bytes in the J row
     if constexpr (!kJ2) {
-      t = static_cast<int64_t>(tt) * kTT + RowMap<kJ2>::time(q, 8 * RowMap<kJ2>::swap(g) + g);
-      jrow = P.J + (bj * 2 + (q & 1)) * P.jpitch + t;
+      at = static_cast<int64_t>(tt) * kTT + RowMap<kJ2>::time(q, 8 * RowMap<kJ2>::swap(g) + g);
+      jrow = P.J + (bj * 2 + (q & 1)) * P.rpitch + at;
+      bstride = static_cast<int64_t>(P.F) * 2 * P.rpitch;
     } else {
-      t = static_cast<int64_t>(tt) * kTT + 16 * q + 2 * static_cast<int>(g);
-      jrow = P.J + bj * 2 * P.jpitch + 2 * t;
+      at = 2 * (static_cast<int64_t>(tt) * kTT + 16 * q + 2 * static_cast<int>(g));
+      jrow = P.J + bj * P.rpitch + at;
+      bstride = static_cast<int64_t>(P.F) * P.rpitch;
     }
-    t_ok = t < P.T;
-    bstride = static_cast<int64_t>(P.F) * 2 * P.jpitch;  // bytes between beams, both layouts
+    nbytes = static_cast<int>(max(int64_t(0), min(int64_t(4), P.rlen - at)));
+    bytes = P.bytes != 0;
     blim = P.B - b0 - static_cast<int>(cb);              // beam offsets below this exist
   }
 
@@ -214,13 +217,20 @@ struct EpilogueTile {
     if constexpr (kFull) {
       __stcs(reinterpret_cast<uint32_t *>(dst), w[0]);
       __stcs(reinterpret_cast<uint32_t *>(dst + 4 * bstride), w[1]);
-    } else if (t_ok) {
-      if (8 * c < blim) __stcs(reinterpret_cast<uint32_t *>(dst), w[0]);
-      if (8 * c + 4 < blim) __stcs(reinterpret_cast<uint32_t *>(dst + 4 * bstride), w[1]);
+    } else if (!bytes) {  // rows are multiples of 4 bytes
+      if (nbytes > 0 && 8 * c < blim) __stcs(reinterpret_cast<uint32_t *>(dst), w[0]);
+      if (nbytes > 0 && 8 * c + 4 < blim) __stcs(reinterpret_cast<uint32_t *>(dst + 4 * bstride), w[1]);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (i < nbytes && 8 * c + 4 * k < blim) dst[4 * k * bstride + i] = static_cast<uint8_t>(w[k] >> (8 * i));
     }
     if constexpr (kAdler) {  // only the bytes stored count
-      const uint32_t w0 = kFull || (t_ok && 8 * c < blim) ? w[0] : 0u;
-      const uint32_t w1 = kFull || (t_ok && 8 * c + 4 < blim) ? w[1] : 0u;
+      const uint32_t in = kFull || nbytes == 4 ? 0xFFFFFFFFu : (1u << (8 * nbytes)) - 1u;
+      const uint32_t w0 = kFull || 8 * c < blim ? w[0] & in : 0u;
+      const uint32_t w1 = kFull || 8 * c + 4 < blim ? w[1] & in : 0u;
       const uint32_t s1 = __dp4a(w1, 0x01010101u, 0u);
       const uint32_t s01 = __dp4a(w0, 0x01010101u, s1);
       a.a0 += s01;
@@ -256,7 +266,7 @@ struct EpilogueTile {
     Sums a;
     bool ok;
     if (!wide) {
-      ok = __all_sync(0xffffffffu, t_ok && 8 * c_end - 4 < blim)
+      ok = __all_sync(0xffffffffu, !bytes && nbytes == 4 && 8 * c_end - 4 < blim)
                ? chunks<kC, true>(acc_addr, c_begin, c_end, a, wait, release)
                : chunks<kC, false>(acc_addr, c_begin, c_end, a, wait, release);
     } else {
