@@ -636,87 +636,123 @@ __global__ void __launch_bounds__(Roles<kEpiW, kGroups>::kThreads, kHalf ? 2 : 1
 }
 
 // Builds the E4M3 operand W[f][n][k] and the digit rows of the row sums
-// sum_k W[f][n][k] from A[f][b][d]; one warp per row n, four k per lane-step.
+// sum_k W[f][n][k] from A[f][b][d].
 //   n = 2*b + cj                   (cj: 0 = real output, 1 = imaginary output)
 //   k = 8*(d/4)  + 4*c  + d%4      (c:  0 = real input,  1 = imaginary input)
 // W = Ar, -Ai for the real output and Ai, Ar for the imaginary output.
-constexpr int kPrepRows = 8;  // rows per 256-thread block
-__global__ void __launch_bounds__(32 * kPrepRows) bf_prep_weights(const uint8_t *__restrict__ A,
-                                                                   uint8_t *__restrict__ W,
-                                                                   uint8_t *__restrict__ dig,
-                                                                   const float *__restrict__ G, float *__restrict__ gs,
-                                                                   int *__restrict__ gwide, int B, int D, int Dk, int nw,
-                                                                   int nw_pad, int a_layout) {
-  // the E4M3 code of v * 2^-9, |v| <= 15, is |v| with a sign bit
-  const int rblocks = (nw_pad + kPrepRows - 1) / kPrepRows;  // blocks per frequency
-  const int f = static_cast<int>(blockIdx.x) / rblocks;
-  const int n = (static_cast<int>(blockIdx.x) % rblocks) * kPrepRows + static_cast<int>(threadIdx.x >> 5);
+//
+// One warp per beam: both of its rows hold the same numbers, so a lane turns 16
+// dishes into the codes of Ar, Ai and -Ai four bytes at a time and stores 32
+// bytes of each row.  Bound by the bytes of W (f=16 b=512 d=1024: 33.5 MB and
+// 8.4 MB of A); a warp per row and a byte per load took 42 us there, this 14.4
+// (f=16 b=96 d=512: 9.1 and 4.5 us, launch included).
+constexpr int kPrepBeams = 8;  // beams per 256-thread block
+
+// The E4M3 codes of v * 2^-9 (a sign bit and |v|) of four stored nibbles u = v + 8.
+__device__ __forceinline__ uint32_t w_codes(uint32_t u) {
+  const uint32_t x = u ^ 0x08080808u;                // two's complement nibbles
+  const uint32_t n = (x >> 3) & 0x01010101u;         // 1 where negative
+  return ((x ^ (n * 15u)) + n) | (n << 7);           // 15 - x + 1 there
+}
+__device__ __forceinline__ uint32_t w_negate(uint32_t codes) {  // zero stays zero
+  return codes ^ (((codes & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) & 0x80808080u);
+}
+
+__global__ void __launch_bounds__(32 * kPrepBeams) bf_prep_weights(const uint8_t *__restrict__ A,
+                                                                    uint8_t *__restrict__ W,
+                                                                    uint8_t *__restrict__ dig,
+                                                                    const float *__restrict__ G, float *__restrict__ gs,
+                                                                    int *__restrict__ gwide, int B, int D, int Dk,
+                                                                    int nw, int nw_pad, int a_layout) {
+  const int beams = nw_pad / 2;
+  const int fblocks = (beams + kPrepBeams - 1) / kPrepBeams;  // blocks per frequency
+  const int f = static_cast<int>(blockIdx.x) / fblocks;
+  const int b = (static_cast<int>(blockIdx.x) % fblocks) * kPrepBeams + static_cast<int>(threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  if (static_cast<int>(blockIdx.x) % rblocks == 0) {  // the frequency's scaled gains: 2^18 G, zero past B
-    const int ng = nw_pad / 2;
+  if (static_cast<int>(blockIdx.x) % fblocks == 0) {  // the frequency's scaled gains: 2^18 G, zero past B
     // |raw| <= 128 D, so with |G| * 128 D < 2^30 every product G * raw stays
     // below 2^31 and the plain requantisation is exact; otherwise (or for a
     // non-finite gain) the frequency takes the narrowing one of cpu.cxx:38
     const float wide_at = 1073741824.0f / (128.0f * static_cast<float>(D));
     int wide = 0;
-    for (int i = threadIdx.x; i < ng; i += blockDim.x) {
+    for (int i = threadIdx.x; i < beams; i += blockDim.x) {
       const float g = i < B ? G[static_cast<int64_t>(f) * B + i] : 0.0f;
-      gs[static_cast<int64_t>(f) * ng + i] = 262144.0f * g;
+      gs[static_cast<int64_t>(f) * beams + i] = 262144.0f * g;
       wide |= !(fabsf(g) < wide_at);
     }
     wide = __syncthreads_or(wide);
     if (threadIdx.x == 0) gwide[f] = wide;
   }
-  if (n >= nw_pad) return;  // the whole warp
-  int sum = 0;
-  if (n < nw) {
-    const int b = n >> 1;
-    const int cj = n & 1;
-    // rows of 2 Dk bytes, Dk % 8 == 0: 4-byte aligned words
-    uint32_t *wrow = reinterpret_cast<uint32_t *>(W + (static_cast<int64_t>(f) * nw + n) * (2 * Dk));
-    for (int k4 = lane; k4 < Dk / 2; k4 += 32) {  // k = 4 k4 .. 4 k4 + 3: dishes d0 .. d0 + 3, input part c
-      const int c = k4 & 1;
-      const int d0 = 4 * (k4 >> 1);
-      uint32_t word = 0;
+  if (b >= beams) return;  // the whole warp
+  int s_re = 0, s_im = 0;  // sums of Ar and Ai
+  if (b < nw / 2) {
+    const uint8_t *row = A + (static_cast<int64_t>(f) * B + b) * D;  // linear layout
+    const bool vec = a_layout == kALinear && b < B && D % 16 == 0 && (reinterpret_cast<uintptr_t>(A) & 15u) == 0;
+    // rows 2 b and 2 b + 1 of 2 Dk bytes, Dk a multiple of 8: 16-byte aligned
+    uint4 *w0 = reinterpret_cast<uint4 *>(W + (static_cast<int64_t>(f) * nw + 2 * b) * (2 * Dk));
+    uint4 *w1 = w0 + Dk / 8;
+    for (int i = lane; i < (Dk + 15) / 16; i += 32) {  // dishes 16 i .. 16 i + 15
+      uint32_t w[4];
+      if (vec) {
+        const uint4 q = __ldg(reinterpret_cast<const uint4 *>(row) + i);
+        w[0] = q.x, w[1] = q.y, w[2] = q.z, w[3] = q.w;
+      } else {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        int v = 0;
-        if (b < B && d0 + j < D) {
-          int ar, ai;
-          load_a(A, a_layout, f, b, d0 + j, B, D, ar, ai);
-          v = cj == 0 ? (c == 0 ? ar : -ai) : (c == 0 ? ai : ar);
+        for (int j = 0; j < 4; ++j) {
+          w[j] = 0;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const int d = 16 * i + 4 * j + k;
+            int re = 0, im = 0;
+            if (b < B && d < D) load_a(A, a_layout, f, b, d, B, D, re, im);
+            w[j] |= static_cast<uint32_t>(((re + 8) << 4) | (im + 8)) << (8 * k);
+          }
         }
-        const int av = v < 0 ? -v : v;
-        word |= static_cast<uint32_t>(av | (v < 0 ? 0x80 : 0x00)) << (8 * j);
-        sum += v;
       }
-      wrow[k4] = word;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {  // 8 dishes: 16 bytes of each row
+        if (16 * i + 8 * h >= Dk) break;
+        uint32_t re[2], im[2], ni[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const uint32_t ur = (w[2 * h + j] >> 4) & 0x0F0F0F0Fu, ui = w[2 * h + j] & 0x0F0F0F0Fu;
+          s_re += static_cast<int>(__dp4a(ur, 0x01010101u, 0u)) - 32;
+          s_im += static_cast<int>(__dp4a(ui, 0x01010101u, 0u)) - 32;
+          re[j] = w_codes(ur);
+          im[j] = w_codes(ui);
+          ni[j] = w_negate(im[j]);
+        }
+        w0[2 * i + h] = make_uint4(re[0], ni[0], re[1], ni[1]);
+        w1[2 * i + h] = make_uint4(im[0], re[0], im[1], re[1]);
+      }
     }
   }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-  if (lane == 0) {
+  for (int o = 16; o > 0; o >>= 1) {
+    s_re += __shfl_xor_sync(0xffffffffu, s_re, o);
+    s_im += __shfl_xor_sync(0xffffffffu, s_im, o);
+  }
+  if (lane < 2) {  // row 2 b + lane
     // s = sum_k W[n][k], |s| <= 16 D <= 2^15, in balanced base-16 digits
     // d0..d3 in [-8, 7] and d4 in {-1, 0, 1}; the digit row holds the E4M3
     // codes of d0, d1, d2, d3, 4 d4 (see kDigitScaleLo)
-    uint32_t w0 = 0, w1 = 0;
-    int rest = sum;
+    uint32_t d03 = 0;
+    int rest = lane == 0 ? s_re - s_im : s_im + s_re;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int r = rest & 15;
       const int dj = r >= 8 ? r - 16 : r;
       rest = (rest - dj) >> 4;
       const int av = dj < 0 ? -dj : dj;
-      w0 |= static_cast<uint32_t>(av | (dj < 0 ? 0x80 : 0x00)) << (8 * j);
+      d03 |= static_cast<uint32_t>(av | (dj < 0 ? 0x80 : 0x00)) << (8 * j);
     }
-    w1 = rest == 0 ? 0u : (rest > 0 ? 0x04u : 0x84u);  // 4 * d4: +-4 or 0
-    uint32_t *row = reinterpret_cast<uint32_t *>(dig + (static_cast<int64_t>(f) * nw_pad + n) * kDigitRow);
-    row[0] = w0;
-    row[1] = w1;
-#pragma unroll
-    for (int j = 2; j < kDigitRow / 4; ++j) row[j] = 0u;
+    const uint32_t d4 = rest == 0 ? 0u : (rest > 0 ? 0x04u : 0x84u);  // 4 * d4: +-4 or 0
+    uint4 *row = reinterpret_cast<uint4 *>(dig + (static_cast<int64_t>(f) * nw_pad + 2 * b + lane) * kDigitRow);
+    row[0] = make_uint4(d03, d4, 0u, 0u);
+    row[1] = make_uint4(0u, 0u, 0u, 0u);
   }
 }
+static_assert(kDigitRow == 32, "two 16-byte stores per digit row");
 
 PFN_cuTensorMapEncodeTiled_v12000 get_encode_fn() {
   // initialised once, thread-safely (the server thread encodes maps too)
@@ -890,9 +926,9 @@ cudaError_t launch_pad_e(const bf_dims &d, const uint8_t *E, size_t avail, int64
 }
 
 cudaError_t launch_prep_weights(const TcWeights &w, const uint8_t *A, cudaStream_t s, int a_layout) {
-  const int64_t blocks = static_cast<int64_t>((w.nw_pad + kPrepRows - 1) / kPrepRows) * w.F;
+  const int64_t blocks = static_cast<int64_t>((w.nw_pad / 2 + kPrepBeams - 1) / kPrepBeams) * w.F;
   if (blocks > 0x7FFFFFFF) return cudaErrorInvalidValue;
-  bf_prep_weights<<<static_cast<unsigned>(blocks), 32 * kPrepRows, 0, s>>>(
+  bf_prep_weights<<<static_cast<unsigned>(blocks), 32 * kPrepBeams, 0, s>>>(
       A, w.W, w.dig, w.G, w.gs, w.gwide, static_cast<int>(w.B), static_cast<int>(w.D), static_cast<int>(w.Dk),
       w.nw, w.nw_pad, a_layout);
   return cudaGetLastError();
