@@ -71,6 +71,27 @@ bool simt_four_multiply();
 cudaError_t launch_simt(const bf_dims &d, uint8_t *J, const uint8_t *E, const uint8_t *A, const float *G,
                         cudaStream_t s, int64_t jpitch = 0, int a_layout = kALinear, int j_layout = kJLinear);
 
+#ifdef __CUDACC__
+// Launches a kernel that calls grid_wait() before it touches memory: its launch
+// and set-up (barriers, tensor memory; 2 us of 10 on one channel's chunk) overlap
+// the end of the kernel before it on the stream.
+template <class... Params, class... Args>
+cudaError_t launch_overlapped(void (*kern)(Params...), unsigned grid, unsigned block, size_t smem, cudaStream_t s,
+                              Args &&...args) {
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<Params>(args)...);
+}
+#endif
+
 // Tensor-core path ------------------------------------------------------------
 
 // Layout of the resident operand built from A: for each frequency, nw rows of

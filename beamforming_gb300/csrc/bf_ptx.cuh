@@ -170,11 +170,23 @@ __device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t mapped) {
 __device__ __forceinline__ void st_cluster_u32(uint32_t mapped, uint32_t v) {
   asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(mapped), "r"(v) : "memory");
 }
-// Every thread of both CTAs arrives and waits.
-__device__ __forceinline__ void cluster_sync() {
+// Every thread of both CTAs arrives and, sooner or later, waits.
+__device__ __forceinline__ void cluster_arrive() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_sync() {
+  cluster_arrive();
+  cluster_wait();
+}
+
+// ---------------------------------------------------------------- launches
+// A launch with programmatic serialization (launch_overlapped) starts while the
+// kernel before it on the stream ends: it sets itself up, then waits here until
+// that kernel and its memory are complete.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Lets the next such launch start once every CTA of this grid has come here.
+__device__ __forceinline__ void grid_launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---------------------------------------------------------------- proxies
 __device__ __forceinline__ void fence_proxy_async_smem() {

@@ -664,6 +664,8 @@ __global__ void __launch_bounds__(32 * kPrepBeams) bf_prep_weights(const uint8_t
                                                                     const float *__restrict__ G, float *__restrict__ gs,
                                                                     int *__restrict__ gwide, int B, int D, int Dk,
                                                                     int nw, int nw_pad, int a_layout) {
+  grid_launch_next();
+  grid_wait();
   const int beams = nw_pad / 2;
   const int fblocks = (beams + kPrepBeams - 1) / kPrepBeams;  // blocks per frequency
   const int f = static_cast<int>(blockIdx.x) / fblocks;
@@ -854,6 +856,8 @@ __device__ __forceinline__ uint4 load16_any(const uint8_t *__restrict__ E, int64
 // One warp per row, 16 bytes per lane and step: bound by the bytes it moves.
 __global__ void __launch_bounds__(256) bf_pad_e(const uint8_t *__restrict__ E, int64_t avail, uint8_t *__restrict__ out,
                                                 int64_t T, int64_t F, int64_t D, int64_t Dk, int P) {
+  grid_launch_next();
+  grid_wait();
   const int64_t rows = (P == 2 ? T : (T + 1) / 2) * F;
   const int lane = threadIdx.x & 31;
   for (int64_t row = blockIdx.x * 8ll + (threadIdx.x >> 5); row < rows; row += gridDim.x * 8ll) {
@@ -920,18 +924,16 @@ cudaError_t launch_pad_e(const bf_dims &d, const uint8_t *E, size_t avail, int64
   const int64_t Dk = (d.ndishes + 7) / 8 * 8;
   const int64_t rows = (d.npolarizations == 2 ? times : (times + 1) / 2) * d.nfrequencies;
   const int64_t blocks = std::min<int64_t>((rows + 7) / 8, 16ll * num_sms());
-  bf_pad_e<<<static_cast<unsigned>(blocks), 256, 0, s>>>(E, static_cast<int64_t>(avail), out, times, d.nfrequencies,
-                                                         d.ndishes, Dk, static_cast<int>(d.npolarizations));
-  return cudaGetLastError();
+  return launch_overlapped(bf_pad_e, static_cast<unsigned>(blocks), 256, 0, s, E, static_cast<int64_t>(avail), out, times,
+                           d.nfrequencies, d.ndishes, Dk, static_cast<int>(d.npolarizations));
 }
 
 cudaError_t launch_prep_weights(const TcWeights &w, const uint8_t *A, cudaStream_t s, int a_layout) {
   const int64_t blocks = static_cast<int64_t>((w.nw_pad / 2 + kPrepBeams - 1) / kPrepBeams) * w.F;
   if (blocks > 0x7FFFFFFF) return cudaErrorInvalidValue;
-  bf_prep_weights<<<static_cast<unsigned>(blocks), 32 * kPrepBeams, 0, s>>>(
-      A, w.W, w.dig, w.G, w.gs, w.gwide, static_cast<int>(w.B), static_cast<int>(w.D), static_cast<int>(w.Dk),
-      w.nw, w.nw_pad, a_layout);
-  return cudaGetLastError();
+  return launch_overlapped(bf_prep_weights, static_cast<unsigned>(blocks), 32 * kPrepBeams, 0, s, A, w.W, w.dig, w.G,
+                           w.gs, w.gwide, static_cast<int>(w.B), static_cast<int>(w.D), static_cast<int>(w.Dk), w.nw,
+                           w.nw_pad, a_layout);
 }
 
 // Rows that start or end between words are stored byte by byte.

@@ -169,29 +169,29 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
   const int ncols = p.ncols;
   const int per_half = (kPairAcc - ncols) / kStageCols;
 
-  if (threadIdx.x == 0) {
-    for (int r = 0; r < R; ++r) {
-      mbar_init(raw_full(r), 1);
-      mbar_init(raw_empty(r), kStageWarps);
+  // Each producer sets up its own barriers and starts its copies without waiting
+  // for the CTAs of the pair to meet (setup_sync, some 2700 cycles in).
+  if (warp == kEProdWarp) {
+    for (int i = lane; i < 2 * R; i += 32) mbar_init(raw_full(i), i < R ? 1 : kStageWarps);
+    if (!kGrouped && lane == 0) tma_prefetch_desc(&p.one.tm_e);
+  } else if (warp == kWProdWarp) {
+    for (int i = lane; i < 3 * SW; i += 32) mbar_init(w_full(i), 1);
+    if (lane < 3 * kDigSlots) mbar_init(d_full(0) + 8u * lane, 1);
+    if (!kGrouped && lane == 0) {
+      tma_prefetch_desc(&p.one.tm_w);
+      tma_prefetch_desc(&p.one.tm_d);
     }
-    for (int s = 0; s < SW; ++s) {
-      mbar_init(w_full(s), 1);
-      mbar_init(w_peer(s), 1);
-      mbar_init(w_empty(s), 1);
-    }
-    for (int s = 0; s < S; ++s) {
-      mbar_init(a_full(s), 2 * kStageWarps);  // the leader's: the unpack warps of a stage in both CTAs
-      mbar_init(empty(s), 1);
-    }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(accfull(i), 1);
-      mbar_init(accempty(i), 2 * kEpiW);  // the leader's: both CTAs' epilogue warps
-      mbar_init(d_full(i), 1);
-      mbar_init(d_peer(i), 1);
-      mbar_init(d_empty(i), 1);
-    }
-    for (int i = 0; i < 4; ++i) counts[i] = 0;
-    fence_barrier_init();
+  } else if (warp == 0) {
+    // a_full, accempty (the leader's): the unpack warps of a stage, the epilogue
+    // warps, in both CTAs
+    if (lane < 2 * S) mbar_init(a_full(lane), lane < S ? 2 * kStageWarps : 1);
+    if (lane < 4) mbar_init(accfull(lane), lane < 2 ? 1 : 2 * kEpiW);
+    if (lane < 4) counts[lane] = 0;
+  }
+  fence_barrier_init();
+  if (warp == kMmaWarp) {
+    tmem_alloc_pair(smem_u32(tmem_holder), 512);
+    tmem_relinquish_pair();
   }
   // constant A tile of the offset MMA: every row the same, so the 32-byte
   // swizzle leaves it unchanged
@@ -200,15 +200,26 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     reinterpret_cast<uint32_t *>(sA)[i] = (w == 0 || w == 4) ? kDigitScaleLo : (w == 1 || w == 5) ? kDigitScaleHi : 0u;
   }
   fence_proxy_async_smem();
-  if (warp == kMmaWarp) {
-    tmem_alloc_pair(smem_u32(tmem_holder), 512);
-    tmem_relinquish_pair();
-  }
-  tc_fence_before();
-  __syncthreads();
-  cluster_sync();
-  tc_fence_after();
-  const uint32_t tmem_base = *tmem_holder;
+  grid_launch_next();
+  grid_wait();
+  auto setup_sync = [&]() {
+    tc_fence_before();
+    cluster_sync();
+    tc_fence_after();
+  };
+  static_assert(2 * kPairMaxStages <= 32, "one lane per stage barrier");
+  // waits for the last phase committed on every barrier
+  auto drain_commits = [&](uint32_t nstage, uint32_t nw, uint32_t ndig, uint32_t nacc) {
+    const uint32_t uS = static_cast<uint32_t>(S), uW = static_cast<uint32_t>(SW), uD = static_cast<uint32_t>(kDigSlots);
+    for (uint32_t k = nstage > uS ? nstage - uS : 0; k < nstage; ++k)
+      mbar_wait_drain(empty(static_cast<int>(k % uS)), (k / uS) & 1u);
+    for (uint32_t k = nw > uW ? nw - uW : 0; k < nw; ++k)
+      mbar_wait_drain(w_empty(static_cast<int>(k % uW)), (k / uW) & 1u);
+    for (uint32_t k = ndig > uD ? ndig - uD : 0; k < ndig; ++k)
+      mbar_wait_drain(d_empty(static_cast<int>(k % uD)), (k / uD) & 1u);
+    for (uint32_t k = nacc > 2u ? nacc - 2u : 0u; k < nacc; ++k)
+      mbar_wait_drain(accfull(static_cast<int>(k & 1u)), (k >> 1) & 1u);
+  };
   int *err = p.err;
 
   const int64_t ncl = gridDim.x >> 1, cl = blockIdx.x >> 1;
@@ -217,84 +228,90 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 
   if (warp == kEProdWarp) {
     // ------------------------------------------------------------ E producer
-    if (lane == 0 && !p.test_stall) {
-      const uint64_t pol_e = policy_evict_first();
-      Ring rr(R);
-      uint32_t issued = 0;
-      bool ok = true;
-      const TcProblem *seen = nullptr;
-      PairCursor<kGrouped> cur(p, first);
-      for (int tile = first; ok && tile < end; ++tile, cur.next(p)) {
-        if (kGrouped && cur.P != seen) {  // a table entry the host rewrites between launches
-          tensormap_acquire(&cur.P->tm_e);
-          seen = cur.P;
-        }
-        for (int ks = 0; ks < nk; ++ks, rr.advance(), ++issued) {
-          const int r = static_cast<int>(rr.idx);
-          if (!mbar_wait(raw_empty(r), rr.phase ^ 1u, err, kDevTimeoutEmpty)) {
-            ok = false;
-            break;
-          }
+    const uint64_t pol_e = policy_evict_first();
+    Ring rr(R);
+    uint32_t issued = 0;
+    bool ok = !p.test_stall;
+    cluster_arrive();
+    const TcProblem *seen = nullptr;
+    PairCursor<kGrouped> cur(p, first);
+    for (int tile = first; ok && tile < end; ++tile, cur.next(p)) {
+      if (kGrouped && cur.P != seen) {  // a table entry the host rewrites between launches
+        tensormap_acquire(&cur.P->tm_e);
+        seen = cur.P;
+      }
+      for (int ks = 0; ks < nk; ++ks, rr.advance(), ++issued) {
+        const int r = static_cast<int>(rr.idx);
+        ok = __all_sync(0xffffffffu, mbar_wait(raw_empty(r), rr.phase ^ 1u, err, kDevTimeoutEmpty));
+        if (!ok) break;
+        if (lane == 0) {
           mbar_arrive_expect_tx(raw_full(r), kRawBytes);
 #pragma unroll
           for (int h = 0; h < kSub; ++h)
             tma_load_3d(smem_u32(sR + r * kRawBytes + h * kRawBox), &cur.P->tm_e, raw_full(r), (ks * kSub + h) * kKC,
                         cur.f, (2 * cur.tp + rank) * kTT, pol_e);
         }
+        __syncwarp();
       }
-      // let the copies already issued land before the CTA exits, on every exit
-      for (uint32_t k = (issued >= static_cast<uint32_t>(R) ? issued - R : 0); k < issued; ++k)
-        mbar_wait_drain(raw_full(static_cast<int>(k % R)), (k / R) & 1u);
     }
+    cluster_wait();
+    // let the copies already issued land before the CTA exits, on every exit
+    for (uint32_t k = (issued >= static_cast<uint32_t>(R) ? issued - R : 0); k < issued; ++k)
+      mbar_wait_drain(raw_full(static_cast<int>(k % R)), (k / R) & 1u);
   } else if (warp == kWProdWarp) {
     // ------------------------------------------------------------ W producer
-    if (lane == 0 && !p.test_stall) {
-      const uint64_t pol_w = policy_evict_last();
-      Ring wr(SW), dr(kDigSlots);
-      uint32_t it = 0, dit = 0;
-      bool ok = true, fresh = true;
-      const TcProblem *seen = nullptr;
-      PairCursor<kGrouped> cur(p, first);
-      for (int tile = first; ok && tile < end; ++tile) {
-        if (fresh || stream_w) {
-          if (kGrouped && cur.P != seen) {
-            tensormap_acquire(&cur.P->tm_w);
-            tensormap_acquire(&cur.P->tm_d);
-            seen = cur.P;
-          }
-          const int row0 = cur.pass * 2 * cur.P->nb_pass + rank * (cur.n() / 2);
-          const int wbox = cur.P->w_rows * kKC;
-          if (fresh) {  // the digit rows, for the offset MMA
-            const int ds = static_cast<int>(dr.idx);
-            if (!mbar_wait(d_empty(ds), dr.phase ^ 1u, err, kDevTimeoutEmpty)) break;
+    const uint64_t pol_w = policy_evict_last();
+    Ring wr(SW), dr(kDigSlots);
+    uint32_t it = 0, dit = 0;
+    bool ok = !p.test_stall, fresh = true;
+    cluster_arrive();
+    const TcProblem *seen = nullptr;
+    PairCursor<kGrouped> cur(p, first);
+    for (int tile = first; ok && tile < end; ++tile) {
+      if (fresh || stream_w) {
+        if (kGrouped && cur.P != seen) {
+          tensormap_acquire(&cur.P->tm_w);
+          tensormap_acquire(&cur.P->tm_d);
+          seen = cur.P;
+        }
+        const int row0 = cur.pass * 2 * cur.P->nb_pass + rank * (cur.n() / 2);
+        const int wbox = cur.P->w_rows * kKC;
+        if (fresh) {  // the digit rows, for the offset MMA
+          const int ds = static_cast<int>(dr.idx);
+          ok = __all_sync(0xffffffffu, mbar_wait(d_empty(ds), dr.phase ^ 1u, err, kDevTimeoutEmpty));
+          if (!ok) break;
+          if (lane == 0) {
             mbar_arrive_expect_tx(d_full(ds), cur.P->w_rows * kDigitRow);
             tma_load_3d(smem_u32(sD + ds * sp.dbytes), &cur.P->tm_d, d_full(ds), 0, row0, cur.f, pol_w);
-            dr.advance();
-            ++dit;
           }
-          for (int ks = 0; ks < nk; ++ks, ++it, wr.advance()) {
-            const int s = static_cast<int>(wr.idx);
-            if (!mbar_wait(w_empty(s), wr.phase ^ 1u, err, kDevTimeoutEmpty)) {
-              ok = false;
-              break;
-            }
+          dr.advance();
+          ++dit;
+        }
+        for (int ks = 0; ks < nk; ++ks, ++it, wr.advance()) {
+          const int s = static_cast<int>(wr.idx);
+          ok = __all_sync(0xffffffffu, mbar_wait(w_empty(s), wr.phase ^ 1u, err, kDevTimeoutEmpty));
+          if (!ok) break;
+          if (lane == 0) {
             mbar_arrive_expect_tx(w_full(s), kSub * wbox);
 #pragma unroll
             for (int h = 0; h < kSub; ++h)
               tma_load_3d(smem_u32(sW + s * sp.wbytes + h * wbox), &cur.P->tm_w, w_full(s), (ks * kSub + h) * kKC,
                           row0, cur.f, pol_w);
           }
+          __syncwarp();
         }
-        fresh = cur.last_of_w();
-        cur.next(p);
       }
-      for (uint32_t k = (it >= static_cast<uint32_t>(SW) ? it - SW : 0); k < it; ++k)
-        mbar_wait_drain(w_full(static_cast<int>(k % SW)), (k / SW) & 1u);
-      for (uint32_t k = (dit >= static_cast<uint32_t>(kDigSlots) ? dit - kDigSlots : 0); k < dit; ++k)
-        mbar_wait_drain(d_full(static_cast<int>(k % kDigSlots)), (k / kDigSlots) & 1u);
+      fresh = cur.last_of_w();
+      cur.next(p);
     }
+    cluster_wait();
+    for (uint32_t k = (it >= static_cast<uint32_t>(SW) ? it - SW : 0); k < it; ++k)
+      mbar_wait_drain(w_full(static_cast<int>(k % SW)), (k / SW) & 1u);
+    for (uint32_t k = (dit >= static_cast<uint32_t>(kDigSlots) ? dit - kDigSlots : 0); k < dit; ++k)
+      mbar_wait_drain(d_full(static_cast<int>(k % kDigSlots)), (k / kDigSlots) & 1u);
   } else if (warp == kMmaWarp && rank == 1) {
     // ------------------------------------- peer: this CTA's W and digits landed
+    setup_sync();
     if (lane == 0 && !p.test_stall) {
       Ring wr(SW), dr(kDigSlots);
       bool ok = true, fresh = true;
@@ -325,6 +342,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     // idles whenever a stage costs this warp more than its MMAs take, so the
     // loop of the common tile -- resident W, neither loaded nor given back --
     // holds nothing but the wait, the MMAs and the commit.
+    setup_sync();
+    const uint32_t tmem_base = *tmem_holder;
     Ring ar(S), wr(SW), dr(kDigSlots);
     const uint64_t a_const = smem_desc_sw32(smem_u32(sA));
     const uint64_t w_desc0 = smem_desc_sw128(smem_u32(sW));
@@ -422,11 +441,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
       st_cluster_u32(at + 4, nw);
       st_cluster_u32(at + 8, ndig);
       st_cluster_u32(at + 12, nacc);
-      counts[0] = nstage;
-      counts[1] = nw;
-      counts[2] = ndig;
-      counts[3] = nacc;
     }
+    drain_commits(nstage, nw, ndig, nacc);
     __syncwarp();
   } else if (warp >= kUnpackWarp0 && warp < kEProdWarp) {
     // ------------------------------------------------------------ unpack
@@ -434,6 +450,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     // holds both polarizations, and keeps its own (RowMap).  The groups take
     // stages in turn (R and S are multiples of their number, so a slot always
     // belongs to one group).
+    setup_sync();
+    const uint32_t tmem_base = *tmem_holder;
     const int group = (warp - kUnpackWarp0) / kStageWarps;
     const int box0 = ((warp - kUnpackWarp0) % kStageWarps >> 2) * kBoxes;
     const int q = warp & 3;
@@ -484,6 +502,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     // share no barrier: a slow one does not hold up the others.
     const int q = warp & 3;
     const int part = warp >> 2;
+    setup_sync();
+    const uint32_t tmem_base = *tmem_holder;
     const uint32_t lane_addr = static_cast<uint32_t>(32 * q) << 16;
     uint32_t local = 0;
     unsigned long long ad_s1 = 0, ad_s2 = 0;  // fused adler32 (kAdler): sums of the J bytes this lane stores
@@ -510,27 +530,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     if constexpr (kAdler) add_adler(p.one.adler, ad_s1, ad_s2, lane);
   }
 
-  // Both CTAs wait for the leader's last commits to arrive (see the MMA issuer)
-  // and for each other before either frees tensor memory or exits.
+  // Both CTAs meet once more: neither frees tensor memory or exits while the
+  // other's threads or the leader's MMAs may still reach into it.  What can still
+  // come after that are the arrivals of the leader's last commits at the peer's
+  // own barriers, which the peer waits for here.
   __syncwarp();
-  cluster_sync();
-  if (warp == kMmaWarp) {
-    const uint32_t uS = static_cast<uint32_t>(S), uW = static_cast<uint32_t>(SW), uD = static_cast<uint32_t>(kDigSlots);
-    const uint32_t c0 = counts[0], c1 = counts[1], c2 = counts[2], c3 = counts[3];
-    for (uint32_t k = c0 > uS ? c0 - uS : 0; k < c0; ++k) mbar_wait_drain(empty(static_cast<int>(k % uS)), (k / uS) & 1u);
-    for (uint32_t k = c1 > uW ? c1 - uW : 0; k < c1; ++k)
-      mbar_wait_drain(w_empty(static_cast<int>(k % uW)), (k / uW) & 1u);
-    for (uint32_t k = c2 > uD ? c2 - uD : 0; k < c2; ++k)
-      mbar_wait_drain(d_empty(static_cast<int>(k % uD)), (k / uD) & 1u);
-    for (uint32_t k = c3 > 2u ? c3 - 2u : 0u; k < c3; ++k) mbar_wait_drain(accfull(static_cast<int>(k & 1u)), (k >> 1) & 1u);
-    __syncwarp();
-  }
   tc_fence_before();
-  __syncthreads();
   cluster_sync();
   if (warp == kMmaWarp) {
+    if (rank == 1) drain_commits(counts[0], counts[1], counts[2], counts[3]);
+    __syncwarp();
     tc_fence_after();
-    tmem_dealloc_pair(tmem_base, 512);
+    tmem_dealloc_pair(*tmem_holder, 512);
   }
 }
 
@@ -571,8 +582,7 @@ cudaError_t launch_inst(const PairParams &p, int smem_bytes, cudaStream_t s) {
   }
   const int grid = 2 * std::min(p.ntiles, pair_clusters());
   if (grid <= 0) return cudaSuccess;
-  kern<<<grid, kPairThreads, smem_bytes, s>>>(p);
-  return cudaGetLastError();
+  return launch_overlapped(kern, grid, kPairThreads, smem_bytes, s, p);
 }
 
 }  // namespace
