@@ -144,6 +144,10 @@ __device__ __forceinline__ bool mbar_wait_drain(uint32_t bar, uint32_t parity) {
   }
 }
 
+// Barrier 1 of the CTA: every warp arrives, those that sync wait for the rest.
+__device__ __forceinline__ void cta_arrive(int threads) { asm volatile("bar.arrive 1, %0;" ::"r"(threads) : "memory"); }
+__device__ __forceinline__ void cta_sync(int threads) { asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory"); }
+
 // ---------------------------------------------------------------- clusters
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;

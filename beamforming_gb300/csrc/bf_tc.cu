@@ -268,28 +268,27 @@ __global__ void __launch_bounds__(Roles<kEpiW, kGroups>::kThreads, kHalf ? 2 : 1
   const int ncols = 2 * p.max_nb_pass;                 // accumulator columns reserved (largest GEMM N)
   const int per_half = (kAcc - ncols) / kStageCols;  // unpacked stages beside each accumulator
 
-  if (threadIdx.x == 0) {
-    for (int r = 0; r < R; ++r) {
-      mbar_init(raw_full(r), 1);
-      mbar_init(raw_empty(r), 128);
+  // Each producer sets up its own barriers and starts its copies at once; the
+  // other warps meet while those are under way.
+  if (warp == kEProdWarp) {
+    for (int i = lane; i < 2 * R; i += 32) mbar_init(raw_full(i), i < R ? 1 : 128);
+    if (!kGrouped && lane == 0) tma_prefetch_desc(&p.one.tm_e);
+  } else if (warp == kWProdWarp) {
+    for (int i = lane; i < 2 * SW; i += 32) mbar_init(w_full(i), 1);
+    if (lane < 2 * kDigSlots) mbar_init(d_full(lane), 1);
+    if (!kGrouped && lane == 0) {
+      tma_prefetch_desc(&p.one.tm_w);
+      tma_prefetch_desc(&p.one.tm_d);
     }
-    for (int s = 0; s < SW; ++s) {
-      mbar_init(w_full(s), 1);
-      mbar_init(w_empty(s), 1);
-    }
-    for (int s = 0; s < S; ++s) {
-      mbar_init(a_full(s), 128 + (RL::kForwarder ? 1 : 0));  // one unpack group (+ the W forwarder)
-      mbar_init(empty(s), 1);
-    }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(accfull(i), 1);
-      mbar_init(accempty(i), kEpiThreads);
-    }
-    for (int i = 0; i < kDigSlots; ++i) {
-      mbar_init(d_full(i), 1);
-      mbar_init(d_empty(i), 1);
-    }
-    fence_barrier_init();
+  } else if (warp == 0) {
+    if (lane < 2 * S) mbar_init(a_full(lane), lane < S ? 128 + (RL::kForwarder ? 1 : 0) : 1);  // one group (+ forwarder)
+    if (lane < 4) mbar_init(accfull(lane), lane < 2 ? 1 : kEpiThreads);
+  }
+  static_assert(2 * kMaxStages <= 32, "one lane per stage barrier");
+  fence_barrier_init();
+  if (warp == kMmaWarp) {
+    tmem_alloc(smem_u32(tmem_holder), 2 * kAcc);
+    tmem_relinquish();
   }
   // constant A tile of the offset MMA: every row the same, so the 32-byte
   // swizzle leaves it unchanged
@@ -298,18 +297,15 @@ __global__ void __launch_bounds__(Roles<kEpiW, kGroups>::kThreads, kHalf ? 2 : 1
     reinterpret_cast<uint32_t *>(sA)[i] = (w == 0 || w == 4) ? kDigitScaleLo : (w == 1 || w == 5) ? kDigitScaleHi : 0u;
   }
   fence_proxy_async_smem();
-  if (warp == kMmaWarp) {
-    tmem_alloc(smem_u32(tmem_holder), 2 * kAcc);
-    tmem_relinquish();
-  }
-  if (!kGrouped && warp == kEProdWarp && lane == 0) {
-    tma_prefetch_desc(&p.one.tm_e);
-    tma_prefetch_desc(&p.one.tm_w);
-  }
+  grid_launch_next();
+  grid_wait();
   tc_fence_before();
-  __syncthreads();
+  if (warp == kEProdWarp || warp == kWProdWarp)
+    cta_arrive(RL::kThreads);
+  else
+    cta_sync(RL::kThreads);
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_holder;
+  const uint32_t tmem_base = warp == kEProdWarp || warp == kWProdWarp ? 0u : *tmem_holder;  // the producers need none
   int *err = p.err;
 
   if (warp == kEProdWarp) {
@@ -631,7 +627,7 @@ __global__ void __launch_bounds__(Roles<kEpiW, kGroups>::kThreads, kHalf ? 2 : 1
   __syncthreads();
   if (warp == kMmaWarp) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, 2 * kAcc);
+    tmem_dealloc(*tmem_holder, 2 * kAcc);
   }
 }
 
@@ -1055,8 +1051,7 @@ static cudaError_t launch_inst(const TcParams &p, int smem_bytes, cudaStream_t s
   }
   const int grid = std::min(p.ntiles, (kHalf ? 2 : 1) * num_sms());
   if (grid <= 0) return cudaSuccess;
-  kern<<<grid, Roles<kEpiW, kGroups>::kThreads, smem_bytes, s>>>(p);
-  return cudaGetLastError();
+  return launch_overlapped(kern, grid, Roles<kEpiW, kGroups>::kThreads, smem_bytes, s, p);
 }
 
 // Warp layout of a launch: passes of at most kHalfPass beams run two CTAs per
