@@ -202,6 +202,15 @@ struct TcProblem {  // 128-byte aligned through its tensor maps
   int w_rows;        // rows of the W and digit boxes: the pass's 2 * nb_pass, or a CTA's half of N in a pair launch
 };
 
+// Whether the weights of passes this wide are stored as W + 8 rather than as
+// signed codes (see bf_prep_weights).  A launch sums the rows of E if its widest
+// pass asks for it; the digit rows of narrower ones ignore the sums.  The sums
+// cost the unpack the same at any width, the codes save in proportion to it:
+// f=64 d=512, 32768 times, 512 -> 474 us at 72 beams and 457 -> 444 at 64, but
+// 2048 times x 16 channels 14.0 -> 14.5 and 13.2 -> 14.5 us, and narrower passes
+// are the smaller calls.
+inline bool tc_w_offset(int nb_pass) { return nb_pass > 64; }
+
 // Shared-memory ring depths of a launch (0: planner default).
 struct TcRingPlan {
   int wslots = 0;

@@ -282,11 +282,11 @@ __device__ __forceinline__ void mma_f8f6f4_ts(uint32_t d_tmem, uint32_t a_tmem, 
 // call it from a warp-uniform loop behind elect_one(), so that the operands
 // stay in uniform registers.
 __device__ __forceinline__ void mma_ts_stage8(uint32_t d_tmem, uint32_t a_tmem, uint64_t b0, uint64_t b1,
-                                              uint32_t idesc) {
+                                              uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t.reg .b64 b;\n\t.reg .b32 a;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], [%1], %2, %4, p;\n\t"
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 b;\n\t.reg .b32 a;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], [%1], %2, %4, q;\n\t"
       "add.u32 a, %1, 8;\n\tadd.s64 b, %2, 2;\n\t"
       "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], [a], b, %4, p;\n\t"
       "add.u32 a, %1, 16;\n\tadd.s64 b, %2, 4;\n\t"
@@ -301,7 +301,7 @@ __device__ __forceinline__ void mma_ts_stage8(uint32_t d_tmem, uint32_t a_tmem, 
       "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], [a], b, %4, p;\n\t"
       "add.u32 a, %1, 56;\n\tadd.s64 b, %3, 6;\n\t"
       "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], [a], b, %4, p;\n\t}" ::"r"(d_tmem),
-      "r"(a_tmem), "l"(b0), "l"(b1), "r"(idesc)
+      "r"(a_tmem), "l"(b0), "l"(b1), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 
@@ -330,19 +330,20 @@ __device__ __forceinline__ void mma_f8f6f4_pair(uint32_t d_tmem, uint64_t a_desc
 }
 // The four MMAs of one 128-byte W box: K step kk reads TMEM columns a + 8 kk
 // and byte 32 kk of the box's rows.
-__device__ __forceinline__ void mma_ts_box_pair(uint32_t d_tmem, uint32_t a_tmem, uint64_t b0, uint32_t idesc) {
+__device__ __forceinline__ void mma_ts_box_pair(uint32_t d_tmem, uint32_t a_tmem, uint64_t b0, uint32_t idesc,
+                                                uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t.reg .b64 b;\n\t.reg .b32 a, l, h;\n\t"
-      "setp.ne.b32 p, %3, 0;\n\t"
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 b;\n\t.reg .b32 a, l, h;\n\t"
+      "setp.ne.b32 p, %3, 0;\n\tsetp.ne.b32 q, %4, 0;\n\t"
       "mov.b64 {l, h}, %2;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], [%1], %2, %3, p;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], [%1], %2, %3, q;\n\t"
       "add.u32 a, %1, 8;\n\tadd.u32 l, l, 2;\n\tmov.b64 b, {l, h};\n\t"
       "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], [a], b, %3, p;\n\t"
       "add.u32 a, %1, 16;\n\tadd.u32 l, l, 2;\n\tmov.b64 b, {l, h};\n\t"
       "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], [a], b, %3, p;\n\t"
       "add.u32 a, %1, 24;\n\tadd.u32 l, l, 2;\n\tmov.b64 b, {l, h};\n\t"
       "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], [a], b, %3, p;\n\t}" ::"r"(d_tmem),
-      "r"(a_tmem), "l"(b0), "r"(idesc)
+      "r"(a_tmem), "l"(b0), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 // Arrive once on the mbarrier at this offset in both CTAs of the pair when

@@ -13,17 +13,18 @@
 // [0, 15] is, read as E4M3, exactly u * 2^-9 (exponent field 0 or 1: the
 // subnormal and the first normal binade share the step 2^-9).  So the raw
 // ucomplex4 nibbles (value x stored as u = x + 8) become tensor-core operands
-// with one AND per 4 values.  The offset goes into the accumulator's start
-// value, set by one extra MMA that opens every tile (digit rows of the row
-// sums times a constant tile, see kDigitScaleLo):
+// with one AND per 4 values.  The offset goes into the accumulator with one extra
+// MMA per tile (digit rows of the row sums of W times a constant tile, see
+// kDigitScaleLo):
 //
 //   acc[n] = 2^-18 (-8 sum_k W[n][k] + sum_k u_k W[n][k])
 //          = 2^-18 sum_k (u_k - 8) W[n][k] = 2^-18 raw
 //
 // W holds the integers Ar, -Ai, Ai in [-8, 8] in the same form, w * 2^-9 (a sign
-// and the low nibble).  The start value and every partial sum are integer
-// multiples of 2^-18 below 2^1 in magnitude (at most 19 significant bits), exact
-// in the f32 accumulator.  As normal numbers (w itself) the products are just
+// and the low nibble), or for wide passes w + 8 in [0, 16], when the extra MMA
+// also takes off 8 sum_k u_k (see bf_prep_weights).  Every partial sum is an
+// integer multiple of 2^-18 below 2^2 in magnitude (ndishes <= 2048: at most 20
+// significant bits), exact in the f32 accumulator.  As normal numbers (w itself) the products are just
 // as exact, but the codes' exponent bits toggle from column to column, and the
 // chip runs at its power limit: the full chunk took 745 us with them, 719
 // with subnormals (the wide array 743, 726; sustained).  The
@@ -218,12 +219,12 @@ __host__ __device__ inline SmemPlan smem_plan(int stages, int wslots, int raw, i
   s.dbytes = (2 * nb_pass * kDigitRow + 1023) / 1024 * 1024;
   s.off_w = 0;
   s.off_a = s.off_w + wslots * s.wbytes;  // constant A tile of the offset MMA
-  s.off_d = s.off_a + kConstABytes;       // digit-row slots
+  s.off_d = s.off_a + 2 * kConstABytes;       // digit-row slots
   s.off_r = s.off_d + kDigSlots * s.dbytes;
   s.off_bar = s.off_r + raw * kRawBytes;
   // raw_full[R], raw_empty[R], w_full[SW], w_empty[SW], a_full[S], empty[S], accfull[2], accempty[2],
-  // d_full[2], d_empty[2]
-  s.nbar = 2 * raw + 2 * wslots + 2 * stages + 4 + 2 * kDigSlots;
+  // d_full[2], d_empty[2], rs_full[2]
+  s.nbar = 2 * raw + 2 * wslots + 2 * stages + 4 + 2 * kDigSlots + 2;
   s.total = s.off_bar + 8 * s.nbar + 16;
   return s;
 }
@@ -242,6 +243,7 @@ __global__ void __launch_bounds__(Roles<kEpiW, kGroups>::kThreads, kHalf ? 2 : 1
   constexpr int kEpiThreads = RL::kEpiThreads, kEpiParts = RL::kEpiParts, kEProdWarp = RL::kEProdWarp;
   constexpr int kMmaWarp = RL::kMmaWarp, kWProdWarp = RL::kWProdWarp, kUnpackWarp0 = RL::kUnpackWarp0;
   constexpr int kUnpackGroups = RL::kUnpackGroups;
+  constexpr bool kSums = !kHalf;  // passes of the half-SM layout are too narrow for W + 8 (tc_w_offset)
   extern __shared__ uint8_t smem_dyn[];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
   const int S = p.stages, SW = p.wslots, R = p.raw;
@@ -261,6 +263,7 @@ __global__ void __launch_bounds__(Roles<kEpiW, kGroups>::kThreads, kHalf ? 2 : 1
   auto accempty = [&](int i) { return bar0 + 8u * (2 * R + 2 * SW + 2 * S + 2 + i); };
   auto d_full = [&](int i) { return bar0 + 8u * (2 * R + 2 * SW + 2 * S + 4 + i); };
   auto d_empty = [&](int i) { return bar0 + 8u * (2 * R + 2 * SW + 2 * S + 4 + kDigSlots + i); };
+  auto rs_full = [&](int i) { return bar0 + 8u * (2 * R + 2 * SW + 2 * S + 4 + 2 * kDigSlots + i); };
   uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(smem + sp.off_bar + 8 * sp.nbar);
 
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);  // known to be warp-uniform
@@ -283,6 +286,7 @@ __global__ void __launch_bounds__(Roles<kEpiW, kGroups>::kThreads, kHalf ? 2 : 1
   } else if (warp == 0) {
     if (lane < 2 * S) mbar_init(a_full(lane), lane < S ? 128 + (RL::kForwarder ? 1 : 0) : 1);  // one group (+ forwarder)
     if (lane < 4) mbar_init(accfull(lane), lane < 2 ? 1 : kEpiThreads);
+    if (lane < 2) mbar_init(rs_full(lane), 4 * kUnpackGroups);
   }
   static_assert(2 * kMaxStages <= 32, "one lane per stage barrier");
   fence_barrier_init();
@@ -290,12 +294,7 @@ __global__ void __launch_bounds__(Roles<kEpiW, kGroups>::kThreads, kHalf ? 2 : 1
     tmem_alloc(smem_u32(tmem_holder), 2 * kAcc);
     tmem_relinquish();
   }
-  // constant A tile of the offset MMA: every row the same, so the 32-byte
-  // swizzle leaves it unchanged
-  for (int i = threadIdx.x; i < kConstABytes / 4; i += blockDim.x) {
-    const int w = i & 7;
-    reinterpret_cast<uint32_t *>(sA)[i] = (w == 0 || w == 4) ? kDigitScaleLo : (w == 1 || w == 5) ? kDigitScaleHi : 0u;
-  }
+  fill_offset_tiles<kSums ? 2 : 1>(sA);
   fence_proxy_async_smem();
   grid_launch_next();
   grid_wait();
@@ -428,7 +427,7 @@ __global__ void __launch_bounds__(Roles<kEpiW, kGroups>::kThreads, kHalf ? 2 : 1
     // 128 / 256) and 309 / 365 in this form (152 SMs, 400 stages, clock64).
     {
       Ring ar(S), wr(SW), dr(kDigSlots);
-      const uint64_t a_const = smem_desc_sw32(smem_u32(sA));
+      const uint64_t a_off = smem_desc_sw32(smem_u32(sA));
       const uint64_t w_desc0 = smem_desc_sw128(smem_u32(sW));
       uint32_t local = 0;
       uint32_t nstage = 0, ndig = 0, nacc = 0;  // commits issued on empty, d_empty, accfull
@@ -447,14 +446,15 @@ __global__ void __launch_bounds__(Roles<kEpiW, kGroups>::kThreads, kHalf ? 2 : 1
         if (!__all_sync(0xffffffffu, mbar_wait(d_full(ds), dr.phase, err, kDevTimeoutFull))) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + ab * kAcc;
-        // the offset MMA starts the accumulator at -8 sum_k W[n][k] 2^-18
-        if (elect_one()) {
-          mma_f8f6f4(d_tmem, a_const, smem_desc_sw32(smem_u32(sD + ds * sp.dbytes)), idesc, 0u);
+        // the offset MMA: -8 sum_k W[n][k] 2^-18, with the row sums also
+        // -8 sum_k u[m][k] 2^-18, which are there last
+        auto offset_mma = [&]() {
+          mma_f8f6f4(d_tmem, a_off + (kSums ? ab * (kConstABytes >> 4) : 0u), smem_desc_sw32(smem_u32(sD + ds * sp.dbytes)), idesc,
+                     kSums ? 1u : 0u);
           mma_commit(d_empty(ds));
-        }
+        };
+        if (!kSums && elect_one()) offset_mma();
         __syncwarp();
-        ++ndig;
-        dr.advance();
         for (int ks = 0; ks < p.nk; ++ks, ar.advance(), wr.advance()) {
           const int s = static_cast<int>(ar.idx);
           const int sw = static_cast<int>(wr.idx);
@@ -467,14 +467,24 @@ __global__ void __launch_bounds__(Roles<kEpiW, kGroups>::kThreads, kHalf ? 2 : 1
           const uint32_t a_tmem = tmem_base + stage_col(s, ncols, per_half, kAcc);
           const uint64_t b_desc = w_desc0 + static_cast<uint64_t>((sw * sp.wbytes) >> 4);
           if (elect_one()) {
-            mma_ts_stage8(d_tmem, a_tmem, b_desc, b_desc + static_cast<uint64_t>(wbox >> 4), idesc);
+            mma_ts_stage8(d_tmem, a_tmem, b_desc, b_desc + static_cast<uint64_t>(wbox >> 4), idesc, !kSums || ks > 0);
             mma_commit(empty(s));  // also frees the W slot: the unpack passes it on
-            if (ks + 1 == p.nk) mma_commit(accfull(ab));
           }
           __syncwarp();
           ++nstage;
         }
         if (!ok) break;
+        if constexpr (kSums) {
+          if (!__all_sync(0xffffffffu, mbar_wait(rs_full(ab), aph, err, kDevTimeoutUnpacked))) break;
+          tc_fence_after();
+        }
+        if (elect_one()) {
+          if constexpr (kSums) offset_mma();
+          mma_commit(accfull(ab));
+        }
+        __syncwarp();
+        ++ndig;
+        dr.advance();
         ++nacc;
       }
       // A commit's arrival is an asynchronous write into this CTA's shared
@@ -537,7 +547,14 @@ __global__ void __launch_bounds__(Roles<kEpiW, kGroups>::kThreads, kHalf ? 2 : 1
       ar.advance();
       wr.advance();
     }
-    bool ok = true;
+    RowSums rs(sA, group, group, 32 * q + lane);
+    auto rs_free = [&](int tile) {
+      return __all_sync(0xffffffffu, mbar_wait(accfull(tile & 1), ((tile >> 1) & 1) ^ 1, err, kDevTimeoutAccFull));
+    };
+    auto rs_arrive = [&](int tile) {
+      if (lane == 0) mbar_arrive(rs_full(tile & 1));
+    };
+    bool ok = !kSums || rs.settle(p.nk, static_cast<int>(my_tiles), rs_free, rs_arrive);
     for (uint32_t it = group; ok && it < total; it += kUnpackGroups) {
       {
         const int r = static_cast<int>(rr.idx);
@@ -551,7 +568,7 @@ __global__ void __launch_bounds__(Roles<kEpiW, kGroups>::kThreads, kHalf ? 2 : 1
         // stores wait for the tensor core to release the stage
         uint32_t out[kSub][32];
 #pragma unroll
-        for (int h = 0; h < kSub; ++h) unpack_box(smem_u32(sR) + r * kRawBytes + h * kRawBox, row, sel, out[h]);
+        for (int h = 0; h < kSub; ++h) rs.sum += unpack_box<kSums>(smem_u32(sR) + r * kRawBytes + h * kRawBox, row, sel, out[h]);
         // the raw slot is in registers now; the next TMA into it is an async-proxy
         // write after these generic reads, so order them across proxies first
         fence_proxy_async_smem();
@@ -571,6 +588,10 @@ __global__ void __launch_bounds__(Roles<kEpiW, kGroups>::kThreads, kHalf ? 2 : 1
         if (!__all_sync(0xffffffffu, ok)) break;
         tc_fence_before();
         mbar_arrive(a_full(s));
+        if constexpr (kSums) {
+          rs.kpos += kUnpackGroups;
+          ok = rs.settle(p.nk, static_cast<int>(my_tiles), rs_free, rs_arrive);
+        }
       }
 #pragma unroll
       for (int g = 0; g < kUnpackGroups; ++g) {
@@ -631,19 +652,6 @@ __global__ void __launch_bounds__(Roles<kEpiW, kGroups>::kThreads, kHalf ? 2 : 1
   }
 }
 
-// Builds the E4M3 operand W[f][n][k] and the digit rows of the row sums
-// sum_k W[f][n][k] from A[f][b][d].
-//   n = 2*b + cj                   (cj: 0 = real output, 1 = imaginary output)
-//   k = 8*(d/4)  + 4*c  + d%4      (c:  0 = real input,  1 = imaginary input)
-// W = Ar, -Ai for the real output and Ai, Ar for the imaginary output.
-//
-// One warp per beam: both of its rows hold the same numbers, so a lane turns 16
-// dishes into the codes of Ar, Ai and -Ai four bytes at a time and stores 32
-// bytes of each row.  Bound by the bytes of W (f=16 b=512 d=1024: 33.5 MB and
-// 8.4 MB of A); a warp per row and a byte per load took 42 us there, this 14.4
-// (f=16 b=96 d=512: 9.1 and 4.5 us, launch included).
-constexpr int kPrepBeams = 8;  // beams per 256-thread block
-
 // The E4M3 codes of v * 2^-9 (a sign bit and |v|) of four stored nibbles u = v + 8.
 __device__ __forceinline__ uint32_t w_codes(uint32_t u) {
   const uint32_t x = u ^ 0x08080808u;                // two's complement nibbles
@@ -654,6 +662,26 @@ __device__ __forceinline__ uint32_t w_negate(uint32_t codes) {  // zero stays ze
   return codes ^ (((codes & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) & 0x80808080u);
 }
 
+// Builds the E4M3 operand W[f][n][k] and the digit rows of the row sums
+// sum_k W[f][n][k] from A[f][b][d].
+//   n = 2*b + cj                   (cj: 0 = real output, 1 = imaginary output)
+//   k = 8*(d/4)  + 4*c  + d%4      (c:  0 = real input,  1 = imaginary input)
+// W = Ar, -Ai for the real output and Ai, Ar for the imaginary output, stored as
+// E4M3 (W + 8) * 2^-9, all codes 0..16.  The accumulator is then too large by
+// 8 sum_k u_k in every column of a row, which the unpack sums and the offset MMA
+// takes off (RowSums).  Signed codes are as exact and need no sums, but the
+// chip runs at its power limit and operands whose sign changes from column to
+// column cost the most of it: the full chunk (f=84 t=32768 b=96 d=512) took 735 us
+// with them and 661 so, at 1.40 and 1.63 GHz; the wide array 711 and 693.
+//
+// One warp per beam: both of its rows hold the same numbers, so a lane turns 16
+// dishes into the codes of Ar, Ai and -Ai four bytes at a time and stores 32
+// bytes of each row.  Bound by the bytes of W (f=16 b=512 d=1024: 33.5 MB and
+// 8.4 MB of A); a warp per row and a byte per load took 42 us there, this 14.4
+// (f=16 b=96 d=512: 9.1 and 4.5 us, launch included).
+constexpr int kPrepBeams = 8;  // beams per 256-thread block
+
+template <bool kOffset>
 __global__ void __launch_bounds__(32 * kPrepBeams) bf_prep_weights(const uint8_t *__restrict__ A,
                                                                     uint8_t *__restrict__ W,
                                                                     uint8_t *__restrict__ dig,
@@ -716,9 +744,15 @@ __global__ void __launch_bounds__(32 * kPrepBeams) bf_prep_weights(const uint8_t
           const uint32_t ur = (w[2 * h + j] >> 4) & 0x0F0F0F0Fu, ui = w[2 * h + j] & 0x0F0F0F0Fu;
           s_re += static_cast<int>(__dp4a(ur, 0x01010101u, 0u)) - 32;
           s_im += static_cast<int>(__dp4a(ui, 0x01010101u, 0u)) - 32;
-          re[j] = w_codes(ur);
-          im[j] = w_codes(ui);
-          ni[j] = w_negate(im[j]);
+          if constexpr (kOffset) {  // the stored nibbles are Ar + 8 and Ai + 8
+            re[j] = ur;
+            im[j] = ui;
+            ni[j] = 0x10101010u - ui;
+          } else {
+            re[j] = w_codes(ur);
+            im[j] = w_codes(ui);
+            ni[j] = w_negate(im[j]);
+          }
         }
         w0[2 * i + h] = make_uint4(re[0], ni[0], re[1], ni[1]);
         w1[2 * i + h] = make_uint4(im[0], re[0], im[1], re[1]);
@@ -746,7 +780,7 @@ __global__ void __launch_bounds__(32 * kPrepBeams) bf_prep_weights(const uint8_t
     }
     const uint32_t d4 = rest == 0 ? 0u : (rest > 0 ? 0x04u : 0x84u);  // 4 * d4: +-4 or 0
     uint4 *row = reinterpret_cast<uint4 *>(dig + (static_cast<int64_t>(f) * nw_pad + 2 * b + lane) * kDigitRow);
-    row[0] = make_uint4(d03, d4, 0u, 0u);
+    row[0] = make_uint4(d03, d4, kOffset ? kDigitScaleLo : 0u, kOffset ? kDigitScaleLo : 0u);
     row[1] = make_uint4(0u, 0u, 0u, 0u);
   }
 }
@@ -927,7 +961,8 @@ cudaError_t launch_pad_e(const bf_dims &d, const uint8_t *E, size_t avail, int64
 cudaError_t launch_prep_weights(const TcWeights &w, const uint8_t *A, cudaStream_t s, int a_layout) {
   const int64_t blocks = static_cast<int64_t>((w.nw_pad / 2 + kPrepBeams - 1) / kPrepBeams) * w.F;
   if (blocks > 0x7FFFFFFF) return cudaErrorInvalidValue;
-  return launch_overlapped(bf_prep_weights, static_cast<unsigned>(blocks), 32 * kPrepBeams, 0, s, A, w.W, w.dig, w.G,
+  auto kern = tc_w_offset(w.nb_pass) ? bf_prep_weights<true> : bf_prep_weights<false>;
+  return launch_overlapped(kern, static_cast<unsigned>(blocks), 32 * kPrepBeams, 0, s, A, w.W, w.dig, w.G,
                            w.gs, w.gwide, static_cast<int>(w.B), static_cast<int>(w.D), static_cast<int>(w.Dk), w.nw,
                            w.nw_pad, a_layout);
 }

@@ -20,11 +20,11 @@ constexpr int kRawBytes = kSub * kRawBox;
 constexpr int kStageCols = kStageK / 4;  // TMEM columns per unpacked stage
 constexpr int kDigSlots = 2;            // digit-row slots (one per tile in flight)
 // Offset correction: one extra MMA per tile, issued first (it also clears the
-// accumulator), multiplies a constant A tile by the tile's digit rows.  The
-// constant row holds -2^-6, -2^-2, -4, -64, -256 at K = 0..4 (again at 16..20,
+// accumulator) or, with row sums (RowSums), last, multiplies a constant A tile by
+// the tile's digit rows.  The constant row holds -2^-6, -2^-2, -4, -64, -256 at K = 0..4 (again at 16..20,
 // so the 32-byte swizzle cannot move them), the digit row of n holds d0..d3 and
-// 4 d4, all times 2^-9, with sum_k W[n][k] = d0 + 16 d1 + 256 d2 + 4096 d3 + 65536 d4, so the
-// accumulator starts at -2^-15 sum_k W[n][k] = -8 sum_k W[n][k] 2^-18 exactly.
+// 4 d4, all times 2^-9, with sum_k W[n][k] = d0 + 16 d1 + 256 d2 + 4096 d3 + 65536 d4, so it
+// adds -2^-15 sum_k W[n][k] = -8 sum_k W[n][k] 2^-18 exactly.
 constexpr uint32_t kDigitScaleLo = 0xE8C8A888u;  // E4M3 -2^-6, -2^-2, -4, -64
 constexpr uint32_t kDigitScaleHi = 0x000000F8u;  // E4M3 -256
 constexpr int kConstABytes = kBM * kDigitRow;
@@ -93,8 +93,10 @@ struct UnpackRow {
 
 // One raw E box (64 times x 64 dishes x 2 polarizations, 128-byte swizzle) in
 // shared memory -> the 128 operand bytes of this lane's row, of the polarization
-// that `sel` picks (0x6420: even bytes, 0x7531: odd ones).
-__device__ __forceinline__ void unpack_box(uint32_t raw, const UnpackRow &row, uint32_t sel, uint32_t (&out)[32]) {
+// that `sel` picks (0x6420: even bytes, 0x7531: odd ones).  Returns
+// the sum of those 128 nibbles with kSums.
+template <bool kSums>
+__device__ __forceinline__ uint32_t unpack_box(uint32_t raw, const UnpackRow &row, uint32_t sel, uint32_t (&out)[32]) {
   uint32_t e[16];  // this row's polarization, dishes 4m..4m+3 of the box in word m
 #pragma unroll
   for (uint32_t j = 0; j < 8; ++j) {
@@ -112,7 +114,54 @@ __device__ __forceinline__ void unpack_box(uint32_t raw, const UnpackRow &row, u
     out[2 * m] = (e[m] >> 4) & msk;  // real nibbles u (E4M3 bytes = u * 2^-9)
     out[2 * m + 1] = e[m] & msk;     // imaginary nibbles
   }
+  if (!kSums) return 0;
+  uint32_t s[2] = {0, 0};  // byte sums of 16 words: at most 240
+#pragma unroll
+  for (int m = 0; m < 16; ++m) s[m >> 3] += out[2 * m] + out[2 * m + 1];
+  return __dp4a(s[0], 0x01010101u, __dp4a(s[1], 0x01010101u, 0u));
 }
+
+// The A tile of the offset MMA: 128 rows of 32 bytes (32-byte swizzle), one tile
+// per accumulator.  Words 0, 1, 4 and 5 of a row hold the digit scales; words 2
+// and 3 of its first 16 bytes take -- against kDigitScaleLo in the digit rows --
+// the sum of the row's nibbles u as base-16 digits, from the two parts of its
+// K stages (or boxes) that the unpack warps of its lane quarter take.
+template <int kTiles>
+__device__ __forceinline__ void fill_offset_tiles(uint8_t *sA) {
+  for (int i = threadIdx.x; i < kTiles * kConstABytes / 4; i += blockDim.x) {
+    const int w = i & 3;
+    reinterpret_cast<uint32_t *>(sA)[i] = w == 0 ? kDigitScaleLo : w == 1 ? kDigitScaleHi : 0u;
+  }
+}
+
+// One unpack warp's walk over the tiles: it takes the K stages kpos, kpos +
+// groups, ... of tile after tile, and hands over its rows' sums at the end of each.
+struct RowSums {
+  uint32_t *at;  // this lane's word in the first tile
+  int tile = 0, kpos;
+  uint32_t sum = 0;  // < 2^16: at most 2 * 2048 nibbles
+  __device__ RowSums(uint8_t *sA, int group, int part, int row)
+      : at(reinterpret_cast<uint32_t *>(sA) + row * (kDigitRow / 4) + ((row >> 2) & 1) * 4 + 2 + part), kpos(group) {}
+  // After each stage (and once before the first: with fewer stages a tile than
+  // groups a warp has none of some tiles).  `free` waits for the MMAs of the tile
+  // two before, `arrive` tells the issuer.
+  template <class Free, class Arrive>
+  __device__ __forceinline__ bool settle(int nk, int ntiles, Free free, Arrive arrive) {
+    while (kpos >= nk && tile < ntiles) {
+      if (!free(tile)) return false;
+      uint32_t w = (sum | (sum << 8)) & 0x00FF00FFu;
+      w = (w | (w << 4)) & 0x0F0F0F0Fu;
+      at[(tile & 1) * (kConstABytes / 4)] = w;
+      fence_proxy_async_smem();
+      __syncwarp();
+      arrive(tile);
+      sum = 0;
+      ++tile;
+      kpos -= nk;
+    }
+    return true;
+  }
+};
 
 // The epilogue of one accumulator for one warp: lane quarter q of the tile's
 // rows and a range of its 8-beam column chunks.  Thread (g, cb) = (lane / 4,

@@ -71,12 +71,12 @@ __host__ __device__ inline PairSmem pair_smem(int stages, int wslots, int raw, i
   s.wbytes = kSub * (ncols / 2) * kKC;  // this CTA's half of the rows
   s.dbytes = (ncols / 2 * kDigitRow + 1023) / 1024 * 1024;
   s.off_a = wslots * s.wbytes;
-  s.off_d = s.off_a + kConstABytes;
+  s.off_d = s.off_a + 2 * kConstABytes;
   s.off_r = s.off_d + kDigSlots * s.dbytes;
   s.off_bar = s.off_r + raw * kRawBytes;
   // raw_full[R] raw_empty[R] w_full[SW] w_peer[SW] w_empty[SW] a_full[S] empty[S] accfull[2] accempty[2]
-  // d_full[2] d_peer[2] d_empty[2]
-  s.nbar = 2 * raw + 3 * wslots + 2 * stages + 4 + 3 * kDigSlots;
+  // d_full[2] d_peer[2] d_empty[2] rs_full[2]
+  s.nbar = 2 * raw + 3 * wslots + 2 * stages + 4 + 3 * kDigSlots + 2;
   s.total = s.off_bar + 8 * s.nbar + 32;  // + the TMEM address and the leader's commit counts
   return s;
 }
@@ -130,7 +130,7 @@ __host__ __device__ inline uint32_t pair_stage_col(uint32_t i, int ncols, int pe
          (i < static_cast<uint32_t>(per_half) ? 0u : static_cast<uint32_t>(kPairAcc - per_half * cols));
 }
 
-template <bool kGrouped, bool kJ2, bool kAdler, int kGroups>
+template <bool kGrouped, bool kJ2, bool kAdler, int kGroups, bool kSums>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     bf_form_beams_pair(const __grid_constant__ PairParams p) {
   constexpr int kUnpackWarp0 = kEpiW, kEProdWarp = kEpiW + kUnpackWarps, kMmaWarp = kEProdWarp + 1;
@@ -160,6 +160,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
   auto d_full = [&](int i) { return bc + 32u + 8u * i; };
   auto d_peer = [&](int i) { return bc + 48u + 8u * i; };
   auto d_empty = [&](int i) { return bc + 64u + 8u * i; };
+  auto rs_full = [&](int i) { return bc + 80u + 8u * i; };
   uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(smem + sp.off_bar + 8 * sp.nbar);
   uint32_t *counts = tmem_holder + 1;  // commits the leader issued on empty, w_empty, d_empty, accfull
 
@@ -186,6 +187,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     // warps, in both CTAs
     if (lane < 2 * S) mbar_init(a_full(lane), lane < S ? 2 * kStageWarps : 1);
     if (lane < 4) mbar_init(accfull(lane), lane < 2 ? 1 : 2 * kEpiW);
+    if (lane < 2) mbar_init(rs_full(lane), 2 * kUnpackWarps);
     if (lane < 4) counts[lane] = 0;
   }
   fence_barrier_init();
@@ -193,12 +195,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     tmem_alloc_pair(smem_u32(tmem_holder), 512);
     tmem_relinquish_pair();
   }
-  // constant A tile of the offset MMA: every row the same, so the 32-byte
-  // swizzle leaves it unchanged
-  for (int i = threadIdx.x; i < kConstABytes / 4; i += blockDim.x) {
-    const int w = i & 7;
-    reinterpret_cast<uint32_t *>(sA)[i] = (w == 0 || w == 4) ? kDigitScaleLo : (w == 1 || w == 5) ? kDigitScaleHi : 0u;
-  }
+  fill_offset_tiles<kSums ? 2 : 1>(sA);
   fence_proxy_async_smem();
   grid_launch_next();
   grid_wait();
@@ -345,7 +342,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     setup_sync();
     const uint32_t tmem_base = *tmem_holder;
     Ring ar(S), wr(SW), dr(kDigSlots);
-    const uint64_t a_const = smem_desc_sw32(smem_u32(sA));
+    const uint64_t a_off = smem_desc_sw32(smem_u32(sA));
     const uint64_t w_desc0 = smem_desc_sw128(smem_u32(sW));
     const uint32_t w_step = static_cast<uint32_t>(sp.wbytes) >> 4;
     uint32_t local = 0;
@@ -364,16 +361,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
         break;
       tc_fence_after();
       const uint32_t d_tmem = tmem_base + ab * kPairAcc;
-      // the offset MMA starts the accumulator at -8 sum_k W[n][k] 2^-18
-      if (elect_one()) {
-        mma_f8f6f4_pair(d_tmem, a_const, smem_desc_sw32(smem_u32(sD + ds * sp.dbytes)), idesc, 0u);
+      // the offset MMA: -8 sum_k W[n][k] 2^-18, with the row sums also
+      // -8 sum_k u[m][k] 2^-18, which are there last
+      auto offset_mma = [&]() {
+        mma_f8f6f4_pair(d_tmem, a_off + (kSums ? ab * (kConstABytes >> 4) : 0u), smem_desc_sw32(smem_u32(sD + ds * sp.dbytes)), idesc,
+                        kSums ? 1u : 0u);
         if (last) mma_commit_pair(d_empty(ds));
-      }
+      };
+      if (!kSums && elect_one()) offset_mma();
       __syncwarp();
-      if (last) {
-        ++ndig;
-        dr.advance();
-      }
       if (!fresh && !last && !stream_w) {
         uint64_t b_desc = w_desc0;
         for (int ks = 0; ks < nk; ++ks, b_desc += w_step) {
@@ -385,16 +381,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
           tc_fence_after();
           const uint32_t a_tmem = tmem_base + pair_stage_col(ar.idx, ncols, per_half, kStageCols);
           if (elect_one()) {
-            mma_ts_box_pair(d_tmem, a_tmem, b_desc, idesc);
-            mma_ts_box_pair(d_tmem, a_tmem + 32, b_desc + wbox, idesc);
+            mma_ts_box_pair(d_tmem, a_tmem, b_desc, idesc, !kSums || ks > 0);
+            mma_ts_box_pair(d_tmem, a_tmem + 32, b_desc + wbox, idesc, 1u);
             mma_commit_pair(bar + 8u * S);  // empty
           }
           __syncwarp();
           ++nstage;
           ar.advance();
         }
-        if (ok && elect_one()) mma_commit_pair(accfull(ab));
-        __syncwarp();
       } else {
         const bool reload = fresh || stream_w, release = last || stream_w;
         for (int ks = 0; ks < nk; ++ks, ar.advance()) {
@@ -415,11 +409,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
           const uint32_t a_tmem = tmem_base + pair_stage_col(ar.idx, ncols, per_half, kStageCols);
           const uint64_t b_desc = w_desc0 + static_cast<uint32_t>(sw) * w_step;
           if (elect_one()) {
-            mma_ts_box_pair(d_tmem, a_tmem, b_desc, idesc);
-            mma_ts_box_pair(d_tmem, a_tmem + 32, b_desc + wbox, idesc);
+            mma_ts_box_pair(d_tmem, a_tmem, b_desc, idesc, !kSums || ks > 0);
+            mma_ts_box_pair(d_tmem, a_tmem + 32, b_desc + wbox, idesc, 1u);
             mma_commit_pair(bar + 8u * S);  // empty
             if (release) mma_commit_pair(w_empty(sw));
-            if (ks + 1 == nk) mma_commit_pair(accfull(ab));
           }
           __syncwarp();
           ++nstage;
@@ -428,6 +421,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
         }
       }
       if (!ok) break;
+      if constexpr (kSums) {
+        if (!__all_sync(0xffffffffu, mbar_wait(rs_full(ab), (local >> 1) & 1u, err, kDevTimeoutUnpacked))) break;
+        tc_fence_after();
+      }
+      if (elect_one()) {
+        if constexpr (kSums) offset_mma();
+        mma_commit_pair(accfull(ab));
+      }
+      __syncwarp();
+      if (last) {
+        ++ndig;
+        dr.advance();
+      }
       ++nacc;
       fresh = last;
       cur.next(p);
@@ -464,7 +470,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
       rr.advance();
       ar.advance();
     }
-    for (uint32_t it = group; it < total; it += kGroups) {
+    const int my_tiles = end - first;
+    RowSums rs(sA, group, (warp - kUnpackWarp0) >> 2, 32 * q + lane);
+    auto rs_free = [&](int tile) {
+      return __all_sync(0xffffffffu, mbar_wait(accfull(tile & 1), ((tile >> 1) & 1) ^ 1, err, kDevTimeoutAccFull));
+    };
+    auto rs_arrive = [&](int tile) {
+      if (lane == 0) mbar_arrive_cluster(map_cta(rs_full(tile & 1), 0));
+    };
+    bool live = !kSums || rs.settle(nk, my_tiles, rs_free, rs_arrive);
+    for (uint32_t it = group; live && it < total; it += kGroups) {
       const int r = static_cast<int>(rr.idx);
       const int s = static_cast<int>(ar.idx);
       if (!__all_sync(0xffffffffu, mbar_wait(raw_full(r), rr.phase, err, kDevTimeoutFull))) break;
@@ -476,7 +491,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 #pragma unroll
       for (int h = 0; h < kBoxes; ++h) {
         uint32_t out[32];
-        unpack_box(raw + h * kRawBox, row, sel, out);
+        rs.sum += unpack_box<kSums>(raw + h * kRawBox, row, sel, out);
         if (h == 0) free = __all_sync(0xffffffffu, mbar_wait(empty(s), ar.phase ^ 1u, err, kDevTimeoutEmpty));
         if (!free) break;
         tmem_st_32x32b_x32(col + 32 * h, out);
@@ -490,6 +505,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster_relaxed(map_cta(a_full(s), 0));
+      if constexpr (kSums) {
+        rs.kpos += kGroups;
+        live = rs.settle(nk, my_tiles, rs_free, rs_arrive);
+      }
 #pragma unroll
       for (int g = 0; g < kGroups; ++g) {
         rr.advance();
@@ -546,8 +565,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 }
 
 // Ring depths and shared memory of a launch whose widest GEMM N is ncols.
-cudaError_t plan_pair(PairParams &p, int64_t D, int ncols, int groups, int *smem_bytes) {
+cudaError_t plan_pair(PairParams &p, int64_t D, int max_nb_pass, int groups, int *smem_bytes) {
   p.nk = tc_stages_per_tile(D);
+  p.ncols = pair_cols(max_nb_pass);
+  const int ncols = p.ncols;
   int stages = std::min(kPairMaxStages, 2 * ((kPairAcc - ncols) / kStageCols));
   stages -= stages % groups;  // so does a TMEM stage
   if (stages < 2) return cudaErrorInvalidValue;
@@ -563,7 +584,6 @@ cudaError_t plan_pair(PairParams &p, int64_t D, int ncols, int groups, int *smem
   int raw = 2;
   while (raw < kPairMaxRaw && total(wslots, raw + 1) <= kPairSmem) ++raw;
   raw -= raw % groups;  // a raw slot stays with one unpack group
-  p.ncols = ncols;
   p.stages = stages;
   p.wslots = wslots;
   p.raw = raw;
@@ -571,9 +591,9 @@ cudaError_t plan_pair(PairParams &p, int64_t D, int ncols, int groups, int *smem
   return *smem_bytes > kPairSmem ? cudaErrorInvalidValue : cudaSuccess;
 }
 
-template <bool kGrouped, bool kJ2, bool kAdler, int kGroups>
+template <bool kGrouped, bool kJ2, bool kAdler, int kGroups, bool kSums>
 cudaError_t launch_inst(const PairParams &p, int smem_bytes, cudaStream_t s) {
-  auto kern = bf_form_beams_pair<kGrouped, kJ2, kAdler, kGroups>;
+  auto kern = bf_form_beams_pair<kGrouped, kJ2, kAdler, kGroups, kSums>;
   static std::atomic<bool> attr_set{false};
   if (!attr_set.load()) {
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem);
@@ -583,6 +603,16 @@ cudaError_t launch_inst(const PairParams &p, int smem_bytes, cudaStream_t s) {
   const int grid = 2 * std::min(p.ntiles, pair_clusters());
   if (grid <= 0) return cudaSuccess;
   return launch_overlapped(kern, grid, kPairThreads, smem_bytes, s, p);
+}
+
+template <bool kSums>
+cudaError_t launch_plain(const PairParams &p, int smem_bytes, cudaStream_t s) {
+  const bool adler = p.one.adler != nullptr;
+  if (p.one.jlayout == kJ2)
+    return adler ? launch_inst<false, true, true, 2, kSums>(p, smem_bytes, s)
+                 : launch_inst<false, true, false, 2, kSums>(p, smem_bytes, s);
+  return adler ? launch_inst<false, false, true, 2, kSums>(p, smem_bytes, s)
+               : launch_inst<false, false, false, 2, kSums>(p, smem_bytes, s);
 }
 
 }  // namespace
@@ -595,7 +625,7 @@ int pair_clusters() {
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
       return 0;
-    auto kern = bf_form_beams_pair<false, false, false, 2>;
+    auto kern = bf_form_beams_pair<false, false, false, 2, true>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem) != cudaSuccess) {
       (void)cudaGetLastError();
       return 0;
@@ -623,7 +653,7 @@ int pair_clusters() {
 cudaError_t pair_launch_shape(int64_t D, int max_nb_pass, int groups, int *stages) {
   PairParams p{};
   int smem_bytes = 0;
-  const cudaError_t e = plan_pair(p, D, pair_cols(max_nb_pass), groups, &smem_bytes);
+  const cudaError_t e = plan_pair(p, D, max_nb_pass, groups, &smem_bytes);
   *stages = p.stages;
   return e;
 }
@@ -638,12 +668,9 @@ cudaError_t launch_pair(const TcProblem &one, int64_t D, int test_stall, int *er
   p.err = err;
   p.test_stall = test_stall;
   int smem_bytes = 0;
-  const cudaError_t e = plan_pair(p, D, pair_cols(one.nb_pass), 2, &smem_bytes);
+  const cudaError_t e = plan_pair(p, D, one.nb_pass, 2, &smem_bytes);
   if (e != cudaSuccess) return e;
-  const bool j2 = one.jlayout == kJ2, adler = one.adler != nullptr;
-  if (j2)
-    return adler ? launch_inst<false, true, true, 2>(p, smem_bytes, s) : launch_inst<false, true, false, 2>(p, smem_bytes, s);
-  return adler ? launch_inst<false, false, true, 2>(p, smem_bytes, s) : launch_inst<false, false, false, 2>(p, smem_bytes, s);
+  return tc_w_offset(one.nb_pass) ? launch_plain<true>(p, smem_bytes, s) : launch_plain<false>(p, smem_bytes, s);
 }
 
 cudaError_t launch_pair_grouped(const TcProblem *table, int nprob, int ntiles, int64_t D, int max_nb_pass, int groups,
@@ -655,10 +682,11 @@ cudaError_t launch_pair_grouped(const TcProblem *table, int nprob, int ntiles, i
   p.err = err;
   p.test_stall = test_stall;
   int smem_bytes = 0;
-  const cudaError_t e = plan_pair(p, D, pair_cols(max_nb_pass), groups, &smem_bytes);
+  const cudaError_t e = plan_pair(p, D, max_nb_pass, groups, &smem_bytes);
   if (e != cudaSuccess) return e;
-  return groups == 1 ? launch_inst<true, false, false, 1>(p, smem_bytes, s)
-                     : launch_inst<true, false, false, 2>(p, smem_bytes, s);
+  if (groups == 1) return launch_inst<true, false, false, 1, true>(p, smem_bytes, s);  // only beside two TMEM stages
+  return tc_w_offset(max_nb_pass) ? launch_inst<true, false, false, 2, true>(p, smem_bytes, s)
+                                  : launch_inst<true, false, false, 2, false>(p, smem_bytes, s);
 }
 
 }  // namespace bf
