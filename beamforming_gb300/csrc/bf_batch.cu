@@ -23,6 +23,7 @@ namespace {
 // One grouped launch of a batch: a range of the device problem table.
 struct BatchLaunch {
   int first = 0, nprob = 0, ntiles = 0, max_nb_pass = 0, stages = 0, groups = 0, ctas_per_sm = 0;
+  bool two_pass = false;  // of two beam passes, some of them
 };
 constexpr int kMaxLaunches = 3;  // one per pass-width class
 }  // namespace
@@ -96,6 +97,7 @@ Schedule schedule_of(const std::vector<Records> &probs, const std::vector<int> &
       if (launch_of(class_of(probs[i].one), cuts) != l) continue;
       TcProblem P = pair ? probs[i].pair : probs[i].one;
       P.tile_begin = static_cast<int>(begin);
+      L.two_pass |= P.npass == 2;
       begin += tc_problem_tiles(P);
       sc.table.push_back(P);
     }
@@ -123,7 +125,7 @@ cudaError_t launch_schedule(const bf_batch *b, const BatchLaunch *ls, int n, con
                             cudaStream_t s) {
   for (int i = 0; i < n; ++i) {
     const cudaError_t e =
-        launch_tc_grouped(b->table + ls[i].first, ls[i].nprob, ls[i].ntiles, b->D, ls[i].max_nb_pass, plan, b->err, s);
+        launch_tc_grouped(b->table + ls[i].first, ls[i].nprob, ls[i].ntiles, b->D, ls[i].max_nb_pass, ls[i].two_pass, plan, b->err, s);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;

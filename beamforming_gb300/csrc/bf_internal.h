@@ -229,9 +229,10 @@ int64_t tc_problem_tiles(const TcProblem &P);
 int tc_stages_per_tile(int64_t D);
 
 // One persistent launch over nprob problems (records in device memory; all
-// with D dishes).  max_nb_pass = the largest nb_pass among them.
+// with D dishes).  max_nb_pass = the largest nb_pass among them; two_pass: some
+// have two passes.
 cudaError_t launch_tc_grouped(const TcProblem *table, int nprob, int ntiles, int64_t D, int max_nb_pass,
-                              const TcRingPlan &plan, int *err, cudaStream_t s);
+                              bool two_pass, const TcRingPlan &plan, int *err, cudaStream_t s);
 
 // The whole ring layout of a launch with these sizes: out[0..11] = stages,
 // W slots, raw E slots, unpack groups, CTAs per SM, K stages per tile,
@@ -246,8 +247,8 @@ int pair_clusters();
 int pair_cols(int nb_pass);
 cudaError_t pair_launch_shape(int64_t D, int max_nb_pass, int groups, int *stages);
 cudaError_t launch_pair(const TcProblem &one, int64_t D, int test_stall, int *err, cudaStream_t s);
-cudaError_t launch_pair_grouped(const TcProblem *table, int nprob, int ntiles, int64_t D, int max_nb_pass, int groups,
-                                int test_stall, int *err, cudaStream_t s);
+cudaError_t launch_pair_grouped(const TcProblem *table, int nprob, int ntiles, int64_t D, int max_nb_pass, bool two_pass,
+                                int groups, int test_stall, int *err, cudaStream_t s);
 
 // TMEM stages, unpack groups and CTAs per SM of a grouped launch with these sizes.
 cudaError_t tc_launch_shape(int64_t D, int max_nb_pass, const TcRingPlan &plan, int *stages, int *groups,

@@ -241,7 +241,7 @@ bool bf_server::launch(Flight &fl, const std::vector<Request> &reqs, int *ntiles
   if (cudaMemcpyAsync(fl.table_dev, fl.table_host, sizeof(TcProblem) * n, cudaMemcpyHostToDevice, fl.s) !=
       cudaSuccess)
     return false;
-  if (launch_tc_grouped(fl.table_dev, n, static_cast<int>(begin), w.D, w.nb_pass, TcRingPlan{}, fl.err_dev,
+  if (launch_tc_grouped(fl.table_dev, n, static_cast<int>(begin), w.D, w.nb_pass, w.npass == 2, TcRingPlan{}, fl.err_dev,
                         fl.s) != cudaSuccess)
     return false;
   if (cudaMemcpyAsync(fl.err_host, fl.err_dev, sizeof(int), cudaMemcpyDeviceToHost, fl.s) != cudaSuccess)

@@ -1187,10 +1187,10 @@ cudaError_t tc_launch_shape(int64_t D, int max_nb_pass, const TcRingPlan &plan, 
 }
 
 cudaError_t launch_tc_grouped(const TcProblem *table, int nprob, int ntiles, int64_t D, int max_nb_pass,
-                              const TcRingPlan &plan, int *err, cudaStream_t s) {
+                              bool two_pass, const TcRingPlan &plan, int *err, cudaStream_t s) {
   if (tc_pair_launch(max_nb_pass))
-    return launch_pair_grouped(table, nprob, ntiles, D, max_nb_pass, pair_groups(max_nb_pass, plan), g_test_stall, err,
-                               s);
+    return launch_pair_grouped(table, nprob, ntiles, D, max_nb_pass, two_pass, pair_groups(max_nb_pass, plan),
+                               g_test_stall, err, s);
   TcParams p{};
   p.table = table;
   p.nprob = nprob;

@@ -14,8 +14,12 @@
 // Tiles of a cluster are contiguous: beam pass fastest, then time, then
 // frequency (then problem).  W stage ks of a new (problem, frequency, pass) is
 // loaded as soon as the tensor cores finished the last tile that used slot ks.
-// Where W does not fit (deep K), or the next tile is another pass, the slots are
-// an ordinary ring.
+// Where W does not fit (deep K, or more passes than fit) the slots are an ordinary
+// ring.  A problem of two passes (97 to 128 beams) keeps the W of both, and where
+// the tile's K stages all fit in tensor memory (ndishes <= 512 there) the second
+// pass reads the operand that was unpacked for the first, whose E is then neither
+// loaded nor unpacked again: f=64 d=512 b=128, 32768 times, 956 -> 707 us (581 at
+// twice the measured bf16 rate), 128 problems of 8192 times 496 -> 330.
 //
 // Warp roles of each CTA (kEpiW epilogue warps):
 //   epilogue     as in bf_tc.cu
@@ -57,6 +61,8 @@ struct PairParams {
   int nk;                   // K stages per tile
   int ncols;                // widest GEMM N of the launch (a multiple of 32)
   int stages, wslots, raw;  // TMEM stages, W slots, raw E slots
+  int sets;                 // passes whose W (unless streamed) and digit rows stay resident
+  int share;                // nonzero: the passes of a tile share its unpacked operand
   int test_stall;
   int *err;
 };
@@ -103,8 +109,19 @@ struct PairCursor {
     tp = (lt / P->npass) % ntp;
     f = lt / (P->npass * ntp);
   }
-  // the next tile has other W rows
-  __device__ __forceinline__ bool last_of_w() const { return P->npass > 1 || tp + 1 == ntp; }
+  // This is the first (last) of its tiles with these W and digit rows, `n` tiles
+  // after the start (before the end) of the cluster's range: those of up to `sets`
+  // passes stay for a frequency.  They are given back together and only where
+  // tiles follow, so the releases of all slots run through the ring in rounds
+  // (drain_commits), although a range that starts with an odd pass loads that first.
+  __device__ __forceinline__ bool first_of_w(int n, int sets) const { return P->npass > sets || n < P->npass || tp == 0; }
+  __device__ __forceinline__ bool last_of_w(int n, int sets) const {
+    return P->npass > sets || (tp + 1 == ntp && n > P->npass - pass);
+  }
+  // This tile's operand is unpacked for it (and not for the pass before), and
+  // free after it.
+  __device__ __forceinline__ bool first_of_a(bool share, bool range_first) const { return !share || pass == 0 || range_first; }
+  __device__ __forceinline__ bool last_of_a(bool share, bool range_last) const { return !share || pass + 1 == P->npass || range_last; }
   __device__ __forceinline__ void next(const PairParams &p) {
     if (++pass < P->npass) return;
     pass = 0;
@@ -123,6 +140,21 @@ struct PairCursor {
   __device__ __forceinline__ int beams() const { return min(P->nb_pass, (P->B + 7) / 8 * 8 - pass * P->nb_pass); }
   __device__ __forceinline__ int n() const { return (2 * beams() + 31) & ~31; }
 };
+
+// Operands to unpack for tiles first .. end - 1 (first < end).
+template <bool kGrouped>
+__device__ __forceinline__ int operands_of(const PairParams &p, int first, int end) {
+  if (!p.share) return end - first;
+  auto span = [](int a, int b, int np) { return (b - 1) / np - a / np + 1; };  // a < b
+  if constexpr (!kGrouped) return span(first, end, p.one.npass);
+  int n = 0;
+  for (int i = PairCursor<kGrouped>(p, first).idx; i < p.nprob; ++i) {
+    const int t0 = p.table[i].tile_begin, t1 = i + 1 < p.nprob ? p.table[i + 1].tile_begin : p.ntiles;
+    if (t0 >= end) break;
+    n += span(max(first, t0) - t0, min(end, t1) - t0, p.table[i].npass);
+  }
+  return n;
+}
 
 // TMEM column of unpacked stage i: the columns left beside the two accumulators.
 __host__ __device__ inline uint32_t pair_stage_col(uint32_t i, int ncols, int per_half, int cols) {
@@ -222,6 +254,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
   const int64_t ncl = gridDim.x >> 1, cl = blockIdx.x >> 1;
   const int first = static_cast<int>(cl * p.ntiles / ncl), end = static_cast<int>((cl + 1) * p.ntiles / ncl);
   const bool stream_w = SW < nk;  // W slots are an ordinary ring
+  const int sets = p.sets;
+  const bool share = !kSums && p.share != 0;
 
   if (warp == kEProdWarp) {
     // ------------------------------------------------------------ E producer
@@ -233,6 +267,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     const TcProblem *seen = nullptr;
     PairCursor<kGrouped> cur(p, first);
     for (int tile = first; ok && tile < end; ++tile, cur.next(p)) {
+      if (!cur.first_of_a(share, tile == first)) continue;
       if (kGrouped && cur.P != seen) {  // a table entry the host rewrites between launches
         tensormap_acquire(&cur.P->tm_e);
         seen = cur.P;
@@ -260,11 +295,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     const uint64_t pol_w = policy_evict_last();
     Ring wr(SW), dr(kDigSlots);
     uint32_t it = 0, dit = 0;
-    bool ok = !p.test_stall, fresh = true;
+    bool ok = !p.test_stall;
     cluster_arrive();
     const TcProblem *seen = nullptr;
     PairCursor<kGrouped> cur(p, first);
-    for (int tile = first; ok && tile < end; ++tile) {
+    for (int tile = first; ok && tile < end; ++tile, cur.next(p)) {
+      const bool fresh = cur.first_of_w(tile - first, sets);
       if (fresh || stream_w) {
         if (kGrouped && cur.P != seen) {
           tensormap_acquire(&cur.P->tm_w);
@@ -298,8 +334,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
           __syncwarp();
         }
       }
-      fresh = cur.last_of_w();
-      cur.next(p);
     }
     cluster_wait();
     for (uint32_t k = (it >= static_cast<uint32_t>(SW) ? it - SW : 0); k < it; ++k)
@@ -311,9 +345,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     setup_sync();
     if (lane == 0 && !p.test_stall) {
       Ring wr(SW), dr(kDigSlots);
-      bool ok = true, fresh = true;
+      bool ok = true;
       PairCursor<kGrouped> cur(p, first);
-      for (int tile = first; ok && tile < end; ++tile) {
+      for (int tile = first; ok && tile < end; ++tile, cur.next(p)) {
+        const bool fresh = cur.first_of_w(tile - first, sets);
         if (fresh) {
           if (!mbar_wait(d_full(dr.idx), dr.phase, err, kDevTimeoutFull)) break;
           mbar_arrive_cluster(map_cta(d_peer(dr.idx), 0));
@@ -328,8 +363,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
             mbar_arrive_cluster(map_cta(w_peer(wr.idx), 0));
           }
         }
-        fresh = cur.last_of_w();
-        cur.next(p);
       }
     }
     __syncwarp();
@@ -347,18 +380,26 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     const uint32_t w_step = static_cast<uint32_t>(sp.wbytes) >> 4;
     uint32_t local = 0;
     uint32_t nstage = 0, nw = 0, ndig = 0, nacc = 0;  // commits issued on empty, w_empty, d_empty, accfull
-    bool ok = true, fresh = true;
+    bool ok = true;
+    int w_at[2] = {0, 0}, d_at[2] = {0, 0};  // first W slot and digit slot of even and odd passes
+    Ring a0(S);                              // the first stage of the tile's operand
     PairCursor<kGrouped> cur(p, first);
-    for (int tile = first; ok && tile < end; ++tile, ++local) {
+    for (int tile = first; ok && tile < end; ++tile, ++local, cur.next(p)) {
       const uint32_t idesc = idesc_e4m3_f32(2 * kBM, static_cast<uint32_t>(cur.n()));
       const uint32_t wbox = static_cast<uint32_t>(cur.P->w_rows * kKC) >> 4;
-      const bool last = cur.last_of_w();
+      const bool fresh = cur.first_of_w(tile - first, sets), last = cur.last_of_w(end - tile, sets);
+      const bool new_a = cur.first_of_a(share, tile == first), last_a = cur.last_of_a(share, tile + 1 == end);
+      const bool odd = cur.pass & 1;
+      if (new_a) a0 = ar; else ar = a0;
+      if (fresh) (odd ? w_at[1] : w_at[0]) = stream_w ? 0 : static_cast<int>(wr.idx);
+      if (fresh) (odd ? d_at[1] : d_at[0]) = static_cast<int>(dr.idx);
+      const int w0 = odd ? w_at[1] : w_at[0], ds = odd ? d_at[1] : d_at[0];
       const uint32_t ab = local & 1u;
       if (!__all_sync(0xffffffffu, mbar_wait(accempty(ab), ((local >> 1) & 1u) ^ 1u, err, kDevTimeoutAccEmpty))) break;
-      const int ds = static_cast<int>(dr.idx);
       if (fresh && !__all_sync(0xffffffffu, mbar_wait(d_full(ds), dr.phase, err, kDevTimeoutFull) &&
                                                 mbar_wait(d_peer(ds), dr.phase, err, kDevTimeoutFull)))
         break;
+      if (fresh) dr.advance();
       tc_fence_after();
       const uint32_t d_tmem = tmem_base + ab * kPairAcc;
       // the offset MMA: -8 sum_k W[n][k] 2^-18, with the row sums also
@@ -371,10 +412,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
       if (!kSums && elect_one()) offset_mma();
       __syncwarp();
       if (!fresh && !last && !stream_w) {
-        uint64_t b_desc = w_desc0;
+        uint64_t b_desc = w_desc0 + static_cast<uint32_t>(w0) * w_step;
         for (int ks = 0; ks < nk; ++ks, b_desc += w_step) {
           const uint32_t bar = a_full(ar.idx);
-          if (!__all_sync(0xffffffffu, mbar_wait(bar, ar.phase, err, kDevTimeoutUnpacked))) {
+          if (new_a && !__all_sync(0xffffffffu, mbar_wait(bar, ar.phase, err, kDevTimeoutUnpacked))) {
             ok = false;
             break;
           }
@@ -383,10 +424,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
           if (elect_one()) {
             mma_ts_box_pair(d_tmem, a_tmem, b_desc, idesc, !kSums || ks > 0);
             mma_ts_box_pair(d_tmem, a_tmem + 32, b_desc + wbox, idesc, 1u);
-            mma_commit_pair(bar + 8u * S);  // empty
+            if (last_a) mma_commit_pair(bar + 8u * S);  // empty
           }
           __syncwarp();
-          ++nstage;
+          nstage += last_a ? 1u : 0u;
           ar.advance();
         }
       } else {
@@ -394,14 +435,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
         for (int ks = 0; ks < nk; ++ks, ar.advance()) {
           // the parity of a W slot's current load: resident slots (SW == nk) step
           // with the loads, not with the tiles
-          const int sw = stream_w ? static_cast<int>(wr.idx) : ks;
+          const int sw = stream_w ? static_cast<int>(wr.idx) : w0 + ks;
           if (reload && !__all_sync(0xffffffffu, mbar_wait(w_full(sw), wr.phase, err, kDevTimeoutFull) &&
                                                      mbar_wait(w_peer(sw), wr.phase, err, kDevTimeoutFull))) {
             ok = false;
             break;
           }
           const uint32_t bar = a_full(ar.idx);
-          if (!__all_sync(0xffffffffu, mbar_wait(bar, ar.phase, err, kDevTimeoutUnpacked))) {
+          if (new_a && !__all_sync(0xffffffffu, mbar_wait(bar, ar.phase, err, kDevTimeoutUnpacked))) {
             ok = false;
             break;
           }
@@ -411,11 +452,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
           if (elect_one()) {
             mma_ts_box_pair(d_tmem, a_tmem, b_desc, idesc, !kSums || ks > 0);
             mma_ts_box_pair(d_tmem, a_tmem + 32, b_desc + wbox, idesc, 1u);
-            mma_commit_pair(bar + 8u * S);  // empty
+            if (last_a) mma_commit_pair(bar + 8u * S);  // empty
             if (release) mma_commit_pair(w_empty(sw));
           }
           __syncwarp();
-          ++nstage;
+          nstage += last_a ? 1u : 0u;
           nw += release ? 1u : 0u;
           if (reload) wr.advance();
         }
@@ -430,13 +471,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
         mma_commit_pair(accfull(ab));
       }
       __syncwarp();
-      if (last) {
-        ++ndig;
-        dr.advance();
-      }
+      if (last) ++ndig;
       ++nacc;
-      fresh = last;
-      cur.next(p);
     }
     // A commit's arrival is an asynchronous write into both CTAs' shared memory:
     // wait (bounded) for the last phase committed on every barrier before the
@@ -464,7 +500,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     const UnpackRow row(RowMap<kJ2>::time(q, lane));
     const uint32_t sel = RowMap<kJ2>::pol(q, lane) ? 0x7531u : 0x6420u;  // odd or even bytes
     const uint32_t lane_addr = static_cast<uint32_t>(32 * q) << 16;
-    const uint32_t total = static_cast<uint32_t>(end - first) * static_cast<uint32_t>(nk);
+    const int operands = kSums ? end - first : operands_of<kGrouped>(p, first, end);
+    const uint32_t total = static_cast<uint32_t>(operands) * static_cast<uint32_t>(nk);
     Ring rr(R), ar(S);
     for (int g = 0; g < group; ++g) {
       rr.advance();
@@ -565,7 +602,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 }
 
 // Ring depths and shared memory of a launch whose widest GEMM N is ncols.
-cudaError_t plan_pair(PairParams &p, int64_t D, int max_nb_pass, int groups, int *smem_bytes) {
+cudaError_t plan_pair(PairParams &p, int64_t D, int max_nb_pass, bool two_pass, int groups, int *smem_bytes) {
   p.nk = tc_stages_per_tile(D);
   p.ncols = pair_cols(max_nb_pass);
   const int ncols = p.ncols;
@@ -581,6 +618,13 @@ cudaError_t plan_pair(PairParams &p, int64_t D, int max_nb_pass, int groups, int
     wslots = 2;
     while (wslots < p.nk - 1 && total(wslots + 1, 4) <= kPairSmem) ++wslots;
   }
+  // two passes' W where that leaves as much: neither is loaded per tile then
+  // (f=32 d=256 b=192, 16384 times: 191 -> 164 us)
+  if (two_pass && total(2 * p.nk, 4) <= kPairSmem) wslots = 2 * p.nk;
+  p.sets = wslots < p.nk ? kDigSlots : std::min(kDigSlots, wslots / p.nk);
+  // a tile's whole operand fits the TMEM stages: its passes take it in turn
+  // (with row sums, one per tile of the accumulator, they do not)
+  p.share = two_pass && p.nk <= stages && !tc_w_offset(max_nb_pass) ? 1 : 0;
   int raw = 2;
   while (raw < kPairMaxRaw && total(wslots, raw + 1) <= kPairSmem) ++raw;
   raw -= raw % groups;  // a raw slot stays with one unpack group
@@ -653,7 +697,7 @@ int pair_clusters() {
 cudaError_t pair_launch_shape(int64_t D, int max_nb_pass, int groups, int *stages) {
   PairParams p{};
   int smem_bytes = 0;
-  const cudaError_t e = plan_pair(p, D, max_nb_pass, groups, &smem_bytes);
+  const cudaError_t e = plan_pair(p, D, max_nb_pass, false, groups, &smem_bytes);
   *stages = p.stages;
   return e;
 }
@@ -668,13 +712,13 @@ cudaError_t launch_pair(const TcProblem &one, int64_t D, int test_stall, int *er
   p.err = err;
   p.test_stall = test_stall;
   int smem_bytes = 0;
-  const cudaError_t e = plan_pair(p, D, one.nb_pass, 2, &smem_bytes);
+  const cudaError_t e = plan_pair(p, D, one.nb_pass, one.npass == 2, 2, &smem_bytes);
   if (e != cudaSuccess) return e;
   return tc_w_offset(one.nb_pass) ? launch_plain<true>(p, smem_bytes, s) : launch_plain<false>(p, smem_bytes, s);
 }
 
-cudaError_t launch_pair_grouped(const TcProblem *table, int nprob, int ntiles, int64_t D, int max_nb_pass, int groups,
-                                int test_stall, int *err, cudaStream_t s) {
+cudaError_t launch_pair_grouped(const TcProblem *table, int nprob, int ntiles, int64_t D, int max_nb_pass, bool two_pass,
+                                int groups, int test_stall, int *err, cudaStream_t s) {
   PairParams p{};
   p.table = table;
   p.nprob = nprob;
@@ -682,7 +726,7 @@ cudaError_t launch_pair_grouped(const TcProblem *table, int nprob, int ntiles, i
   p.err = err;
   p.test_stall = test_stall;
   int smem_bytes = 0;
-  const cudaError_t e = plan_pair(p, D, max_nb_pass, groups, &smem_bytes);
+  const cudaError_t e = plan_pair(p, D, max_nb_pass, two_pass, groups, &smem_bytes);
   if (e != cudaSuccess) return e;
   if (groups == 1) return launch_inst<true, false, false, 1, true>(p, smem_bytes, s);  // only beside two TMEM stages
   return tc_w_offset(max_nb_pass) ? launch_inst<true, false, false, 2, true>(p, smem_bytes, s)

@@ -22,6 +22,10 @@ SHAPES = [
     (16, 1, 64, 96), (64, 3, 8, 72), (80, 3, 128, 96), (128, 2, 128, 17), (144, 2, 256, 88), (192, 9, 376, 65),
     (272, 1, 384, 64), (208, 2, 512, 41), (1040, 3, 512, 96), (528, 2, 1024, 200), (336, 2, 1024, 96), (272, 1, 2048, 96),
     (144, 1, 2048, 130), (80, 160, 128, 80),
+    # two passes that share the unpacked operand and keep both W (and neighbours
+    # that only keep W, or neither): ranges that start and end between the passes
+    (16, 1, 512, 97), (528, 2, 512, 128), (8208, 3, 512, 128), (80, 160, 256, 112), (272, 50, 8, 104), (400, 77, 384, 120),
+    (528, 20, 256, 192), (528, 20, 520, 128),
 ]
 
 
@@ -74,16 +78,23 @@ def test_pair_extreme_sums(bflib, cuda, oracle, shape, fill):
     np.testing.assert_array_equal(J.cpu().numpy(), _oracle_J(oracle, d, E, A, G))
 
 
+@pytest.mark.parametrize("wide", [True, False])
 @pytest.mark.parametrize("dd", [64, 128, 384, 512, 2048])
-def test_pair_batch_mixes_signed_and_offset_weights(bflib, cuda, oracle, dd):
-    """One launch over problems whose weights are stored in either form."""
+def test_pair_batch_mixes_widths_and_weights(bflib, cuda, oracle, dd, wide):
+    """One launch over problems of one and two passes, without and (wide) with
+    weights of both forms."""
     probs = []
     for i, (t, b) in enumerate([(272, 96), (64, 16), (528, 64), (80, 128), (16, 72), (144, 41)]):
+        if not wide and b in (96, 72):
+            continue
         d = bflib.Dims(t, 1, dd, 2, b)
         E, A, G = _host_inputs(bflib, d, 50 + i)
         W = bflib.ResidentWeights(1, b, dd, A, G)
         J = cuda.full((d.jsize,), 0x5A, dtype=cuda.uint8, device="cuda")
         probs.append((d, (E, A, G), W, cuda.from_numpy(E).cuda(), J))
+        if b == 128:  # more tiles than clusters: ranges start anywhere
+            for k in range(40):
+                probs.append((d, (E, A, G), W, probs[-1][3], cuda.full((d.jsize,), 0x5A, dtype=cuda.uint8, device="cuda")))
     batch = bflib.Batch([(W, d.ntimes, Ed, J) for d, _, W, Ed, J in probs])
     for _ in range(2):
         batch.run()
