@@ -547,7 +547,7 @@ def run_ours(args):
     assert bf.adler32_device(J) == checksum
     W.close()
     alg_bytes = d.esize + d.jsize + d.asize + 4 * d.gsize
-    roofline = roofline_of(bf, stream, d.cmacs, alg_bytes, k_ms, "bf_form_beams_tc")
+    roofline = roofline_of(bf, stream, d.cmacs, alg_bytes, k_ms, "bf_form_beams_pair")
     roofline["traffic"] = profile_traffic()
     # clock-normalised kernel time, comparable across runs whose power-capped
     # SM clock differs: kernel ms x median SM MHz of this run = kilocycles
@@ -953,7 +953,7 @@ def run_batched(args, emit=True):
         "per_problem_launches": {"value": total_cmac / (ms_loop * 1e-3), "ms_per_step": round(ms_loop, 4),
                                  "launches": len(probs)},
         "speedup_vs_per_problem": round(ms_loop / ms_batch, 3),
-        "roofline": roofline_of(bf, stream, total_cmac, alg_bytes, ms_batch, "bf_form_beams_tc (grouped)"),
+        "roofline": roofline_of(bf, stream, total_cmac, alg_bytes, ms_batch, "bf_form_beams_pair (grouped)"),
         "autotune": batch.info(),
         "parity": "every problem's J equals the oracle's (all 128, bytewise) and the per-problem launches' "
                   "(adler32)",
@@ -1301,7 +1301,7 @@ def run_wide(args, emit=True):
     bf.stream_status(stream)
     k_ms = statistics.mean(a.elapsed_time(b) for a, b in evs)
     alg_bytes = d.esize + d.jsize + d.asize + 4 * d.gsize
-    roofline = roofline_of(bf, stream, d.cmacs, alg_bytes, k_ms, "bf_form_beams_tc")
+    roofline = roofline_of(bf, stream, d.cmacs, alg_bytes, k_ms, "bf_form_beams_pair")
     ref.close()
 
     W = bf.ResidentWeights(d.nfrequencies, d.nbeams, d.ndishes, As[0], G, stream=stream)
