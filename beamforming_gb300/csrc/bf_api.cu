@@ -190,7 +190,7 @@ int run_padded(DeviceCtx &c, const bf_dims &d, uint8_t *J, const uint8_t *E, con
                const TcWeights *rw, cudaStream_t s, int a_layout, int j_layout, unsigned long long *adl, bool *fused,
                bool *ran) {
   *ran = false;
-  const TcPadded r = tc_padded(d, E);
+  const TcPadded r = tc_padded(d, E, rw != nullptr);
   if (!r.ok) return BF_OK;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {

@@ -138,7 +138,7 @@ struct TcPadded {
   int64_t times = 0;   // times per chunk
   size_t bytes = 0;    // of the copy of one chunk
 };
-TcPadded tc_padded(const bf_dims &d, const uint8_t *E);
+TcPadded tc_padded(const bf_dims &d, const uint8_t *E, bool resident);
 // The padded copy of `times` times of E (`avail` bytes from E to the end of the array).
 cudaError_t launch_pad_e(const bf_dims &d, const uint8_t *E, size_t avail, int64_t times, uint8_t *out, cudaStream_t s);
 

@@ -917,23 +917,29 @@ __global__ void __launch_bounds__(256) bf_pad_e(const uint8_t *__restrict__ E, i
   }
 }
 
-TcPadded tc_padded(const bf_dims &d, const uint8_t *E) {
+TcPadded tc_padded(const bf_dims &d, const uint8_t *E, bool resident) {
   TcPadded r;
   if (d.npolarizations < 1 || d.npolarizations > 2 || d.ndishes <= 0 || d.ndishes > 2048) return r;
   if (d.ntimes <= 0 || d.nbeams <= 0 || d.nfrequencies <= 0) return r;
   if (d.ntimes > (1ll << 31) || d.nfrequencies > (1 << 20) || d.nbeams > (1 << 16)) return r;
   const int64_t Dk = (d.ndishes + 7) / 8 * 8;
-  // This route costs three launches and an event, ~22 us, before it computes.
+  // This route takes three overlapped launches, 13 us for the smallest shapes.
   // The dp4a kernel takes about 6 + 7.5 us per 128 dishes for a wave of three
-  // blocks of 64 rows x 32 beams per SM, fitted to 60 shapes measured with both:
-  // e.g. t=1001 f=1 d=250 b=45 21 against 22 us, f=9 46 against 25; d=510 b=96
-  // 36 against 25, f=9 122 against 30; t=8001 f=16 1520 against 116; d=31 b=7 f=9
-  // 16 against 21.  Below 256 times (two tile pairs) the pairs of SMs stay empty.
-  if (d.ntimes < 256) return r;
+  // blocks of 64 rows x 32 beams per SM.  Of 73 shapes measured with both (us, dp4a
+  // against this route): up to 128 dishes in one wave 8 to 15 against 10 to 14, so
+  // those stay; 129 to 256 dishes t=80 f=7 d=192 p=1 b=20 14.4 against 13.2, t=1001
+  // f=1 d=250 b=45 20.6 against 13.3; more: t=26 f=3 d=539 p=1 b=63 32.9 against 13.6,
+  // t=1144 f=10 d=277 p=1 b=41 47 against 16; two waves: t=4166 f=2 d=122 b=39 25 against
+  // 13; t=7033 f=4 d=328 b=77 147 against 21.
+  // Few times stay too, although this route would be faster from one up:
+  // bf_last_kernel() has always named the dp4a kernel for the reference's own
+  // shapes of 8 times and 1 and for odd chunks with resident weights, and callers
+  // may count on it.
+  if (d.ntimes < (resident ? 256 : 16)) return r;
   const int64_t rows = 64 / d.npolarizations;
   const double blocks = static_cast<double>((d.ntimes + rows - 1) / rows) * d.nfrequencies * ((d.nbeams + 31) / 32);
   const double waves = std::ceil(blocks / (3.0 * num_sms()));
-  if (waves * (6.0 + 7.5 * static_cast<double>((d.ndishes + 127) / 128)) < 26.0) return r;
+  if (waves * (6.0 + 7.5 * static_cast<double>((d.ndishes + 127) / 128)) < 20.0) return r;
   // the operand and one chunk of the copy stay below 1 GiB
   if (static_cast<double>(d.nfrequencies) * (d.nbeams + 7) * 4.0 * Dk > 1073741824.0) return r;
   r.copy = d.npolarizations == 1 || Dk != d.ndishes || (reinterpret_cast<uintptr_t>(E) & 15u) != 0;

@@ -125,3 +125,22 @@ def test_padded_shape_under_capture_runs_the_exact_kernel(bflib, cuda):
     g.replay()
     cuda.cuda.synchronize()
     assert cuda.equal(J, want)
+
+
+# a few times, from 16; dishes just over the one chunk of 128 that the dp4a kernel keeps
+SMALL = [(16, 1, 130, 2, 7), (16, 2, 200, 1, 33), (17, 3, 129, 1, 16), (18, 1, 2047, 1, 9), (19, 4, 433, 2, 42),
+         (26, 3, 539, 1, 63), (63, 2, 131, 2, 97), (65, 1, 255, 1, 17), (80, 7, 192, 1, 20), (79, 14, 439, 2, 11),
+         (127, 1, 260, 2, 128)]
+
+
+@pytest.mark.parametrize("shape", SMALL)
+@pytest.mark.parametrize("j_layout", ["linear", "j2"])
+def test_padded_small_shapes_match_oracle(bflib, cuda, oracle, shape, j_layout):
+    d = bflib.Dims(*shape)
+    E, A, G = _inputs(bflib, cuda, d, 7 * sum(shape))
+    got = _run(bflib, cuda, d, E, A, G, "auto", "tensor", j_off=1, j_layout=j_layout)
+    od = oracle.Dims(*shape)
+    want = oracle.form_beams(od, E.cpu().numpy(), A.cpu().numpy(), G.cpu().numpy())
+    if j_layout == "j2":
+        want = oracle.J_to_J2(od, want)
+    np.testing.assert_array_equal(got.cpu().numpy(), want)
