@@ -217,15 +217,13 @@ int run_padded(DeviceCtx &c, const bf_dims &d, uint8_t *J, const uint8_t *E, con
   t_last_kernel = "tensor";
   c.pad_used = true;
   const int st = [&]() -> int {
-    if (adl) {
-      BF_TRY(cudaMemsetAsync(adl, 0, 2 * sizeof(unsigned long long), s));
-      if (fused) *fused = true;
-    }
+    if (adl && rw) BF_TRY(cudaMemsetAsync(adl, 0, 2 * sizeof(unsigned long long), s));
+    if (adl && fused) *fused = true;
     if (!rw) {
       w.W = c.padW.as<uint8_t>();
       tc_set_extra(w, c.padDig.as<uint8_t>());
       w.G = G;
-      BF_TRY(launch_prep_weights(w, A, s, a_layout));
+      BF_TRY(launch_prep_weights(w, A, s, a_layout, adl));
     }
     const int64_t P = d.npolarizations, per_t = d.nfrequencies * d.ndishes * P;
     for (int64_t t0 = 0; t0 < d.ntimes; t0 += r.times) {
@@ -290,11 +288,8 @@ int run_device_bufs(const bf_dims &d, uint8_t *J, const uint8_t *E, const uint8_
   w.W = Wb.as<uint8_t>();
   tc_set_extra(w, digb.as<uint8_t>());
   w.G = G;
-  if (adl) {  // before the preparation, whose end the main kernel's launch overlaps
-    BF_TRY(cudaMemsetAsync(adl, 0, 2 * sizeof(unsigned long long), s));
-    if (fused) *fused = true;
-  }
-  BF_TRY(launch_prep_weights(w, A, s, a_layout));
+  if (adl && fused) *fused = true;
+  BF_TRY(launch_prep_weights(w, A, s, a_layout, adl));
   t_last_kernel = "tensor";
   return to_status(launch_tc(w, d.ntimes, J, E, err, s, 0, j_layout, adl, J));
 }
@@ -410,11 +405,9 @@ int run_host_pipelined(DeviceCtx &c, const bf_dims &d, uint8_t *J, const uint8_t
     w.W = c.W.as<uint8_t>();
     tc_set_extra(w, c.dig.as<uint8_t>());
     w.G = c.G.as<float>();
-    BF_TRY(launch_prep_weights(w, c.A.as<uint8_t>(), l0.s, a_layout));
-    if (adl) {  // every chunk's launch adds into the same sums, positions from the start of J
-      BF_TRY(cudaMemsetAsync(adl, 0, 2 * sizeof(unsigned long long), l0.s));
-      if (fused) *fused = true;
-    }
+    // every chunk's launch adds into the same sums, positions from the start of J
+    BF_TRY(launch_prep_weights(w, c.A.as<uint8_t>(), l0.s, a_layout, adl));
+    if (adl && fused) *fused = true;
   }
   BF_TRY(cudaEventRecord(l0.done, l0.s));
   for (int i = 1; i < kLanes; ++i) BF_TRY(cudaStreamWaitEvent(c.lanes[i].s, l0.done, 0));

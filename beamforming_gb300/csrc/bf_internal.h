@@ -147,8 +147,10 @@ cudaError_t launch_pad_e(const bf_dims &d, const uint8_t *E, size_t avail, int64
 // are five passes of 96 and one of 32 instead of six of 88, each padded to 96.
 void tc_plan_beams(int64_t B, int *nb_pass, int *npass, int granule = 16);
 
-// Fills w.W, w.dig and w.gs from device A and w.G (w's sizes and buffers already set).
-cudaError_t launch_prep_weights(const TcWeights &w, const uint8_t *A, cudaStream_t s, int a_layout = kALinear);
+// Fills w.W, w.dig and w.gs from device A and w.G (w's sizes and buffers already set),
+// and zeroes the two adler32 sums of the launch that follows, if any.
+cudaError_t launch_prep_weights(const TcWeights &w, const uint8_t *A, cudaStream_t s, int a_layout = kALinear,
+                                unsigned long long *adler = nullptr);
 
 // Beamforms T times of device E into device J with prepared weights.  `err`
 // is a device int that receives a nonzero DeviceError on an expired wait.

@@ -687,9 +687,11 @@ __global__ void __launch_bounds__(32 * kPrepBeams) bf_prep_weights(const uint8_t
                                                                     uint8_t *__restrict__ dig,
                                                                     const float *__restrict__ G, float *__restrict__ gs,
                                                                     int *__restrict__ gwide, int B, int D, int Dk,
-                                                                    int nw, int nw_pad, int a_layout) {
+                                                                    int nw, int nw_pad, int a_layout,
+                                                                    unsigned long long *adler) {
   grid_launch_next();
   grid_wait();
+  if (adler && blockIdx.x == 0 && threadIdx.x < 2) adler[threadIdx.x] = 0;
   const int beams = nw_pad / 2;
   const int fblocks = (beams + kPrepBeams - 1) / kPrepBeams;  // blocks per frequency
   const int f = static_cast<int>(blockIdx.x) / fblocks;
@@ -964,13 +966,14 @@ cudaError_t launch_pad_e(const bf_dims &d, const uint8_t *E, size_t avail, int64
                            d.nfrequencies, d.ndishes, Dk, static_cast<int>(d.npolarizations));
 }
 
-cudaError_t launch_prep_weights(const TcWeights &w, const uint8_t *A, cudaStream_t s, int a_layout) {
+cudaError_t launch_prep_weights(const TcWeights &w, const uint8_t *A, cudaStream_t s, int a_layout,
+                                unsigned long long *adler) {
   const int64_t blocks = static_cast<int64_t>((w.nw_pad / 2 + kPrepBeams - 1) / kPrepBeams) * w.F;
   if (blocks > 0x7FFFFFFF) return cudaErrorInvalidValue;
   auto kern = tc_w_offset(w.nb_pass) ? bf_prep_weights<true> : bf_prep_weights<false>;
   return launch_overlapped(kern, static_cast<unsigned>(blocks), 32 * kPrepBeams, 0, s, A, w.W, w.dig, w.G,
                            w.gs, w.gwide, static_cast<int>(w.B), static_cast<int>(w.D), static_cast<int>(w.Dk), w.nw,
-                           w.nw_pad, a_layout);
+                           w.nw_pad, a_layout, adler);
 }
 
 // Rows that start or end between words are stored byte by byte.
