@@ -8,6 +8,7 @@
 // to a and b.  A first kernel reduces every 64 KiB chunk to (S1, sum (i-s) x_i)
 // mod 65521; a one-block kernel combines them.
 #include "bf_internal.h"
+#include "bf_ptx.cuh"
 
 #include <algorithm>
 
@@ -124,6 +125,15 @@ __global__ void fill_random_kernel(uint8_t *__restrict__ dst, size_t n, uint64_t
   }
 }
 
+// Up to 32 words to pinned host memory, behind the kernels before it.  It is
+// resident by the time they end (a launch that overlaps them), where a copy of the
+// same bytes starts only then: the smallest checked call 33.6 -> 28.0 us, t=8192 f=16
+// d=256 b=64 46.9 -> 45.3.
+__global__ void __launch_bounds__(32) write_words(const uint32_t *__restrict__ src, uint32_t *__restrict__ dst, int n) {
+  grid_wait();
+  if (static_cast<int>(threadIdx.x) < n) dst[threadIdx.x] = src[threadIdx.x];
+}
+
 }  // namespace
 
 int adler_nchunks(size_t len) { return static_cast<int>((len + kChunk - 1) / kChunk); }
@@ -171,6 +181,10 @@ uint32_t adler32_host(const uint8_t *p, size_t n) {
     b %= kAdlerMod;
   }
   return (b << 16) | a;
+}
+
+cudaError_t launch_write_words(const void *src, void *pinned, int n, cudaStream_t s) {
+  return launch_overlapped(write_words, 1u, 32u, 0, s, static_cast<const uint32_t *>(src), static_cast<uint32_t *>(pinned), n);
 }
 
 }  // namespace bf

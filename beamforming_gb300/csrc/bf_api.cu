@@ -295,10 +295,16 @@ int run_device_bufs(const bf_dims &d, uint8_t *J, const uint8_t *E, const uint8_
 }
 
 // Waits for the stream and reads the device results; a kernel's error clears the
-// error word and is the status.
-int read_and_clear_err(DeviceCtx &c, cudaStream_t s, DevResult *out = nullptr) {
+// error word and is the status.  `behind_kernel`: the stream's last work is a
+// kernel, and another one writes the results faster than a copy; behind a copy a
+// copy is faster (host call 294 against 296 us).
+int read_and_clear_err(DeviceCtx &c, cudaStream_t s, DevResult *out = nullptr, bool behind_kernel = false) {
   DevResult *h = t_result.get();
-  BF_TRY(cudaMemcpyAsync(h, c.err, sizeof(DevResult), cudaMemcpyDeviceToHost, s));
+  static_assert(sizeof(DevResult) % 4 == 0 && sizeof(DevResult) <= 128, "words of one warp");
+  if (behind_kernel && h == t_result.p)
+    BF_TRY(launch_write_words(c.err, h, sizeof(DevResult) / 4, s));
+  else
+    BF_TRY(cudaMemcpyAsync(h, c.err, sizeof(DevResult), cudaMemcpyDeviceToHost, s));
   BF_TRY(cudaStreamSynchronize(s));
   if (out) *out = *h;
   if (h->err != 0) {
@@ -531,14 +537,15 @@ namespace {
 // Ends a checked call: the adler32 of the n bytes of device J, from the fused
 // sums when the tensor-core kernel ran, else by the separate two-kernel pass, and
 // the call's status.  Synchronises the stream.
-int finish_adler(DeviceCtx &c, bool fused, const uint8_t *Jdev, size_t n, cudaStream_t s, uint32_t *out) {
+int finish_adler(DeviceCtx &c, bool fused, const uint8_t *Jdev, size_t n, cudaStream_t s, uint32_t *out,
+                 bool behind_kernel = false) {
   if (!fused) {
     BF_TRY(c.partials.reserve(static_cast<size_t>(adler_nchunks(n)) * 2 * sizeof(uint32_t)));
     BF_TRY(launch_adler_partials(Jdev, n, c.partials.as<uint32_t>(), s));
     BF_TRY(launch_adler_combine(c.partials.as<uint32_t>(), n, c.adler, s));
   }
   DevResult r{};
-  const int st = read_and_clear_err(c, s, &r);
+  const int st = read_and_clear_err(c, s, &r, behind_kernel || !fused);
   if (st == BF_OK) *out = fused ? adler_finish(r.adl[0], r.adl[1], n) : r.adler;
   return st;
 }
@@ -579,7 +586,7 @@ static int form_beams_impl(const bf_dims *dims, uint8_t *J, const uint8_t *E, co
   if (ptr_kind == BF_PTR_DEVICE) {
     st = run_device(*c, d, J, E, A, G, s, a_layout, j_layout, adl, &fused);
     if (st != BF_OK || !adler_out) return st;
-    return finish_adler(*c, fused, J, jsize(d), s, adler_out);
+    return finish_adler(*c, fused, J, jsize(d), s, adler_out, true);
   }
 
   // Host pointers: stage in, compute, stage out, synchronously (cuda.cu:274-314 does the same around its

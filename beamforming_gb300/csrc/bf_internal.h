@@ -277,6 +277,8 @@ void tc_set_ring_plan(int wslots, int raw);
 int adler_nchunks(size_t len);
 cudaError_t launch_adler_partials(const uint8_t *data, size_t len, uint32_t *partials, cudaStream_t s);
 // Combines the partials into one adler32 value in *out (device).
+// n (at most 32) words of device memory into pinned host memory.
+cudaError_t launch_write_words(const void *src, void *pinned, int n, cudaStream_t s);
 cudaError_t launch_adler_combine(const uint32_t *partials, size_t len, uint32_t *out, cudaStream_t s);
 // adler32 of n bytes of host memory (adler32.c:7-20).
 uint32_t adler32_host(const uint8_t *p, size_t n);
