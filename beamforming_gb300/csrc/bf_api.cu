@@ -671,12 +671,46 @@ int bf_weights_create(bf_weights **out, int64_t nfrequencies, int64_t nbeams, in
   return BF_OK;
 }
 
+// Whether all n bytes at p lie in one allocation of this device: what a copy from
+// there would check.
+static bool on_device(const void *p, size_t n, int device) {
+  using Fn = CUresult (*)(unsigned int, CUpointer_attribute *, void **, CUdeviceptr);
+  static const Fn fn = []() -> Fn {
+    void *q = nullptr;
+    cudaDriverEntryPointQueryResult r{};
+    if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &q, 12000, cudaEnableDefault, &r) != cudaSuccess ||
+        r != cudaDriverEntryPointSuccess)
+      return nullptr;
+    return reinterpret_cast<Fn>(q);
+  }();
+  unsigned type = 0;
+  int ordinal = -1;
+  CUdeviceptr start = 0;
+  size_t size = 0;
+  CUpointer_attribute at[4] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL,
+                               CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+  void *out[4] = {&type, &ordinal, &start, &size};
+  const CUdeviceptr at0 = reinterpret_cast<CUdeviceptr>(p);
+  if (!fn || fn(4, at, out, at0) != CUDA_SUCCESS) return false;
+  return type == CU_MEMORYTYPE_DEVICE && ordinal == device && at0 >= start && n <= size && at0 - start <= size - n;
+}
+
 int bf_weights_update(bf_weights *w, const uint8_t *A, const float *G, int ptr_kind, bf_stream_t stream) {
   if (!w || !A || !G) return BF_ERR_INVALID_ARGUMENT;
   if (ptr_kind != BF_PTR_HOST && ptr_kind != BF_PTR_DEVICE) return BF_ERR_INVALID_ARGUMENT;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const size_t na = static_cast<size_t>(w->tc.F) * w->tc.B * w->tc.D;
   const size_t ng = static_cast<size_t>(w->tc.F) * w->tc.B;
+  // The preparation reads every byte of A and G once: it writes the copies on the
+  // way where it can read them in place, instead of two device copies in front of
+  // it (update and pass, t=80 f=1 d=416 b=19 15.0 -> 10.8 us, t=1024 f=16 d=1024 b=512
+  // 75.1 -> 67.9).
+  if (ptr_kind == BF_PTR_DEVICE && (reinterpret_cast<uintptr_t>(G) & 3u) == 0 && on_device(A, na, w->device) &&
+      on_device(G, ng * sizeof(float), w->device)) {
+    TcWeights t = w->tc;
+    t.G = G;
+    return to_status(launch_prep_weights(t, A, s, kALinear, nullptr, w->A, w->G));
+  }
   const cudaMemcpyKind k = ptr_kind == BF_PTR_HOST ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice;
   BF_TRY(cudaMemcpyAsync(w->A, A, na, k, s));
   BF_TRY(cudaMemcpyAsync(w->G, G, ng * sizeof(float), k, s));

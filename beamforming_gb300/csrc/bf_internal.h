@@ -148,9 +148,11 @@ cudaError_t launch_pad_e(const bf_dims &d, const uint8_t *E, size_t avail, int64
 void tc_plan_beams(int64_t B, int *nb_pass, int *npass, int granule = 16);
 
 // Fills w.W, w.dig and w.gs from device A and w.G (w's sizes and buffers already set),
-// and zeroes the two adler32 sums of the launch that follows, if any.
+// and zeroes the two adler32 sums of the launch that follows, if any.  A_copy and
+// G_copy, if given, receive A (of the linear layout) and w.G as they are read.
 cudaError_t launch_prep_weights(const TcWeights &w, const uint8_t *A, cudaStream_t s, int a_layout = kALinear,
-                                unsigned long long *adler = nullptr);
+                                unsigned long long *adler = nullptr, uint8_t *A_copy = nullptr,
+                                float *G_copy = nullptr);
 
 // Beamforms T times of device E into device J with prepared weights.  `err`
 // is a device int that receives a nonzero DeviceError on an expired wait.

@@ -688,7 +688,9 @@ __global__ void __launch_bounds__(32 * kPrepBeams) bf_prep_weights(const uint8_t
                                                                     const float *__restrict__ G, float *__restrict__ gs,
                                                                     int *__restrict__ gwide, int B, int D, int Dk,
                                                                     int nw, int nw_pad, int a_layout,
-                                                                    unsigned long long *adler) {
+                                                                    unsigned long long *adler,
+                                                                    uint8_t *__restrict__ A_copy,
+                                                                    float *__restrict__ G_copy) {
   grid_launch_next();
   grid_wait();
   if (adler && blockIdx.x == 0 && threadIdx.x < 2) adler[threadIdx.x] = 0;
@@ -705,6 +707,7 @@ __global__ void __launch_bounds__(32 * kPrepBeams) bf_prep_weights(const uint8_t
     int wide = 0;
     for (int i = threadIdx.x; i < beams; i += blockDim.x) {
       const float g = i < B ? G[static_cast<int64_t>(f) * B + i] : 0.0f;
+      if (G_copy && i < B) G_copy[static_cast<int64_t>(f) * B + i] = g;
       gs[static_cast<int64_t>(f) * beams + i] = 262144.0f * g;
       wide |= !(fabsf(g) < wide_at);
     }
@@ -724,6 +727,7 @@ __global__ void __launch_bounds__(32 * kPrepBeams) bf_prep_weights(const uint8_t
       if (vec) {
         const uint4 q = __ldg(reinterpret_cast<const uint4 *>(row) + i);
         w[0] = q.x, w[1] = q.y, w[2] = q.z, w[3] = q.w;
+        if (A_copy) reinterpret_cast<uint4 *>(A_copy + (static_cast<int64_t>(f) * B + b) * D)[i] = q;
       } else {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -733,7 +737,10 @@ __global__ void __launch_bounds__(32 * kPrepBeams) bf_prep_weights(const uint8_t
             const int d = 16 * i + 4 * j + k;
             int re = 0, im = 0;
             if (b < B && d < D) load_a(A, a_layout, f, b, d, B, D, re, im);
-            w[j] |= static_cast<uint32_t>(((re + 8) << 4) | (im + 8)) << (8 * k);
+            const uint32_t byte = static_cast<uint32_t>(((re + 8) << 4) | (im + 8));  // as stored
+            w[j] |= byte << (8 * k);
+            if (A_copy && b < B && d < D)
+              A_copy[(static_cast<int64_t>(f) * B + b) * D + d] = static_cast<uint8_t>(byte);
           }
         }
       }
@@ -967,13 +974,13 @@ cudaError_t launch_pad_e(const bf_dims &d, const uint8_t *E, size_t avail, int64
 }
 
 cudaError_t launch_prep_weights(const TcWeights &w, const uint8_t *A, cudaStream_t s, int a_layout,
-                                unsigned long long *adler) {
+                                unsigned long long *adler, uint8_t *A_copy, float *G_copy) {
   const int64_t blocks = static_cast<int64_t>((w.nw_pad / 2 + kPrepBeams - 1) / kPrepBeams) * w.F;
   if (blocks > 0x7FFFFFFF) return cudaErrorInvalidValue;
   auto kern = tc_w_offset(w.nb_pass) ? bf_prep_weights<true> : bf_prep_weights<false>;
   return launch_overlapped(kern, static_cast<unsigned>(blocks), 32 * kPrepBeams, 0, s, A, w.W, w.dig, w.G,
                            w.gs, w.gwide, static_cast<int>(w.B), static_cast<int>(w.D), static_cast<int>(w.Dk), w.nw,
-                           w.nw_pad, a_layout, adler);
+                           w.nw_pad, a_layout, adler, A_copy, G_copy);
 }
 
 // Rows that start or end between words are stored byte by byte.
