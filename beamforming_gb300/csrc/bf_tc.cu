@@ -681,7 +681,7 @@ __device__ __forceinline__ uint32_t w_negate(uint32_t codes) {  // zero stays ze
 // (f=16 b=96 d=512: 9.1 and 4.5 us, launch included).
 constexpr int kPrepBeams = 8;  // beams per 256-thread block
 
-template <bool kOffset>
+template <bool kOffset, bool kCopy>
 __global__ void __launch_bounds__(32 * kPrepBeams) bf_prep_weights(const uint8_t *__restrict__ A,
                                                                     uint8_t *__restrict__ W,
                                                                     uint8_t *__restrict__ dig,
@@ -707,7 +707,7 @@ __global__ void __launch_bounds__(32 * kPrepBeams) bf_prep_weights(const uint8_t
     int wide = 0;
     for (int i = threadIdx.x; i < beams; i += blockDim.x) {
       const float g = i < B ? G[static_cast<int64_t>(f) * B + i] : 0.0f;
-      if (G_copy && i < B) G_copy[static_cast<int64_t>(f) * B + i] = g;
+      if (kCopy && G_copy && i < B) G_copy[static_cast<int64_t>(f) * B + i] = g;
       gs[static_cast<int64_t>(f) * beams + i] = 262144.0f * g;
       wide |= !(fabsf(g) < wide_at);
     }
@@ -727,7 +727,7 @@ __global__ void __launch_bounds__(32 * kPrepBeams) bf_prep_weights(const uint8_t
       if (vec) {
         const uint4 q = __ldg(reinterpret_cast<const uint4 *>(row) + i);
         w[0] = q.x, w[1] = q.y, w[2] = q.z, w[3] = q.w;
-        if (A_copy) reinterpret_cast<uint4 *>(A_copy + (static_cast<int64_t>(f) * B + b) * D)[i] = q;
+        if (kCopy && A_copy) reinterpret_cast<uint4 *>(A_copy + (static_cast<int64_t>(f) * B + b) * D)[i] = q;
       } else {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -739,7 +739,7 @@ __global__ void __launch_bounds__(32 * kPrepBeams) bf_prep_weights(const uint8_t
             if (b < B && d < D) load_a(A, a_layout, f, b, d, B, D, re, im);
             const uint32_t byte = static_cast<uint32_t>(((re + 8) << 4) | (im + 8));  // as stored
             w[j] |= byte << (8 * k);
-            if (A_copy && b < B && d < D)
+            if (kCopy && A_copy && b < B && d < D)
               A_copy[(static_cast<int64_t>(f) * B + b) * D + d] = static_cast<uint8_t>(byte);
           }
         }
@@ -977,7 +977,11 @@ cudaError_t launch_prep_weights(const TcWeights &w, const uint8_t *A, cudaStream
                                 unsigned long long *adler, uint8_t *A_copy, float *G_copy) {
   const int64_t blocks = static_cast<int64_t>((w.nw_pad / 2 + kPrepBeams - 1) / kPrepBeams) * w.F;
   if (blocks > 0x7FFFFFFF) return cudaErrorInvalidValue;
-  auto kern = tc_w_offset(w.nb_pass) ? bf_prep_weights<true> : bf_prep_weights<false>;
+  // Signed codes: without the copies' code where none are asked for (t=2001 f=9 d=250
+  // b=45 19.9 against 20.4 us).  W + 8 is no slower with it (b=96 20.2 against 20.7).
+  auto kern = tc_w_offset(w.nb_pass) ? bf_prep_weights<true, true>
+              : A_copy               ? bf_prep_weights<false, true>
+                                     : bf_prep_weights<false, false>;
   return launch_overlapped(kern, static_cast<unsigned>(blocks), 32 * kPrepBeams, 0, s, A, w.W, w.dig, w.G,
                            w.gs, w.gwide, static_cast<int>(w.B), static_cast<int>(w.D), static_cast<int>(w.Dk), w.nw,
                            w.nw_pad, a_layout, adler, A_copy, G_copy);
