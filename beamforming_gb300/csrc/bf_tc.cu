@@ -290,6 +290,7 @@ __global__ void __launch_bounds__(Roles<kEpiW, kGroups>::kThreads, kHalf ? 2 : 1
   }
   static_assert(2 * kMaxStages <= 32, "one lane per stage barrier");
   fence_barrier_init();
+  __syncwarp();  // a producer's lane 0 uses barriers that its other lanes set up, and waits for no other warp
   if (warp == kMmaWarp) {
     tmem_alloc(smem_u32(tmem_holder), 2 * kAcc);
     tmem_relinquish();

@@ -223,6 +223,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     if (lane < 4) counts[lane] = 0;
   }
   fence_barrier_init();
+  __syncwarp();  // a producer's lane 0 uses barriers that its other lanes set up, and waits for no other warp
   if (warp == kMmaWarp) {
     tmem_alloc_pair(smem_u32(tmem_holder), 512);
     tmem_relinquish_pair();

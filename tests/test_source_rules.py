@@ -1,0 +1,42 @@
+"""Rules of the kernels' sources that no run can show to be broken: what they
+guard against needs a schedule, or a state of the caches, that a test cannot ask for."""
+from __future__ import annotations
+
+import os
+import re
+
+import pytest
+
+from conftest import ROOT
+
+CSRC = os.path.join(ROOT, "beamforming_gb300", "csrc")
+
+
+def _source(name):
+    """The file without its comments."""
+    with open(os.path.join(CSRC, name)) as f:
+        text = f.read()
+    return re.sub(r"//[^\n]*|/\*.*?\*/", "", text, flags=re.S)
+
+
+def _body(text, name):
+    """The body of kernel `name`."""
+    at = re.search(r"\b%s\s*\([^;{]*\)\s*\{" % name, text)
+    assert at, name
+    depth, i = 1, at.end()
+    while depth:
+        depth += {"{": 1, "}": -1}.get(text[i], 0)
+        i += 1
+    return text[at.end():i]
+
+
+@pytest.mark.parametrize("name,kernel", [("bf_tc.cu", "bf_form_beams_tc"), ("bf_tc_pair.cu", "bf_form_beams_pair")])
+def test_barriers_are_set_up_before_their_warp_uses_them(name, kernel):
+    """The lanes of a producer warp initialise its barriers together and lane 0
+    goes on without waiting for another warp, so the warp meets in between."""
+    body = _body(_source(name), kernel)
+    inits = [m.end() for m in re.finditer(r"\bmbar_init\(", body)]
+    fence = body.index("fence_barrier_init();")
+    used = min(body.index(x) for x in ("cluster_arrive();", "cta_arrive(") if x in body)
+    assert inits and max(inits) < fence < used
+    assert "__syncwarp();" in body[fence:used]
