@@ -181,7 +181,9 @@ __device__ __forceinline__ void cluster_sync() {
 // ---------------------------------------------------------------- launches
 // A launch with programmatic serialization (launch_overlapped) starts while the
 // kernel before it on the stream ends: it sets itself up, then waits here until
-// that kernel and its memory are complete.
+// that kernel and its memory are complete.  What an earlier kernel writes is then
+// not constant for the life of this grid, which the read-only path (__ldg, const
+// __restrict__) asks for: kernels that wait here use plain loads.
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Lets the next such launch start once every CTA of this grid has come here.
 __device__ __forceinline__ void grid_launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -683,10 +683,10 @@ __device__ __forceinline__ uint32_t w_negate(uint32_t codes) {  // zero stays ze
 constexpr int kPrepBeams = 8;  // beams per 256-thread block
 
 template <bool kOffset, bool kCopy>
-__global__ void __launch_bounds__(32 * kPrepBeams) bf_prep_weights(const uint8_t *__restrict__ A,
+__global__ void __launch_bounds__(32 * kPrepBeams) bf_prep_weights(const uint8_t *A,
                                                                     uint8_t *__restrict__ W,
                                                                     uint8_t *__restrict__ dig,
-                                                                    const float *__restrict__ G, float *__restrict__ gs,
+                                                                    const float *G, float *__restrict__ gs,
                                                                     int *__restrict__ gwide, int B, int D, int Dk,
                                                                     int nw, int nw_pad, int a_layout,
                                                                     unsigned long long *adler,
@@ -726,7 +726,7 @@ __global__ void __launch_bounds__(32 * kPrepBeams) bf_prep_weights(const uint8_t
     for (int i = lane; i < (Dk + 15) / 16; i += 32) {  // dishes 16 i .. 16 i + 15
       uint32_t w[4];
       if (vec) {
-        const uint4 q = __ldg(reinterpret_cast<const uint4 *>(row) + i);
+        const uint4 q = reinterpret_cast<const uint4 *>(row)[i];
         w[0] = q.x, w[1] = q.y, w[2] = q.z, w[3] = q.w;
         if (kCopy && A_copy) reinterpret_cast<uint4 *>(A_copy + (static_cast<int64_t>(f) * B + b) * D)[i] = q;
       } else {
@@ -868,7 +868,7 @@ bool tc_supported(const bf_dims &d) {
 
 // 16 bytes of E from byte `off`, `valid` of them (the rest 0).  Unaligned words
 // where all of them lie inside the array, else byte by byte.
-__device__ __forceinline__ uint4 load16_any(const uint8_t *__restrict__ E, int64_t off, int valid, int64_t avail) {
+__device__ __forceinline__ uint4 load16_any(const uint8_t *E, int64_t off, int valid, int64_t avail) {
   uint32_t w[4];
   if (valid >= 16 && off >= 4 && off + 20 <= avail) {
     const uintptr_t at = reinterpret_cast<uintptr_t>(E + off);
@@ -876,7 +876,7 @@ __device__ __forceinline__ uint4 load16_any(const uint8_t *__restrict__ E, int64
     const uint32_t sh = 8u * static_cast<uint32_t>(at & 3u);
     uint32_t v[5];
 #pragma unroll
-    for (int i = 0; i < 5; ++i) v[i] = __ldg(p + i);
+    for (int i = 0; i < 5; ++i) v[i] = p[i];
 #pragma unroll
     for (int i = 0; i < 4; ++i) w[i] = __funnelshift_r(v[i], v[i + 1], sh);
   } else {
@@ -885,7 +885,7 @@ __device__ __forceinline__ uint4 load16_any(const uint8_t *__restrict__ E, int64
       w[i] = 0;
 #pragma unroll
       for (int k = 0; k < 4; ++k)
-        if (4 * i + k < valid) w[i] |= static_cast<uint32_t>(__ldg(E + off + 4 * i + k)) << (8 * k);
+        if (4 * i + k < valid) w[i] |= static_cast<uint32_t>(E[off + 4 * i + k]) << (8 * k);
     }
   }
   return make_uint4(w[0], w[1], w[2], w[3]);
@@ -894,7 +894,7 @@ __device__ __forceinline__ uint4 load16_any(const uint8_t *__restrict__ E, int64
 // The padded copy of E (TcPadded): rows [t][f] of Dk dishes x 2 bytes.  One
 // polarization: row [t'][f] interleaves the rows of times 2 t' and 2 t' + 1.
 // One warp per row, 16 bytes per lane and step: bound by the bytes it moves.
-__global__ void __launch_bounds__(256) bf_pad_e(const uint8_t *__restrict__ E, int64_t avail, uint8_t *__restrict__ out,
+__global__ void __launch_bounds__(256) bf_pad_e(const uint8_t *E, int64_t avail, uint8_t *__restrict__ out,
                                                 int64_t T, int64_t F, int64_t D, int64_t Dk, int P) {
   grid_launch_next();
   grid_wait();
@@ -919,7 +919,7 @@ __global__ void __launch_bounds__(256) bf_pad_e(const uint8_t *__restrict__ E, i
           const int64_t off = ((2 * t + q) * F + f) * D + 8 * c;
 #pragma unroll
           for (int k = 0; k < 8; ++k)
-            if (k < valid) w[k >> 1] |= static_cast<uint32_t>(__ldg(E + off + k)) << (16 * (k & 1) + 8 * q);
+            if (k < valid) w[k >> 1] |= static_cast<uint32_t>(E[off + k]) << (16 * (k & 1) + 8 * q);
         }
         dst[c] = make_uint4(w[0], w[1], w[2], w[3]);
       }

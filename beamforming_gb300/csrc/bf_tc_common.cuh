@@ -169,7 +169,7 @@ struct RowSums {
 // RowMap) of every fourth beam.
 template <bool kJ2, bool kAdler>
 struct EpilogueTile {
-  const float *gcur;
+  const float *gcur;  // written by the launch before this one: plain loads (grid_wait)
   uint8_t *jrow;  // the thread's bytes for beam b0 + cb
   int64_t bstride;
   int blim;
@@ -187,7 +187,7 @@ struct EpilogueTile {
     gcur = P.gs + static_cast<int64_t>(f) * P.npass * P.nb_pass + b0 + cb;
     // huge or non-finite gains of this frequency: requantise with the
     // narrowing of cpu.cxx:38 (tile-uniform branch, normally not taken)
-    wide = __ldg(P.gwide + f) != 0;
+    wide = P.gwide[f] != 0;
     const int64_t bj = static_cast<int64_t>(b0 + static_cast<int>(cb)) * P.F + f;  // beam row b0 + cb
     int64_t at;  // the thread's 4 bytes in the J row
     if constexpr (!kJ2) {
@@ -326,7 +326,7 @@ struct EpilogueTile {
         uint32_t r[16], w[2];
         tmem_ld_rows4_x2(acc_addr + 16u * c, r);
         tmem_ld_wait(r);
-        words<true>(r, __ldg(gcur + 8 * c), __ldg(gcur + 8 * c + 4), w);
+        words<true>(r, gcur[8 * c], gcur[8 * c + 4], w);
         put<false>(dst, c, c - c_begin, w, a);
         dst += 8 * bstride;
       }
@@ -369,8 +369,8 @@ struct EpilogueTile {
     for (int i = 0; i < kC; ++i) tmem_ld_rows4_x2(acc_addr + 16u * (c + i), r[i]);
 #pragma unroll
     for (int i = 0; i < kC; ++i) {
-      g[2 * i] = __ldg(gcur + 8 * (c + i));
-      g[2 * i + 1] = __ldg(gcur + 8 * (c + i) + 4);
+      g[2 * i] = gcur[8 * (c + i)];
+      g[2 * i + 1] = gcur[8 * (c + i) + 4];
     }
 #pragma unroll
     for (int i = 0; i < kC; ++i) tmem_ld_wait(r[i]);  // the first waits for all; each ties its registers to the wait

@@ -40,3 +40,18 @@ def test_barriers_are_set_up_before_their_warp_uses_them(name, kernel):
     used = min(body.index(x) for x in ("cluster_arrive();", "cta_arrive(") if x in body)
     assert inits and max(inits) < fence < used
     assert "__syncwarp();" in body[fence:used]
+
+
+def test_overlapped_kernels_use_plain_loads():
+    """A launch that overlaps the one before it may be resident while that one
+    writes what it reads, so nothing in it may go through the read-only path."""
+    for name in ("bf_tc.cu", "bf_tc_pair.cu", "bf_tc_common.cuh", "bf_ptx.cuh"):
+        text = _source(name)
+        assert "__ldg" not in text and ".nc." not in text, name
+        assert not re.search(r"\bconst\s+\w+\s*\*\s*__restrict__", text), name
+    launched = set()
+    for name in os.listdir(CSRC):
+        launched |= set(re.findall(r"launch_overlapped\(\s*(\w+)\s*,", _source(name)))
+    assert launched == {"kern", "bf_pad_e", "write_words"}  # `kern`: of the files above
+    head = re.search(r"\bwrite_words\(([^)]*)\)\s*\{", _source("bf_adler.cu"))
+    assert "__restrict__" not in head.group(1)
