@@ -12,6 +12,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <new>
 #include <thread>
 #include <vector>
 
@@ -59,6 +60,14 @@ struct Lane {
 
 constexpr int kLanes = 3;
 
+// Scratch of a captured call (Scratch), once its graph is gone: a CUDA call cannot
+// be made where that is noticed, so the next call on the device frees it.
+struct GraphScratch {
+  struct DeviceCtx *c;
+  void *p;
+  GraphScratch *next;
+};
+
 struct DeviceCtx {
   std::mutex mu;
   bool ready = false;
@@ -68,8 +77,11 @@ struct DeviceCtx {
   int *err = nullptr;              // error word written by kernels
   uint32_t *adler = nullptr;       // adler32 result of the separate pass
   unsigned long long *adl = nullptr;  // fused adler32 sums {sum d_i, sum i d_i} of the last checked call
+  cudaMemPool_t pool = nullptr;    // of the calls' operands (Scratch)
+  cudaStream_t pool_s = nullptr;   // allocations that belong to no caller's stream
+  std::atomic<GraphScratch *> dropped{nullptr};
   DevBuf E, A, G, J;        // staging for host-pointer calls
-  DevBuf W, dig;            // tensor-core operand for non-resident calls
+  DevBuf W;                 // operand of synchronous calls, which end before they let go of mu
   DevBuf partials;          // adler32 partial sums
   // Scratch of the padded route (run_padded): operand and E copy of the call
   // that used it last, on whatever stream; the next one waits for pad_done.
@@ -104,6 +116,110 @@ thread_local HostResult t_result;
 constexpr int kMaxDevices = 64;
 DeviceCtx g_ctx[kMaxDevices];
 
+// Lets this thread allocate and free while another one captures a graph in global
+// mode, which would refuse it and lose that capture.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+// Unused memory the pool of a device keeps from one call to the next; what is above
+// goes back to the device when a stream is waited for.
+constexpr uint64_t kPoolKeep = uint64_t(1) << 30;
+
+cudaError_t make_pool(int dev, DeviceCtx &c) {
+  cudaMemPoolProps props{};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = dev;
+  if (!c.pool_s) {
+    const cudaError_t e = cudaStreamCreateWithFlags(&c.pool_s, cudaStreamNonBlocking);
+    if (e != cudaSuccess) return e;
+  }
+  if (c.pool) return cudaSuccess;
+  cudaMemPool_t pool = nullptr;
+  uint64_t keep = kPoolKeep;
+  int off = 0;  // streams stay independent: one does not wait for another's memory
+  cudaError_t e = cudaMemPoolCreate(&pool, &props);
+  if (e == cudaSuccess) e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+  if (e == cudaSuccess) e = cudaMemPoolSetAttribute(pool, cudaMemPoolReuseAllowInternalDependencies, &off);
+  if (e == cudaSuccess) c.pool = pool;
+  else if (pool) (void)cudaMemPoolDestroy(pool);
+  return e;
+}
+
+void CUDART_CB drop_graph_scratch(void *arg) {
+  GraphScratch *g = static_cast<GraphScratch *>(arg);
+  g->next = g->c->dropped.load();
+  while (!g->c->dropped.compare_exchange_weak(g->next, g)) {
+  }
+}
+
+// Device memory of one asynchronous call on stream s, in stream order: calls on one
+// stream use the same memory one after the other, calls on several streams never
+// share it (one operand per device let the second call's preparation overwrite what
+// the first one's kernel still read).  Allocation and free cost 0.5 us of host time
+// together and no launch.  A call under capture gets memory that belongs to its
+// graph: a replay reads it at any later time, beside any other call.
+class Scratch {
+ public:
+  Scratch() = default;
+  Scratch(const Scratch &) = delete;
+  Scratch &operator=(const Scratch &) = delete;
+  ~Scratch() {
+    if (!p_ || graph_) return;
+    RelaxedCapture relaxed;
+    (void)cudaFreeAsync(p_, s_);
+  }
+  cudaError_t reserve(DeviceCtx &c, size_t n, cudaStream_t s) {
+    RelaxedCapture relaxed;
+    for (GraphScratch *g = c.dropped.exchange(nullptr); g;) {
+      GraphScratch *const next = g->next;
+      (void)cudaFreeAsync(g->p, c.pool_s);
+      delete g;
+      g = next;
+    }
+    s_ = s;
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    cudaGraph_t graph = nullptr;
+    cudaError_t e = cudaStreamGetCaptureInfo(s, &st, nullptr, &graph, nullptr, nullptr, nullptr);
+    if (e == cudaSuccess)
+      e = st == cudaStreamCaptureStatusNone     ? cudaMallocFromPoolAsync(&p_, n, c.pool, s)
+          : st == cudaStreamCaptureStatusActive ? of_graph(c, n, graph)
+                                                : cudaErrorStreamCaptureInvalidated;
+    if (e != cudaSuccess) (void)cudaGetLastError();
+    return e;
+  }
+  uint8_t *get() const { return static_cast<uint8_t *>(p_); }
+
+ private:
+  cudaError_t of_graph(DeviceCtx &c, size_t n, cudaGraph_t graph) {
+    graph_ = true;
+    GraphScratch *const g = new (std::nothrow) GraphScratch{&c, nullptr, nullptr};
+    if (!g) return cudaErrorMemoryAllocation;
+    cudaError_t e = cudaMallocFromPoolAsync(&g->p, n, c.pool, c.pool_s);
+    if (e != cudaSuccess) {
+      delete g;
+      return e;
+    }
+    p_ = g->p;
+    cudaUserObject_t owner = nullptr;
+    e = cudaStreamSynchronize(c.pool_s);  // any stream may use it from here on
+    if (e == cudaSuccess) e = cudaUserObjectCreate(&owner, g, drop_graph_scratch, 1, cudaUserObjectNoDestructorSync);
+    if (e != cudaSuccess) {
+      drop_graph_scratch(g);
+      return e;
+    }
+    e = cudaGraphRetainUserObject(graph, owner, 1, cudaGraphUserObjectMove);
+    if (e != cudaSuccess) (void)cudaUserObjectRelease(owner, 1);
+    return e;
+  }
+  void *p_ = nullptr;
+  cudaStream_t s_ = nullptr;
+  bool graph_ = false;  // the graph's memory, not the call's
+};
+
 int current_ctx(DeviceCtx **out) {
   int dev = -1;
   const cudaError_t e = cudaGetDevice(&dev);
@@ -113,6 +229,7 @@ int current_ctx(DeviceCtx **out) {
   if (!c.ready) {
     std::lock_guard<std::mutex> lk(c.mu);
     if (!c.ready) {
+      BF_TRY(make_pool(dev, c));
       DevResult *res = nullptr;
       BF_TRY(cudaMalloc(&res, sizeof(DevResult)));
       BF_TRY(cudaMemset(res, 0, sizeof(DevResult)));
@@ -162,6 +279,13 @@ void plan_weights(TcWeights &w, int64_t F, int64_t B, int64_t D) {
 
 size_t weights_bytes(const TcWeights &w) { return static_cast<size_t>(w.F) * w.nw * 2 * w.Dk; }
 
+// The operand in one block: W, then (on a 256-byte boundary) the digit rows and gains.
+size_t extra_at(const TcWeights &w) { return (weights_bytes(w) + 255) / 256 * 256; }
+size_t operand_bytes(const TcWeights &w) { return extra_at(w) + tc_extra_bytes(w); }
+void set_operand(TcWeights &w, uint8_t *p) {
+  w.W = p;
+  tc_set_extra(w, p + extra_at(w));
+}
 
 int choose_tensor(const bf_dims &d, bool *use_tc) {
   const int k = g_kernel.load();
@@ -173,13 +297,6 @@ int choose_tensor(const bf_dims &d, bool *use_tc) {
   *use_tc = (k == BF_KERNEL_TENSOR) || (k == BF_KERNEL_AUTO && ok);
   return BF_OK;
 }
-
-// All four arrays on the device; the tensor-core operand goes to W / dig.
-// With `adl` set (zeroed here), a tensor-core launch also sums J for its
-// adler32 and *fused reports that it did; the SIMT kernel does not.
-int run_device_bufs(const bf_dims &d, uint8_t *J, const uint8_t *E, const uint8_t *A, const float *G, DevBuf &W,
-                    DevBuf &dig, int *err, cudaStream_t s, int a_layout = kALinear, int j_layout = kJLinear,
-                    unsigned long long *adl = nullptr, bool *fused = nullptr);
 
 // A shape the tensor-core kernel does not take in place, on it all the same
 // (TcPadded); *ran = false where the dp4a kernel has to take it: the rule or the
@@ -247,8 +364,13 @@ int run_padded(DeviceCtx &c, const bf_dims &d, uint8_t *J, const uint8_t *E, con
   return st != BF_OK ? st : to_status(re);
 }
 
-// All four arrays on the device.  Operand scratch comes from ctx (caller holds ctx.mu).
-int run_device(DeviceCtx &c, const bf_dims &d, uint8_t *J, const uint8_t *E, const uint8_t *A, const float *G,
+// All four arrays on the device; asynchronous on s.  With `adl` set, a tensor-core
+// launch also sums J for its adler32 (into sums that it zeroes) and *fused reports
+// that it did; the SIMT kernel does not.  The prepared weights go to memory of the
+// call's own, or with `ends_here` (the caller waits for the stream before it lets go
+// of c.mu, also after an error) to a buffer of the device: the pool's first allocation
+// after a wait costs a checked call 3 us of 52.  The caller holds c.mu.
+int run_device(DeviceCtx &c, bool ends_here, const bf_dims &d, uint8_t *J, const uint8_t *E, const uint8_t *A, const float *G,
                cudaStream_t s, int a_layout = kALinear, int j_layout = kJLinear, unsigned long long *adl = nullptr,
                bool *fused = nullptr) {
   if (fused) *fused = false;
@@ -257,41 +379,27 @@ int run_device(DeviceCtx &c, const bf_dims &d, uint8_t *J, const uint8_t *E, con
   const int st = choose_tensor(d, &use_tc);
   if (st != BF_OK) return st;
   const bool aligned = ((reinterpret_cast<uintptr_t>(E) | reinterpret_cast<uintptr_t>(J)) & 15u) == 0;
-  if (g_kernel.load() == BF_KERNEL_AUTO && !(use_tc && aligned)) {
-    bool ran = false;
-    const int ps = run_padded(c, d, J, E, A, G, nullptr, s, a_layout, j_layout, adl, fused, &ran);
-    if (ran || ps != BF_OK) return ps;
-  }
-  return run_device_bufs(d, J, E, A, G, c.W, c.dig, c.err, s, a_layout, j_layout, adl, fused);
-}
-
-int run_device_bufs(const bf_dims &d, uint8_t *J, const uint8_t *E, const uint8_t *A, const float *G, DevBuf &Wb,
-                    DevBuf &digb, int *err, cudaStream_t s, int a_layout, int j_layout, unsigned long long *adl,
-                    bool *fused) {
-  if (fused) *fused = false;
-  if (jsize(d) == 0) return BF_OK;
-  bool use_tc = false;
-  const int st = choose_tensor(d, &use_tc);
-  if (st != BF_OK) return st;
-  if (use_tc && ((reinterpret_cast<uintptr_t>(E) | reinterpret_cast<uintptr_t>(J)) & 15u)) {
-    if (g_kernel.load() == BF_KERNEL_TENSOR) return BF_ERR_UNSUPPORTED;
-    use_tc = false;
-  }
+  if (use_tc && !aligned && g_kernel.load() == BF_KERNEL_TENSOR) return BF_ERR_UNSUPPORTED;
+  use_tc = use_tc && aligned;
   if (!use_tc) {
+    if (g_kernel.load() == BF_KERNEL_AUTO) {
+      bool ran = false;
+      const int ps = run_padded(c, d, J, E, A, G, nullptr, s, a_layout, j_layout, adl, fused, &ran);
+      if (ran || ps != BF_OK) return ps;
+    }
     t_last_kernel = simt_name();
     return to_status(launch_simt(d, J, E, A, G, s, 0, a_layout, j_layout));
   }
   TcWeights w;
   plan_weights(w, d.nfrequencies, d.nbeams, d.ndishes);
-  BF_TRY(Wb.reserve(weights_bytes(w)));
-  BF_TRY(digb.reserve(tc_extra_bytes(w)));
-  w.W = Wb.as<uint8_t>();
-  tc_set_extra(w, digb.as<uint8_t>());
+  Scratch own;
+  BF_TRY(ends_here ? c.W.reserve(operand_bytes(w)) : own.reserve(c, operand_bytes(w), s));
+  set_operand(w, ends_here ? c.W.as<uint8_t>() : own.get());
   w.G = G;
   if (adl && fused) *fused = true;
   BF_TRY(launch_prep_weights(w, A, s, a_layout, adl));
   t_last_kernel = "tensor";
-  return to_status(launch_tc(w, d.ntimes, J, E, err, s, 0, j_layout, adl, J));
+  return to_status(launch_tc(w, d.ntimes, J, E, c.err, s, 0, j_layout, adl, J));
 }
 
 // Waits for the stream and reads the device results; a kernel's error clears the
@@ -406,10 +514,8 @@ int run_host_pipelined(DeviceCtx &c, const bf_dims &d, uint8_t *J, const uint8_t
   TcWeights w;
   if (use_tc) {
     plan_weights(w, d.nfrequencies, d.nbeams, d.ndishes);
-    BF_TRY(c.W.reserve(weights_bytes(w)));
-    BF_TRY(c.dig.reserve(tc_extra_bytes(w)));
-    w.W = c.W.as<uint8_t>();
-    tc_set_extra(w, c.dig.as<uint8_t>());
+    BF_TRY(c.W.reserve(operand_bytes(w)));
+    set_operand(w, c.W.as<uint8_t>());
     w.G = c.G.as<float>();
     // every chunk's launch adds into the same sums, positions from the start of J
     BF_TRY(launch_prep_weights(w, c.A.as<uint8_t>(), l0.s, a_layout, adl));
@@ -550,9 +656,10 @@ int finish_adler(DeviceCtx &c, bool fused, const uint8_t *Jdev, size_t n, cudaSt
   return st;
 }
 
-// After a failed synchronous host-pointer call: wait for what it had already
-// queued (copies from the caller's E, drains into the caller's J) so that
-// nothing touches the caller's buffers once the call has returned.
+// After a failed synchronous call: wait for what it had already queued (copies
+// from the caller's E, drains into the caller's J, the operand's preparation) so
+// that nothing touches the caller's buffers, or the device's, once the call has
+// returned.
 void settle_after_error(DeviceCtx &c, cudaStream_t s) {
   (void)cudaStreamSynchronize(s);
   if (c.lanes_ready)
@@ -584,9 +691,11 @@ static int form_beams_impl(const bf_dims *dims, uint8_t *J, const uint8_t *E, co
   unsigned long long *adl = adler_out ? c->adl : nullptr;
   bool fused = false;
   if (ptr_kind == BF_PTR_DEVICE) {
-    st = run_device(*c, d, J, E, A, G, s, a_layout, j_layout, adl, &fused);
-    if (st != BF_OK || !adler_out) return st;
-    return finish_adler(*c, fused, J, jsize(d), s, adler_out, true);
+    st = run_device(*c, adler_out != nullptr, d, J, E, A, G, s, a_layout, j_layout, adl, &fused);
+    if (!adler_out) return st;
+    if (st == BF_OK) st = finish_adler(*c, fused, J, jsize(d), s, adler_out, true);
+    if (st != BF_OK && st != BF_ERR_UNSUPPORTED) settle_after_error(*c, s);  // a refused shape queued nothing
+    return st;
   }
 
   // Host pointers: stage in, compute, stage out, synchronously (cuda.cu:274-314 does the same around its
@@ -604,7 +713,7 @@ static int form_beams_impl(const bf_dims *dims, uint8_t *J, const uint8_t *E, co
     BF_TRY(cudaMemcpyAsync(c->E.p, E, esize(d), cudaMemcpyHostToDevice, s));
     BF_TRY(cudaMemcpyAsync(c->A.p, A, asize(d), cudaMemcpyHostToDevice, s));
     BF_TRY(cudaMemcpyAsync(c->G.p, G, gsize(d) * sizeof(float), cudaMemcpyHostToDevice, s));
-    const int rs = run_device(*c, d, c->J.as<uint8_t>(), c->E.as<uint8_t>(), c->A.as<uint8_t>(), c->G.as<float>(),
+    const int rs = run_device(*c, true, d, c->J.as<uint8_t>(), c->E.as<uint8_t>(), c->A.as<uint8_t>(), c->G.as<float>(),
                               s, a_layout, j_layout, adl, &fused);
     if (rs != BF_OK) return rs;
     BF_TRY(cudaMemcpyAsync(J, c->J.p, jsize(d), cudaMemcpyDeviceToHost, s));

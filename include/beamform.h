@@ -104,7 +104,9 @@ BF_API const char *bf_status_string(int status);
 
 /* One beamforming pass with explicit sizes.  ptr_kind says whether E, A, G and
  * J are host or device pointers.  Device pointers: asynchronous on `stream`;
- * call bf_stream_status() (or synchronize) before reading J.  Host pointers:
+ * call bf_stream_status() (or synchronize) before reading J; calls on several
+ * streams are independent of each other, and a captured one belongs to its
+ * graph, the memory of its prepared weights too.  Host pointers:
  * synchronous (copies in, computes, copies out). */
 BF_API int bf_form_beams_ex(const bf_dims *dims, uint8_t *J, const uint8_t *E, const uint8_t *A, const float *G,
                      int ptr_kind, bf_stream_t stream);

@@ -1,0 +1,124 @@
+"""Explicit device-pointer calls are asynchronous: calls on several streams and
+captured calls prepare their weights into memory that no other call touches."""
+from __future__ import annotations
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+SHAPE = (2048, 16, 512, 2, 96)
+
+
+def _set(bf, torch, shape, seed):
+    """(dims, E, A, G, J of the exact kernel)."""
+    d = bf.Dims(*shape)
+    E = torch.empty(d.esize, dtype=torch.uint8, device="cuda")
+    A = torch.empty(d.asize, dtype=torch.uint8, device="cuda")
+    bf.fill_random_device(E, seed, 0)
+    bf.fill_random_device(A, seed, 1)
+    G = torch.from_numpy(bf.gains(d)).cuda() * (1.0 + seed % 3)
+    return d, E, A, G, _exact(bf, torch, d, E, A, G)
+
+
+def _exact(bf, torch, d, E, A, G):
+    J = torch.empty(d.jsize, dtype=torch.uint8, device="cuda")
+    bf.set_kernel("simt")
+    try:
+        bf.form_beams_ex(d, J, E, A, G)
+        bf.stream_status()
+    finally:
+        bf.set_kernel("auto")
+    return J
+
+
+@pytest.mark.parametrize("shape", [SHAPE, (4096, 1, 512, 2, 128), (8192, 2, 256, 2, 16)])
+def test_calls_on_streams_do_not_share_weights(bflib, cuda, shape):
+    sets = [_set(bflib, cuda, shape, k) for k in range(3)]
+    streams = [cuda.cuda.Stream() for _ in sets]
+    cuda.cuda.synchronize()
+    out = []
+    for _ in range(20):
+        for (d, E, A, G, want), s in zip(sets, streams):
+            with cuda.cuda.stream(s):
+                J = cuda.empty(d.jsize, dtype=cuda.uint8, device="cuda")
+                bflib.form_beams_ex(d, J, E, A, G, stream=s)
+            assert bflib.last_kernel() == "tensor"
+            out.append((J, want))
+    cuda.cuda.synchronize()
+    bflib.stream_status()
+    for J, want in out:
+        assert cuda.equal(J, want)
+
+
+def _capture(bf, torch, d, E, A, G):
+    J = torch.zeros(d.jsize, dtype=torch.uint8, device="cuda")
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        bf.form_beams_ex(d, J, E, A, G)
+        assert bf.last_kernel() == "tensor"
+    return g, J
+
+
+def test_captured_calls_keep_their_scratch(bflib, cuda):
+    """Replays beside larger and other calls, with the graph's inputs changed, and
+    after other graphs are gone."""
+    d, E, A, G, want = _set(bflib, cuda, SHAPE, 1)
+    big = _set(bflib, cuda, (1024, 32, 1024, 2, 256), 2)
+    gone, _ = _capture(bflib, cuda, d, E, A, G)
+    g, J = _capture(bflib, cuda, d, E, A, G)
+    other = _set(bflib, cuda, SHAPE, 3)
+    g2, J2 = _capture(bflib, cuda, *other[:4])
+    del gone
+    s1, s2 = cuda.cuda.Stream(), cuda.cuda.Stream()
+    cuda.cuda.synchronize()
+    Jb = cuda.empty(big[0].jsize, dtype=cuda.uint8, device="cuda")
+    for rep in range(6):
+        if rep == 3:  # new voltages and weights in the captured buffers
+            bflib.fill_random_device(E, 9, 0)
+            bflib.fill_random_device(A, 9, 1)
+            want = _exact(bflib, cuda, d, E, A, G)
+        J.zero_(), J2.zero_(), Jb.zero_()
+        cuda.cuda.synchronize()
+        with cuda.cuda.stream(s1):
+            g.replay()
+        with cuda.cuda.stream(s2):
+            g2.replay()
+        bflib.form_beams_ex(big[0], Jb, *big[1:4])
+        cuda.cuda.synchronize()
+        bflib.stream_status()
+        assert cuda.equal(J, want) and cuda.equal(J2, other[4]) and cuda.equal(Jb, big[4])
+
+
+def test_capture_while_other_threads_call(bflib, cuda):
+    """Calls on other threads go on, and their scratch grows, while this one captures
+    in global mode; the capture survives them."""
+    import threading
+
+    d, E, A, G, want = _set(bflib, cuda, (512, 4, 512, 2, 96), 4)
+    big = [_set(bflib, cuda, (256, 40 + 20 * k, 1024, 2, 200), 5 + k) for k in range(2)]
+    s = cuda.cuda.Stream()
+    Jb = [cuda.empty(x[0].jsize, dtype=cuda.uint8, device="cuda") for x in big]
+    failed = []
+
+    def call():
+        try:
+            for x, j in zip(big, Jb):
+                bflib.form_beams_ex(x[0], j, *x[1:4], stream=s)
+        except Exception as e:  # noqa: BLE001 - reported below
+            failed.append(e)
+
+    cuda.cuda.synchronize()
+    J = cuda.zeros(d.jsize, dtype=cuda.uint8, device="cuda")
+    g = cuda.cuda.CUDAGraph()
+    with cuda.cuda.graph(g):
+        bflib.form_beams_ex(d, J, E, A, G)
+        th = threading.Thread(target=call)
+        th.start()
+        th.join()
+        bflib.form_beams_ex(d, J, E, A, G)
+    assert not failed
+    g.replay()
+    cuda.cuda.synchronize()
+    assert cuda.equal(J, want)
+    for x, j in zip(big, Jb):
+        assert cuda.equal(j, x[4])
