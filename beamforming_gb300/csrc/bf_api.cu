@@ -81,13 +81,8 @@ struct DeviceCtx {
   cudaStream_t pool_s = nullptr;   // allocations that belong to no caller's stream
   std::atomic<GraphScratch *> dropped{nullptr};
   DevBuf E, A, G, J;        // staging for host-pointer calls
-  DevBuf W;                 // operand of synchronous calls, which end before they let go of mu
+  DevBuf W;                 // what synchronous calls prepare: they end before they let go of mu
   DevBuf partials;          // adler32 partial sums
-  // Scratch of the padded route (run_padded): operand and E copy of the call
-  // that used it last, on whatever stream; the next one waits for pad_done.
-  DevBuf padE, padW, padDig;
-  cudaEvent_t pad_done = nullptr;
-  bool pad_used = false;
 };
 
 // Device results and where a thread reads them: pinned, so that the copy back is
@@ -127,6 +122,8 @@ struct RelaxedCapture {
 // Unused memory the pool of a device keeps from one call to the next; what is above
 // goes back to the device when a stream is waited for.
 constexpr uint64_t kPoolKeep = uint64_t(1) << 30;
+// The most a synchronous call prepares in the device's buffer, which lives until exit.
+constexpr size_t kKeptBytes = size_t(256) << 20;
 
 cudaError_t make_pool(int dev, DeviceCtx &c) {
   cudaMemPoolProps props{};
@@ -298,14 +295,25 @@ int choose_tensor(const bf_dims &d, bool *use_tc) {
   return BF_OK;
 }
 
+// Memory for what one call prepares: the call's own, or with `ends_here` (the caller
+// waits for the stream before it lets go of c.mu, also after an error) a buffer of the
+// device: the pool's first allocation after a wait costs a checked call 3 us of 52.
+cudaError_t call_memory(DeviceCtx &c, Scratch &own, bool ends_here, size_t n, cudaStream_t s, uint8_t **p) {
+  const bool kept = ends_here && n <= kKeptBytes;
+  const cudaError_t e = kept ? c.W.reserve(n) : own.reserve(c, n, s);
+  *p = kept ? c.W.as<uint8_t>() : own.get();
+  if (e != cudaSuccess) (void)cudaGetLastError();
+  return e;
+}
+
 // A shape the tensor-core kernel does not take in place, on it all the same
-// (TcPadded); *ran = false where the dp4a kernel has to take it: the rule or the
-// memory says so, or the stream is being captured (the scratch is shared with
-// later calls, which a graph cannot wait for).  `rw`: resident weights, whose
-// operand is used instead of preparing A.  The caller holds c.mu.
-int run_padded(DeviceCtx &c, const bf_dims &d, uint8_t *J, const uint8_t *E, const uint8_t *A, const float *G,
-               const TcWeights *rw, cudaStream_t s, int a_layout, int j_layout, unsigned long long *adl, bool *fused,
-               bool *ran) {
+// (TcPadded); *ran = false where the dp4a kernel has to take it: the rule says so,
+// the memory cannot be had, or the stream is being captured (a graph would hold the
+// copy of E for as long as it lives).  `rw`: resident weights, whose operand is used
+// instead of preparing A; no checksum then.  The caller holds c.mu if `ends_here`.
+int run_padded(DeviceCtx &c, bool ends_here, const bf_dims &d, uint8_t *J, const uint8_t *E, const uint8_t *A,
+               const float *G, const TcWeights *rw, cudaStream_t s, int a_layout, int j_layout,
+               unsigned long long *adl, bool *fused, bool *ran) {
   *ran = false;
   const TcPadded r = tc_padded(d, E, rw != nullptr);
   if (!r.ok) return BF_OK;
@@ -320,56 +328,41 @@ int run_padded(DeviceCtx &c, const bf_dims &d, uint8_t *J, const uint8_t *E, con
   } else {
     plan_weights(w, d.nfrequencies, d.nbeams, d.ndishes);
   }
-  if (!c.pad_done) BF_TRY(cudaEventCreateWithFlags(&c.pad_done, cudaEventDisableTiming));
-  if (c.pad_used) BF_TRY(cudaStreamWaitEvent(s, c.pad_done, 0));
-  cudaError_t e = r.copy ? c.padE.reserve(r.bytes) : cudaSuccess;
-  if (!rw && e == cudaSuccess) e = c.padW.reserve(weights_bytes(w));
-  if (!rw && e == cudaSuccess) e = c.padDig.reserve(tc_extra_bytes(w));
-  if (e == cudaErrorMemoryAllocation) {
-    (void)cudaGetLastError();
-    return BF_OK;
-  }
-  BF_TRY(e);
+  const size_t copy = r.copy ? (r.bytes + 255) / 256 * 256 : 0;  // the copy of E first, then the operand
+  const size_t need = copy + (rw ? 0 : operand_bytes(w));
+  Scratch own;
+  uint8_t *mem = nullptr;
+  if (need && call_memory(c, own, ends_here, need, s, &mem) != cudaSuccess) return BF_OK;
   *ran = true;
   t_last_kernel = "tensor";
-  c.pad_used = true;
-  const int st = [&]() -> int {
-    if (adl && rw) BF_TRY(cudaMemsetAsync(adl, 0, 2 * sizeof(unsigned long long), s));
-    if (adl && fused) *fused = true;
-    if (!rw) {
-      w.W = c.padW.as<uint8_t>();
-      tc_set_extra(w, c.padDig.as<uint8_t>());
-      w.G = G;
-      BF_TRY(launch_prep_weights(w, A, s, a_layout, adl));
+  if (adl && fused) *fused = true;
+  if (!rw) {
+    set_operand(w, mem + copy);
+    w.G = G;
+    BF_TRY(launch_prep_weights(w, A, s, a_layout, adl));
+  }
+  const int64_t P = d.npolarizations, per_t = d.nfrequencies * d.ndishes * P;
+  for (int64_t t0 = 0; t0 < d.ntimes; t0 += r.times) {
+    const int64_t nt = std::min(r.times, d.ntimes - t0);
+    const uint8_t *Ec = E + t0 * per_t;
+    if (r.copy) {
+      BF_TRY(launch_pad_e(d, Ec, esize(d) - static_cast<size_t>(t0 * per_t), nt, mem, s));
+      Ec = mem;
     }
-    const int64_t P = d.npolarizations, per_t = d.nfrequencies * d.ndishes * P;
-    for (int64_t t0 = 0; t0 < d.ntimes; t0 += r.times) {
-      const int64_t nt = std::min(r.times, d.ntimes - t0);
-      const uint8_t *Ec = E + t0 * per_t;
-      if (r.copy) {
-        BF_TRY(launch_pad_e(d, Ec, esize(d) - static_cast<size_t>(t0 * per_t), nt, c.padE.as<uint8_t>(), s));
-        Ec = c.padE.as<uint8_t>();
-      }
-      if (P == 1) {
-        const TcRows rows{d.ntimes, nt};
-        const int64_t pairs = (nt + 1) / 2;
-        BF_TRY(launch_tc(w, pairs, J + t0, Ec, c.err, s, (d.ntimes + 1) / 2, kJ2, adl, J, &rows));
-      } else {
-        BF_TRY(launch_tc(w, nt, J + (j_layout == kJ2 ? 2 * t0 : t0), Ec, c.err, s, d.ntimes, j_layout, adl, J));
-      }
+    if (P == 1) {
+      const TcRows rows{d.ntimes, nt};
+      const int64_t pairs = (nt + 1) / 2;
+      BF_TRY(launch_tc(w, pairs, J + t0, Ec, c.err, s, (d.ntimes + 1) / 2, kJ2, adl, J, &rows));
+    } else {
+      BF_TRY(launch_tc(w, nt, J + (j_layout == kJ2 ? 2 * t0 : t0), Ec, c.err, s, d.ntimes, j_layout, adl, J));
     }
-    return BF_OK;
-  }();
-  const cudaError_t re = cudaEventRecord(c.pad_done, s);
-  return st != BF_OK ? st : to_status(re);
+  }
+  return BF_OK;
 }
 
 // All four arrays on the device; asynchronous on s.  With `adl` set, a tensor-core
 // launch also sums J for its adler32 (into sums that it zeroes) and *fused reports
-// that it did; the SIMT kernel does not.  The prepared weights go to memory of the
-// call's own, or with `ends_here` (the caller waits for the stream before it lets go
-// of c.mu, also after an error) to a buffer of the device: the pool's first allocation
-// after a wait costs a checked call 3 us of 52.  The caller holds c.mu.
+// that it did; the SIMT kernel does not.  The caller holds c.mu.
 int run_device(DeviceCtx &c, bool ends_here, const bf_dims &d, uint8_t *J, const uint8_t *E, const uint8_t *A, const float *G,
                cudaStream_t s, int a_layout = kALinear, int j_layout = kJLinear, unsigned long long *adl = nullptr,
                bool *fused = nullptr) {
@@ -384,7 +377,7 @@ int run_device(DeviceCtx &c, bool ends_here, const bf_dims &d, uint8_t *J, const
   if (!use_tc) {
     if (g_kernel.load() == BF_KERNEL_AUTO) {
       bool ran = false;
-      const int ps = run_padded(c, d, J, E, A, G, nullptr, s, a_layout, j_layout, adl, fused, &ran);
+      const int ps = run_padded(c, ends_here, d, J, E, A, G, nullptr, s, a_layout, j_layout, adl, fused, &ran);
       if (ran || ps != BF_OK) return ps;
     }
     t_last_kernel = simt_name();
@@ -393,8 +386,9 @@ int run_device(DeviceCtx &c, bool ends_here, const bf_dims &d, uint8_t *J, const
   TcWeights w;
   plan_weights(w, d.nfrequencies, d.nbeams, d.ndishes);
   Scratch own;
-  BF_TRY(ends_here ? c.W.reserve(operand_bytes(w)) : own.reserve(c, operand_bytes(w), s));
-  set_operand(w, ends_here ? c.W.as<uint8_t>() : own.get());
+  uint8_t *mem = nullptr;
+  BF_TRY(call_memory(c, own, ends_here, operand_bytes(w), s, &mem));
+  set_operand(w, mem);
   w.G = G;
   if (adl && fused) *fused = true;
   BF_TRY(launch_prep_weights(w, A, s, a_layout, adl));
@@ -858,9 +852,8 @@ int bf_form_beams_resident(const bf_weights *w, int64_t ntimes, uint8_t *J, cons
     return to_status(launch_tc(w->tc, ntimes, J, E, c->err, s));
   }
   if (g_kernel.load() == BF_KERNEL_AUTO) {
-    std::lock_guard<std::mutex> lk(c->mu);
     bool ran = false;
-    const int ps = run_padded(*c, d, J, E, nullptr, nullptr, &w->tc, s, kALinear, kJLinear, nullptr, nullptr, &ran);
+    const int ps = run_padded(*c, false, d, J, E, nullptr, nullptr, &w->tc, s, kALinear, kJLinear, nullptr, nullptr, &ran);
     if (ran || ps != BF_OK) return ps;
   }
   t_last_kernel = simt_name();

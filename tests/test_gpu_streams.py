@@ -122,3 +122,81 @@ def test_capture_while_other_threads_call(bflib, cuda):
     assert cuda.equal(J, want)
     for x, j in zip(big, Jb):
         assert cuda.equal(j, x[4])
+
+
+def test_odd_resident_calls_while_another_thread_captures(bflib, cuda):
+    """A call on a shape that takes the padded copy needs new scratch: neither it nor
+    the other thread's capture, in global mode, is lost."""
+    import threading
+
+    T, F, D, B = 3001, 12, 253, 45
+    d, E, A, G, want = _set(bflib, cuda, (T, F, D, 2, B), 11)
+    W = bflib.ResidentWeights(F, B, D, A, G)
+    s = cuda.cuda.Stream()
+    J = cuda.empty(d.jsize, dtype=cuda.uint8, device="cuda")
+    x = cuda.ones(64, device="cuda")
+    failed = []
+
+    def call():
+        try:
+            W.form_beams(J, E, T, stream=s)
+            if bflib.last_kernel() != "tensor":
+                failed.append(bflib.last_kernel())
+        except Exception as e:  # noqa: BLE001 - reported below
+            failed.append(e)
+
+    cuda.cuda.synchronize()
+    g = cuda.cuda.CUDAGraph()
+    with cuda.cuda.graph(g):
+        y = x + 1
+        th = threading.Thread(target=call)
+        th.start()
+        th.join()
+        y = y + 1
+    assert not failed
+    g.replay()
+    cuda.cuda.synchronize()
+    assert cuda.equal(J, want) and bool((y == 3).all())
+
+
+def test_odd_resident_calls_wait_for_no_other_thread(bflib, cuda):
+    """A checked call holds the device's lock until its stream is through (here for as
+    long as a stalled launch takes to give up, 1.5 s); a call on resident weights has
+    no use for the lock, whichever kernel takes its shape."""
+    import threading
+    import time
+
+    T, F, D, B = 201, 2, 61, 9
+    d, E, A, G, want = _set(bflib, cuda, (T, F, D, 2, B), 12)
+    W = bflib.ResidentWeights(F, B, D, A, G)
+    J = cuda.empty(d.jsize, dtype=cuda.uint8, device="cuda")
+    d2, E2, A2, G2, _ = _set(bflib, cuda, (64, 1, 64, 2, 40), 13)
+    J2 = cuda.empty(d2.jsize, dtype=cuda.uint8, device="cuda")
+    s1, s2 = cuda.cuda.Stream(), cuda.cuda.Stream()
+    W.form_beams(J, E, T, stream=s2)
+    cuda.cuda.synchronize()
+    status = []
+
+    def stalled():
+        try:
+            bflib.form_beams_adler(d2, J2, E2, A2, G2, stream=s1)
+            status.append(bflib.OK)
+        except bflib.BeamformError as e:
+            status.append(e.status)
+
+    bflib.lib().bf_set_test_stall(1)
+    th = threading.Thread(target=stalled)
+    try:
+        th.start()
+        time.sleep(0.3)  # the stalled launch is queued, its call waits
+    finally:
+        bflib.lib().bf_set_test_stall(0)
+    t0 = time.monotonic()
+    W.form_beams(J, E, T, stream=s2)
+    took = time.monotonic() - t0
+    assert th.is_alive()
+    th.join()
+    assert status == [bflib.ERR_DEVICE_TIMEOUT]
+    assert bflib.last_kernel() == "simt" and took < 0.3, took
+    cuda.cuda.synchronize()
+    assert cuda.equal(J, want)
