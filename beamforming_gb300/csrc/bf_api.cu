@@ -68,15 +68,31 @@ struct GraphScratch {
   GraphScratch *next;
 };
 
+// What the host reads back after a call, and the blocks of pinned memory it is read
+// from: pinned, so that the copy back is one asynchronous transfer and the call waits
+// once; the device's, so that a thread neither pins memory on its first call nor frees
+// it, which waits for the device, at its end.
+struct DevResult {
+  int err;
+  uint32_t adler;
+  unsigned long long adl[2];
+};
+struct alignas(64) HostBlock {
+  DevResult r;
+};
+constexpr int kHostBlocks = 32;  // calls of a device that read at the same time; more read into their stack
+
 struct DeviceCtx {
   std::mutex mu;
   bool ready = false;
   bool lanes_ready = false;
   Lane lanes[kLanes];
-  // What the host reads back after a call, in one device block (DevResult).
+  // The fields of the device's DevResult.
   int *err = nullptr;              // error word written by kernels
   uint32_t *adler = nullptr;       // adler32 result of the separate pass
   unsigned long long *adl = nullptr;  // fused adler32 sums {sum d_i, sum i d_i} of the last checked call
+  HostBlock *host = nullptr;       // null: no pinned memory to be had
+  std::atomic<uint32_t> host_used{0};
   cudaMemPool_t pool = nullptr;    // of the calls' operands (Scratch)
   cudaStream_t pool_s = nullptr;   // allocations that belong to no caller's stream
   std::atomic<GraphScratch *> dropped{nullptr};
@@ -84,29 +100,6 @@ struct DeviceCtx {
   DevBuf W;                 // what synchronous calls prepare: they end before they let go of mu
   DevBuf partials;          // adler32 partial sums
 };
-
-// Device results and where a thread reads them: pinned, so that the copy back is
-// one asynchronous transfer and the call waits once.
-struct DevResult {
-  int err;
-  uint32_t adler;
-  unsigned long long adl[2];
-};
-struct HostResult {
-  DevResult *p = nullptr;
-  DevResult pageable{};
-  DevResult *get() {
-    if (!p && cudaMallocHost(&p, sizeof(DevResult)) != cudaSuccess) {
-      (void)cudaGetLastError();
-      p = nullptr;
-    }
-    return p ? p : &pageable;
-  }
-  ~HostResult() {
-    if (p) (void)cudaFreeHost(p);
-  }
-};
-thread_local HostResult t_result;
 
 constexpr int kMaxDevices = 64;
 DeviceCtx g_ctx[kMaxDevices];
@@ -217,6 +210,36 @@ class Scratch {
   bool graph_ = false;  // the graph's memory, not the call's
 };
 
+// A host block for one call: pinned where one is free.
+class HostResult {
+ public:
+  explicit HostResult(DeviceCtx &c) : c_(c) {
+    if (!c.host) return;
+    for (uint32_t used = c.host_used.load(); used != ~uint32_t(0);) {
+      const uint32_t bit = ~used & (used + 1);  // the lowest free one
+      if (c.host_used.compare_exchange_weak(used, used | bit)) {
+        bit_ = bit;
+        int i = 0;
+        while (!(bit >> i & 1)) ++i;
+        p_ = &c.host[i].r;
+        return;
+      }
+    }
+  }
+  HostResult(const HostResult &) = delete;
+  HostResult &operator=(const HostResult &) = delete;
+  ~HostResult() { c_.host_used.fetch_and(~bit_); }
+  DevResult *get() { return p_; }
+  bool pinned() const { return bit_ != 0; }
+
+ private:
+  DeviceCtx &c_;
+  DevResult stack_{};
+  DevResult *p_ = &stack_;
+  uint32_t bit_ = 0;
+};
+static_assert(kHostBlocks == 32, "one bit each");
+
 int current_ctx(DeviceCtx **out) {
   int dev = -1;
   const cudaError_t e = cudaGetDevice(&dev);
@@ -230,6 +253,10 @@ int current_ctx(DeviceCtx **out) {
       DevResult *res = nullptr;
       BF_TRY(cudaMalloc(&res, sizeof(DevResult)));
       BF_TRY(cudaMemset(res, 0, sizeof(DevResult)));
+      if (cudaMallocHost(&c.host, kHostBlocks * sizeof(HostBlock)) != cudaSuccess) {
+        (void)cudaGetLastError();
+        c.host = nullptr;
+      }
       c.err = &res->err;
       c.adler = &res->adler;
       c.adl = res->adl;
@@ -401,9 +428,10 @@ int run_device(DeviceCtx &c, bool ends_here, const bf_dims &d, uint8_t *J, const
 // kernel, and another one writes the results faster than a copy; behind a copy a
 // copy is faster (host call 294 against 296 us).
 int read_and_clear_err(DeviceCtx &c, cudaStream_t s, DevResult *out = nullptr, bool behind_kernel = false) {
-  DevResult *h = t_result.get();
+  HostResult block(c);
+  DevResult *const h = block.get();
   static_assert(sizeof(DevResult) % 4 == 0 && sizeof(DevResult) <= 128, "words of one warp");
-  if (behind_kernel && h == t_result.p)
+  if (behind_kernel && block.pinned())
     BF_TRY(launch_write_words(c.err, h, sizeof(DevResult) / 4, s));
   else
     BF_TRY(cudaMemcpyAsync(h, c.err, sizeof(DevResult), cudaMemcpyDeviceToHost, s));
@@ -874,7 +902,8 @@ int bf_adler32_device(const uint8_t *data, size_t len, uint32_t *out, bf_stream_
   BF_TRY(c->partials.reserve(static_cast<size_t>(adler_nchunks(len)) * 2 * sizeof(uint32_t)));
   BF_TRY(launch_adler_partials(data, len, c->partials.as<uint32_t>(), s));
   BF_TRY(launch_adler_combine(c->partials.as<uint32_t>(), len, c->adler, s));
-  DevResult *h = t_result.get();
+  HostResult block(*c);
+  DevResult *const h = block.get();
   BF_TRY(cudaMemcpyAsync(&h->adler, c->adler, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
   BF_TRY(cudaStreamSynchronize(s));
   *out = h->adler;

@@ -200,3 +200,33 @@ def test_odd_resident_calls_wait_for_no_other_thread(bflib, cuda):
     assert bflib.last_kernel() == "simt" and took < 0.3, took
     cuda.cuda.synchronize()
     assert cuda.equal(J, want)
+
+
+def test_threads_that_end_wait_for_no_other_stream(bflib, cuda):
+    """A thread whose only call reads the status of an idle stream is not held up by
+    another stream's work (a stalled launch, which gives up after 1.5 s), neither in
+    the call nor at its end."""
+    import ctypes
+    import time
+
+    d, E, A, G, _ = _set(bflib, cuda, (64, 1, 64, 2, 40), 14)
+    J = cuda.empty(d.jsize, dtype=cuda.uint8, device="cuda")
+    s1, s2 = cuda.cuda.Stream(), cuda.cuda.Stream()
+    libc = ctypes.CDLL(None)
+    libc.pthread_create.argtypes = [ctypes.POINTER(ctypes.c_void_p)] + 3 * [ctypes.c_void_p]
+    libc.pthread_join.argtypes = [ctypes.c_void_p, ctypes.POINTER(ctypes.c_void_p)]
+    status = ctypes.cast(bflib.lib().bf_stream_status, ctypes.c_void_p)  # int (void *), as a thread's function
+    bflib.stream_status(s2)
+    bflib.lib().bf_set_test_stall(1)
+    try:
+        bflib.form_beams_ex(d, J, E, A, G, stream=s1)
+    finally:
+        bflib.lib().bf_set_test_stall(0)
+    t0 = time.monotonic()
+    tid, out = ctypes.c_void_p(), ctypes.c_void_p()
+    assert libc.pthread_create(ctypes.byref(tid), None, status, s2.cuda_stream) == 0
+    assert libc.pthread_join(tid, ctypes.byref(out)) == 0
+    took = time.monotonic() - t0
+    with pytest.raises(bflib.BeamformError):
+        bflib.stream_status(s1)
+    assert (out.value or 0) & 0xFFFFFFFF == bflib.OK and took < 0.3, took
