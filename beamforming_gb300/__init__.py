@@ -244,14 +244,13 @@ def _ptr(x, dtype, nbytes_min: int, writable: bool = False) -> tuple[int, int]:
 
 def _stream_handle(stream) -> int | None:
     if stream is None:  # the caller's current torch stream, if torch has been started on the device
-        torch = sys.modules.get("torch")
-        try:
-            if torch is not None and torch.cuda.is_initialized():
-                # what torch.cuda.current_stream().cuda_stream looks up, 3.5 us sooner
-                return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
-        except Exception:
-            pass
-        return None
+        cuda = getattr(sys.modules.get("torch"), "cuda", None)
+        if cuda is None or not cuda.is_initialized():
+            return None
+        # what torch.cuda.current_stream().cuda_stream looks up, 3.5 us sooner where torch has it
+        core = sys.modules["torch"]._C
+        raw, device = getattr(core, "_cuda_getCurrentRawStream", None), getattr(core, "_cuda_getDevice", None)
+        return raw(device()) if raw and device else cuda.current_stream().cuda_stream
     if isinstance(stream, int):
         return stream
     return stream.cuda_stream
