@@ -456,16 +456,6 @@ int64_t chunk_times(const bf_dims &d) {
   return tc * 3 / 2 >= d.ntimes ? d.ntimes : tc;
 }
 
-int num_sms_api() {
-  static const int n = [] {
-    int dev = 0, v = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-      v = 1;
-    return v > 0 ? v : 1;
-  }();
-  return n;
-}
-
 // Copies bytes [off, off + len) of each of `rows` rows (`pitch` bytes apart)
 // from the device J to the caller's J in pinned host memory (its device
 // mapping): one 16-byte load and streaming store per step, so a warp writes
@@ -565,7 +555,7 @@ int run_host_pipelined(DeviceCtx &c, const bf_dims &d, uint8_t *J, const uint8_t
       BF_TRY(launch_simt(dc, Jc, l.E.as<uint8_t>(), c.A.as<uint8_t>(), c.G.as<float>(), l.s, T, a_layout, j_layout));
     }
     if (jmap) {
-      const int grid = 2 * std::max(1, num_sms_api());
+      const int grid = 2 * num_sms();
       drain_rows<<<grid, 256, 0, l.s>>>(c.J.as<uint8_t>(), jmap, jrows, jpitch, t0 * jscale, nt * jscale);
       BF_TRY(cudaGetLastError());
     }

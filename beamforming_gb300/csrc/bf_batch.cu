@@ -23,6 +23,7 @@ namespace {
 // One grouped launch of a batch: a range of the device problem table.
 struct BatchLaunch {
   int first = 0, nprob = 0, ntiles = 0, max_nb_pass = 0, stages = 0, groups = 0, ctas_per_sm = 0;
+  bool pair = false;      // on pairs of SMs
   bool two_pass = false;  // of two beam passes, some of them
 };
 constexpr int kMaxLaunches = 3;  // one per pass-width class
@@ -84,29 +85,30 @@ int launch_of(int cls, int cuts) { return (cls >= 1 && (cuts & 1)) + (cls >= 2 &
 
 // Problems in `order`, one launch per group of classes that `cuts` keeps
 // together (wider classes first); empty launches are dropped.
-Schedule schedule_of(const std::vector<Records> &probs, const std::vector<int> &order, int cuts) {
-  Schedule sc;
+cudaError_t schedule_of(Schedule &sc, const std::vector<Records> &probs, const std::vector<int> &order, int cuts) {
+  sc = Schedule{};
   for (int l = 0; l < kMaxLaunches; ++l) {
     BatchLaunch L;
     L.first = static_cast<int>(sc.table.size());
     for (int i : order)
       if (launch_of(class_of(probs[i].one), cuts) == l) L.max_nb_pass = std::max(L.max_nb_pass, probs[i].one.nb_pass);
-    const bool pair = tc_pair_launch(L.max_nb_pass);
+    const cudaError_t e = tc_pair_launch(L.max_nb_pass, &L.pair);
+    if (e != cudaSuccess) return e;
     int64_t begin = 0;
     for (int i : order) {
       if (launch_of(class_of(probs[i].one), cuts) != l) continue;
-      TcProblem P = pair ? probs[i].pair : probs[i].one;
+      TcProblem P = L.pair ? probs[i].pair : probs[i].one;
       P.tile_begin = static_cast<int>(begin);
       L.two_pass |= P.npass == 2;
       begin += tc_problem_tiles(P);
       sc.table.push_back(P);
     }
-    sc.ring_plans |= !pair && static_cast<int>(sc.table.size()) > L.first;
+    sc.ring_plans |= !L.pair && static_cast<int>(sc.table.size()) > L.first;
     L.nprob = static_cast<int>(sc.table.size()) - L.first;
     L.ntiles = static_cast<int>(begin);
     if (L.nprob > 0) sc.launches[sc.nlaunch++] = L;
   }
-  return sc;
+  return cudaSuccess;
 }
 
 // The device error word after the tuning launches: a bounded wait that gave
@@ -124,8 +126,8 @@ int take_device_error(int *err, cudaStream_t s) {
 cudaError_t launch_schedule(const bf_batch *b, const BatchLaunch *ls, int n, const TcRingPlan &plan,
                             cudaStream_t s) {
   for (int i = 0; i < n; ++i) {
-    const cudaError_t e =
-        launch_tc_grouped(b->table + ls[i].first, ls[i].nprob, ls[i].ntiles, b->D, ls[i].max_nb_pass, ls[i].two_pass, plan, b->err, s);
+    const cudaError_t e = launch_tc_grouped(b->table + ls[i].first, ls[i].nprob, ls[i].ntiles, b->D, ls[i].max_nb_pass,
+                                            ls[i].pair, ls[i].two_pass, plan, b->err, s);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
@@ -193,8 +195,9 @@ int bf_batch_create(bf_batch **out, const bf_problem *problems, int nproblems, b
   for (int cuts = 0; cuts < 4 && st == BF_OK; ++cuts) {
     if (((cuts & 1) && !cut_ok[0]) || ((cuts & 2) && !cut_ok[1])) continue;
     for (int o = 0; o < 2 && st == BF_OK; ++o) {
-      const Schedule sc = schedule_of(probs, *orders[o], cuts);
-      cudaError_t e = cudaMemcpyAsync(b->table, sc.table.data(), sizeof(TcProblem) * sc.table.size(),
+      Schedule sc;
+      cudaError_t e = schedule_of(sc, probs, *orders[o], cuts);
+      if (e == cudaSuccess) e = cudaMemcpyAsync(b->table, sc.table.data(), sizeof(TcProblem) * sc.table.size(),
                                       cudaMemcpyHostToDevice, s);
       for (int pl = 0; pl < (sc.ring_plans ? 3 : 1) && e == cudaSuccess; ++pl) {
         e = launch_schedule(b, sc.launches, sc.nlaunch, plans[pl], s);  // warm-up
@@ -219,7 +222,8 @@ int bf_batch_create(bf_batch **out, const bf_problem *problems, int nproblems, b
   cudaEventDestroy(e1);
   if (st == BF_OK) st = take_device_error(err, s);
   if (st == BF_OK) {
-    const Schedule sc = schedule_of(probs, *orders[b->order], b->cuts);
+    Schedule sc;
+    cudaError_t e = schedule_of(sc, probs, *orders[b->order], b->cuts);
     b->tuned_ms = best / 3.0f;
     b->nlaunch = sc.nlaunch;
     b->ntiles = 0;
@@ -227,11 +231,11 @@ int bf_batch_create(bf_batch **out, const bf_problem *problems, int nproblems, b
       b->launches[i] = sc.launches[i];
       b->ntiles += sc.launches[i].ntiles;
       BatchLaunch &L = b->launches[i];
-      if (tc_launch_shape(D, L.max_nb_pass, b->plan, &L.stages, &L.groups, &L.ctas_per_sm) != cudaSuccess)
+      if (tc_launch_shape(D, L.max_nb_pass, L.pair, b->plan, &L.stages, &L.groups, &L.ctas_per_sm) != cudaSuccess)
         st = BF_ERR_UNSUPPORTED;
     }
-    cudaError_t e = cudaMemcpyAsync(b->table, sc.table.data(), sizeof(TcProblem) * sc.table.size(),
-                                    cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(b->table, sc.table.data(), sizeof(TcProblem) * sc.table.size(), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     // capture the chosen launches in a graph
     cudaStream_t cap = nullptr;

@@ -223,7 +223,7 @@ struct TcRingPlan {
 };
 
 // Whether a launch whose widest pass has max_nb_pass beams runs on pairs of SMs.
-bool tc_pair_launch(int max_nb_pass);
+cudaError_t tc_pair_launch(int max_nb_pass, bool *pair);
 // Fills a problem record (tile_begin left 0) for T times of E with weights w,
 // for a launch on pairs of SMs or not.
 cudaError_t tc_make_problem(TcProblem &P, const TcWeights &w, int64_t T, uint8_t *J, const uint8_t *E,
@@ -233,10 +233,10 @@ int64_t tc_problem_tiles(const TcProblem &P);
 int tc_stages_per_tile(int64_t D);
 
 // One persistent launch over nprob problems (records in device memory; all
-// with D dishes).  max_nb_pass = the largest nb_pass among them; two_pass: some
-// have two passes.
+// with D dishes), made for pairs of SMs or not.  max_nb_pass = the largest nb_pass
+// among them; two_pass: some have two passes.
 cudaError_t launch_tc_grouped(const TcProblem *table, int nprob, int ntiles, int64_t D, int max_nb_pass,
-                              bool two_pass, const TcRingPlan &plan, int *err, cudaStream_t s);
+                              bool pair, bool two_pass, const TcRingPlan &plan, int *err, cudaStream_t s);
 
 // The whole ring layout of a launch with these sizes: out[0..11] = stages,
 // W slots, raw E slots, unpack groups, CTAs per SM, K stages per tile,
@@ -245,9 +245,12 @@ cudaError_t launch_tc_grouped(const TcProblem *table, int nprob, int ntiles, int
 // the last TMEM column a stage uses.
 cudaError_t tc_plan_rings(int64_t D, int max_nb_pass, const TcRingPlan &plan, int *out);
 
+// SMs of the device.
+int num_sms();
+
 // Pair launches (bf_tc_pair.cu): clusters of two CTAs the device runs at once
 // (0: none), the GEMM N of a pass, the TMEM stages of a launch, and the launches.
-int pair_clusters();
+cudaError_t pair_clusters(int *n);
 int pair_cols(int nb_pass);
 cudaError_t pair_launch_shape(int64_t D, int max_nb_pass, int groups, int *stages);
 cudaError_t launch_pair(const TcProblem &one, int64_t D, int test_stall, int *err, cudaStream_t s);
@@ -255,7 +258,7 @@ cudaError_t launch_pair_grouped(const TcProblem *table, int nprob, int ntiles, i
                                 int groups, int test_stall, int *err, cudaStream_t s);
 
 // TMEM stages, unpack groups and CTAs per SM of a grouped launch with these sizes.
-cudaError_t tc_launch_shape(int64_t D, int max_nb_pass, const TcRingPlan &plan, int *stages, int *groups,
+cudaError_t tc_launch_shape(int64_t D, int max_nb_pass, bool pair, const TcRingPlan &plan, int *stages, int *groups,
                             int *ctas_per_sm);
 
 // Beam passes of at most kNarrowPass beams leave room for four or more
@@ -269,10 +272,6 @@ constexpr int kHalfPass = 16;
 // Failure-path test hook: nonzero makes the producer of later tensor-core
 // launches issue nothing, so the kernel's bounded waits expire.
 void tc_set_test_stall(int on);
-
-// Shared-memory ring depths of the tensor-core kernel (0 = planner default):
-// W slots and raw E slots.
-void tc_set_ring_plan(int wslots, int raw);
 
 // Checksum ----------------------------------------------------------------------
 // Partial adler sums over chunks; `partials` holds 2 * nchunks uint32.

@@ -218,7 +218,8 @@ void CUDART_CB flight_landed(void *arg) {
 // host function that marks the flight landed.  Runs without the mutex.
 bool bf_server::launch(Flight &fl, const std::vector<Request> &reqs, int *ntiles) {
   const TcWeights &w = weights->tc;
-  const bool pair = tc_pair_launch(w.nb_pass);
+  bool pair = false;
+  if (tc_pair_launch(w.nb_pass, &pair) != cudaSuccess) return false;
   int64_t begin = 0;
   unsigned waited = 0;  // versions whose refresh this stream already waits for
   for (size_t i = 0; i < reqs.size(); ++i) {
@@ -241,8 +242,8 @@ bool bf_server::launch(Flight &fl, const std::vector<Request> &reqs, int *ntiles
   if (cudaMemcpyAsync(fl.table_dev, fl.table_host, sizeof(TcProblem) * n, cudaMemcpyHostToDevice, fl.s) !=
       cudaSuccess)
     return false;
-  if (launch_tc_grouped(fl.table_dev, n, static_cast<int>(begin), w.D, w.nb_pass, w.npass == 2, TcRingPlan{}, fl.err_dev,
-                        fl.s) != cudaSuccess)
+  if (launch_tc_grouped(fl.table_dev, n, static_cast<int>(begin), w.D, w.nb_pass, pair, w.npass == 2, TcRingPlan{},
+                        fl.err_dev, fl.s) != cudaSuccess)
     return false;
   if (cudaMemcpyAsync(fl.err_host, fl.err_dev, sizeof(int), cudaMemcpyDeviceToHost, fl.s) != cudaSuccess)
     return false;

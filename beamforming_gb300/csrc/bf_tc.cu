@@ -55,6 +55,7 @@
 // RowMap.  TMEM columns: accumulators at [0, N) and [256, 256 + N), unpacked
 // E stages (64 columns = 256 K bytes each) in the remaining columns.
 #include "bf_internal.h"
+#include "bf_once.h"
 #include "bf_tc_common.cuh"
 
 #include <algorithm>
@@ -822,27 +823,21 @@ bool make_map(CUtensorMap *m, const void *base, int rank, const cuuint64_t *dims
 }
 
 int g_test_stall = 0;
-int g_plan_wslots = 0;  // nonzero: W slots to use (tuning)
-int g_plan_raw = 0;     // nonzero: raw E slots to use (tuning)
-
-int num_sms() {
-  static const int n = []() {
-    int dev = 0, k = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&k, cudaDevAttrMultiProcessorCount, dev);
-    return k > 0 ? k : 1;
-  }();
-  return n;
-}
 
 }  // namespace
 
-void tc_set_test_stall(int on) { g_test_stall = on; }
-
-void tc_set_ring_plan(int wslots, int raw) {
-  g_plan_wslots = wslots;
-  g_plan_raw = raw;
+int num_sms() {
+  static AskedOnce<int> asked;
+  int n = 1;
+  (void)asked.get(&n, [](int *k) {
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    return e != cudaSuccess ? e : cudaDeviceGetAttribute(k, cudaDevAttrMultiProcessorCount, dev);
+  });
+  return n;
 }
+
+void tc_set_test_stall(int on) { g_test_stall = on; }
 
 void tc_plan_beams(int64_t B, int *nb_pass, int *npass, int granule) {
   // at most 96 beams (192 accumulator columns) per pass, so that two
@@ -1062,13 +1057,11 @@ static cudaError_t plan_launch(TcParams &p, int max_nb_pass, const TcRingPlan &p
   // so at least S slots keep it moving.
   const int groups = stages >= 4 && !half ? 2 : 1;  // the half-SM layout has one group
   // shared memory: W slots first (their loads gate the MMA), then raw E slots
-  const int want_w = plan.wslots > 0 ? plan.wslots : g_plan_wslots;
-  const int want_r = plan.raw > 0 ? plan.raw : g_plan_raw;
-  int wslots = want_w > 0 ? want_w : kMaxWSlots;
+  int wslots = plan.wslots > 0 ? plan.wslots : kMaxWSlots;
   if (groups == 2) wslots = std::min(wslots, stages);
-  int raw = want_r > 0 ? want_r : kMinRaw;
+  int raw = plan.raw > 0 ? plan.raw : kMinRaw;
   while (wslots > 2 && smem_plan(stages, wslots, raw, max_nb_pass).total + 1024 > smem_limit) --wslots;
-  while (raw < kMaxRaw && smem_plan(stages, wslots, raw + 1, max_nb_pass).total + 1024 <= smem_limit && want_r <= 0)
+  while (raw < kMaxRaw && smem_plan(stages, wslots, raw + 1, max_nb_pass).total + 1024 <= smem_limit && plan.raw <= 0)
     ++raw;
   while (raw > 2 && smem_plan(stages, wslots, raw, max_nb_pass).total + 1024 > smem_limit) --raw;
   // Two groups take alternate sequences, and raw slot k % R serves sequences
@@ -1144,7 +1137,12 @@ static cudaError_t launch_kernel(const TcParams &p, int smem_bytes, cudaStream_t
 // Passes of at most kHalfPass beams run two CTAs on each SM instead: their MMAs
 // take a few cycles, so two of everything else on an SM is worth more than
 // sharing W (b = 16: DRAM at 0.87 of the copy bandwidth).
-bool tc_pair_launch(int max_nb_pass) { return max_nb_pass > kHalfPass && pair_clusters() > 0; }
+cudaError_t tc_pair_launch(int max_nb_pass, bool *pair) {
+  int clusters = 0;
+  const cudaError_t e = max_nb_pass > kHalfPass ? pair_clusters(&clusters) : cudaSuccess;
+  *pair = clusters > 0;
+  return e;
+}
 
 cudaError_t tc_make_problem(TcProblem &P, const TcWeights &w, int64_t T, uint8_t *J, const uint8_t *E,
                             int64_t jpitch, int j_layout, bool pair) {
@@ -1189,9 +1187,9 @@ static int pair_groups(int max_nb_pass, const TcRingPlan &plan) {
   return plan.one_group && max_nb_pass > kNarrowPass ? 1 : 2;
 }
 
-cudaError_t tc_launch_shape(int64_t D, int max_nb_pass, const TcRingPlan &plan, int *stages, int *groups,
+cudaError_t tc_launch_shape(int64_t D, int max_nb_pass, bool pair, const TcRingPlan &plan, int *stages, int *groups,
                             int *ctas_per_sm) {
-  if (tc_pair_launch(max_nb_pass)) {
+  if (pair) {
     *ctas_per_sm = 1;
     *groups = pair_groups(max_nb_pass, plan);
     return pair_launch_shape(D, max_nb_pass, *groups, stages);
@@ -1208,8 +1206,8 @@ cudaError_t tc_launch_shape(int64_t D, int max_nb_pass, const TcRingPlan &plan, 
 }
 
 cudaError_t launch_tc_grouped(const TcProblem *table, int nprob, int ntiles, int64_t D, int max_nb_pass,
-                              bool two_pass, const TcRingPlan &plan, int *err, cudaStream_t s) {
-  if (tc_pair_launch(max_nb_pass))
+                              bool pair, bool two_pass, const TcRingPlan &plan, int *err, cudaStream_t s) {
+  if (pair)
     return launch_pair_grouped(table, nprob, ntiles, D, max_nb_pass, two_pass, pair_groups(max_nb_pass, plan),
                                g_test_stall, err, s);
   TcParams p{};
@@ -1228,8 +1226,10 @@ cudaError_t launch_tc(const TcWeights &w, int64_t T, uint8_t *J, const uint8_t *
                       int64_t jpitch, int j_layout, unsigned long long *adler, const uint8_t *jbase,
                       const TcRows *rows) {
   TcParams p{};
-  const bool pair = tc_pair_launch(w.nb_pass);
-  cudaError_t e = make_problem(p.one, w, T, J, E, jpitch, j_layout, pair);
+  bool pair = false;
+  cudaError_t e = tc_pair_launch(w.nb_pass, &pair);
+  if (e != cudaSuccess) return e;
+  e = make_problem(p.one, w, T, J, E, jpitch, j_layout, pair);
   if (e != cudaSuccess) return e;
   p.one.adler = adler;
   if (jbase) p.one.jbase = jbase;

@@ -36,6 +36,7 @@
 //                in short bursts).  More warps only contend for the integer pipe
 //                (16 unpack warps 712, 12 epilogue warps 693 us).
 #include "bf_internal.h"
+#include "bf_once.h"
 #include "bf_tc_common.cuh"
 
 #include <algorithm>
@@ -645,7 +646,11 @@ cudaError_t launch_inst(const PairParams &p, int smem_bytes, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     attr_set.store(true);
   }
-  const int grid = 2 * std::min(p.ntiles, pair_clusters());
+  int clusters = 0;
+  const cudaError_t e = pair_clusters(&clusters);
+  if (e != cudaSuccess) return e;
+  if (clusters <= 0) return cudaErrorInvalidConfiguration;
+  const int grid = 2 * std::min(p.ntiles, clusters);
   if (grid <= 0) return cudaSuccess;
   return launch_overlapped(kern, grid, kPairThreads, smem_bytes, s, p);
 }
@@ -664,17 +669,14 @@ cudaError_t launch_plain(const PairParams &p, int smem_bytes, cudaStream_t s) {
 
 int pair_cols(int nb_pass) { return (2 * nb_pass + 31) / 32 * 32; }
 
-int pair_clusters() {
-  static const int n = []() {
+cudaError_t pair_clusters(int *n) {
+  static AskedOnce<int> asked;
+  return asked.get(n, [](int *k) {
     int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-      return 0;
     auto kern = bf_form_beams_pair<false, false, false, 2, true>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem) != cudaSuccess) {
-      (void)cudaGetLastError();
-      return 0;
-    }
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(2);
     cfg.blockDim = dim3(kPairThreads);
@@ -685,14 +687,11 @@ int pair_clusters() {
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    int k = 0;
-    if (cudaOccupancyMaxActiveClusters(&k, kern, &cfg) != cudaSuccess) {
-      (void)cudaGetLastError();
-      return 0;
-    }
-    return std::min(k, sms / 2);
-  }();
-  return n;
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(k, kern, &cfg);
+    *k = std::min(*k, sms / 2);
+    if (e != cudaSuccess) (void)cudaGetLastError();
+    return e;
+  });
 }
 
 cudaError_t pair_launch_shape(int64_t D, int max_nb_pass, int groups, int *stages) {
