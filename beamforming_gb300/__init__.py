@@ -51,6 +51,7 @@ EXPORTED_SYMBOLS = (
     "bf_set_kernel",
     "bf_plan_rings",
     "bf_set_test_stall",
+    "bf_set_test_one_cta",
     "bf_last_kernel",
     "bf_weights_create",
     "bf_weights_update",
@@ -163,6 +164,7 @@ def lib() -> ctypes.CDLL:
         L.bf_plan_rings.argtypes = [ctypes.c_int64, ctypes.c_int, ctypes.c_int, ctypes.c_int,
                                     ctypes.POINTER(ctypes.c_int)]
         L.bf_set_test_stall.argtypes = [ctypes.c_int]
+        L.bf_set_test_one_cta.argtypes = [ctypes.c_int]
         L.bf_last_kernel.argtypes = []
         L.bf_last_kernel.restype = ctypes.c_char_p
         L.bf_weights_create.argtypes = [
@@ -366,6 +368,11 @@ def set_test_stall(on: bool) -> None:
     """Failure-path test hook: tensor-core launches issue no copies while on,
     so their bounded waits expire and the call raises ERR_DEVICE_TIMEOUT."""
     _check(lib().bf_set_test_stall(1 if on else 0), "bf_set_test_stall")
+
+
+def set_test_one_cta(on: bool) -> None:
+    """Test hook: tensor-core launches keep off pairs of SMs while on."""
+    _check(lib().bf_set_test_one_cta(1 if on else 0), "bf_set_test_one_cta")
 
 
 def last_kernel() -> str:

@@ -631,6 +631,11 @@ int bf_set_test_stall(int on) {
   return BF_OK;
 }
 
+int bf_set_test_one_cta(int on) {
+  tc_set_test_one_cta(on);
+  return BF_OK;
+}
+
 int bf_form_beams_ex(const bf_dims *dims, uint8_t *J, const uint8_t *E, const uint8_t *A, const float *G,
                      int ptr_kind, bf_stream_t stream) {
   return bf_form_beams_layout(dims, J, E, A, G, BF_A_LINEAR, BF_J_LINEAR, ptr_kind, stream);

@@ -273,6 +273,10 @@ constexpr int kHalfPass = 16;
 // launches issue nothing, so the kernel's bounded waits expire.
 void tc_set_test_stall(int on);
 
+// Test hook: nonzero keeps launches planned from then on off pairs of SMs, as on a
+// device with no room for a cluster of two.
+void tc_set_test_one_cta(int on);
+
 // Checksum ----------------------------------------------------------------------
 // Partial adler sums over chunks; `partials` holds 2 * nchunks uint32.
 int adler_nchunks(size_t len);

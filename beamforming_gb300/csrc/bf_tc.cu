@@ -823,6 +823,7 @@ bool make_map(CUtensorMap *m, const void *base, int rank, const cuuint64_t *dims
 }
 
 int g_test_stall = 0;
+std::atomic<int> g_test_one_cta{0};
 
 }  // namespace
 
@@ -838,6 +839,7 @@ int num_sms() {
 }
 
 void tc_set_test_stall(int on) { g_test_stall = on; }
+void tc_set_test_one_cta(int on) { g_test_one_cta.store(on); }
 
 void tc_plan_beams(int64_t B, int *nb_pass, int *npass, int granule) {
   // at most 96 beams (192 accumulator columns) per pass, so that two
@@ -1140,7 +1142,7 @@ static cudaError_t launch_kernel(const TcParams &p, int smem_bytes, cudaStream_t
 cudaError_t tc_pair_launch(int max_nb_pass, bool *pair) {
   int clusters = 0;
   const cudaError_t e = max_nb_pass > kHalfPass ? pair_clusters(&clusters) : cudaSuccess;
-  *pair = clusters > 0;
+  *pair = clusters > 0 && !g_test_one_cta.load();
   return e;
 }
 

@@ -124,6 +124,11 @@ BF_API int bf_set_kernel(int kernel);
  * out of bounds and the CUDA context stays usable. */
 BF_API int bf_set_test_stall(int on);
 
+/* Test hook: while `on` is nonzero, tensor-core launches (and batches created)
+ * run one CTA per tile at every beam pass width, as on a device that has no
+ * room for a cluster of two SMs. */
+BF_API int bf_set_test_one_cta(int on);
+
 /* Name of the kernel family the last launch on this thread used:
  * "tensor", "simt" or "none". */
 BF_API const char *bf_last_kernel(void);
