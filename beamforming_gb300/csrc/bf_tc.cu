@@ -455,7 +455,10 @@ __global__ void __launch_bounds__(Roles<kEpiW, kGroups>::kThreads, kHalf ? 2 : 1
                      kSums ? 1u : 0u);
           mma_commit(d_empty(ds));
         };
-        if (!kSums && elect_one()) offset_mma();
+        if constexpr (!kSums) {
+          if (elect_one()) offset_mma();
+          ++ndig;  // with its commit: the tile may end early
+        }
         __syncwarp();
         for (int ks = 0; ks < p.nk; ++ks, ar.advance(), wr.advance()) {
           const int s = static_cast<int>(ar.idx);
@@ -480,12 +483,12 @@ __global__ void __launch_bounds__(Roles<kEpiW, kGroups>::kThreads, kHalf ? 2 : 1
           if (!__all_sync(0xffffffffu, mbar_wait(rs_full(ab), aph, err, kDevTimeoutUnpacked))) break;
           tc_fence_after();
         }
-        if (elect_one()) {
-          if constexpr (kSums) offset_mma();
-          mma_commit(accfull(ab));
+        if constexpr (kSums) {
+          if (elect_one()) offset_mma();
+          ++ndig;
         }
+        if (elect_one()) mma_commit(accfull(ab));
         __syncwarp();
-        ++ndig;
         dr.advance();
         ++nacc;
       }

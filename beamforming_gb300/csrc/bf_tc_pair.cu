@@ -411,7 +411,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
                         kSums ? 1u : 0u);
         if (last) mma_commit_pair(d_empty(ds));
       };
-      if (!kSums && elect_one()) offset_mma();
+      if constexpr (!kSums) {
+        if (elect_one()) offset_mma();
+        ndig += last ? 1u : 0u;  // with its commit: the tile may end early
+      }
       __syncwarp();
       if (!fresh && !last && !stream_w) {
         uint64_t b_desc = w_desc0 + static_cast<uint32_t>(w0) * w_step;
@@ -468,12 +471,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
         if (!__all_sync(0xffffffffu, mbar_wait(rs_full(ab), (local >> 1) & 1u, err, kDevTimeoutUnpacked))) break;
         tc_fence_after();
       }
-      if (elect_one()) {
-        if constexpr (kSums) offset_mma();
-        mma_commit_pair(accfull(ab));
+      if constexpr (kSums) {
+        if (elect_one()) offset_mma();
+        ndig += last ? 1u : 0u;
       }
+      if (elect_one()) mma_commit_pair(accfull(ab));
       __syncwarp();
-      if (last) ++ndig;
       ++nacc;
     }
     // A commit's arrival is an asynchronous write into both CTAs' shared memory:

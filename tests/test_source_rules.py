@@ -55,3 +55,16 @@ def test_overlapped_kernels_use_plain_loads():
     assert launched == {"kern", "bf_pad_e", "write_words"}  # `kern`: of the files above
     head = re.search(r"\bwrite_words\(([^)]*)\)\s*\{", _source("bf_adler.cu"))
     assert "__restrict__" not in head.group(1)
+
+
+@pytest.mark.parametrize("name,kernel", [("bf_tc.cu", "bf_form_beams_tc"), ("bf_tc_pair.cu", "bf_form_beams_pair")])
+def test_commits_are_counted_where_they_are_issued(name, kernel):
+    """The issuer waits at its end for the commits that it counted.  A wait that gives
+    up ends a tile early, so no wait may lie between a commit and its count: the arrival
+    that was left out would land in the shared memory of a CTA that has gone."""
+    body = _body(_source(name), kernel)
+    calls = [m.end() for m in re.finditer(r"\boffset_mma\(\);", body)]
+    assert len(calls) == 2
+    for at in calls:
+        until = re.search(r"\bmbar_wait\(|\bmbar_wait_drain\(", body[at:]).start()
+        assert "ndig" in body[at:at + until]
