@@ -50,6 +50,7 @@ EXPORTED_SYMBOLS = (
     "bf_stream_status",
     "bf_set_kernel",
     "bf_plan_rings",
+    "bf_plan_pair",
     "bf_set_test_stall",
     "bf_set_test_one_cta",
     "bf_last_kernel",
@@ -163,6 +164,7 @@ def lib() -> ctypes.CDLL:
         L.bf_set_kernel.argtypes = [ctypes.c_int]
         L.bf_plan_rings.argtypes = [ctypes.c_int64, ctypes.c_int, ctypes.c_int, ctypes.c_int,
                                     ctypes.POINTER(ctypes.c_int)]
+        L.bf_plan_pair.argtypes = [ctypes.c_int64, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.POINTER(ctypes.c_int)]
         L.bf_set_test_stall.argtypes = [ctypes.c_int]
         L.bf_set_test_one_cta.argtypes = [ctypes.c_int]
         L.bf_last_kernel.argtypes = []
@@ -358,6 +360,17 @@ def plan_rings(ndishes: int, max_nb_pass: int, wslots: int = 0, raw: int = 0) ->
         return None
     return dict(zip(("stages", "wslots", "raw", "groups", "ctas_per_sm", "nk", "smem_bytes", "tmem_cols",
                      "acc_cols", "acc2_col", "stages_per_acc", "stage_end_col"), list(out)))
+
+
+def plan_pair(ndishes: int, max_nb_pass: int, two_pass: bool = False, groups: int = 2) -> dict | None:
+    """The layout of a launch on pairs of SMs (host only, no GPU), or None where
+    none fits: as plan_rings, with the passes whose digit rows (and W, unless W is
+    a ring) stay resident and whether the passes of a tile share its operand."""
+    out = (ctypes.c_int * 12)()
+    if lib().bf_plan_pair(ndishes, max_nb_pass, 1 if two_pass else 0, groups, out) != 0:
+        return None
+    return dict(zip(("stages", "wslots", "raw", "sets", "share", "nk", "smem_bytes", "tmem_cols", "acc_cols",
+                     "acc2_col", "stages_per_acc", "stage_end_col"), list(out)))
 
 
 def set_kernel(kind: str) -> None:

@@ -282,6 +282,13 @@ int bf_plan_rings(int64_t ndishes, int max_nb_pass, int wslots, int raw, int *ou
   return bf::tc_plan_rings(ndishes, max_nb_pass, plan, out) == cudaSuccess ? BF_OK : BF_ERR_INVALID_ARGUMENT;
 }
 
+int bf_plan_pair(int64_t ndishes, int max_nb_pass, int two_pass, int groups, int *out) {
+  if (!out || ndishes <= 0 || ndishes > 2048 || max_nb_pass <= kHalfPass || max_nb_pass > 128 || groups < 1 ||
+      groups > 2 || (groups == 1 && max_nb_pass <= kNarrowPass))
+    return BF_ERR_INVALID_ARGUMENT;
+  return bf::pair_plan(ndishes, max_nb_pass, two_pass != 0, groups, out) == cudaSuccess ? BF_OK : BF_ERR_INVALID_ARGUMENT;
+}
+
 int bf_batch_shape(const bf_batch *b, int *nlaunches, int *nproblems, int *ntiles, int *max_nb_pass, int *stages,
                    int *unpack_groups, int *ctas_per_sm) {
   if (!b || !nlaunches) return BF_ERR_INVALID_ARGUMENT;

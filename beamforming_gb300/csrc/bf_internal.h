@@ -253,6 +253,8 @@ int num_sms();
 cudaError_t pair_clusters(int *n);
 int pair_cols(int nb_pass);
 cudaError_t pair_launch_shape(int64_t D, int max_nb_pass, int groups, int *stages);
+// (out[0..11] of bf_plan_pair)
+cudaError_t pair_plan(int64_t D, int max_nb_pass, bool two_pass, int groups, int *out);
 cudaError_t launch_pair(const TcProblem &one, int64_t D, int test_stall, int *err, cudaStream_t s);
 cudaError_t launch_pair_grouped(const TcProblem *table, int nprob, int ntiles, int64_t D, int max_nb_pass, bool two_pass,
                                 int groups, int test_stall, int *err, cudaStream_t s);

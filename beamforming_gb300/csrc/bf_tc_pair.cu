@@ -46,6 +46,7 @@ namespace bf {
 namespace {
 
 constexpr int kPairAcc = 256;        // TMEM column of the second accumulator
+constexpr int kPairCols = 512;       // TMEM columns of a CTA: all
 constexpr int kPairSmem = 232448;    // 227 KiB opt-in per block
 constexpr int kPairMaxRaw = 16;
 constexpr int kPairMaxStages = 8;
@@ -226,7 +227,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
   fence_barrier_init();
   __syncwarp();  // a producer's lane 0 uses barriers that its other lanes set up, and waits for no other warp
   if (warp == kMmaWarp) {
-    tmem_alloc_pair(smem_u32(tmem_holder), 512);
+    tmem_alloc_pair(smem_u32(tmem_holder), kPairCols);
     tmem_relinquish_pair();
   }
   fill_offset_tiles<kSums ? 2 : 1>(sA);
@@ -602,7 +603,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     if (rank == 1) drain_commits(counts[0], counts[1], counts[2], counts[3]);
     __syncwarp();
     tc_fence_after();
-    tmem_dealloc_pair(*tmem_holder, 512);
+    tmem_dealloc_pair(*tmem_holder, kPairCols);
   }
 }
 
@@ -703,6 +704,21 @@ cudaError_t pair_launch_shape(int64_t D, int max_nb_pass, int groups, int *stage
   const cudaError_t e = plan_pair(p, D, max_nb_pass, false, groups, &smem_bytes);
   *stages = p.stages;
   return e;
+}
+
+cudaError_t pair_plan(int64_t D, int max_nb_pass, bool two_pass, int groups, int *out) {
+  PairParams p{};
+  int smem_bytes = 0;
+  const cudaError_t e = plan_pair(p, D, max_nb_pass, two_pass, groups, &smem_bytes);
+  if (e != cudaSuccess) return e;
+  const int per_half = (kPairAcc - p.ncols) / kStageCols;  // the kernel's
+  uint32_t last_col = 0;
+  for (int i = 0; i < p.stages; ++i)
+    last_col = std::max(last_col, pair_stage_col(i, p.ncols, per_half, kStageCols) + kStageCols);
+  const int v[12] = {p.stages, p.wslots, p.raw,    p.sets,   p.share,  p.nk,
+                     smem_bytes, kPairCols, p.ncols, kPairAcc, per_half, static_cast<int>(last_col)};
+  std::copy(v, v + 12, out);
+  return cudaSuccess;
 }
 
 cudaError_t launch_pair(const TcProblem &one, int64_t D, int test_stall, int *err, cudaStream_t s) {

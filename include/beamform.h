@@ -213,6 +213,17 @@ BF_API int bf_batch_destroy(bf_batch *batch);
  * reference. */
 BF_API int bf_plan_rings(int64_t ndishes, int max_nb_pass, int wslots, int raw, int *out);
 
+/* The same for a launch on pairs of SMs (passes of more than 16 beams): out[0..11]
+ * = unpacked stages in tensor memory, W slots (fewer than K stages: an ordinary
+ * ring), raw E slots, passes whose digit rows (and W, unless a ring) stay resident,
+ * 1 where the passes of a tile share its unpacked operand, K stages per tile,
+ * dynamic shared memory bytes per CTA, tensor-memory columns allocated per CTA,
+ * columns of each accumulator, column of the second accumulator, stages beside
+ * each accumulator, one past the last column a stage uses.  two_pass: problems of
+ * two passes are among the launch's; groups: unpack warp groups, 2, or 1 in a batch
+ * with passes wider than 64 beams. */
+BF_API int bf_plan_pair(int64_t ndishes, int max_nb_pass, int two_pass, int groups, int *out);
+
 /* Array layouts (for bf_form_beams_layout).  BF_A_LINEAR / BF_J_LINEAR are the
  * reference's A[f][b][d] and J[b][f][p][t] (Alinear, Jlinear; arraysizes.hxx:92,
  * 115) used everywhere else in this API.  BF_A_A2 is the lossy kernel family's
