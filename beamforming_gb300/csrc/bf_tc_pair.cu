@@ -53,6 +53,7 @@ constexpr int kPairMaxStages = 8;
 constexpr int kEpiW = 8;       // epilogue warps
 constexpr int kEpiChunks = 2;  // chunks of 8 beams in flight per epilogue warp
 constexpr int kUnpackWarps = 8;
+constexpr int kCounts = 5;  // what the leader leaves for the peer's exit
 constexpr int kPairThreads = 32 * (kEpiW + kUnpackWarps + 3);
 
 struct PairParams {
@@ -83,9 +84,10 @@ __host__ __device__ inline PairSmem pair_smem(int stages, int wslots, int raw, i
   s.off_r = s.off_d + kDigSlots * s.dbytes;
   s.off_bar = s.off_r + raw * kRawBytes;
   // raw_full[R] raw_empty[R] w_full[SW] w_peer[SW] w_empty[SW] a_full[S] empty[S] accfull[2] accempty[2]
-  // d_full[2] d_peer[2] d_empty[2] rs_full[2]
-  s.nbar = 2 * raw + 3 * wslots + 2 * stages + 4 + 3 * kDigSlots + 2;
+  // d_full[2] d_peer[2] d_empty[2] rs_full[2] cut_done
+  s.nbar = 2 * raw + 3 * wslots + 2 * stages + 4 + 3 * kDigSlots + 3;
   s.total = s.off_bar + 8 * s.nbar + 32;  // + the TMEM address and the leader's commit counts
+  static_assert(4 * (1 + kCounts) <= 32, "they fit");
   return s;
 }
 
@@ -195,8 +197,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
   auto d_peer = [&](int i) { return bc + 48u + 8u * i; };
   auto d_empty = [&](int i) { return bc + 64u + 8u * i; };
   auto rs_full = [&](int i) { return bc + 80u + 8u * i; };
+  const uint32_t cut_done = bc + 96u;  // the MMAs of a tile that a failed wait cut short
   uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(smem + sp.off_bar + 8 * sp.nbar);
-  uint32_t *counts = tmem_holder + 1;  // commits the leader issued on empty, w_empty, d_empty, accfull
+  uint32_t *counts = tmem_holder + 1;  // commits the leader issued on empty, w_empty, d_empty, accfull, cut_done
 
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);  // known to be warp-uniform
   const int lane = threadIdx.x & 31;
@@ -222,7 +225,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     if (lane < 2 * S) mbar_init(a_full(lane), lane < S ? 2 * kStageWarps : 1);
     if (lane < 4) mbar_init(accfull(lane), lane < 2 ? 1 : 2 * kEpiW);
     if (lane < 2) mbar_init(rs_full(lane), 2 * kUnpackWarps);
-    if (lane < 4) counts[lane] = 0;
+    if (lane < kCounts) counts[lane] = 0;
+    if (lane == 0) mbar_init(cut_done, 1);
   }
   fence_barrier_init();
   __syncwarp();  // a producer's lane 0 uses barriers that its other lanes set up, and waits for no other warp
@@ -241,7 +245,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
   };
   static_assert(2 * kPairMaxStages <= 32, "one lane per stage barrier");
   // waits for the last phase committed on every barrier
-  auto drain_commits = [&](uint32_t nstage, uint32_t nw, uint32_t ndig, uint32_t nacc) {
+  auto drain_commits = [&](uint32_t nstage, uint32_t nw, uint32_t ndig, uint32_t nacc, uint32_t cut) {
+    if (cut) mbar_wait_drain(cut_done, 0u);
     const uint32_t uS = static_cast<uint32_t>(S), uW = static_cast<uint32_t>(SW), uD = static_cast<uint32_t>(kDigSlots);
     for (uint32_t k = nstage > uS ? nstage - uS : 0; k < nstage; ++k)
       mbar_wait_drain(empty(static_cast<int>(k % uS)), (k / uS) & 1u);
@@ -387,7 +392,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     int w_at[2] = {0, 0}, d_at[2] = {0, 0};  // first W slot and digit slot of even and odd passes
     Ring a0(S);                              // the first stage of the tile's operand
     PairCursor<kGrouped> cur(p, first);
-    for (int tile = first; ok && tile < end; ++tile, ++local, cur.next(p)) {
+    int tile = first;
+    for (; ok && tile < end; ++tile, ++local, cur.next(p)) {
       const uint32_t idesc = idesc_e4m3_f32(2 * kBM, static_cast<uint32_t>(cur.n()));
       const uint32_t wbox = static_cast<uint32_t>(cur.P->w_rows * kKC) >> 4;
       const bool fresh = cur.first_of_w(tile - first, sets), last = cur.last_of_w(end - tile, sets);
@@ -480,6 +486,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
       __syncwarp();
       ++nacc;
     }
+    // A tile that a failed wait cut short has MMAs that no commit covers (the offset
+    // MMA, stages that the next pass would read too): one more commit does.
+    const uint32_t cut = tile < end ? 1u : 0u;
+    if (cut && elect_one()) mma_commit_pair(cut_done);
+    __syncwarp();
     // A commit's arrival is an asynchronous write into both CTAs' shared memory:
     // wait (bounded) for the last phase committed on every barrier before the
     // CTAs can exit, here and, from the counts, in the peer.
@@ -489,8 +500,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
       st_cluster_u32(at + 4, nw);
       st_cluster_u32(at + 8, ndig);
       st_cluster_u32(at + 12, nacc);
+      st_cluster_u32(at + 16, cut);
     }
-    drain_commits(nstage, nw, ndig, nacc);
+    drain_commits(nstage, nw, ndig, nacc, cut);
     __syncwarp();
   } else if (warp >= kUnpackWarp0 && warp < kEProdWarp) {
     // ------------------------------------------------------------ unpack
@@ -600,7 +612,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
   tc_fence_before();
   cluster_sync();
   if (warp == kMmaWarp) {
-    if (rank == 1) drain_commits(counts[0], counts[1], counts[2], counts[3]);
+    if (rank == 1) drain_commits(counts[0], counts[1], counts[2], counts[3], counts[4]);
     __syncwarp();
     tc_fence_after();
     tmem_dealloc_pair(*tmem_holder, kPairCols);

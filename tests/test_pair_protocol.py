@@ -150,7 +150,8 @@ class Pair(Model):
         self.readers, self.events, self.mma_queue, self.commits = {}, [], [], []
         self.mma_issued = self.mma_done = 0
         self.acc_tile_done = {}
-        self.counts = (0, 0, 0, 0)
+        self.cut_done = [Barrier(f"cut_done@{c}", 1) for c in (0, 1)]
+        self.counts = (0, 0, 0, 0, 0)
         self.planted = None
 
     # ------------------------------------------------------------- slots
@@ -308,7 +309,7 @@ class Pair(Model):
     def issuer(self):
         nk, S, SW = self.nk, self.S, self.SW
         ar = a0 = it = dit = 0
-        nstage = nw = ndig = nacc = 0
+        nstage = nw = ndig = nacc = finished = 0
         w_at, d_at = [0, 0], [0, 0]
         for n, t in enumerate(self.tiles):
             fresh, last = t.first_of_w(n, self.sets), t.last_of_w(len(self.tiles) - n, self.sets)
@@ -342,7 +343,8 @@ class Pair(Model):
                 return int(last)
 
             if not self.sums:
-                ndig += offset()
+                late = offset()
+                ndig += 0 if self.planted == "count" else late
             ok = True
             for ks in range(nk):
                 reload, release = fresh or self.stream, last or self.stream
@@ -371,13 +373,21 @@ class Pair(Model):
                 if not (yield self.wait(self.rs_full[ab], n // 2)):
                     break
                 ndig += offset()
+            elif self.planted == "count":
+                ndig += late
             self.commit([self.accfull[0][ab], self.accfull[1][ab]])
             nacc += 1
-        self.counts = (nstage, nw, ndig, nacc)
+            finished += 1
+        cut = int(finished < len(self.tiles) and self.planted != "cut")
+        if cut:
+            self.commit(self.cut_done)
+        self.counts = (nstage, nw, ndig, nacc, cut)
         yield from self.drain(0)
 
     def drain(self, c):
-        nstage, nw, ndig, nacc = self.counts
+        nstage, nw, ndig, nacc, cut = self.counts
+        if cut:
+            yield ("drain", self.cut_done[c], 0)
         for bars, n, ring in ((self.empty[c], nstage, self.S), (self.w_empty[c], nw, self.SW),
                               (self.d_empty[c], ndig, 2), (self.accfull[c], nacc, 2)):
             for q in range(max(0, n - ring), n):
@@ -400,6 +410,10 @@ class Pair(Model):
                           f"unpack{c}0": self.unpack(c, 0), f"unpack{c}1": self.unpack(c, 1)})
         peer = None if self.planted == "peer" else lambda: {"exit": self.drain(1)}
         return drive(self, roles, self.rng, inorder, fail, peer)
+
+
+ROLES = ["MMA", "relay"] + [r + str(c) for c in (0, 1) for r in ("E", "W", "epi")] + \
+    [f"unpack{c}{u}" for c in (0, 1) for u in (0, 1)]
 
 
 def _range(rng, table, limit):
@@ -463,19 +477,35 @@ def test_small_rings(name, inorder):
         Pair(_range(rng, _table(rng, True), 16), *SMALL[name], rng).explore(inorder)
 
 
-@pytest.mark.parametrize("planted,name", [
-    ("relay", "W of one pass"),         # the peer tells the leader before its W has landed
-    ("rs", "one stage a tile, W of two passes"),  # row sums written over a tile still in use
-    ("release", "shared operand"),      # W given back where no tiles follow, each pass on its own
-    ("peer", "W of one pass"),          # the peer leaves without waiting for its commits
+@pytest.mark.parametrize("name", sorted(SMALL))
+@pytest.mark.parametrize("inorder", [True, False])
+def test_one_role_gives_up(name, inorder):
+    """One role's wait gives up, the others at later polls: nothing is left to land,
+    and no MMA to run, when the CTAs have gone.  Problems of one pass."""
+    failed = 0
+    for seed in range(150):
+        rng = random.Random(_seed("fail", name, inorder, seed))
+        m = Pair(_range(rng, _table(rng, False), 10), *SMALL[name], rng)
+        failed += m.explore(inorder, (rng.choice(ROLES), rng.randint(1, 12)))
+    assert failed > 50
+
+
+@pytest.mark.parametrize("planted,name,fails", [
+    ("relay", "W of one pass", False),         # the peer tells the leader before its W has landed
+    ("rs", "one stage a tile, W of two passes", False),  # row sums written over a tile still in use
+    ("release", "shared operand", False),      # W given back where no tiles follow, each pass on its own
+    ("peer", "W of one pass", False),          # the peer leaves without waiting for its commits
+    ("count", "narrow, no sums", True),        # the offset MMA's commit counted at the end of the tile
+    ("cut", "shared operand", True),           # no commit behind the MMAs of a tile that ends early
 ])
-def test_the_model_finds(planted, name):
+def test_the_model_finds(planted, name, fails):
     for seed in range(400):
         rng = random.Random(_seed(planted, seed))
-        m = Pair(_range(rng, _table(rng, True), 16), *SMALL[name], rng)
+        m = Pair(_range(rng, _table(rng, not fails), 16), *SMALL[name], rng)
         m.planted = planted
+        fail = ("MMA" if rng.random() < 0.5 else rng.choice(ROLES), rng.randint(1, 12)) if fails else None
         try:
-            m.explore(inorder=False)
+            m.explore(inorder=False, fail=fail)
         except AssertionError:
             return
     raise AssertionError("the planted mistake was not found")
