@@ -53,7 +53,6 @@ constexpr int kPairMaxStages = 8;
 constexpr int kEpiW = 8;       // epilogue warps
 constexpr int kEpiChunks = 2;  // chunks of 8 beams in flight per epilogue warp
 constexpr int kUnpackWarps = 8;
-constexpr int kCounts = 5;  // what the leader leaves for the peer's exit
 constexpr int kPairThreads = 32 * (kEpiW + kUnpackWarps + 3);
 
 struct PairParams {
@@ -87,7 +86,6 @@ __host__ __device__ inline PairSmem pair_smem(int stages, int wslots, int raw, i
   // d_full[2] d_peer[2] d_empty[2] rs_full[2] cut_done
   s.nbar = 2 * raw + 3 * wslots + 2 * stages + 4 + 3 * kDigSlots + 3;
   s.total = s.off_bar + 8 * s.nbar + 32;  // + the TMEM address and the leader's commit counts
-  static_assert(4 * (1 + kCounts) <= 32, "they fit");
   return s;
 }
 
@@ -117,7 +115,8 @@ struct PairCursor {
   // after the start (before the end) of the cluster's range: those of up to `sets`
   // passes stay for a frequency.  They are given back together and only where
   // tiles follow, so the releases of all slots run through the ring in rounds
-  // (drain_commits), although a range that starts with an odd pass loads that first.
+  // (drain_commits), although a range that starts with an odd pass loads that first
+  // -- unless a failed wait cuts it short (cut_commits).
   __device__ __forceinline__ bool first_of_w(int n, int sets) const { return P->npass > sets || n < P->npass || tp == 0; }
   __device__ __forceinline__ bool last_of_w(int n, int sets) const {
     return P->npass > sets || (tp + 1 == ntp && n > P->npass - pass);
@@ -144,6 +143,78 @@ struct PairCursor {
   __device__ __forceinline__ int beams() const { return min(P->nb_pass, (P->B + 7) / 8 * 8 - pass * P->nb_pass); }
   __device__ __forceinline__ int n() const { return (2 * beams() + 31) & ~31; }
 };
+
+// Commits the leader issued, for the exits of both CTAs (in the shared memory of each).
+struct Commits {
+  uint32_t nstage, nw, ndig, nacc;  // on empty, w_empty, d_empty, accfull
+  uint32_t cut;                     // a failed wait ended a tile: cut_done too
+  uint32_t w1, d1;                  // then: of nw and ndig, on the second resident W, the second digit slot
+};
+
+// `w1` and `d1` of an issuer whose tile `cut` a failed wait ended: its walk over the
+// tiles once more, on the failure path alone.  (Counting slot by slot as the commits
+// are issued: the wide array 698 -> 714 us in one form, t=8208 f=21 d=328 b=41 34.6 ->
+// 35.0 in another.)  One lane.
+template <bool kGrouped>
+__device__ __noinline__ void cut_commits(const PairParams &p, int first, int cut, int end, Commits &c) {
+  uint32_t w = 0, d = 0;  // of the tiles before
+  int it = 0, dit = 0;    // slots loaded
+  int w_at[2] = {0, 0}, d_at[2] = {0, 0};
+  const int nk = p.nk, SW = p.wslots;
+  PairCursor<kGrouped> cur(p, first);
+#pragma unroll 1
+  for (int tile = first; tile <= cut; ++tile, cur.next(p)) {
+    const bool odd = cur.pass & 1;
+    if (cur.first_of_w(tile - first, p.sets)) {
+      (odd ? w_at[1] : w_at[0]) = it % SW;
+      (odd ? d_at[1] : d_at[0]) = dit % kDigSlots;
+      it += nk;
+      ++dit;
+    }
+    const bool last = cur.last_of_w(end - tile, p.sets);
+    // the cut tile's: what is left of the counts
+    const uint32_t tw = tile == cut ? c.nw - w : last ? static_cast<uint32_t>(nk) : 0u;
+    const uint32_t td = tile == cut ? c.ndig - d : last ? 1u : 0u;
+    w += tw;
+    d += td;
+    if (SW >= nk && (odd ? w_at[1] : w_at[0]) != 0) c.w1 += tw;
+    if ((odd ? d_at[1] : d_at[0]) != 0) c.d1 += td;
+  }
+}
+
+static_assert(sizeof(Commits) + 4 <= 32, "they fit behind the TMEM address (pair_smem)");
+
+// A CTA's exit: waits (bounded) for the last phase that the leader committed on each
+// barrier, one to a lane.  `bw`, `ba`, `bc`: the first W, stage and accumulator barrier.
+// A function, for leader and peer: inlined, its waits push the kernel's loops out of
+// the instruction cache (t=8208 f=21 d=328 b=41 34.3 -> 35.1 us).
+__device__ __noinline__ void drain_commits(uint32_t bw, uint32_t ba, uint32_t bc, int S, int SW, int nk,
+                                           const Commits &n) {
+  auto phases = [](uint32_t n, int ring, int i) { return (n + ring - 1 - i) / ring; };  // of slot i of a ring
+  const int ring = SW < nk ? SW : nk;  // a resident W gives its slots back in order
+#pragma unroll 1
+  for (int i = threadIdx.x & 31; i < S + SW + 2 * kDigSlots + 1; i += 32) {
+    uint32_t bar, done;
+    if (const int w = i - S; w < 0) {
+      bar = ba + 8u * (S + i);
+      done = phases(n.nstage, S, i);
+    } else if (const int d = w - SW; d < 0) {
+      bar = bw + 8u * (2 * SW + w);
+      done = !n.cut ? phases(n.nw, SW, w) : w < ring ? phases(n.nw - n.w1, ring, w) : phases(n.w1, ring, w - ring);
+    } else if (const int a = d - kDigSlots; a < 0) {
+      bar = bc + 64u + 8u * d;
+      done = !n.cut ? phases(n.ndig, kDigSlots, d) : d ? n.d1 : n.ndig - n.d1;
+    } else if (a < 2) {
+      bar = bc + 8u * a;
+      done = phases(n.nacc, 2, a);
+    } else {
+      bar = bc + 96u;
+      done = n.cut;
+    }
+    if (done) mbar_wait_drain(bar, (done - 1u) & 1u);
+  }
+  __syncwarp();
+}
 
 // Operands to unpack for tiles first .. end - 1 (first < end).
 template <bool kGrouped>
@@ -199,7 +270,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
   auto rs_full = [&](int i) { return bc + 80u + 8u * i; };
   const uint32_t cut_done = bc + 96u;  // the MMAs of a tile that a failed wait cut short
   uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(smem + sp.off_bar + 8 * sp.nbar);
-  uint32_t *counts = tmem_holder + 1;  // commits the leader issued on empty, w_empty, d_empty, accfull, cut_done
+  Commits *counts = reinterpret_cast<Commits *>(tmem_holder + 1);
 
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);  // known to be warp-uniform
   const int lane = threadIdx.x & 31;
@@ -225,7 +296,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     if (lane < 2 * S) mbar_init(a_full(lane), lane < S ? 2 * kStageWarps : 1);
     if (lane < 4) mbar_init(accfull(lane), lane < 2 ? 1 : 2 * kEpiW);
     if (lane < 2) mbar_init(rs_full(lane), 2 * kUnpackWarps);
-    if (lane < kCounts) counts[lane] = 0;
+    if (lane == 0) *counts = Commits{};
     if (lane == 0) mbar_init(cut_done, 1);
   }
   fence_barrier_init();
@@ -244,19 +315,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     tc_fence_after();
   };
   static_assert(2 * kPairMaxStages <= 32, "one lane per stage barrier");
-  // waits for the last phase committed on every barrier
-  auto drain_commits = [&](uint32_t nstage, uint32_t nw, uint32_t ndig, uint32_t nacc, uint32_t cut) {
-    if (cut) mbar_wait_drain(cut_done, 0u);
-    const uint32_t uS = static_cast<uint32_t>(S), uW = static_cast<uint32_t>(SW), uD = static_cast<uint32_t>(kDigSlots);
-    for (uint32_t k = nstage > uS ? nstage - uS : 0; k < nstage; ++k)
-      mbar_wait_drain(empty(static_cast<int>(k % uS)), (k / uS) & 1u);
-    for (uint32_t k = nw > uW ? nw - uW : 0; k < nw; ++k)
-      mbar_wait_drain(w_empty(static_cast<int>(k % uW)), (k / uW) & 1u);
-    for (uint32_t k = ndig > uD ? ndig - uD : 0; k < ndig; ++k)
-      mbar_wait_drain(d_empty(static_cast<int>(k % uD)), (k / uD) & 1u);
-    for (uint32_t k = nacc > 2u ? nacc - 2u : 0u; k < nacc; ++k)
-      mbar_wait_drain(accfull(static_cast<int>(k & 1u)), (k >> 1) & 1u);
-  };
   int *err = p.err;
 
   const int64_t ncl = gridDim.x >> 1, cl = blockIdx.x >> 1;
@@ -492,18 +550,24 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     if (cut && elect_one()) mma_commit_pair(cut_done);
     __syncwarp();
     // A commit's arrival is an asynchronous write into both CTAs' shared memory:
-    // wait (bounded) for the last phase committed on every barrier before the
-    // CTAs can exit, here and, from the counts, in the peer.
+    // wait for the last phase committed on every barrier before the CTAs can exit,
+    // here and, from the counts, in the peer.
     if (lane == 0) {
+      *counts = Commits{nstage, nw, ndig, nacc, cut, 0u, 0u};
+      if (cut) cut_commits<kGrouped>(p, first, tile, end, *counts);
       const uint32_t at = map_cta(smem_u32(counts), 1);
       st_cluster_u32(at, nstage);
       st_cluster_u32(at + 4, nw);
       st_cluster_u32(at + 8, ndig);
       st_cluster_u32(at + 12, nacc);
       st_cluster_u32(at + 16, cut);
+      if (cut) {
+        st_cluster_u32(at + 20, counts->w1);
+        st_cluster_u32(at + 24, counts->d1);
+      }
     }
-    drain_commits(nstage, nw, ndig, nacc, cut);
     __syncwarp();
+    drain_commits(bw, ba, bc, S, SW, nk, *counts);
   } else if (warp >= kUnpackWarp0 && warp < kEProdWarp) {
     // ------------------------------------------------------------ unpack
     // Each lane fills one GEMM row: it reads the raw row of its time, which
@@ -612,8 +676,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
   tc_fence_before();
   cluster_sync();
   if (warp == kMmaWarp) {
-    if (rank == 1) drain_commits(counts[0], counts[1], counts[2], counts[3], counts[4]);
-    __syncwarp();
+    if (rank == 1) drain_commits(bw, ba, bc, S, SW, nk, *counts);
     tc_fence_after();
     tmem_dealloc_pair(*tmem_holder, kPairCols);
   }

@@ -151,7 +151,7 @@ class Pair(Model):
         self.mma_issued = self.mma_done = 0
         self.acc_tile_done = {}
         self.cut_done = [Barrier(f"cut_done@{c}", 1) for c in (0, 1)]
-        self.counts = (0, 0, 0, 0, 0)
+        self.counts = (0, [0, 0], [0, 0], 0, 0)
         self.planted = None
 
     # ------------------------------------------------------------- slots
@@ -309,12 +309,13 @@ class Pair(Model):
     def issuer(self):
         nk, S, SW = self.nk, self.S, self.SW
         ar = a0 = it = dit = 0
-        nstage = nw = ndig = nacc = finished = 0
+        nstage = nacc = finished = 0
+        nw, nd = [0, 0], [0, 0]  # of each resident W (or ring: the first), of each digit slot
         w_at, d_at = [0, 0], [0, 0]
         for n, t in enumerate(self.tiles):
             fresh, last = t.first_of_w(n, self.sets), t.last_of_w(len(self.tiles) - n, self.sets)
             if self.planted == "release":
-                last = self.sets < t.npass or t.tp + 1 == t.ntp
+                last = self.sets < t.npass or t.tp + 2 == t.ntp
             new_a = t.first_of_a(self.share, n == 0)
             last_a = t.last_of_a(self.share, n + 1 == len(self.tiles))
             odd, ab = t.ps & 1, n & 1
@@ -344,7 +345,7 @@ class Pair(Model):
 
             if not self.sums:
                 late = offset()
-                ndig += 0 if self.planted == "count" else late
+                nd[ds] += 0 if self.planted == "count" else late
             ok = True
             for ks in range(nk):
                 reload, release = fresh or self.stream, last or self.stream
@@ -364,7 +365,7 @@ class Pair(Model):
                     nstage += 1
                 if release:
                     self.commit([self.w_empty[0][sw], self.w_empty[1][sw]])
-                    nw += 1
+                    nw[int(w0 > 0)] += 1
                 it += int(reload)
                 ar += 1
             if not ok:
@@ -372,26 +373,55 @@ class Pair(Model):
             if self.sums:
                 if not (yield self.wait(self.rs_full[ab], n // 2)):
                     break
-                ndig += offset()
+                nd[ds] += offset()
             elif self.planted == "count":
-                ndig += late
+                nd[ds] += late
             self.commit([self.accfull[0][ab], self.accfull[1][ab]])
             nacc += 1
             finished += 1
         cut = int(finished < len(self.tiles) and self.planted != "cut")
         if cut:
             self.commit(self.cut_done)
-        self.counts = (nstage, nw, ndig, nacc, cut)
+            assert self.cut_commits(finished, sum(nw), sum(nd)) == (nw[1], nd[1])
+        self.counts = (nstage, nw, nd, nacc, cut)
         yield from self.drain(0)
 
+    def cut_commits(self, cut, nw, nd):
+        """The kernel's walk over the tiles: from the totals, the commits on the second
+        resident W and on the second digit slot."""
+        it = dit = w = d = w1 = d1 = 0
+        w_at, d_at = [0, 0], [0, 0]
+        for n, t in enumerate(self.tiles[:cut + 1]):
+            odd = t.ps & 1
+            if t.first_of_w(n, self.sets):
+                w_at[odd], d_at[odd] = it % self.SW, dit % 2
+                it, dit = it + self.nk, dit + 1
+            last = t.last_of_w(len(self.tiles) - n, self.sets)
+            tw, td = (nw - w, nd - d) if n == cut else (self.nk * last, int(last))
+            w, d = w + tw, d + td
+            w1 += tw if self.SW >= self.nk and w_at[odd] else 0
+            d1 += td if d_at[odd] else 0
+        return w1, d1
+
     def drain(self, c):
-        nstage, nw, ndig, nacc, cut = self.counts
+        nstage, nw, nd, nacc, cut = self.counts
         if cut:
             yield ("drain", self.cut_done[c], 0)
-        for bars, n, ring in ((self.empty[c], nstage, self.S), (self.w_empty[c], nw, self.SW),
-                              (self.d_empty[c], ndig, 2), (self.accfull[c], nacc, 2)):
-            for q in range(max(0, n - ring), n):
-                yield ("drain", bars[q % ring], q // ring)
+        for q in range(max(0, nstage - self.S), nstage):
+            yield ("drain", self.empty[c][q % self.S], q // self.S)
+        if not cut or self.planted == "rounds":  # the releases run through the rings in rounds
+            for bars, n, ring in ((self.w_empty[c], sum(nw), self.SW), (self.d_empty[c], sum(nd), 2)):
+                for q in range(max(0, n - ring), n):
+                    yield ("drain", bars[q % ring], q // ring)
+        else:
+            ring = min(self.SW, self.nk)
+            for w in (0, 1):
+                for q in range(max(0, nw[w] - ring), nw[w]):
+                    yield ("drain", self.w_empty[c][w * ring + q % ring], q // ring)
+                if nd[w]:
+                    yield ("drain", self.d_empty[c][w], nd[w] - 1)
+        for q in range(max(0, nacc - 2), nacc):
+            yield ("drain", self.accfull[c][q % 2], q // 2)
 
     def epilogue(self, c):
         for n in range(len(self.tiles)):
@@ -445,15 +475,20 @@ def _planned(bflib):
 
 def test_every_planned_layout_passes_the_model(bflib):
     """Random ranges of random tables under random schedules, commits in and out of
-    order."""
+    order, and with one role's wait giving up."""
     layouts = _planned(bflib)
     assert len(layouts) >= 40
+    failed = 0
     for S, SW, R, sets, share, nk, groups, sums, two_pass in layouts:
         key = (S, SW, R, sets, share, nk, groups, sums, two_pass)
         for seed in range(10 if nk <= 4 else 4):
-            rng = random.Random(_seed(*key, seed))
-            m = Pair(_range(rng, _table(rng, two_pass), 14 if nk <= 4 else 6), S, SW, R, sets, share, nk, groups, sums, rng)
-            m.explore(inorder=bool(seed % 2))
+            for fail in (False, True):
+                rng = random.Random(_seed(*key, seed, fail))
+                m = Pair(_range(rng, _table(rng, two_pass), 14 if nk <= 4 else 6), S, SW, R, sets, share, nk, groups, sums,
+                         rng)
+                failed += m.explore(inorder=bool(seed % 2),
+                                    fail=(rng.choice(ROLES), rng.randint(1, 10)) if fail else None)
+    assert failed > 200
 
 
 # sizes that make the rings and the rounds short: S, SW, R, sets, share, nk, groups, sums
@@ -481,11 +516,11 @@ def test_small_rings(name, inorder):
 @pytest.mark.parametrize("inorder", [True, False])
 def test_one_role_gives_up(name, inorder):
     """One role's wait gives up, the others at later polls: nothing is left to land,
-    and no MMA to run, when the CTAs have gone.  Problems of one pass."""
+    and no MMA to run, when the CTAs have gone."""
     failed = 0
     for seed in range(150):
         rng = random.Random(_seed("fail", name, inorder, seed))
-        m = Pair(_range(rng, _table(rng, False), 10), *SMALL[name], rng)
+        m = Pair(_range(rng, _table(rng, True), 10), *SMALL[name], rng)
         failed += m.explore(inorder, (rng.choice(ROLES), rng.randint(1, 12)))
     assert failed > 50
 
@@ -493,15 +528,17 @@ def test_one_role_gives_up(name, inorder):
 @pytest.mark.parametrize("planted,name,fails", [
     ("relay", "W of one pass", False),         # the peer tells the leader before its W has landed
     ("rs", "one stage a tile, W of two passes", False),  # row sums written over a tile still in use
-    ("release", "shared operand", False),      # W given back where no tiles follow, each pass on its own
+    ("release", "shared operand", False),      # W given back a tile too early
     ("peer", "W of one pass", False),          # the peer leaves without waiting for its commits
     ("count", "narrow, no sums", True),        # the offset MMA's commit counted at the end of the tile
     ("cut", "shared operand", True),           # no commit behind the MMAs of a tile that ends early
+    ("rounds", "shared operand", True),        # W's commits waited for in ring order, odd pass first or not
 ])
 def test_the_model_finds(planted, name, fails):
     for seed in range(400):
         rng = random.Random(_seed(planted, seed))
-        m = Pair(_range(rng, _table(rng, not fails), 16), *SMALL[name], rng)
+        tiles = _range(rng, _table(rng, True), 16) if planted != "rounds" else tiles_of([(2, 3, 2)])[1:]
+        m = Pair(tiles, *SMALL[name], rng)
         m.planted = planted
         fail = ("MMA" if rng.random() < 0.5 else rng.choice(ROLES), rng.randint(1, 12)) if fails else None
         try:
