@@ -349,7 +349,7 @@ def stream_status(stream=None) -> None:
 
 
 def plan_rings(ndishes: int, max_nb_pass: int, wslots: int = 0, raw: int = 0) -> dict | None:
-    """The ring layout the tensor-core kernel plans (host only, no GPU), or
+    """The ring layout of a launch on single CTAs (host only, no GPU), or
     None where no layout fits: TMEM stages, W slots, raw E slots, unpack
     groups, CTAs per SM, K stages per tile, and the resources: shared memory
     bytes per CTA and the tensor-memory columns (allocated, per accumulator,

@@ -127,8 +127,8 @@ __global__ void fill_random_kernel(uint8_t *__restrict__ dst, size_t n, uint64_t
 
 // Up to 32 words to pinned host memory, behind the kernels before it.  It is
 // resident by the time they end (a launch that overlaps them), where a copy of the
-// same bytes starts only then: the smallest checked call 33.6 -> 28.0 us, t=8192 f=16
-// d=256 b=64 46.9 -> 45.3.
+// same bytes starts only then: the smallest checked call 33.8 -> 28.1 us, t=8192 f=16
+// d=256 b=64 52.8 -> 49.3.
 __global__ void __launch_bounds__(32) write_words(const uint32_t *src, uint32_t *dst, int n) {
   grid_wait();
   if (static_cast<int>(threadIdx.x) < n) dst[threadIdx.x] = src[threadIdx.x];

@@ -45,6 +45,9 @@
 //                de-interleaved E4M3 operand rows written straight into tensor
 //                memory (tcgen05.st); no shared-memory operand
 //
+// It runs passes of at most 16 beams (two CTAs per SM), and wider ones only where
+// the device has no room for a cluster of two SMs (bf_tc_pair.cu takes them).
+//
 // Launches with four or more unpacked stages in TMEM (beam passes of at most
 // 64 beams) run two unpack groups, which take the stages in turn, and one more
 // warp, the W forwarder: it arrives on a stage's a_full once that stage's W slot
@@ -676,8 +679,8 @@ __device__ __forceinline__ uint32_t w_negate(uint32_t codes) {  // zero stays ze
 // 8 sum_k u_k in every column of a row, which the unpack sums and the offset MMA
 // takes off (RowSums).  Signed codes are as exact and need no sums, but the
 // chip runs at its power limit and operands whose sign changes from column to
-// column cost the most of it: the full chunk (f=84 t=32768 b=96 d=512) took 735 us
-// with them and 661 so, at 1.40 and 1.63 GHz; the wide array 711 and 693.
+// column cost the most of it: the full chunk (f=84 t=32768 b=96 d=512) took 716 us
+// with them and 661 so, at 1.40 and 1.63 GHz; the wide array 731 and 690.
 //
 // One warp per beam: both of its rows hold the same numbers, so a lane turns 16
 // dishes into the codes of Ar, Ai and -Ai four bytes at a time and stores 32

@@ -201,7 +201,8 @@ BF_API int bf_batch_shape(const bf_batch *batch, int *nlaunches, int *nproblems,
 
 BF_API int bf_batch_destroy(bf_batch *batch);
 
-/* The ring layout the tensor-core kernel plans for a launch over ndishes
+/* The ring layout of a tensor-core launch on single CTAs (passes of at most 16
+ * beams, and wider ones on a device without room for pairs of SMs) over ndishes
  * dishes whose widest beam pass has max_nb_pass beams, with wslots W slots
  * and raw raw-E slots asked for (0: the planner's choice).  out[0..11] =
  * unpacked stages in tensor memory, W slots, raw E slots, unpack warp
