@@ -190,27 +190,24 @@ static_assert(sizeof(Commits) + 4 <= 32, "they fit behind the TMEM address (pair
 // the instruction cache (t=8208 f=21 d=328 b=41 34.3 -> 35.1 us).
 __device__ __noinline__ void drain_commits(uint32_t bw, uint32_t ba, uint32_t bc, int S, int SW, int nk,
                                            const Commits &n) {
-  auto phases = [](uint32_t n, int ring, int i) { return (n + ring - 1 - i) / ring; };  // of slot i of a ring
-  const int ring = SW < nk ? SW : nk;  // a resident W gives its slots back in order
 #pragma unroll 1
   for (int i = threadIdx.x & 31; i < S + SW + 2 * kDigSlots + 1; i += 32) {
-    uint32_t bar, done;
-    if (const int w = i - S; w < 0) {
-      bar = ba + 8u * (S + i);
-      done = phases(n.nstage, S, i);
-    } else if (const int d = w - SW; d < 0) {
-      bar = bw + 8u * (2 * SW + w);
-      done = !n.cut ? phases(n.nw, SW, w) : w < ring ? phases(n.nw - n.w1, ring, w) : phases(n.w1, ring, w - ring);
-    } else if (const int a = d - kDigSlots; a < 0) {
-      bar = bc + 64u + 8u * d;
-      done = !n.cut ? phases(n.ndig, kDigSlots, d) : d ? n.d1 : n.ndig - n.d1;
-    } else if (a < 2) {
-      bar = bc + 8u * a;
-      done = phases(n.nacc, 2, a);
-    } else {
-      bar = bc + 96u;
-      done = n.cut;
+    // slot `at` of a ring that `count` commits went round
+    const int w = i - S, d = w - SW, a = d - kDigSlots;
+    uint32_t bar = ba + 8u * (S + i), count = n.nstage;
+    int ring = S, at = i;
+    if (w >= 0) bar = bw + 8u * (2 * SW + w), count = n.nw, ring = SW, at = w;
+    if (d >= 0) bar = bc + 64u + 8u * d, count = n.ndig, ring = kDigSlots, at = d;
+    if (a >= 0) bar = bc + 8u * a, count = n.nacc, ring = 2, at = a;
+    if (a >= 2) bar = bc + 96u, count = n.cut, ring = 1, at = 0;
+    if (n.cut && w >= 0 && d < 0) {  // each resident W by itself, its slots in order
+      ring = SW < nk ? SW : nk;
+      count = w < ring ? n.nw - n.w1 : n.w1;
+      at = w < ring ? w : w - ring;
+    } else if (n.cut && d >= 0 && a < 0) {
+      count = d ? n.d1 : n.ndig - n.d1, ring = 1, at = 0;
     }
+    const uint32_t done = (count + ring - 1 - at) / ring;
     if (done) mbar_wait_drain(bar, (done - 1u) & 1u);
   }
   __syncwarp();
