@@ -82,6 +82,16 @@ struct alignas(64) HostBlock {
 };
 constexpr int kHostBlocks = 32;  // calls of a device that read at the same time; more read into their stack
 
+// Memory that stays with one stream (its id, which no later stream gets) from call to
+// call: in stream order each call can use what the one before prepared into.
+struct Home {
+  unsigned long long id = 0;
+  bool taken = false;
+  void *p = nullptr;
+  size_t cap = 0;
+};
+constexpr int kHomes = 4;
+
 struct DeviceCtx {
   std::mutex mu;
   bool ready = false;
@@ -96,6 +106,7 @@ struct DeviceCtx {
   cudaMemPool_t pool = nullptr;    // of the calls' operands (Scratch)
   cudaStream_t pool_s = nullptr;   // allocations that belong to no caller's stream
   std::atomic<GraphScratch *> dropped{nullptr};
+  Home homes[kHomes];              // of the first streams that made calls; under mu
   DevBuf E, A, G, J;        // staging for host-pointer calls
   DevBuf W;                 // what synchronous calls prepare: they end before they let go of mu
   DevBuf partials;          // adler32 partial sums
@@ -115,8 +126,9 @@ struct RelaxedCapture {
 // Unused memory the pool of a device keeps from one call to the next; what is above
 // goes back to the device when a stream is waited for.
 constexpr uint64_t kPoolKeep = uint64_t(1) << 30;
-// The most a synchronous call prepares in the device's buffer, which lives until exit.
+// The most that is kept until exit: of synchronous calls, and of each stream with a home.
 constexpr size_t kKeptBytes = size_t(256) << 20;
+constexpr size_t kHomeBytes = size_t(64) << 20;
 
 cudaError_t make_pool(int dev, DeviceCtx &c) {
   cudaMemPoolProps props{};
@@ -150,7 +162,7 @@ void CUDART_CB drop_graph_scratch(void *arg) {
 // stream use the same memory one after the other, calls on several streams never
 // share it (one operand per device let the second call's preparation overwrite what
 // the first one's kernel still read).  Allocation and free cost 0.5 us of host time
-// together and no launch.  A call under capture gets memory that belongs to its
+// together and no launch, the first ones after a wait 3 us more.  A call under capture gets memory that belongs to its
 // graph: a replay reads it at any later time, beside any other call.
 class Scratch {
  public:
@@ -164,12 +176,6 @@ class Scratch {
   }
   cudaError_t reserve(DeviceCtx &c, size_t n, cudaStream_t s) {
     RelaxedCapture relaxed;
-    for (GraphScratch *g = c.dropped.exchange(nullptr); g;) {
-      GraphScratch *const next = g->next;
-      (void)cudaFreeAsync(g->p, c.pool_s);
-      delete g;
-      g = next;
-    }
     s_ = s;
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     cudaGraph_t graph = nullptr;
@@ -322,14 +328,62 @@ int choose_tensor(const bf_dims &d, bool *use_tc) {
   return BF_OK;
 }
 
-// Memory for what one call prepares: the call's own, or with `ends_here` (the caller
-// waits for the stream before it lets go of c.mu, also after an error) a buffer of the
-// device: the pool's first allocation after a wait costs a checked call 3 us of 52.
-cudaError_t call_memory(DeviceCtx &c, Scratch &own, bool ends_here, size_t n, cudaStream_t s, uint8_t **p) {
-  const bool kept = ends_here && n <= kKeptBytes;
-  const cudaError_t e = kept ? c.W.reserve(n) : own.reserve(c, n, s);
-  *p = kept ? c.W.as<uint8_t>() : own.get();
-  if (e != cudaSuccess) (void)cudaGetLastError();
+// The home of stream s for n bytes: null where it has none, is being captured, or the
+// memory cannot be had.  The caller holds c.mu until its launches are queued.
+uint8_t *home_memory(DeviceCtx &c, size_t n, cudaStream_t s) {
+  unsigned long long id = 0;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone ||
+      cudaStreamGetId(s, &id) != cudaSuccess)
+    return nullptr;
+  for (Home &h : c.homes) {
+    if (h.taken && h.id != id) continue;
+    h.taken = true;
+    h.id = id;
+    if (h.cap < n) {
+      RelaxedCapture relaxed;
+      if (h.p) (void)cudaFreeAsync(h.p, s);
+      h.p = nullptr;
+      h.cap = 0;
+      if (cudaMallocFromPoolAsync(&h.p, n, c.pool, s) != cudaSuccess) {
+        h.p = nullptr;
+        return nullptr;
+      }
+      h.cap = n;
+    }
+    return static_cast<uint8_t *>(h.p);
+  }
+  return nullptr;
+}
+
+// Memory for what one call prepares.  Synchronous calls (`ends_here`: the caller waits
+// for the stream before it lets go of c.mu, also after an error) share a buffer of the
+// device, the first streams keep theirs (`locked`: the caller holds c.mu until its
+// launches are queued), any other call has its own: from the pool in every call,
+// checked calls took 55 us for 52, and an explicit call on an idle stream 55 for 50.
+cudaError_t call_memory(DeviceCtx &c, Scratch &own, bool locked, bool ends_here, size_t n, cudaStream_t s, uint8_t **p) {
+  if (c.dropped.load(std::memory_order_relaxed)) {
+    RelaxedCapture relaxed;
+    for (GraphScratch *g = c.dropped.exchange(nullptr); g;) {
+      GraphScratch *const next = g->next;
+      (void)cudaFreeAsync(g->p, c.pool_s);
+      delete g;
+      g = next;
+    }
+  }
+  cudaError_t e = cudaSuccess;
+  *p = nullptr;
+  if (ends_here && n <= kKeptBytes) {
+    e = c.W.reserve(n);
+    *p = c.W.as<uint8_t>();
+  } else {
+    if (locked && n <= kHomeBytes) *p = home_memory(c, n, s);
+    if (!*p) {
+      e = own.reserve(c, n, s);
+      *p = own.get();
+    }
+  }
+  if (e != cudaSuccess || !*p) (void)cudaGetLastError();
   return e;
 }
 
@@ -337,8 +391,8 @@ cudaError_t call_memory(DeviceCtx &c, Scratch &own, bool ends_here, size_t n, cu
 // (TcPadded); *ran = false where the dp4a kernel has to take it: the rule says so,
 // the memory cannot be had, or the stream is being captured (a graph would hold the
 // copy of E for as long as it lives).  `rw`: resident weights, whose operand is used
-// instead of preparing A; no checksum then.  The caller holds c.mu if `ends_here`.
-int run_padded(DeviceCtx &c, bool ends_here, const bf_dims &d, uint8_t *J, const uint8_t *E, const uint8_t *A,
+// instead of preparing A; no checksum then.  `locked`: the caller holds c.mu.
+int run_padded(DeviceCtx &c, bool locked, bool ends_here, const bf_dims &d, uint8_t *J, const uint8_t *E, const uint8_t *A,
                const float *G, const TcWeights *rw, cudaStream_t s, int a_layout, int j_layout,
                unsigned long long *adl, bool *fused, bool *ran) {
   *ran = false;
@@ -359,7 +413,7 @@ int run_padded(DeviceCtx &c, bool ends_here, const bf_dims &d, uint8_t *J, const
   const size_t need = copy + (rw ? 0 : operand_bytes(w));
   Scratch own;
   uint8_t *mem = nullptr;
-  if (need && call_memory(c, own, ends_here, need, s, &mem) != cudaSuccess) return BF_OK;
+  if (need && call_memory(c, own, locked, ends_here, need, s, &mem) != cudaSuccess) return BF_OK;
   *ran = true;
   t_last_kernel = "tensor";
   if (adl && fused) *fused = true;
@@ -404,7 +458,7 @@ int run_device(DeviceCtx &c, bool ends_here, const bf_dims &d, uint8_t *J, const
   if (!use_tc) {
     if (g_kernel.load() == BF_KERNEL_AUTO) {
       bool ran = false;
-      const int ps = run_padded(c, ends_here, d, J, E, A, G, nullptr, s, a_layout, j_layout, adl, fused, &ran);
+      const int ps = run_padded(c, true, ends_here, d, J, E, A, G, nullptr, s, a_layout, j_layout, adl, fused, &ran);
       if (ran || ps != BF_OK) return ps;
     }
     t_last_kernel = simt_name();
@@ -414,7 +468,7 @@ int run_device(DeviceCtx &c, bool ends_here, const bf_dims &d, uint8_t *J, const
   plan_weights(w, d.nfrequencies, d.nbeams, d.ndishes);
   Scratch own;
   uint8_t *mem = nullptr;
-  BF_TRY(call_memory(c, own, ends_here, operand_bytes(w), s, &mem));
+  BF_TRY(call_memory(c, own, true, ends_here, operand_bytes(w), s, &mem));
   set_operand(w, mem);
   w.G = G;
   if (adl && fused) *fused = true;
@@ -876,7 +930,9 @@ int bf_form_beams_resident(const bf_weights *w, int64_t ntimes, uint8_t *J, cons
   }
   if (g_kernel.load() == BF_KERNEL_AUTO) {
     bool ran = false;
-    const int ps = run_padded(*c, false, d, J, E, nullptr, nullptr, &w->tc, s, kALinear, kJLinear, nullptr, nullptr, &ran);
+    std::unique_lock<std::mutex> lk(c->mu, std::try_to_lock);  // for the stream's home, where no other call has it
+    const int ps = run_padded(*c, lk.owns_lock(), false, d, J, E, nullptr, nullptr, &w->tc, s, kALinear, kJLinear, nullptr,
+                              nullptr, &ran);
     if (ran || ps != BF_OK) return ps;
   }
   t_last_kernel = simt_name();

@@ -230,3 +230,63 @@ def test_threads_that_end_wait_for_no_other_stream(bflib, cuda):
     with pytest.raises(bflib.BeamformError):
         bflib.stream_status(s1)
     assert (out.value or 0) & 0xFFFFFFFF == bflib.OK and took < 0.3, took
+
+
+def test_more_streams_than_keep_memory_and_calls_of_other_sizes(bflib, cuda):
+    """Seven streams (the first four that call keep their memory), each with calls that
+    need more, less and more again than the one before; in place and through the
+    padded copy."""
+    shapes = [(512, 4, 512, 2, 40), (1024, 8, 1024, 2, 130), (1001, 9, 250, 2, 45), (2048, 16, 512, 2, 96)]
+    sets = [_set(bflib, cuda, shape, 20 + k) for k, shape in enumerate(shapes)]
+    streams = [cuda.cuda.Stream() for _ in range(7)]
+    cuda.cuda.synchronize()
+    out = []
+    for rep in range(8):
+        for k, s in enumerate(streams):
+            d, E, A, G, want = sets[(rep * 3 + k) % len(sets)]
+            with cuda.cuda.stream(s):
+                J = cuda.empty(d.jsize, dtype=cuda.uint8, device="cuda")
+                bflib.form_beams_ex(d, J, E, A, G, stream=s)
+            assert bflib.last_kernel() == "tensor"
+            out.append((J, want))
+    cuda.cuda.synchronize()
+    bflib.stream_status()
+    for J, want in out:
+        assert cuda.equal(J, want)
+
+
+def test_threads_on_one_stream(bflib, cuda):
+    """Threads whose calls (resident weights on an odd shape, and weights with the call)
+    meet on one stream: each has its scratch to itself until its launches are queued."""
+    import threading
+
+    T, F, D, B = 1001, 9, 250, 45
+    sets = [_set(bflib, cuda, (T, F, D, 2, B), 30 + k) for k in range(4)]
+    W = [bflib.ResidentWeights(F, B, D, x[2], x[3]) for x in sets]
+    s = cuda.cuda.Stream()
+    J = [[cuda.empty(x[0].jsize, dtype=cuda.uint8, device="cuda") for _ in range(30)] for x in sets]
+    cuda.cuda.synchronize()
+    failed = []
+
+    def call(k):
+        d, E, A, G, _ = sets[k]
+        try:
+            for i, j in enumerate(J[k]):
+                if (i + k) % 3:
+                    W[k].form_beams(j, E, T, stream=s)
+                else:
+                    bflib.form_beams_ex(d, j, E, A, G, stream=s)
+        except Exception as e:  # noqa: BLE001 - reported below
+            failed.append(e)
+
+    threads = [threading.Thread(target=call, args=(k,)) for k in range(len(sets))]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    cuda.cuda.synchronize()
+    bflib.stream_status()
+    assert not failed
+    for x, js in zip(sets, J):
+        for j in js:
+            assert cuda.equal(j, x[4])
